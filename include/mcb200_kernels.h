@@ -255,6 +255,10 @@ int mcb200_permute(const float* in, float* out, int num_axes, const int* in_shap
 int mcb200_normalize_nhwc(const float* in, float* out, long long pixels, int channels, const float* scale,
                           int scale_shared, float eps, void* stream);
 
+/* Rows of `width` floats, src_stride floats apart in pinned host memory that the device can address,
+ * to packed rows on the device.                                                                  */
+int mcb200_copy_host_rows(const float* src, long long src_stride, float* dst, int rows, int width, void* stream);
+
 /* ------------------------------------------------------------------ RPN proposals */
 typedef struct mcb200_proposal_params {
   int num_anchors, height, width;  /* score map [2A, H, W], delta map [4A, H, W] per image */
@@ -287,6 +291,19 @@ int mcb200_proposal_forward(const mcb200_proposal_params* p, int batch, const fl
                             const float* im_info, const float* anchors, void* workspace, float* rois,
                             float* roi_scores, int* counts, void* stream);
 
+/* The same with the foreground scores' address given by the caller (image b's A x H x W scores lie
+ * score_stride floats behind those of image b - 1), for images first_image .. of a larger batch
+ * (the rois' column 0; all pointers are those of the first of these images).  Scores, deltas and im_info may be pinned host
+ * memory that the device can address; so may rois, roi_scores and counts.                        */
+int mcb200_proposal_forward_from(const mcb200_proposal_params* p, int first_image, int batch, const float* fg_scores,
+                                 long long score_stride, const float* deltas, const float* im_info, const float* anchors, void* workspace,
+                                 float* rois, float* roi_scores, int* counts, void* stream);
+
+/* Copies the images' valid rows one behind the other into other buffers (which may be pinned host
+ * memory); roi_scores and scores_out may be NULL.                                                */
+int mcb200_proposal_gather(const float* rois, const float* roi_scores, const int* counts, int batch, int post_nms_topn,
+                           float* rois_out, float* scores_out, void* stream);
+
 /* Closes the gaps between the images' row blocks of a batched
  * mcb200_proposal_forward result in place: image b's counts[b] valid rows move
  * from row b * post_nms_topn to row counts[0] + ... + counts[b-1] (rois and,
@@ -307,10 +324,10 @@ int mcb200_proposal_compact(float* rois, float* roi_scores, const int* counts, i
  * their hands.
  *
  * The scratch is a fixed 8 MiB array inside the library's device image (each
- * GPU that loads the library holds it until the process exits).  The largest
- * single image the kernels accept (65536 proposals, pre_nms_topn 6000) takes
- * 1.9 MB of it, an image of the stock R-FCN setting (63 x 38 map, 15 anchors)
- * 1.1 MB, and a batch takes that many times as much; a request that needs more
+ * GPU that loads the library holds it until the process exits).  An
+ * image of 65536 proposals takes
+ * 1.3 MB of it, an image of the stock R-FCN setting (63 x 38 map, 15 anchors)
+ * 0.72 MB, and a batch takes that many times as much; a request that needs more
  * than 8 MiB returns -20 and prints the required size.  The function calls no cudaMalloc, cudaFree
  * or any other allocating routine.
  *

@@ -29,11 +29,13 @@ void Context::Release() {
   // At process exit the runtime may already be gone; ignore errors here.
   if (cudaSetDevice(device_) == cudaSuccess) {
     if (stream_) cudaStreamDestroy(stream_);
-    if (status_dev_) cudaFree(status_dev_);
+    if (copy_stream_) cudaStreamDestroy(copy_stream_);
+    if (event_) cudaEventDestroy(event_);
     if (status_host_) cudaFreeHost(status_host_);
   }
   cudaGetLastError();
-  stream_ = nullptr;
+  stream_ = copy_stream_ = nullptr;
+  event_ = nullptr;
   status_dev_ = nullptr;
   status_host_ = nullptr;
   active_ = false;
@@ -62,26 +64,39 @@ void Context::Activate() {
   CHECK_LT(device_, DeviceCount()) << "invalid device id";
   CUDA_CHECK(cudaSetDevice(device_));
   CUDA_CHECK(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
-  CUDA_CHECK(cudaMalloc(reinterpret_cast<void**>(&status_dev_), sizeof(int)));
-  CUDA_CHECK(cudaMemset(status_dev_, 0, sizeof(int)));
-  CUDA_CHECK(cudaMallocHost(reinterpret_cast<void**>(&status_host_), sizeof(int)));
+  CUDA_CHECK(cudaHostAlloc(reinterpret_cast<void**>(&status_host_), sizeof(int), cudaHostAllocMapped));
   *status_host_ = 0;
+  CUDA_CHECK(cudaHostGetDevicePointer(reinterpret_cast<void**>(&status_dev_), status_host_, 0));
   active_ = true;
+}
+
+cudaStream_t Context::CopiesBegin() {
+  Activate();
+  if (!copy_stream_) CUDA_CHECK(cudaStreamCreateWithFlags(&copy_stream_, cudaStreamNonBlocking));
+  if (!event_) CUDA_CHECK(cudaEventCreateWithFlags(&event_, cudaEventDisableTiming));
+  CUDA_CHECK(cudaEventRecord(event_, stream_));
+  CUDA_CHECK(cudaStreamWaitEvent(copy_stream_, event_, 0));
+  return copy_stream_;
+}
+
+void Context::CopiesArrived() {
+  CUDA_CHECK(cudaEventRecord(event_, copy_stream_));
+  CUDA_CHECK(cudaStreamWaitEvent(stream_, event_, 0));
 }
 
 void Context::Sync() {
   if (!active_) return;
+  // (A pass that ended early with an error may have left copies behind that nothing waits for.)
+  if (copy_stream_) CUDA_CHECK(cudaStreamSynchronize(copy_stream_));
   CUDA_CHECK(cudaStreamSynchronize(stream_));
 }
 
 void Context::SyncAndCheck() {
   if (!active_) return;
-  CUDA_CHECK(cudaMemcpyAsync(status_host_, status_dev_, sizeof(int), cudaMemcpyDeviceToHost, stream_));
   CUDA_CHECK(cudaStreamSynchronize(stream_));
-  if (*status_host_ != 0) {
-    const int code = *status_host_;
-    *status_host_ = 0;
-    CUDA_CHECK(cudaMemsetAsync(status_dev_, 0, sizeof(int), stream_));
+  const int code = *static_cast<volatile int*>(status_host_);
+  if (code != 0) {
+    *static_cast<volatile int*>(status_host_) = 0;
     // 3: a region-of-interest layer met a roi whose image index is outside the batch
     // (the reference fails its CHECK_GE / CHECK_LT on roi_batch_ind at that point).
     if (code == 3) LOG(FATAL) << "Check failed: roi_batch_ind is outside [0, batch_size)";

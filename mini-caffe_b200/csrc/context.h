@@ -44,8 +44,16 @@ class Context {
   void* stream_ptr() { return static_cast<void*>(stream()); }
   // The stream if this thread has one already, else NULL (never creates one, never throws).
   void* stream_if_active() const { return active_ ? static_cast<void*>(stream_) : nullptr; }
-  // Device int that kernels raise on a timed-out wait; checked by Net::Forward.
+  // Word that kernels raise on a timed-out wait; checked by Net::Forward.  It lies in pinned host
+  // memory that the device writes through its mapped address: kernels touch it only when something
+  // went wrong, and a pass does not pay a device-to-host copy to learn that nothing did.
   int* status_word() { Activate(); return status_dev_; }
+  // Copies of new input that run beside the kernels, on a second stream.  CopiesBegin: copies queued
+  // from here on start after the work queued so far (which may still use their destinations), and
+  // the stream to queue them on is returned.  CopiesArrived: work queued on stream() from here on
+  // starts after the copies queued so far.
+  cudaStream_t CopiesBegin();
+  void CopiesArrived();
   // Blocks until the stream is idle and throws if a kernel raised the status word.
   void SyncAndCheck();
   void Sync();
@@ -53,11 +61,13 @@ class Context {
   ~Context();
 
  private:
-  Context() : mode_(GPU), device_(0), active_(false), stream_(nullptr), status_dev_(nullptr), status_host_(nullptr) {}
+  Context() : mode_(GPU), device_(0), active_(false), stream_(nullptr), copy_stream_(nullptr), event_(nullptr),
+              status_dev_(nullptr), status_host_(nullptr) {}
   DeviceMode mode_;
   int device_;
   bool active_;
-  cudaStream_t stream_;
+  cudaStream_t stream_, copy_stream_;
+  cudaEvent_t event_;      // one event serves every hand-over: a wait refers to the record before it
   int* status_dev_;
   int* status_host_;
   void Release();

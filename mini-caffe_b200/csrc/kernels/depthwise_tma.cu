@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(256) depthwise3x3_tma_kernel(const __grid_cons
           if (clock64() - start > kDwWaitLimitCycles / 8) break;
         }
       }
-      if (a.status) atomicExch(a.status, 1);
+      if (a.status) *static_cast<volatile int*>(a.status) = 1;
     }
   }
 }

@@ -1,12 +1,9 @@
 // RPN ProposalLayer on the device, batched over images:
-//   1. decode      anchor + deltas -> clipped box, min-size filter, sort key
-//   2. top-k sort  per image: radix-select the pre_nms_topn best keys, bitonic
-//                  sort them in shared memory, gather boxes in score order
-//   3. greedy NMS  per image: one block walks the boxes 64 at a time and evaluates
-//                  overlaps only for rows that are kept against columns that are
-//                  still alive; stops at post_nms_topn; writes rois (+ scores)
-//                  and the count
-// The host only reads the per-image counts back.
+//   1. decode      anchor + deltas -> clipped box, score (0 for boxes below the minimum size)
+//   2. rank + NMS  a cluster of CTAs per image: takes the best boxes a segment of at most 1024 at a
+//                  time, walks each segment 64 boxes at a time against the kept ones, stops at
+//                  post_nms_topn; writes rois (+ scores) and the count
+// The host only needs the per-image counts.
 //
 // Every float operation that decides which boxes are kept is done with the
 // rounding of the CPU code it replaces (mini-caffe src/layers/proposal_layer.cpp:
@@ -15,6 +12,7 @@
 // multiply and add (no FMA), exp() evaluated in double and the product rounded
 // to float once, IEEE division.  Boxes with equal scores are ordered by
 // proposal index (the CPU quicksort leaves that order unspecified).
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <stdio.h>
@@ -24,27 +22,35 @@
 #include "../../../include/mcb200_kernels.h"
 #include "detection.cuh"
 #include "launch_count.h"
+#include "sm100.cuh"
 
 namespace mcb200 {
 namespace {
 
 using namespace det;
+using sm100::grid_dependency_wait;
+using sm100::grid_launch_dependents;
+
+constexpr int kMaxCluster = 8;     // CTAs that work on one image
 
 struct Workspace {
-  float4* boxes;                 // [batch][n]        decoded boxes, proposal order
-  float* scores;                 // [batch][n]
-  unsigned long long* keys;      // [batch][n]
-  float4* sorted_boxes;          // [batch][k]        score order
-  float* sorted_scores;          // [batch][k]
-  int n, k, col_blocks;
+  float4* boxes;                 // [batch][n]     decoded boxes, proposal order
+  float* scores;                 // [batch][score_ld]
+  uint32_t* score_keys;          // [batch][score_ld]   ascending keys of the descending scores
+  float4* kept_boxes;            // [batch][post], then the areas; used when they do not fit in shared memory
+  int n, k;
+  int score_ld;                  // floats between two images' scores: rows start on 16 bytes
 };
 
 size_t align_up(size_t v) { return (v + 255) & ~static_cast<size_t>(255); }
 
+// Bytes of one image's kept list: boxes, then areas.
+__host__ __device__ inline size_t kept_bytes(int post_nms_topn) {
+  return (static_cast<size_t>(post_nms_topn) * (sizeof(float4) + sizeof(float)) + 15) & ~static_cast<size_t>(15);
+}
+
 size_t carve(const mcb200_proposal_params& p, int batch, char* base, Workspace* ws) {
   const int n = p.num_anchors * p.height * p.width;
-  const int k = n < p.pre_nms_topn ? n : p.pre_nms_topn;
-  const int cb = (k + 63) / 64;
   size_t off = 0;
   auto take = [&](size_t bytes) {
     char* ptr = base ? base + off : nullptr;
@@ -53,35 +59,77 @@ size_t carve(const mcb200_proposal_params& p, int batch, char* base, Workspace* 
   };
   Workspace w;
   w.n = n;
-  w.k = k;
-  w.col_blocks = cb;
+  w.k = n < p.pre_nms_topn ? n : p.pre_nms_topn;
+  w.score_ld = (n + 3) & ~3;
   w.boxes = reinterpret_cast<float4*>(take(sizeof(float4) * n * static_cast<size_t>(batch)));
-  w.scores = reinterpret_cast<float*>(take(sizeof(float) * n * static_cast<size_t>(batch)));
-  w.keys = reinterpret_cast<unsigned long long*>(take(8 * static_cast<size_t>(n) * batch));
-  w.sorted_boxes = reinterpret_cast<float4*>(take(sizeof(float4) * k * static_cast<size_t>(batch)));
-  w.sorted_scores = reinterpret_cast<float*>(take(sizeof(float) * k * static_cast<size_t>(batch)));
+  w.scores = reinterpret_cast<float*>(take(sizeof(float) * w.score_ld * static_cast<size_t>(batch)));
+  w.score_keys = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * w.score_ld * static_cast<size_t>(batch)));
+  w.kept_boxes = reinterpret_cast<float4*>(take(kept_bytes(p.post_nms_topn) * batch));
   if (ws) *ws = w;
   return off;
 }
 
 // ---------------------------------------------------------------- 1. decode
 
-__global__ void proposal_decode_kernel(const float* __restrict__ score_maps, const float* __restrict__ delta_maps,
-                                       const float* __restrict__ im_info, const float* __restrict__ anchors,
-                                       mcb200_proposal_params p, Workspace ws) {
+// A block takes kDecodeCells cells of the map with all their anchors: a warp reads 32 neighbouring
+// cells of one anchor (the maps are anchor-major), the results are turned to proposal order (cell-
+// major) in shared memory and leave as whole rows.  A group of four boxes'
+// values is on its way while the group before it is worked on.
+constexpr int kDecodeCells = 64;
+constexpr int kDecodeThreads = 256;
+constexpr int kDecodeGroup = 4;       // boxes of a thread whose values are asked for together
+
+struct DecodeIn {
+  const float* scores;        // foreground scores of image 0; image stride below
+  long long score_stride;     // floats between the foreground maps of two images
+  const float* deltas;        // [batch][4A][H][W]
+  const float* im_info;       // [batch][3]
+  const float* anchors;       // [A][4]
+};
+
+__global__ void __launch_bounds__(kDecodeThreads)
+proposal_decode_kernel(DecodeIn in, mcb200_proposal_params p, Workspace ws, int turned) {
+  extern __shared__ __align__(16) unsigned char decode_smem[];
   const int image = blockIdx.y;
   const int hw = p.height * p.width;
   const int n = ws.n;
-  // Foreground scores are the second half of the 2A score channels.
-  const float* score = score_maps + static_cast<size_t>(image) * 2 * p.num_anchors * hw + static_cast<size_t>(n);
-  const float* delta = delta_maps + static_cast<size_t>(image) * 4 * p.num_anchors * hw;
-  const float img_h = im_info[image * 3 + 0];
-  const float img_w = im_info[image * 3 + 1];
-  const float min_size = fmul(static_cast<float>(p.min_size), im_info[image * 3 + 2]);
-  // Threads run over (anchor, y, x) with x fastest, so the map reads coalesce.
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-    const int k = t / hw;
-    const int pos = t - k * hw;
+  const float* score = in.scores + static_cast<size_t>(image) * in.score_stride;
+  const float* delta = in.deltas + static_cast<size_t>(image) * 4 * p.num_anchors * hw;
+  const float* anchors = in.anchors;
+  float4* s_box = reinterpret_cast<float4*>(decode_smem);
+  float* s_score = reinterpret_cast<float*>(s_box + (turned ? kDecodeCells * p.num_anchors : 0));
+  __shared__ float info[3];
+  if (threadIdx.x < 3) info[threadIdx.x] = in.im_info[image * 3 + threadIdx.x];
+  const int pos0 = blockIdx.x * kDecodeCells;
+  const int items = kDecodeCells * p.num_anchors;
+  grid_launch_dependents();
+  float in_flight[kDecodeGroup][5];
+  auto load = [&](int group) {
+#pragma unroll
+    for (int u = 0; u < kDecodeGroup; ++u) {
+      const int t = group + u * kDecodeThreads;
+      const int k = t / kDecodeCells;
+      const int pos = pos0 + t % kDecodeCells;
+      if (t >= items || pos >= hw) continue;
+      in_flight[u][0] = score[k * hw + pos];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) in_flight[u][1 + j] = delta[(k * 4 + j) * hw + pos];
+    }
+  };
+  load(threadIdx.x);
+  __syncthreads();
+  const float img_h = info[0], img_w = info[1];
+  const float min_size = fmul(static_cast<float>(p.min_size), info[2]);
+  for (int group = threadIdx.x; group < items; group += kDecodeGroup * kDecodeThreads) {
+#pragma unroll
+   for (int u = 0; u < kDecodeGroup; ++u) {
+    const int t = group + u * kDecodeThreads;
+    if (t >= items) break;
+    const float score_here = in_flight[u][0], dx = in_flight[u][1], dy = in_flight[u][2], dlw = in_flight[u][3],
+                dlh = in_flight[u][4];
+    const int k = t / kDecodeCells;
+    const int pos = pos0 + t % kDecodeCells;
+    if (pos >= hw) continue;
     const int y = pos / p.width;
     const int x = pos - y * p.width;
     const float fx = static_cast<float>(x * p.feat_stride);
@@ -90,11 +138,6 @@ __global__ void proposal_decode_kernel(const float* __restrict__ score_maps, con
     float b1 = fadd(fy, anchors[k * 4 + 1]);
     float b2 = fadd(fx, anchors[k * 4 + 2]);
     float b3 = fadd(fy, anchors[k * 4 + 3]);
-    const float dx = delta[(k * 4 + 0) * hw + pos];
-    const float dy = delta[(k * 4 + 1) * hw + pos];
-    const float dlw = delta[(k * 4 + 2) * hw + pos];
-    const float dlh = delta[(k * 4 + 3) * hw + pos];
-
     const float w = fadd(fsub(b2, b0), 1.f);
     const float h = fadd(fsub(b3, b1), 1.f);
     const float ctr_x = fadd(b0, fmul(0.5f, w));
@@ -117,255 +160,499 @@ __global__ void proposal_decode_kernel(const float* __restrict__ score_maps, con
     const float box_w = fadd(fsub(b2, b0), 1.f);
     const float box_h = fadd(fsub(b3, b1), 1.f);
     const int valid = (box_w >= min_size) && (box_h >= min_size);
-    const float s = fmul(static_cast<float>(valid), score[k * hw + pos]);
+    const float s = fmul(static_cast<float>(valid), score_here);
 
-    const int index = pos * p.num_anchors + k;   // proposal order: (y, x, anchor)
-    const size_t o = static_cast<size_t>(image) * n + index;
-    ws.boxes[o] = make_float4(b0, b1, b2, b3);
-    ws.scores[o] = s;
-    ws.keys[o] = make_key(s, static_cast<uint32_t>(index));
+    const float4 box = make_float4(b0, b1, b2, b3);
+    const int local = (pos - pos0) * p.num_anchors + k;   // proposal order: (y, x, anchor)
+    if (turned) {
+      s_box[local] = box;
+      s_score[local] = s;
+    } else {
+      const size_t o = static_cast<size_t>(pos0) * p.num_anchors + local;
+      ws.boxes[static_cast<size_t>(image) * n + o] = box;
+      ws.scores[static_cast<size_t>(image) * ws.score_ld + o] = s;
+      ws.score_keys[static_cast<size_t>(image) * ws.score_ld + o] = descending_key(s);
+    }
+   }
+   load(group + kDecodeGroup * kDecodeThreads);
   }
-}
-
-// ---------------------------------------------------------------- 2. top-k + sort
-
-// One block per image.  The score halves of the keys (the index half of key i
-// is i itself) are copied to shared memory once, with all loads of a thread in
-// flight together; the passes of the radix select, which test one key after the
-// other with a warp vote in between, and the compaction then run out of shared
-// memory instead of paying an L2 round trip per key and pass.  `staged` = 0 (the
-// keys do not fit beside the sort buffer): they are read from global memory.
-__global__ void __launch_bounds__(1024, 1)
-proposal_topk_sort_kernel(Workspace ws, int padded, int staged) {
-  extern __shared__ unsigned long long sorted[];   // `padded` keys, then (staged) n 32-bit score keys
-  __shared__ int hist[256];
-  __shared__ unsigned long long bcast[2];
-  __shared__ int fill;
-  const int image = blockIdx.x;
-  const unsigned long long* keys = ws.keys + static_cast<size_t>(image) * ws.n;
-  const int n = ws.n, k = ws.k;
-  uint32_t* score_key = reinterpret_cast<uint32_t*>(sorted + padded);
-  if (staged) {
-    for (int i = threadIdx.x; i < n; i += blockDim.x) score_key[i] = static_cast<uint32_t>(keys[i] >> 32);
-  }
-  if (threadIdx.x == 0) fill = 0;
-  for (int i = threadIdx.x; i < padded; i += blockDim.x) sorted[i] = kPadKey;
+  if (!turned) return;
   __syncthreads();
-  auto key_at = [&](int i) {
-    return staged ? ((static_cast<unsigned long long>(score_key[i]) << 32) | static_cast<uint32_t>(i)) : keys[i];
-  };
-
-  unsigned long long threshold = kPadKey;
-  if (k < n) threshold = block_kth_smallest(key_at, n, k, hist, bcast);
-  // Append the selected keys, one update of the shared counter per warp.
-  for (int base = 0; base < n; base += blockDim.x) {
-    const int i = base + threadIdx.x;
-    unsigned long long key = 0;
-    bool take = false;
-    if (i < n) {
-      key = key_at(i);
-      take = key <= threshold;
-    }
-    const unsigned taking = __ballot_sync(0xffffffffu, take);
-    if (taking) {
-      const int lane = threadIdx.x & 31;
-      const int leader = __ffs(taking) - 1;
-      int first = 0;
-      if (lane == leader) first = atomicAdd(&fill, __popc(taking));
-      first = __shfl_sync(0xffffffffu, first, leader);
-      const int slot = first + __popc(taking & ((1u << lane) - 1u));
-      if (take && slot < padded) sorted[slot] = key;
-    }
-  }
-  __syncthreads();
-  block_sort_keys(sorted, padded);
-  const float4* boxes = ws.boxes + static_cast<size_t>(image) * n;
-  const float* scores = ws.scores + static_cast<size_t>(image) * n;
-  // Gather in groups of four per thread: the four box and score loads (random
-  // rows, an L2 round trip each) are issued before the first store.
-  for (int base = threadIdx.x; base < k; base += 4 * blockDim.x) {
-    float4 box[4];
-    float score[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int i = base + u * blockDim.x;
-      if (i < k) {
-        const uint32_t index = static_cast<uint32_t>(sorted[i] & 0xFFFFFFFFull);
-        box[u] = boxes[index];
-        score[u] = scores[index];
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int i = base + u * blockDim.x;
-      if (i < k) {
-        ws.sorted_boxes[static_cast<size_t>(image) * k + i] = box[u];
-        ws.sorted_scores[static_cast<size_t>(image) * k + i] = score[u];
-      }
-    }
+  const int here = min(kDecodeCells, hw - pos0) * p.num_anchors;
+  float4* box_row = ws.boxes + static_cast<size_t>(image) * n + static_cast<size_t>(pos0) * p.num_anchors;
+  const size_t row = static_cast<size_t>(image) * ws.score_ld + static_cast<size_t>(pos0) * p.num_anchors;
+  float* score_row = ws.scores + row;
+  uint32_t* key_row = ws.score_keys + row;
+  for (int t = threadIdx.x; t < here; t += kDecodeThreads) {
+    box_row[t] = s_box[t];
+    score_row[t] = s_score[t];
+    key_row[t] = descending_key(s_score[t]);
   }
 }
 
-// ---------------------------------------------------------------- 3a. overlap test
-
-// IoU with the "+1 pixel" convention; areas[i] + areas[j] - inter, IEEE division.
-__device__ __forceinline__ bool suppresses(const float4& a, float area_a, const float4& b, float area_b,
-                                           float threshold) {
-  const float x1 = fmaxf(a.x, b.x);
-  const float y1 = fmaxf(a.y, b.y);
-  const float x2 = fminf(a.z, b.z);
-  const float y2 = fminf(a.w, b.w);
-  const float w = fmaxf(0.f, fadd(fsub(x2, x1), 1.f));
-  const float h = fmaxf(0.f, fadd(fsub(y2, y1), 1.f));
-  const float inter = fmul(w, h);
-  const float ov = fdiv(inter, fsub(fadd(area_a, area_b), inter));
-  return ov > threshold;
-}
+// ---------------------------------------------------------------- 2a. overlap test
 
 __device__ __forceinline__ float box_area(const float4& b) {
   return fmul(fadd(fsub(b.z, b.x), 1.f), fadd(fsub(b.w, b.y), 1.f));
 }
 
-// ---------------------------------------------------------------- 3b. greedy suppression + output
+// Decides IoU > threshold ("+1 pixel" convention) as the CPU code does: areas[i] + areas[j] -
+// inter, IEEE division.  The division (some forty instructions) runs only where it can matter:
+// with `below` = threshold * (1 - 2^-20) and `above` = threshold * (1 + 2^-20), a float product of
+// either with the union is off by 2^-24 of itself, so an intersection beyond them decides the
+// comparison whatever the quotient's rounding.  A threshold <= 0 or a union that is not a positive
+// finite number passes neither test and takes the division.
+struct OverlapTest {
+  float threshold, below, above;
+  __device__ explicit OverlapTest(float thr)
+      : threshold(thr), below(thr > 0.f ? fmul(thr, 1.f - 0x1p-20f) : -1.f),
+        above(thr > 0.f ? fmul(thr, 1.f + 0x1p-20f) : __builtin_huge_valf()) {}
+  // 1: overlaps by more than the threshold; 0: does not; 2: only the division can tell.
+  __device__ __forceinline__ int quick(const float4& a, float area_a, const float4& b, float area_b) const {
+    const float x1 = fmaxf(a.x, b.x);
+    const float y1 = fmaxf(a.y, b.y);
+    const float x2 = fminf(a.z, b.z);
+    const float y2 = fminf(a.w, b.w);
+    const float w = fmaxf(0.f, fadd(fsub(x2, x1), 1.f));
+    const float h = fmaxf(0.f, fadd(fsub(y2, y1), 1.f));
+    const float inter = fmul(w, h);
+    const float uni = fsub(fadd(area_a, area_b), inter);
+    return inter < fmul(below, uni) ? 0 : (uni > 0.f && inter > fmul(above, uni)) ? 1 : 2;
+  }
+  __device__ __noinline__ bool exact(float4 a, float area_a, float4 b, float area_b) const {
+    const float w = fmaxf(0.f, fadd(fsub(fminf(a.z, b.z), fmaxf(a.x, b.x)), 1.f));
+    const float h = fmaxf(0.f, fadd(fsub(fminf(a.w, b.w), fmaxf(a.y, b.y)), 1.f));
+    const float inter = fmul(w, h);
+    return fdiv(inter, fsub(fadd(area_a, area_b), inter)) > threshold;
+  }
+  __device__ __forceinline__ bool operator()(const float4& a, float area_a, const float4& b, float area_b) const {
+    const int verdict = quick(a, area_a, b, area_b);
+    return verdict == 2 ? exact(a, area_a, b, area_b) : verdict == 1;
+  }
+};
 
-constexpr int kNmsThreads = 1024;
-// Boxes of one image are staged in shared memory when they fit (20 bytes each).
-constexpr int kNmsStagedBoxes = 8192;
+// ---------------------------------------------------------------- 2b. rank + greedy suppression
 
-// Bytes in front of the staged boxes: the indices of the kept boxes (at most
-// post_nms_topn), rounded up so that the float4 array starts on a 16-byte boundary.
-__host__ __device__ constexpr size_t nms_kept_bytes(int post_nms_topn) {
-  return (static_cast<size_t>(post_nms_topn) * 4 + 15) & ~static_cast<size_t>(15);
+namespace cg = cooperative_groups;
+
+constexpr int kRankThreads = 1024;
+constexpr int kSegment = 1024;       // boxes taken at a time, at most: one per thread
+constexpr int kTopBins = 2048;
+// Radix levels of a key (score 32 bits, index 32 bits): 11 + 11 + 10 bits of each half.
+__device__ __forceinline__ int level_shift(int level) {
+  const int in_half = level % 3 == 0 ? 21 : level % 3 == 1 ? 10 : 0;
+  return in_half + (level < 3 ? 32 : 0);
+}
+__device__ __forceinline__ int level_bins(int level) { return level % 3 == 2 ? 1024 : 2048; }
+
+struct RankShared {
+  union {
+    struct {
+      int top[kTopBins];                   // histogram of the first level
+      int bins[kTopBins];                  // histogram of a deeper level
+    };
+    // [w][c]: bit r: box 32 w + r of the segment suppresses its box c (first CTA)
+    uint32_t mask[kSegment / 32][kSegment];
+  };
+  unsigned long long found[kSegment];      // this CTA's finds
+  unsigned long long all[kSegment];        // everybody's, in no order
+  uint32_t high[kSegment + 4];             // their upper halves, then ones
+  unsigned long long sorted[kSegment];
+  float4 boxes[kSegment];
+  float area[kSegment];
+  uint32_t gone[kSegment / 32];            // boxes of the segment that boxes kept earlier suppress (first CTA)
+  uint32_t keep[2][kSegment / 32];         // the walk's set, by the round's parity
+  int kept_total;
+  int part_fill[kMaxCluster];
+  int warp_sum[32];
+  int found_bin, found_before, found_total;
+  int fill;
+};
+
+// Adds one key to a histogram.  Lanes of a warp that all hit one bin (the zero scores of boxes
+// below the minimum size, say) are combined into one update.
+__device__ __forceinline__ void count_key(int* bins, bool live, int bin) {
+  const unsigned lanes = __ballot_sync(0xffffffffu, live);
+  if (!live) return;
+  const int leader = __ffs(lanes) - 1;
+  if (__all_sync(lanes, bin == __shfl_sync(lanes, bin, leader))) {
+    if ((threadIdx.x & 31) == leader) atomicAdd(&bins[bin], __popc(lanes));
+  } else {
+    atomicAdd(&bins[bin], 1);
+  }
 }
 
-// One block per image walks the score-ordered boxes 64 at a time.  Per step:
-//   1. all threads: which of the step's 64 boxes does an already kept box
-//      suppress (kept boxes x 64 columns), and the 64 x 64 overlaps inside the
-//      block (bit c of diag[r] = "row r suppresses column c", c > r);
-//   2. thread 0: resolves the block in order (a box is kept unless an earlier
-//      kept box suppresses it) and stops at post_nms_topn; the kept boxes are
-//      then written out and appended to the kept list in parallel.
-// Overlaps are evaluated lazily, only between kept boxes and the boxes the walk
-// actually reaches: at most post_nms_topn x pre_nms_topn pairs, and far fewer
-// when the walk ends early, instead of the pre_nms_topn^2 / 2 pairs of a full
-// suppression matrix.  The kept set is that of the sequential algorithm
-// (src/layers/proposal_layer.cpp:161-186).
-__global__ void __launch_bounds__(kNmsThreads)
-proposal_nms_kernel(Workspace ws, float threshold, int post_nms_topn, int staged, float* __restrict__ rois,
-                    float* __restrict__ roi_scores, int* __restrict__ counts) {
-  extern __shared__ __align__(16) unsigned char nms_smem[];
-  __shared__ unsigned long long diag[64];
-  __shared__ unsigned long long gone_word;   // columns of the current block that kept boxes suppress
-  __shared__ unsigned long long keep_word;
-  __shared__ int kept_total;
-  __shared__ int stop;
-  const int image = blockIdx.x;
-  const int k = ws.k, cb = ws.col_blocks;
-  const int kpad = cb * 64;
-  const float4* g_boxes = ws.sorted_boxes + static_cast<size_t>(image) * k;
-  const float* scores = ws.sorted_scores + static_cast<size_t>(image) * k;
+// First bin whose inclusive running count (starting from `before`) exceeds `limit`: its number and
+// the count in front of it, or found_bin = -1 and the total when there is none.  Whole block.
+__device__ void find_bin(RankShared& sh, const int* bins, int count, int before, int limit) {
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int a = 2 * t < count ? bins[2 * t] : 0;
+  const int b = 2 * t < count ? bins[2 * t + 1] : 0;
+  int incl = a + b;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  if (lane == 31) sh.warp_sum[warp] = incl;
+  if (t == 0) sh.found_bin = -1;
+  __syncthreads();
+  int base = lane < warp ? sh.warp_sum[lane] : 0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) base += __shfl_xor_sync(0xffffffffu, base, o);
+  const int excl = before + base + incl - (a + b);
+  if (excl <= limit && excl + a + b > limit) {
+    const bool second = excl + a <= limit;
+    sh.found_bin = 2 * t + (second ? 1 : 0);
+    sh.found_before = second ? excl + a : excl;
+  }
+  if (t == kRankThreads - 1) sh.found_total = excl + a + b;
+  __syncthreads();
+}
+
+// A threshold T such that between `lo` and `hi` of the n keys are <= T (their number goes to
+// *count).  It lies on the coarsest bin boundary that the range allows: for ordinary scores the
+// first level's bins decide and no further pass over the keys is needed; ties are cut by index.
+template <typename KeyAt>
+__device__ unsigned long long find_threshold(RankShared& sh, const KeyAt& key_at, int n, int lo, int hi, int* count) {
+  unsigned long long prefix = 0;     // the bits of the levels above, in place
+  int before = 0;
+  for (int level = 0;; ++level) {
+    const int shift = level_shift(level);
+    const int nbins = level_bins(level);
+    const int* bins = sh.top;
+    if (level > 0) {
+      const int above = level_shift(level - 1);
+      for (int i = threadIdx.x; i < nbins; i += kRankThreads) sh.bins[i] = 0;
+      __syncthreads();
+      for (int base = 0; base < n; base += kRankThreads) {
+        const int i = base + threadIdx.x;
+        const unsigned long long key = i < n ? key_at(i) : 0ull;
+        count_key(sh.bins, i < n && (key >> above) == (prefix >> above),
+                  static_cast<int>(key >> shift) & (nbins - 1));
+      }
+      __syncthreads();
+      bins = sh.bins;
+    }
+    find_bin(sh, bins, nbins, before, hi);
+    const int bin = sh.found_bin, in_front = sh.found_before, total = sh.found_total;
+    __syncthreads();                 // the found_* words are rewritten by the next call
+    if (bin < 0) {                   // everything down to here fits
+      *count = total;
+      return level == 0 ? kPadKey : prefix | ((1ull << level_shift(level - 1)) - 1ull);
+    }
+    const unsigned long long start = prefix | (static_cast<unsigned long long>(bin) << shift);
+    if (in_front >= lo) {
+      *count = in_front;
+      return start - 1ull;           // in_front >= lo >= 1: some key lies below `start`
+    }
+    prefix = start;
+    before = in_front;
+  }
+}
+
+// A cluster of `kCluster` CTAs per image, which share every part of the work that can be shared
+// (`part` = this CTA) and keep one copy each of what the others found, so that all of them take the
+// same decisions.  The boxes are needed in score order only as far as the greedy walk gets, which is
+// usually a few hundred boxes beyond post_nms_topn: so they are taken a segment of at most
+// kSegment at a time.  Where a segment ends does not matter as long as it holds the best of what is
+// left:
+//   select  a sample of the score keys says below which key about kAim boxes lie; every CTA looks
+//           through its share of the keys, the finds are exchanged.  When the sample was wrong by too
+//           much (ties, for instance) find_threshold cuts exactly.
+//   sort    by counting: a key's place is the number of smaller keys.  Some 700 keys against 700 are
+//           60 comparisons per thread of the cluster, where a sorting network or a merge of the same
+//           keys is a chain of thirty and more dependent exchanges (5-8 us in one block).
+//   mark    which box of the segment suppresses which: 32 x 32 boxes per warp, the results gathered in
+//           the first CTA's shared memory; and which boxes the ones kept earlier suppress.
+//   walk    the first CTA: keep = not gone and not suppressed by a kept box in front, iterated from
+//           "all that are not gone" until nothing changes.  A box's bit is final once those in front
+//           of it are, so this ends in the sequential algorithm's set, after as many rounds as the
+//           longest chain of suppressions is long.  (A walk in steps of 64 boxes against the kept list
+//           makes half the tests, but a step is 4000 cycles of dependent instructions and barriers.)
+// The kept set is that of the sequential algorithm (src/layers/proposal_layer.cpp:161-186).
+// One block per image that sorted all 6000 boxes and walked them with the division in every test
+// took 157 + 62 us.
+constexpr int kAim = 700;
+
+template <int kCluster>
+__global__ void __launch_bounds__(kRankThreads, 1)
+proposal_rank_nms_kernel(Workspace ws, float threshold, int post_nms_topn, int kept_in_smem, int first_image,
+                         float* __restrict__ rois, float* __restrict__ roi_scores, int* __restrict__ counts) {
+  extern __shared__ __align__(16) unsigned char rank_smem[];
+  RankShared& sh = *reinterpret_cast<RankShared*>(rank_smem);
+  cg::cluster_group cluster = cg::this_cluster();
+  const int part = static_cast<int>(cluster.block_rank());
+  const int image = blockIdx.x / kCluster;
+  const int n = ws.n, k = ws.k;
+  const int t = threadIdx.x, lane = t & 31;
+  // The kept list: a copy per CTA in shared memory or, when it is too long for that, one in the workspace.
+  float4* kept_box = reinterpret_cast<float4*>(
+      kept_in_smem ? rank_smem + ((sizeof(RankShared) + 15) & ~static_cast<size_t>(15))
+                   : reinterpret_cast<unsigned char*>(ws.kept_boxes) + image * kept_bytes(post_nms_topn));
+  float* kept_area = reinterpret_cast<float*>(kept_box + post_nms_topn);
+  const float4* boxes = ws.boxes + static_cast<size_t>(image) * n;
+  const float* scores = ws.scores + static_cast<size_t>(image) * ws.score_ld;
+  const uint32_t* keys = ws.score_keys + static_cast<size_t>(image) * ws.score_ld;
   float* out = rois + static_cast<size_t>(image) * post_nms_topn * 5;
   float* out_scores = roi_scores ? roi_scores + static_cast<size_t>(image) * post_nms_topn : nullptr;
+  const OverlapTest suppresses(threshold);
+  if (t == 0) sh.fill = 0;
+  cluster.sync();   // nobody writes to this CTA's shared memory before it runs
+  grid_dependency_wait();
+  auto key_at = [&](int i) { return (static_cast<unsigned long long>(keys[i]) << 32) | static_cast<uint32_t>(i); };
 
-  int* kept = reinterpret_cast<int*>(nms_smem);
-  float4* s_boxes = reinterpret_cast<float4*>(nms_smem + nms_kept_bytes(post_nms_topn));   // 16-byte aligned
-  float* s_area = reinterpret_cast<float*>(s_boxes + kpad);
-  const int t = threadIdx.x;
-  if (staged) {
-    for (int i = t; i < kpad; i += kNmsThreads) {
-      const float4 b = i < k ? g_boxes[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-      s_boxes[i] = b;
-      s_area[i] = box_area(b);
-    }
-  }
-  if (t == 0) {
-    kept_total = 0;
-    stop = 0;
-  }
-  __syncthreads();
-  auto box_at = [&](int i) { return staged ? s_boxes[i] : g_boxes[i]; };
-  auto area_at = [&](int i, const float4& b) { return staged ? s_area[i] : box_area(b); };
+  // The sample: a key per thread.
+  const int stride = max(n / kRankThreads, 1);
+  const bool sampled = t * stride < n;
+  const uint32_t sample = sampled ? keys[t * stride] : 0u;
 
-  bool done = false;
-  for (int block = 0; block < cb && !done; ++block) {
-    const int base = block * 64;
-    const int rows = min(64, k - base);
-    if (t < 64) diag[t] = 0ull;
-    if (t == 0) gone_word = 0ull;
-    const int total_before = kept_total;   // read before the barrier: thread 0 updates it in step 2
-    __syncthreads();
-    // ---- 1a. kept boxes against this block: thread = (column, every 16th kept box)
-    {
-      const int c = t & 63;
-      if (c < rows) {
-        const float4 b = box_at(base + c);
-        const float area_b = area_at(base + c, b);
-        bool hit = false;
-        for (int q = t >> 6; q < total_before && !hit; q += kNmsThreads / 64) {
-          const int i = kept[q];
-          const float4 a = box_at(i);
-          hit = suppresses(a, area_at(i, a), b, area_b, threshold);
-        }
-        if (hit) atomicOr(&gone_word, 1ull << c);
-      }
-    }
-    // ---- 1b. overlaps inside the block: thread = (row, group of four columns)
-    {
-      const int r = t >> 4;
-      const int c0 = (t & 15) * 4;
-      if (r < rows && c0 + 3 > r) {
-        const float4 a = box_at(base + r);
-        const float area_a = area_at(base + r, a);
-        unsigned long long bits = 0ull;
+  unsigned long long start = 0ull;   // keys below this have been walked
+  int walked = 0, kept_total = 0;
+
+  while (walked < k && kept_total < post_nms_topn) {
+    // ---- select
+    const int hi = min(walked + kSegment, k);
+    uint32_t cut = 0xFFFFFFFFu;                    // n <= hi: everything that is left
+    if (n > hi) {
+      // The upper 22 bits of the `aim`-th smallest sample, by two histograms.
+      const long long wanted = walked + min(kAim, (hi - walked) * 5 / 8);
+      const int aim = max(1, static_cast<int>(wanted * min(kRankThreads, n) / n));
+      uint32_t prefix = 0u;
+      int before = 0;
 #pragma unroll
-        for (int c = c0; c < c0 + 4; ++c) {
-          if (c > r && c < rows) {
-            const float4 b = box_at(base + c);
-            if (suppresses(a, area_a, b, area_at(base + c, b), threshold)) bits |= 1ull << c;
-          }
+      for (int level = 0; level < 2; ++level) {
+        const int shift = level == 0 ? 21 : 10;
+        for (int i = t; i < kTopBins; i += kRankThreads) sh.top[i] = 0;
+        __syncthreads();
+        if (sampled && (level == 0 || (sample >> 21) == (prefix >> 21))) atomicAdd(&sh.top[(sample >> shift) & (kTopBins - 1)], 1);
+        __syncthreads();
+        find_bin(sh, sh.top, kTopBins, before, aim - 1);
+        prefix |= static_cast<uint32_t>(sh.found_bin) << shift;
+        before = sh.found_before;
+        __syncthreads();
+      }
+      cut = prefix | 1023u;
+    }
+    unsigned long long last = (static_cast<unsigned long long>(cut) << 32) | 0xFFFFFFFFull;
+    {
+      const uint32_t floor_key = static_cast<uint32_t>(start >> 32);
+      auto take = [&](uint32_t score_bits, int at) {
+        if (score_bits <= cut && score_bits >= floor_key && at < n) {
+          const unsigned long long key = (static_cast<unsigned long long>(score_bits) << 32) | static_cast<uint32_t>(at);
+          if (key < start) return;
+          const int slot = atomicAdd(&sh.fill, 1);
+          if (slot < kSegment) sh.found[slot] = key;
         }
-        if (bits) atomicOr(&diag[r], bits);
+      };
+      constexpr int kQuads = 3;
+      for (int base = 0; base < n; base += kQuads * 4 * kCluster * kRankThreads) {
+        uint4 v[kQuads];
+#pragma unroll
+        for (int u = 0; u < kQuads; ++u) {
+          const int i = base + ((u * kCluster + part) * kRankThreads + t) * 4;
+          v[u] = i < n ? *reinterpret_cast<const uint4*>(keys + i) : make_uint4(~0u, ~0u, ~0u, ~0u);
+        }
+#pragma unroll
+        for (int u = 0; u < kQuads; ++u) {
+          const int i = base + ((u * kCluster + part) * kRankThreads + t) * 4;
+          if (min(min(v[u].x, v[u].y), min(v[u].z, v[u].w)) > cut) continue;
+          take(v[u].x, i);
+          take(v[u].y, i + 1);
+          take(v[u].z, i + 2);
+          take(v[u].w, i + 3);
+        }
       }
     }
     __syncthreads();
-    // ---- 2. resolve the block in score order
-    if (t == 0) {
-      unsigned long long gone = gone_word;
-      unsigned long long keep = 0ull;
-      int total = total_before;
+    if (t < kCluster) cluster.map_shared_rank(sh.part_fill, t)[part] = sh.fill;
+    cluster.sync();
+    int m = 0, in_front = 0;
+#pragma unroll
+    for (int j = 0; j < kCluster; ++j) {
+      if (j < part) in_front += sh.part_fill[j];
+      m += sh.part_fill[j];
+    }
+    if (m == 0 || walked + m > hi || (walked > 0 && hi == k && k < n)) {
+      // The sample misled, or the cut at pre_nms_topn itself has come: exactly, every CTA by itself.
+      for (int i = t; i < kTopBins; i += kRankThreads) sh.top[i] = 0;
+      __syncthreads();
+      for (int base = 0; base < n; base += kRankThreads) {
+        const int i = base + t;
+        count_key(sh.top, i < n, i < n ? static_cast<int>(keys[i] >> 21) : 0);
+      }
+      if (t == 0) sh.fill = 0;
+      __syncthreads();
+      int count = 0;
+      const int lo = k - walked <= kSegment ? k : walked + kSegment / 2;
+      last = find_threshold(sh, key_at, n, lo, hi, &count);
+      // (the order of the finds differs from CTA to CTA: each ranks all of them)
+      for (int i = t; i < n; i += kRankThreads) {
+        const unsigned long long key = key_at(i);
+        if (key >= start && key <= last) sh.all[atomicAdd(&sh.fill, 1)] = key;
+      }
+      __syncthreads();
+      m = count - walked;
+      for (int i = t; i < m; i += kRankThreads) {
+        const unsigned long long key = sh.all[i];
+        int place = 0;
+        for (int q = 0; q < m; ++q) place += sh.all[q] < key ? 1 : 0;
+        sh.sorted[place] = key;
+      }
+    } else {
+      // Everybody's finds to everybody.
+      for (int i = t; i < sh.part_fill[part]; i += kRankThreads) {
+        const unsigned long long key = sh.found[i];
+#pragma unroll
+        for (int j = 0; j < kCluster; ++j) {
+          cluster.map_shared_rank(sh.all, j)[in_front + i] = key;
+          cluster.map_shared_rank(sh.high, j)[in_front + i] = static_cast<uint32_t>(key >> 32);
+        }
+      }
+      if (t < 4) sh.high[m + t] = 0xFFFFFFFFu;
+      cluster.sync();
+      // ---- sort: `helpers` threads count for one key of this CTA's share, four keys at a time by
+      // their upper halves (equal ones, a rare sight, are told apart in a second pass)
+      const int share = (m + kCluster - 1) / kCluster;
+      int helpers = 32;
+      while (helpers > 1 && share * helpers > kRankThreads) helpers >>= 1;
+      const int sub = t & (helpers - 1);
+      for (int base = 0; base < share; base += kRankThreads / helpers) {
+        const int local = base + t / helpers;
+        const int at = part * share + local;
+        const bool mine = local < share && at < m;
+        const unsigned long long key = mine ? sh.all[at] : 0ull;
+        const uint32_t h = static_cast<uint32_t>(key >> 32);
+        int below = 0, upto = 0;
+#pragma unroll 4
+        for (int q = sub * 4; q < m; q += helpers * 4) {
+          const uint4 v = *reinterpret_cast<const uint4*>(sh.high + q);
+          below += (v.x < h ? 1 : 0) + (v.y < h ? 1 : 0) + (v.z < h ? 1 : 0) + (v.w < h ? 1 : 0);
+          upto += (v.x <= h ? 1 : 0) + (v.y <= h ? 1 : 0) + (v.z <= h ? 1 : 0) + (v.w <= h ? 1 : 0);
+        }
+        for (int o = helpers >> 1; o > 0; o >>= 1) {
+          below += __shfl_xor_sync(0xffffffffu, below, o);
+          upto += __shfl_xor_sync(0xffffffffu, upto, o);
+        }
+        if (mine && upto != below + 1) {
+          below = 0;
+          for (int q = 0; q < m; ++q) below += sh.all[q] < key ? 1 : 0;
+        }
+        for (int j = sub; j < kCluster; j += helpers) {
+          if (mine) cluster.map_shared_rank(sh.sorted, j)[below] = key;
+        }
+      }
+    }
+    cluster.sync();
+    if (t < m) {
+      const float4 b = boxes[sh.sorted[t] & 0xFFFFFFFFull];
+      sh.boxes[t] = b;
+      sh.area[t] = box_area(b);
+    }
+    if (t < kSegment / 32) sh.gone[t] = 0u;
+    if (t == 0) sh.fill = 0;
+    cluster.sync();
+
+    // ---- mark
+    const int blocks = (m + 31) >> 5;
+    const int crew = kCluster * (kRankThreads / 32);
+    uint32_t* mask = cluster.map_shared_rank(&sh.mask[0][0], 0);
+    int column_block = 0, first_tile = 0;      // tiles run over column blocks, then the row blocks up to it
+    for (int tile = (t >> 5) * kCluster + part; tile < blocks * (blocks + 1) / 2; tile += crew) {
+      while (tile > first_tile + column_block) first_tile += ++column_block;
+      const int w = tile - first_tile;
+      const int c = column_block * 32 + lane;
+      const float4 b = sh.boxes[c];
+      const float area_b = sh.area[c];
+      const int rows = min(32, m - w * 32);
+      uint32_t bits = 0u, unsure = 0u;
+#pragma unroll 4
       for (int r = 0; r < rows; ++r) {
-        if (!((gone >> r) & 1ull)) {
-          keep |= 1ull << r;
-          ++total;
-          if (total == post_nms_topn) {
-            stop = 1;
-            break;
-          }
-          gone |= diag[r];
-        }
+        const int verdict = suppresses.quick(sh.boxes[w * 32 + r], sh.area[w * 32 + r], b, area_b);
+        bits |= static_cast<uint32_t>(verdict & 1) << r;
+        unsure |= static_cast<uint32_t>(verdict >> 1) << r;
       }
-      keep_word = keep;
-      kept_total = total;
+      for (; unsure; unsure &= unsure - 1) {
+        const int r = __ffs(unsure) - 1;
+        if (suppresses.exact(sh.boxes[w * 32 + r], sh.area[w * 32 + r], b, area_b)) bits |= 1u << r;
+      }
+      if (w == column_block) bits &= (1u << lane) - 1u;   // only boxes in front suppress
+      if (c < m) mask[w * kSegment + c] = bits;
     }
-    __syncthreads();
-    if (t < rows && ((keep_word >> t) & 1ull)) {
-      const int pos = total_before + __popcll(keep_word & ((1ull << t) - 1ull));
-      const int i = base + t;
-      kept[pos] = i;
-      const float4 b = g_boxes[i];
-      out[pos * 5 + 0] = static_cast<float>(image);
-      out[pos * 5 + 1] = b.x;
-      out[pos * 5 + 2] = b.y;
-      out[pos * 5 + 3] = b.z;
-      out[pos * 5 + 4] = b.w;
-      if (out_scores) out_scores[pos] = scores[i];
+    if (kept_total > 0) {
+      uint32_t* gone = cluster.map_shared_rank(sh.gone, 0);
+      for (int task = (t >> 5) * kCluster + part; task < blocks * 8; task += crew) {
+        const int c = (task >> 3) * 32 + lane;
+        const float4 b = sh.boxes[c];
+        const float area_b = sh.area[c];
+        bool hit = false;
+        for (int q = task & 7; q < kept_total; q += 8) hit = hit || suppresses(kept_box[q], kept_area[q], b, area_b);
+        const unsigned hits = __ballot_sync(0xffffffffu, hit);
+        if (lane == 0 && hits) atomicOr(gone + (task >> 3), hits);
+      }
     }
-    // Everyone takes the same copy of the flag here; thread 0 writes it again
-    // only after the next iteration's first barrier.
-    done = stop != 0;
-    __syncthreads();
+    cluster.sync();
+
+    // ---- walk
+    if (part == 0) {
+      const int own = t >> 5;
+      uint32_t busy = 0u;                     // words of this column that suppress anything at all
+      if (t < m) {
+        for (int w = 0; w <= own; ++w) busy |= (sh.mask[w][t] != 0u ? 1u : 0u) << w;
+      }
+      const bool alive = t < m && !((sh.gone[own] >> lane) & 1u);
+      uint32_t word = __ballot_sync(0xffffffffu, alive);
+      if (lane == 0) sh.keep[0][own] = word;
+      __syncthreads();
+      for (int round = 0;; round ^= 1) {
+        bool stays = alive;
+        for (uint32_t left = busy; left && stays; left &= left - 1) {
+          const int w = __ffs(left) - 1;
+          stays = !(sh.mask[w][t] & sh.keep[round][w]);
+        }
+        const uint32_t next = __ballot_sync(0xffffffffu, stays);
+        if (lane == 0) sh.keep[round ^ 1][own] = next;
+        const int changed = __syncthreads_or(next != word);
+        word = next;
+        if (!changed) break;
+      }
+      // (both copies of the set are the same now)
+      int before = kept_total;
+      for (int w = 0; w < own; ++w) before += __popc(sh.keep[0][w]);
+      const int pos = before + __popc(word & ((1u << lane) - 1u));
+      const bool more = walked + m < k;       // the others need the kept boxes for the next segment
+      if (((word >> lane) & 1u) && pos < post_nms_topn) {
+        const float4 kept = sh.boxes[t];
+#pragma unroll
+        for (int j = 0; j < kCluster; ++j) {
+          if (kept_in_smem && more) {
+            cluster.map_shared_rank(kept_box, j)[pos] = kept;
+            cluster.map_shared_rank(kept_area, j)[pos] = sh.area[t];
+          }
+        }
+        if (!kept_in_smem) {
+          kept_box[pos] = kept;
+          kept_area[pos] = sh.area[t];
+        }
+        out[pos * 5 + 0] = static_cast<float>(first_image + image);
+        out[pos * 5 + 1] = kept.x;
+        out[pos * 5 + 2] = kept.y;
+        out[pos * 5 + 3] = kept.z;
+        out[pos * 5 + 4] = kept.w;
+        if (out_scores) out_scores[pos] = scores[sh.sorted[t] & 0xFFFFFFFFull];
+      }
+      if (t == kRankThreads - 1) {
+        const int total = min(before + __popc(word), post_nms_topn);
+#pragma unroll
+        for (int j = 0; j < kCluster; ++j) *cluster.map_shared_rank(&sh.kept_total, j) = total;
+      }
+    }
+    cluster.sync();
+    kept_total = sh.kept_total;
+    walked += m;
+    start = last + 1ull;
   }
-  if (t == 0) counts[image] = kept_total;
+  if (t == 0 && part == 0) counts[image] = kept_total;
 }
 
 }  // namespace
@@ -381,15 +668,15 @@ static int validate(const mcb200_proposal_params* p, int batch) {
   const long long n = static_cast<long long>(p->num_anchors) * p->height * p->width;
   if (n > (1 << 24)) return -3;
   const int k = n < p->pre_nms_topn ? static_cast<int>(n) : p->pre_nms_topn;
-  // The sorted keys of one image live in shared memory (8 bytes each).
   if (det::next_pow2(k) > 16384) return -4;
   return 0;
 }
 
-constexpr size_t kSortSharedLimit = 220 * 1024;
+// Dynamic shared memory a block may ask for.
+constexpr size_t kRankSharedLimit = 220 * 1024;
+constexpr size_t kDecodeSharedLimit = 48 * 1024;
 
-// The top-k and the NMS kernel use more dynamic shared memory than a kernel gets
-// by default; the opt-in is per device and is made on a device's first call
+// The ranking kernel uses more dynamic shared memory than a kernel gets by default; the opt-in is per device and is made on a device's first call
 // (nets on several host threads may make that call at the same time).
 static cudaError_t configure_kernels() {
   static bool configured[64] = {false};
@@ -399,10 +686,11 @@ static cudaError_t configure_kernels() {
   if (e != cudaSuccess) return e;
   std::lock_guard<std::mutex> lock(mu);
   if (dev < 0 || dev >= 64 || configured[dev]) return cudaSuccess;
-  e = cudaFuncSetAttribute(proposal_topk_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           static_cast<int>(kSortSharedLimit));
+  e = cudaFuncSetAttribute(proposal_rank_nms_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           static_cast<int>(kRankSharedLimit));
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(proposal_nms_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+  e = cudaFuncSetAttribute(proposal_rank_nms_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           static_cast<int>(kRankSharedLimit));
   if (e != cudaSuccess) return e;
   configured[dev] = true;
   return cudaSuccess;
@@ -445,12 +733,13 @@ extern "C" size_t mcb200_proposal_workspace_bytes(const mcb200_proposal_params* 
   return carve(*p, batch, nullptr, nullptr);
 }
 
-extern "C" int mcb200_proposal_forward(const mcb200_proposal_params* p, int batch, const float* scores,
-                                       const float* deltas, const float* im_info, const float* anchors,
-                                       void* workspace, float* rois, float* roi_scores, int* counts, void* stream) {
+extern "C" int mcb200_proposal_forward_from(const mcb200_proposal_params* p, int first_image, int batch,
+                                            const float* fg_scores, long long score_stride, const float* deltas, const float* im_info,
+                                            const float* anchors, void* workspace, float* rois, float* roi_scores,
+                                            int* counts, void* stream) {
   const int rc = validate(p, batch);
   if (rc != 0) return rc;
-  if (!scores || !deltas || !im_info || !anchors || !workspace || !rois || !counts) return -5;
+  if (!fg_scores || !deltas || !im_info || !anchors || !workspace || !rois || !counts) return -5;
   if (reinterpret_cast<uintptr_t>(workspace) & 255) return -6;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const cudaError_t configured = configure_kernels();
@@ -459,31 +748,78 @@ extern "C" int mcb200_proposal_forward(const mcb200_proposal_params* p, int batc
   carve(*p, batch, static_cast<char*>(workspace), &ws);
 
   {
-    const int threads = 256;
-    int blocks = (ws.n + threads - 1) / threads;
-    if (blocks > 148 * 4) blocks = 148 * 4;
-    proposal_decode_kernel<<<dim3(blocks, batch), threads, 0, st>>>(scores, deltas, im_info, anchors, *p, ws);
+    const int hw = p->height * p->width;
+    const size_t smem = static_cast<size_t>(kDecodeCells) * p->num_anchors * (sizeof(float4) + sizeof(float));
+    const int turned = smem <= kDecodeSharedLimit ? 1 : 0;
+    const DecodeIn in = {fg_scores, score_stride, deltas, im_info, anchors};
+    proposal_decode_kernel<<<dim3((hw + kDecodeCells - 1) / kDecodeCells, batch), kDecodeThreads, turned ? smem : 0, st>>>(
+        in, *p, ws, turned);
     count_launch();
   }
-  {
-    const int padded = det::next_pow2(ws.k);
-    const size_t sort_bytes = static_cast<size_t>(padded) * 8;
-    const size_t staged_bytes = sort_bytes + static_cast<size_t>(ws.n) * 4;
-    if (sort_bytes > kSortSharedLimit) return -8;
-    const int staged = staged_bytes <= kSortSharedLimit ? 1 : 0;
-    const size_t smem = staged ? staged_bytes : sort_bytes;
-    proposal_topk_sort_kernel<<<batch, 1024, smem, st>>>(ws, padded, staged);
-    count_launch();
-  }
-  {
-    // Boxes and areas of an image go to shared memory when they fit.
-    const int staged = ws.col_blocks * 64 <= kNmsStagedBoxes ? 1 : 0;
-    const size_t smem = nms_kept_bytes(p->post_nms_topn) + (staged ? static_cast<size_t>(ws.col_blocks) * 64 * 20 : 0);
-    if (smem > 220 * 1024) return -7;   // post_nms_topn beyond 10000 with staged boxes: not a detector's setting
-    proposal_nms_kernel<<<batch, kNmsThreads, smem, st>>>(ws, p->nms_thresh, p->post_nms_topn, staged, rois, roi_scores,
-                                                           counts);
-    count_launch();
-  }
+  // The kept list goes to shared memory where it fits beside the fixed part.
+  size_t smem = (sizeof(RankShared) + 15) & ~static_cast<size_t>(15);
+  const int kept_in_smem = smem + kept_bytes(p->post_nms_topn) <= kRankSharedLimit ? 1 : 0;
+  if (kept_in_smem) smem += kept_bytes(p->post_nms_topn);
+  // Eight CTAs per image while all of them find an SM of their own, else four.
+  const int parts = batch * 8 <= 148 ? 8 : 4;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(batch * parts);
+  cfg.blockDim = dim3(kRankThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // set-up beside the decode kernel's tail
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = parts;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, parts == 8 ? proposal_rank_nms_kernel<8> : proposal_rank_nms_kernel<4>, ws,
+                                           p->nms_thresh, p->post_nms_topn, kept_in_smem, first_image, rois, roi_scores,
+                                           counts);
+  count_launch();
+  return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
+}
+
+extern "C" int mcb200_proposal_forward(const mcb200_proposal_params* p, int batch, const float* scores,
+                                       const float* deltas, const float* im_info, const float* anchors,
+                                       void* workspace, float* rois, float* roi_scores, int* counts, void* stream) {
+  const int rc = validate(p, batch);
+  if (rc != 0) return rc;
+  // Foreground scores are the second half of the 2A score channels.
+  const long long n = static_cast<long long>(p->num_anchors) * p->height * p->width;
+  return mcb200_proposal_forward_from(p, 0, batch, scores ? scores + n : nullptr, 2 * n, deltas, im_info, anchors, workspace,
+                                      rois, roi_scores, counts, stream);
+}
+
+// The images' row blocks (image b's rows start at b * post) one behind the other in another buffer,
+// which may be pinned host memory: one block per image.
+static __global__ void __launch_bounds__(256)
+proposal_gather_kernel(const float* __restrict__ rois, const float* __restrict__ roi_scores, const int* __restrict__ counts,
+                       int post, float* __restrict__ rois_out, float* __restrict__ scores_out) {
+  __shared__ int before;
+  const int image = blockIdx.x;
+  if (threadIdx.x == 0) before = 0;
+  __syncthreads();
+  int sum = 0;
+  for (int i = threadIdx.x; i < image; i += blockDim.x) sum += counts[i];
+  if (sum) atomicAdd(&before, sum);
+  __syncthreads();
+  const int rows = counts[image], first = before;
+  const float* src = rois + static_cast<size_t>(image) * post * 5;
+  for (int i = threadIdx.x; i < rows * 5; i += blockDim.x) rois_out[static_cast<size_t>(first) * 5 + i] = src[i];
+  if (!scores_out) return;
+  for (int i = threadIdx.x; i < rows; i += blockDim.x) scores_out[first + i] = roi_scores[static_cast<size_t>(image) * post + i];
+}
+
+extern "C" int mcb200_proposal_gather(const float* rois, const float* roi_scores, const int* counts, int batch, int post_nms_topn,
+                                      float* rois_out, float* scores_out, void* stream) {
+  if (!rois || !counts || !rois_out || (scores_out && !roi_scores) || batch < 1 || post_nms_topn < 1) return -1;
+  proposal_gather_kernel<<<batch, 256, 0, static_cast<cudaStream_t>(stream)>>>(rois, roi_scores, counts, post_nms_topn,
+                                                                              rois_out, scores_out);
+  count_launch();
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -501,9 +837,8 @@ extern "C" int mcb200_proposal_compact(float* rois, float* roi_scores, const int
 
 // Scratch of mcb200_proposal_forward_static.  It lives in the library's device
 // image: every GPU that loads the library carries these 8 MiB until the process
-// exits.  The largest single image the kernels accept (65536 proposals of which
-// 6000 go to NMS) takes 1.9 MB of it, an image of the stock R-FCN setting (63 x 38
-// map, 15 anchors) 1.1 MB; a call whose batch needs more than the array holds
+// exits.  An image of 65536 proposals takes 1.3 MB of it, one of the stock R-FCN setting (63 x 38
+// map, 15 anchors) 0.72 MB; a call whose batch needs more than the array holds
 // is refused.
 static constexpr size_t kStaticScratchBytes = static_cast<size_t>(8) << 20;
 static __device__ __align__(256) unsigned char g_proposal_static_scratch[kStaticScratchBytes];
@@ -558,8 +893,7 @@ extern "C" int mcb200_proposal_forward_static(const mcb200_proposal_params* p, i
   const int found = static_scratch(&scratch);
   if (found != 0) return found;
   // Every scratch word the kernels read is written earlier in the same call
-  // (keys, boxes and scores for all proposals, the sorted copies for the best
-  // pre_nms_topn), so nothing has to be cleared between calls.
+  // (boxes and scores for all proposals, the kept boxes), so nothing has to be cleared between calls.
   return mcb200_proposal_forward(p, batch, scores, deltas, im_info, anchors, scratch, rois, roi_scores, counts,
                                  stream);
 }

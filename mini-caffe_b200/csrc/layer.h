@@ -113,6 +113,9 @@ class Layer {
   // The net's decision.  operands: read bottoms / residual as bfloat16; top:
   // store top 0 as bfloat16.
   virtual void SetHalfStorage(bool operands, bool top) {}
+  // The net's word that no later layer of the pass reads this layer's tops: the pass ends by
+  // bringing them to the host, so the layer may as well write them there.
+  virtual void SetTopsEndOnHost(bool on_host) {}
   // Sum of host_version() over the parameter blobs: changes when weights do.
   unsigned long long ParamVersion() const {
     unsigned long long v = 0;

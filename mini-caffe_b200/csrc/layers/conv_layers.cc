@@ -5,6 +5,7 @@
 #include <cstring>
 
 #include "../filler.h"
+#include "../syncedmem.h"
 #include "layers.h"
 
 namespace caffe {
@@ -24,6 +25,16 @@ float* DeviceScratch::Reserve(size_t floats) {
     blob_.reset(new Blob(vector<int>(1, static_cast<int>(floats ? floats : 1))));
   }
   return blob_->mutable_gpu_data();
+}
+
+const float* HostInput::Take(const Blob& blob) {
+  const shared_ptr<SyncedMemory>& data = blob.data();
+  const void* host = data ? data->host_only() : nullptr;
+  if (!host) return nullptr;
+  const bool again = memory_ == data.get() && version_ == data->host_version();
+  memory_ = data.get();
+  version_ = data->host_version();
+  return again ? nullptr : static_cast<const float*>(host);
 }
 
 unsigned long long TailVersion(const FusedTail& tail) {

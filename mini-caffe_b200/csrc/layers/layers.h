@@ -29,6 +29,19 @@ class DeviceScratch {
   std::unique_ptr<Blob> blob_;
 };
 
+// Remembers which values of a bottom the layer has read in place from pinned host memory.  New
+// values are read over PCIe by the kernel that needs them; values that come a second time (the
+// caller runs the net again without writing its input) are worth a copy to the device, where they
+// then stay.
+class HostInput {
+ public:
+  // The values' address in host memory if the kernel should read them there, else null.
+  const float* Take(const Blob& blob);
+ private:
+  const void* memory_ = nullptr;
+  unsigned long long version_ = 0;
+};
+
 // ---------------------------------------------------------------- producers
 
 // Convolution, 2-D, any stride / pad / dilation / group.  Depthwise layers
@@ -415,10 +428,14 @@ class ProposalLayer : public Layer {
  protected:
   void Forward_gpu(const vector<Blob*>& bottom, const vector<Blob*>& top) override;
   mcb200_proposal_params params_ = mcb200_proposal_params();
+  void SetTopsEndOnHost(bool on_host) override { tops_end_on_host_ = on_host; }
   DeviceArray anchors_;
   int num_anchors_ = 0;
-  std::unique_ptr<Blob> workspace_, staging_rois_, staging_scores_;
-  std::unique_ptr<BlobInt> counts_;
+  bool tops_end_on_host_ = false;
+  std::unique_ptr<Blob> workspace_;
+  DeviceScratch staging_rois_, staging_scores_, input_copy_;
+  std::unique_ptr<BlobInt> counts_, host_counts_;   // host_counts_: written by the kernel in pinned host memory
+  HostInput host_scores_, host_deltas_, host_info_;
 };
 
 class DetectionOutputLayer : public Layer {

@@ -33,6 +33,7 @@
 #include "google/protobuf/text_format.h"
 #include "io.h"
 #include "layer.h"
+#include "syncedmem.h"
 
 namespace caffe {
 
@@ -47,6 +48,7 @@ struct NetPlan {
   std::vector<NetStep> steps;
   std::vector<std::vector<int> > input_shapes;  // shapes of the Input tops the plan was built for
   std::vector<bool> visible;                    // per blob: guaranteed readable after Forward
+  std::vector<Blob*> marked;                    // visible blobs that are neither inputs nor tops of the last layer
   // Opt-in read when the net is constructed (environment MINICAFFE_PRECISION=bf16):
   // blobs that only tensor-core convolutions read are stored as bfloat16.
   bool half_storage = false;
@@ -212,6 +214,16 @@ void Net::PlaceMemory() {
   for (int b = 0; b < num_blobs; ++b) plan.visible[b] = blob_life_time_[b] >= num_layers;
   for (int b : top_id_vecs_[num_layers - 1]) plan.visible[b] = true;
 
+  plan.marked.clear();
+  for (int b = 0; b < num_blobs; ++b) {
+    const auto& inputs = top_id_vecs_[0];
+    const auto& last = top_id_vecs_[num_layers - 1];
+    if (plan.visible[b] && std::find(inputs.begin(), inputs.end(), b) == inputs.end() &&
+        std::find(last.begin(), last.end(), b) == last.end()) {
+      plan.marked.push_back(blobs_[b].get());
+    }
+  }
+
   // ---- fusion ----
   FusionScan scan{layers_, bottom_id_vecs_, top_id_vecs_, plan.visible, std::vector<bool>(num_layers, false)};
   plan.steps.clear();
@@ -338,6 +350,9 @@ void Net::PlaceMemory() {
     }
   }
 
+  // The last step's tops go to the host and nowhere else.
+  for (const NetStep& step : plan.steps) layers_[step.layer_id]->SetTopsEndOnHost(&step == &plan.steps.back());
+
   // ---- lifetimes over the fused schedule ----
   const int num_steps = static_cast<int>(plan.steps.size());
   std::vector<int> last_use(num_blobs, -1);
@@ -407,11 +422,18 @@ void Net::Forward(bool reshape) {
       profiler->ScopeEnd();
     }
   }
-  // As in the reference: return with the last layer's tops on the host.
+  // As in the reference: return with the last layer's tops on the host.  Marked blobs that the
+  // caller has been reading there come along, so that one wait serves them all.
   if (profiling) profiler->ScopeStart("Sync");
-  const NetStep& last = plan.steps.back();
-  for (Blob* b : last.tops) b->cpu_data();
+  std::vector<SyncedMemory*> copied;
+  for (Blob* b : plan.steps.back().tops) {
+    if (b->data()->BeginHostCopy()) copied.push_back(b->data().get());
+  }
+  for (Blob* b : plan.marked) {
+    if (b->data() && b->data()->host_reads() && b->data()->BeginHostCopy()) copied.push_back(b->data().get());
+  }
   ctx.SyncAndCheck();
+  for (SyncedMemory* m : copied) m->EndHostCopy();
   if (profiling) profiler->ScopeEnd();
 }
 

@@ -202,7 +202,7 @@ MemPoolState MemPoolGetState() { return MemoryPool::Get()->GetState(); }
 // ---------------------------------------------------------------- SyncedMemory
 
 SyncedMemory::SyncedMemory(size_t size)
-    : size_(size), valid_(0), nhwc_aliases_dev_(false), host_version_(1) {
+    : size_(size), valid_(0), nhwc_aliases_dev_(false), host_version_(1), host_reads_(false) {
   dims_[0] = dims_[1] = dims_[2] = dims_[3] = 0;
 }
 
@@ -304,16 +304,30 @@ void SyncedMemory::DeviceFromFreshest() {
 }
 
 const void* SyncedMemory::cpu_data() {
-  EnsureHost();
-  if (!(valid_ & kHost)) {
-    DeviceFromFreshest();
-    Context& ctx = Context::Get();
-    CUDA_CHECK(cudaMemcpyAsync(host_.ptr, dev_.ptr, size_, cudaMemcpyDeviceToHost, ctx.stream()));
-    ctx.SyncAndCheck();
-    valid_ |= kHost;
+  if (BeginHostCopy()) {
+    host_reads_ = true;
+    Context::Get().SyncAndCheck();
+    EndHostCopy();
   }
   return host_.ptr;
 }
+
+bool SyncedMemory::BeginHostCopy() {
+  EnsureHost();
+  if (valid_ & kHost) return false;
+  DeviceFromFreshest();
+  CUDA_CHECK(cudaMemcpyAsync(host_.ptr, dev_.ptr, size_, cudaMemcpyDeviceToHost, Context::Get().stream()));
+  return true;
+}
+
+void* SyncedMemory::overwrite_on_host() {
+  if (!host_.ptr) host_ = MemoryPool::Get()->RequestCPU(size_ ? size_ : 4);
+  valid_ = kHost;
+  ++host_version_;
+  return host_.ptr;
+}
+
+void SyncedMemory::EndHostCopy() { valid_ |= kHost; }
 
 void* SyncedMemory::mutable_cpu_data() {
   cpu_data();

@@ -76,6 +76,19 @@ class SyncedMemory {
   void* mutable_cpu_data();
   const void* gpu_data();
   void* mutable_gpu_data();
+  // cpu_data() in two halves, so that several blobs share one wait for the stream: BeginHostCopy
+  // queues the copy to the host and says whether there was anything to copy; after the caller has
+  // waited, EndHostCopy marks the host copy current.
+  bool BeginHostCopy();
+  void EndHostCopy();
+  // Whether host code has ever fetched the values from the device.
+  bool host_reads() const { return host_reads_; }
+  // For kernels that address pinned host memory themselves.  host_only: the host copy when it is the
+  // only current one (new input that no kernel has asked for yet), else null.  overwrite_on_host:
+  // the host buffer for a kernel to fill; it counts as current at once, so the caller waits for the
+  // stream before anything reads it (as the end of a forward pass does).
+  const void* host_only() const { return valid_ == kHost ? host_.ptr : nullptr; }
+  void* overwrite_on_host();
   // Channels-last copy of the (n, c, h, w) tensor stored here.  When the two
   // orders coincide (c == 1 or h*w == 1) it is the plain device copy.
   const void* gpu_data_nhwc(int n, int c, int h, int w);
@@ -104,6 +117,7 @@ class SyncedMemory {
   bool nhwc_aliases_dev_;   // the channels-last copy is dev_ itself
   int dims_[4];             // (n, c, h, w) the channels-last copy was written with
   unsigned long long host_version_;
+  bool host_reads_;         // cpu_data() had to fetch the values at least once
   DISABLE_COPY_AND_ASSIGN(SyncedMemory);
 };
 

@@ -430,6 +430,35 @@ int mcb200_deconv_as_conv_shape(const mcb200_conv_shape* deconv, mcb200_conv_sha
 int mcb200_deconv_spread_input(const mcb200_conv_shape* deconv, const float* in_nhwc, float* spread, void* stream);
 int mcb200_deconv_flip_weights(const mcb200_conv_shape* deconv, const float* w_iohw, float* w_oihw, void* stream);
 
+/* Deconvolution phase by phase, for strides up to 4 without groups and dilation: output pixels that
+ * leave the same remainders modulo the stride form a stride-1 convolution of the input with every
+ * stride-th tap of the filter, so nothing is multiplied by zeros; all phases run in one launch.  A
+ * single input pixel without padding (the first layer of a generator) runs with one phase per tap
+ * whatever its stride.  packed_weight_count is 0 for shapes it does not take.  The epilogue's
+ * residual must be NULL; out is channels last with out_ld floats per pixel.                       */
+typedef struct mcb200_deconv_plan {
+  mcb200_conv_plan conv;
+  int stride_h, stride_w;            /* phases per axis */
+  int grid_h, grid_w;                /* positions per phase and image */
+  int out_h, out_w;
+  unsigned char off_h[4], off_w[4];  /* where a phase's filter window starts behind the grid's origin */
+} __attribute__((aligned(64))) mcb200_deconv_plan;
+size_t mcb200_deconv_tc_packed_weight_count(const mcb200_conv_shape* deconv);
+int mcb200_deconv_tc_pack_weights(const mcb200_conv_shape* deconv, const float* w_iohw, float* packed, void* stream);
+int mcb200_deconv_tc_plan(const mcb200_conv_shape* deconv, const float* in, const float* packed_w, mcb200_deconv_plan* plan);
+int mcb200_deconv_tc_launch(mcb200_deconv_plan* plan, float* out, int out_ld, const mcb200_epilogue* ep, int* status,
+                            void* stream);
+
+/* The same layer with all phases as output channels (phase-major) of one convolution over the union
+ * of their windows: more zeros to multiply, but one N tile for layers whose phases together have
+ * few channels.  mcb200_deconv_as_window_conv gives that convolution's shape (non-zero: not
+ * expressible, or not a shape that phases take), _window_weights its [cout, c, kh, kw] filter, and
+ * mcb200_depth_to_space brings [n, grid_h, grid_w, stride_h, stride_w, c] into [n, out_h, out_w, c]. */
+int mcb200_deconv_as_window_conv(const mcb200_conv_shape* deconv, mcb200_conv_shape* conv);
+int mcb200_deconv_window_weights(const mcb200_conv_shape* deconv, const float* w_iohw, float* w_oihw, void* stream);
+int mcb200_depth_to_space(const float* src, float* dst, int n, int grid_h, int grid_w, int stride_h, int stride_w, int c,
+                          int out_h, int out_w, void* stream);
+
 /* Crop: out[idx] = in[idx + offsets] over up to six axes
  * (src/layers/crop_layer.cpp:57-100).                                         */
 int mcb200_crop(const float* in, float* out, int num_axes, const int* in_shape, const int* out_shape,
@@ -451,6 +480,13 @@ int mcb200_lrn(const float* in_nchw, float* out_nchw, int n, int c, int h, int w
  * inner + position); inner = 1 for channels-last data.                         */
 int mcb200_channel_batch_stats(const float* x, long long count, int channels, int inner, float eps, float* scale,
                                float* shift, void* stream);
+/* The same for channels-last data (inner = 1, channels % 4 == 0, x 16-byte aligned), by all SMs;
+ * behind it an affine map: scale *= then_scale, shift = shift * then_scale + then_shift per channel
+ * (either may be NULL).  `workspace` is batch_stats_workspace_bytes of device memory whose first
+ * word is zero before the first call; it is zero again after each.                               */
+size_t mcb200_channel_batch_stats_workspace_bytes(int channels);
+int mcb200_channel_batch_stats_nhwc(const float* x, long long count, int channels, float eps, const float* then_scale,
+                                    const float* then_shift, void* workspace, float* scale, float* shift, void* stream);
 
 /* y = tanh(x) or y = 1 / (1 + exp(-x)), elementwise, any layout
  * (src/layers/tanh_layer.cpp:10-18, src/layers/sigmoid_layer.cpp:10-22).      */

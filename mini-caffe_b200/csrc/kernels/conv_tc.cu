@@ -67,6 +67,8 @@ constexpr int kModeMatrix = 0;   // rows of a plain [m, c] matrix (1x1 convoluti
 constexpr int kModeIm2col = 1;   // im2col-mode tensor map: any filter, channels % 4 == 0
 constexpr int kModeRows = 2;     // <= 4 channels: one filter row of 8 pixels x 4 channels per k-iteration
 constexpr int kModeHalo = 3;     // stride-1 filters wider than one tap: the taps of a filter row share one pixel strip
+constexpr int kModePhase = 4;    // deconvolution: one im2col convolution per phase of the output grid
+constexpr int kMaxPhase = 4;      // largest deconvolution stride that phase mode takes
 constexpr int kMaxHaloRows = 16; // extra strip rows ((kw - 1) * dilation) the halo mode takes
 
 struct ConvTcArgs {
@@ -102,6 +104,15 @@ struct ConvTcArgs {
   // its groups span (from `c_origin`, rounded down to 16 bytes) by a block-diagonal weight tile:
   // the packed weights hold zeros where an output column's group does not own the channel.
   int group_cout, group_cin;
+  // Phase mode.  Output pixel (i * stride + py, j * stride + px) of a deconvolution sums the taps whose
+  // row (column) has the remainder that py (px) asks for, over neighbouring input pixels: a
+  // stride-1 convolution of its own per (py, px).  m runs over the (n, i, j) grid (`ho` x `wo`), an N
+  // tile belongs to one phase, whose filter window starts phase_off_h[py] / phase_off_w[px] pixels
+  // behind the grid's own origin.
+  int phase_tiles;               // N tiles per phase
+  int phase_stride_h, phase_stride_w;
+  unsigned char phase_off_h[kMaxPhase], phase_off_w[kMaxPhase];
+  int out_h, out_w;              // the output image, which may cut the last row and column of the grid short
   int l2_prefetch;               // ask L2 for the next tile's activations a tile ahead
   int halo_staged;               // halo mode: results pass through a shared-memory slot so that the stores are
                                  // whole 128-byte rows (fp32 output with 16-byte aligned rows)
@@ -227,6 +238,9 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                const ConvTcArgs args) {
   static_assert(!(kPair && kMode == kModeRows), "row mode runs unpaired");
   static_assert(!(kHalf && kMode == kModeRows), "row mode takes fp32 images");
+  static_assert(!((kPair || kHalf) && kMode == kModePhase), "phase mode runs unpaired on fp32 operands");
+  constexpr bool kIm2col = kMode == kModeIm2col || kMode == kModePhase;     // how activations are fetched
+  constexpr bool kScatter = kMode == kModeHalo || kMode == kModePhase;      // output rows are not one box
   using Plan = SmemPlan<BN, kMode, kPair>;
   constexpr int kElemsK = kHalf ? kBlockKHalf : kBlockK;   // channels per k-iteration
   MCB200_TRACE_CTA(0);
@@ -259,7 +273,8 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int n_tiles = (args.cout + BN - 1) / BN;
+  const int n_tiles = kMode == kModePhase ? args.phase_tiles * args.phase_stride_h * args.phase_stride_w
+                                          : (args.cout + BN - 1) / BN;
   // Row mode: an M tile is (a segment of at most 128 pixels of) one output row of one image.
   const int m_tiles = kMode == kModeRows ? (args.m / args.wo) * args.row_segments : (args.m + kBlockM - 1) / kBlockM;
   // Row mode helpers: image row (n * ho + p) and first pixel of the segment of M tile mt.
@@ -370,7 +385,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           base_h = (row - base_n * args.ho) * args.stride_h;   // row in the spatially padded copy
           base_w = seg_start(mt);                              // first output pixel of the segment
         }
-        if (kMode == kModeIm2col) {
+        if (kIm2col) {
           const int q = m0 % args.wo;
           const int p = (m0 / args.wo) % args.ho;
           base_n = m0 / (args.wo * args.ho);
@@ -436,7 +451,14 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         // Position inside the filter, advanced incrementally: channel block,
         // then tap column, then tap row.
         int c0 = 0, sx = 0;
-        uint16_t off_w = 0, off_h = 0;
+        uint16_t off_w0 = 0, off_h = 0;
+        if (kMode == kModePhase) {
+          const int phase = (tile % n_tiles) / args.phase_tiles;
+          const int py = phase / args.phase_stride_w;
+          off_h = args.phase_off_h[py];
+          off_w0 = args.phase_off_w[phase - py * args.phase_stride_w];
+        }
+        uint16_t off_w = off_w0;
         int row_h = base_h;
         for (int k = 0; k < args.k_iters; k += Plan::kSub) {
           if (!mbar_wait_bounded(&empty_bar[pos.stage], pos.parity ^ 1u, abort, wait_limit)) {
@@ -469,7 +491,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 c0 = 0;
                 off_h = static_cast<uint16_t>(off_h + args.dil_h);
               }
-            } else if (kMode == kModeIm2col) {
+            } else if (kIm2col) {
               if (kPair) {
                 if (live) tma_load_im2col_4d_pair(&map_a, bar_leader, a_dst, c_origin + c0, base_w, base_h, base_n, off_w, off_h);
               } else {
@@ -481,7 +503,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 off_w = static_cast<uint16_t>(off_w + args.dil_w);
                 if (++sx == args.kw) {
                   sx = 0;
-                  off_w = 0;
+                  off_w = off_w0;
                   off_h = static_cast<uint16_t>(off_h + args.dil_h);
                 }
               }
@@ -523,7 +545,12 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       }
       for (int tile = worker; tile < num_tiles && alive; tile += workers) {
         // A CTA of a pair fetches the half of the weight tile that matches its rank.
-        const int n0 = (tile % n_tiles) * BN + static_cast<int>(rank) * Plan::kTileBRows;
+        int n0 = (tile % n_tiles) * BN + static_cast<int>(rank) * Plan::kTileBRows;
+        if (kMode == kModePhase) {
+          // weight rows run over the phases, then their output channels
+          const int phase = (tile % n_tiles) / args.phase_tiles;
+          n0 = phase * args.cout + (tile % n_tiles - phase * args.phase_tiles) * BN;
+        }
         int k0 = 0;
         int halo_cb = 0, halo_row_k0 = 0;   // halo mode: channel block and first packed-weight column of the filter row
         for (int k = 0; k < args.k_iters; k += Plan::kSub) {
@@ -779,7 +806,15 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       const uint32_t use = static_cast<uint32_t>(local >> 1) & 1u;
       const int unit = tile / n_tiles;
       const int mt = unit_to_mt(unit);
-      const int n0 = (tile - unit * n_tiles) * BN;
+      int n0 = (tile - unit * n_tiles) * BN;
+      int phase_y = 0, phase_x = 0;
+      if (kMode == kModePhase) {
+        const int nt = tile - unit * n_tiles;
+        const int phase = nt / args.phase_tiles;
+        n0 = (nt - phase * args.phase_tiles) * BN;
+        phase_y = phase / args.phase_stride_w;
+        phase_x = phase - phase_y * args.phase_stride_w;
+      }
       // First output row (pixel) of this warp's 32-row slice, and how many of the 32 exist.
       const int row0 = (kMode == kModeRows ? row_of(mt) * args.wo + seg_start(mt) : mt * kBlockM) + quad * 32;
       const int rows_here = kMode == kModeRows ? min(args.tile_rows, args.wo - seg_start(mt)) - quad * 32 : args.m - row0;
@@ -791,6 +826,14 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         const int j = out_row - t * args.wp;
         row_ok = row_ok && j < args.wo;
         out_row = t * args.wo + j;
+      }
+      if (kMode == kModePhase) {
+        const int t = out_row / args.wo;           // (image, grid row)
+        const int image = t / args.ho;
+        const int y = (t - image * args.ho) * args.phase_stride_h + phase_y;
+        const int x = (out_row - t * args.wo) * args.phase_stride_w + phase_x;
+        row_ok = row_ok && y < args.out_h && x < args.out_w;
+        out_row = (image * args.out_h + y) * args.out_w + x;
       }
       // tcgen05.ld is warp-collective: the whole warp takes the same branch.
       alive = __all_sync(0xffffffffu, mbar_wait_bounded(&tmem_full_bar[ab], use, abort, wait_limit));
@@ -999,7 +1042,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           const bool whole_chunk = args.vec_store && col0 + 32 <= args.cout;
           // The lane's 32 outputs of its row (128 bytes, 64 as bfloat16), fused tail applied.
           float4 v[8];
-          if (whole_chunk && (row_ok || (kMode == kModeHalo && args.halo_staged))) {
+          if (whole_chunk && (row_ok || (kScatter && args.halo_staged))) {
             const bool add_res = has_res && row_ok;
             auto fill = [&](auto act_tag) {
               if (!add_res) {
@@ -1039,7 +1082,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
               for (int j = 0; j < 8; ++j) round4(v[j]);
             }
           }
-          if (kMode == kModeHalo && args.halo_staged && whole_chunk) {
+          if (kScatter && args.halo_staged && whole_chunk) {
             // Through the warp's shared-memory slot, so that a store instruction writes four whole
             // 128-byte rows (eight lanes each) instead of 16 bytes of 32 different rows: a lane's
             // own row may be a dropped position, its neighbours' rows are not.
@@ -1440,7 +1483,10 @@ cudaError_t launch_variant(const mcb200_conv_plan* plan, ConvTcArgs args, cudaSt
                                 ? static_cast<long long>(plan->shape.n) * plan->shape.ho * args.row_segments
                                 : (static_cast<long long>(args.m) + kBlockM - 1) / kBlockM;   // halo: virtual positions
   const long long m_units = kPair ? (m_tiles + 1) / 2 : m_tiles;
-  const long long tiles = static_cast<long long>((plan->shape.cout + BN - 1) / BN) * m_units;
+  const long long n_tiles = kMode == kModePhase
+                                ? static_cast<long long>(args.phase_tiles) * args.phase_stride_h * args.phase_stride_w
+                                : (plan->shape.cout + BN - 1) / BN;
+  const long long tiles = n_tiles * m_units;
   if (tiles > 0x3fffffffLL) return cudaErrorInvalidConfiguration;
   // One persistent CTA per SM (fewer when there are fewer tiles); a paired
   // launch is a grid of two-CTA clusters, one cluster per tile at a time.
@@ -1491,6 +1537,12 @@ cudaError_t launch_variant(const mcb200_conv_plan* plan, ConvTcArgs args, cudaSt
     args.slots = 1;
     staging_bytes = args.halo_staged ? Plan::staging_bytes(1, 4096) : 0;
   }
+  if (kMode == kModePhase) {
+    // Results pass through one slot per warp, as in halo mode.
+    args.halo_staged = args.vec_store ? 1 : 0;
+    args.slots = 1;
+    staging_bytes = args.halo_staged ? Plan::staging_bytes(1, 4096) : 0;
+  }
   {
     // At most 64 prefetch instructions per tile (long-K tiles take long enough for the ring).
     const int kh = plan->shape.kh, cb = args.c_blocks;
@@ -1499,7 +1551,7 @@ cudaError_t launch_variant(const mcb200_conv_plan* plan, ConvTcArgs args, cudaSt
     // reductions lose 8 %: the requests compete with the loads of the tile at hand), and the
     // layers it was meant for do not gain.
     const char* pf = getenv("MCB200_L2_PREFETCH");
-    args.l2_prefetch = (kMode != kModeRows && count <= 64 && pf && pf[0] == '1') ? 1 : 0;
+    args.l2_prefetch = (kMode != kModeRows && kMode != kModePhase && count <= 64 && pf && pf[0] == '1') ? 1 : 0;
   }
   int stages = (dynamic_limit - 1024 - staging_bytes - resident_bytes) / stage_bytes;
   if (stages > kMaxStages) stages = kMaxStages;
@@ -1648,6 +1700,13 @@ extern "C" int mcb200_bf16_to_f32(const uint16_t* src, float* dst, size_t count,
 
 namespace {
 
+// Drivers up to CUDA 13.1 encode a flag in im2col descriptors of tensors smaller than 128 KiB that
+// makes the load misbehave; NVIDIA's CUTLASS clears it the same way
+// (cute/atom/copy_traits_sm90_im2col.hpp).
+void clear_small_tensor_flag(CUtensorMap* map, unsigned long long bytes) {
+  if (driver_api().driver_version <= 13010 && bytes < 131072ull) reinterpret_cast<uint64_t*>(map)[1] &= ~(1ull << 21);
+}
+
 // Shared by the fp32 (TF32) and the bfloat16 plan: `in` and `packed_w` hold
 // elements of `es` bytes, a k-iteration covers `kelems` channels (128 bytes).
 int plan_core(const mcb200_conv_shape* s, const void* in, const void* packed_w, mcb200_conv_plan* plan, bool half) {
@@ -1747,13 +1806,7 @@ int plan_core(const mcb200_conv_shape* s, const void* in, const void* packed_w, 
     r = api.im2col(ma, dtype, 4, const_cast<void*>(in), dims, strides, lower, upper,
                    static_cast<cuuint32_t>(kelems), halo ? static_cast<cuuint32_t>(plan->strip_rows) : kBlockM, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                    CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    // Drivers up to CUDA 13.1 encode a flag in im2col descriptors of tensors
-    // smaller than 128 KiB that makes the load misbehave; NVIDIA's CUTLASS
-    // clears it the same way (cute/atom/copy_traits_sm90_im2col.hpp).
-    if (r == CUDA_SUCCESS && api.driver_version <= 13010) {
-      const unsigned long long bytes = static_cast<unsigned long long>(pix) * s->w * s->h * s->n;
-      if (bytes < 131072ull) reinterpret_cast<uint64_t*>(ma)[1] &= ~(1ull << 21);
-    }
+    if (r == CUDA_SUCCESS) clear_small_tensor_flag(ma, pix * s->w * s->h * s->n);
   }
   if (r != CUDA_SUCCESS) return -100 - static_cast<int>(r);
   {
@@ -1773,7 +1826,7 @@ int plan_core(const mcb200_conv_shape* s, const void* in, const void* packed_w, 
 }
 
 int launch_core(mcb200_conv_plan* plan, void* out, bool out_half, int out_ld, const mcb200_epilogue* ep, int* status,
-                void* stream);
+                void* stream, const mcb200_deconv_plan* phases = nullptr);
 
 }  // namespace
 
@@ -1801,7 +1854,7 @@ extern "C" int mcb200_conv_tc_launch_bf16(mcb200_conv_plan* plan, void* out, int
 namespace {
 
 int launch_core(mcb200_conv_plan* plan, void* out, bool out_half, int out_ld, const mcb200_epilogue* ep, int* status,
-                void* stream) {
+                void* stream, const mcb200_deconv_plan* phases) {
   if (!plan || !out || out_ld < plan->shape.cout) return -1;
   const bool half = plan->operand_bf16 != 0;
   ConvTcArgs a;
@@ -1849,6 +1902,21 @@ int launch_core(mcb200_conv_plan* plan, void* out, bool out_half, int out_ld, co
     a.m = plan->m_virtual;
     a.wp = plan->m_virtual / (plan->shape.n * plan->shape.ho);
   }
+  a.phase_tiles = 0;
+  if (phases) {
+    a.tma_epilogue = 0;
+    a.phase_tiles = (a.cout + plan->block_n - 1) / plan->block_n;
+    a.phase_stride_h = phases->stride_h;
+    a.phase_stride_w = phases->stride_w;
+    for (int i = 0; i < kMaxPhase; ++i) {
+      a.phase_off_h[i] = phases->off_h[i];
+      a.phase_off_w[i] = phases->off_w[i];
+    }
+    a.out_h = phases->out_h;
+    a.out_w = phases->out_w;
+    a.ho = phases->grid_h;
+    a.wo = phases->grid_w;
+  }
   if (a.tma_epilogue) {
     const bool rows = plan->im2col == kModeRows;
     const long long per_group = rows ? plan->shape.wo : plan->m;
@@ -1879,6 +1947,7 @@ int launch_core(mcb200_conv_plan* plan, void* out, bool out_half, int out_ld, co
   e = mode == kModeRows     ? launch_variant<BN, kModeRows, false, false>(plan, a, st)    \
       : mode == kModeIm2col ? launch_variant<BN, kModeIm2col, false, false>(plan, a, st)  \
       : mode == kModeHalo   ? launch_variant<BN, kModeHalo, false, false>(plan, a, st)    \
+      : mode == kModePhase  ? launch_variant<BN, kModePhase, false, false>(plan, a, st)   \
                             : launch_variant<BN, kModeMatrix, false, false>(plan, a, st)
 #define MCB200_DISPATCH_PAIR(BN)                                                          \
   e = mode == kModeIm2col ? launch_variant<BN, kModeIm2col, true, false>(plan, a, st)     \
@@ -1928,6 +1997,262 @@ int launch_core(mcb200_conv_plan* plan, void* out, bool out_half, int out_ld, co
 }
 
 }  // namespace
+
+// ------------------------------------------------------------------ phase mode (deconvolution)
+
+namespace mcb200 {
+namespace {
+
+// Geometry of one axis: the filter window of phase f covers the input positions
+// i + first[f] .. i + first[f] + taps - 1 for grid position i.
+struct PhaseAxis {
+  int taps, grid, lowest;      // lowest = min over the phases of `first`
+  int first[kMaxPhase];
+};
+
+bool phase_axis(int k, int stride, int pad, int out, PhaseAxis* a) {
+  if (stride < 1 || stride > kMaxPhase || out < 1) return false;
+  a->taps = (k + stride - 1) / stride;
+  a->grid = (out + stride - 1) / stride;
+  for (int f = 0; f < stride; ++f) {
+    // tap r reaches output i * stride + f from input i + (f + pad - r) / stride
+    const int last = (f + pad - (f + pad) % stride) / stride;
+    a->first[f] = last - (a->taps - 1);
+    a->lowest = f == 0 || a->first[f] < a->lowest ? a->first[f] : a->lowest;
+  }
+  return true;
+}
+
+// A single input pixel reaches every output pixel through exactly one tap: the layer is then one
+// phase per tap, whatever its stride.
+void phase_strides(const mcb200_conv_shape& d, int* sh, int* sw) {
+  const bool pixel = d.h == 1 && d.w == 1 && d.pad_h == 0 && d.pad_w == 0;
+  *sh = pixel ? d.kh : d.stride_h;
+  *sw = pixel ? d.kw : d.stride_w;
+}
+
+struct PhaseTable {
+  int first_h[kMaxPhase], first_w[kMaxPhase];
+  int stride_h, stride_w, pad_h, pad_w, kh, kw, taps_h, taps_w;
+};
+
+// [c_in, c_out, kh, kw] -> [phase][c_out][taps][c_pad], zero where a window reaches past the filter.
+__global__ void pack_phase_weights_kernel(const float* __restrict__ w, float* __restrict__ packed, int c, int cout, int c_pad,
+                                          PhaseTable p) {
+  const int taps = p.taps_h * p.taps_w;
+  const size_t total = static_cast<size_t>(p.stride_h) * p.stride_w * cout * taps * c_pad;
+  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total;
+       i += static_cast<size_t>(gridDim.x) * blockDim.x) {
+    const int cc = static_cast<int>(i % c_pad);
+    const int tap = static_cast<int>((i / c_pad) % taps);
+    const size_t row = i / (static_cast<size_t>(c_pad) * taps);
+    const int co = static_cast<int>(row % cout), phase = static_cast<int>(row / cout);
+    const int py = phase / p.stride_w, px = phase % p.stride_w;
+    const int r = py + p.pad_h - p.stride_h * (p.first_h[py] + tap / p.taps_w);
+    const int q = px + p.pad_w - p.stride_w * (p.first_w[px] + tap % p.taps_w);
+    float v = 0.f;
+    if (cc < c && r >= 0 && r < p.kh && q >= 0 && q < p.kw)
+      v = round_to_tf32(w[((static_cast<size_t>(cc) * cout + co) * p.kh + r) * p.kw + q]);
+    packed[i] = v;
+  }
+}
+
+bool phase_geometry(const mcb200_conv_shape* deconv, mcb200_conv_shape* d, PhaseAxis* y, PhaseAxis* x, int* sh, int* sw) {
+  if (!deconv) return false;
+  *d = *deconv;
+  if (mcb200_deconv_out_shape(d) != 0) return false;
+  if (d->group != 1 || d->dil_h != 1 || d->dil_w != 1 || d->c_stride < d->c || (d->c_stride & 3) != 0) return false;
+  phase_strides(*d, sh, sw);
+  if (!phase_axis(d->kh, *sh, d->pad_h, d->ho, y) || !phase_axis(d->kw, *sw, d->pad_w, d->wo, x)) return false;
+  // limits of the im2col tensor map: 8-bit signed box corners
+  const int upper_h = y->grid - d->h + y->lowest, upper_w = x->grid - d->w + x->lowest;
+  return y->lowest >= -128 && x->lowest >= -128 && upper_h >= -128 && upper_h <= 127 && upper_w >= -128 && upper_w <= 127 &&
+         static_cast<long long>(d->n) * y->grid * x->grid <= 0x7fffffffLL;
+}
+
+}  // namespace
+}  // namespace mcb200
+
+extern "C" size_t mcb200_deconv_tc_packed_weight_count(const mcb200_conv_shape* deconv) {
+  mcb200_conv_shape d;
+  PhaseAxis y, x;
+  int sh, sw;
+  if (!phase_geometry(deconv, &d, &y, &x, &sh, &sw)) return 0;
+  return static_cast<size_t>(sh) * sw * d.cout * y.taps * x.taps * ((d.c + kBlockK - 1) / kBlockK * kBlockK);
+}
+
+extern "C" int mcb200_deconv_tc_pack_weights(const mcb200_conv_shape* deconv, const float* w_iohw, float* packed, void* stream) {
+  mcb200_conv_shape d;
+  PhaseAxis y, x;
+  int sh, sw;
+  if (!w_iohw || !packed || !phase_geometry(deconv, &d, &y, &x, &sh, &sw)) return -1;
+  PhaseTable t = {};
+  for (int f = 0; f < kMaxPhase; ++f) {
+    t.first_h[f] = y.first[f];
+    t.first_w[f] = x.first[f];
+  }
+  t.stride_h = sh;
+  t.stride_w = sw;
+  t.pad_h = d.pad_h;
+  t.pad_w = d.pad_w;
+  t.kh = d.kh;
+  t.kw = d.kw;
+  t.taps_h = y.taps;
+  t.taps_w = x.taps;
+  const size_t total = mcb200_deconv_tc_packed_weight_count(deconv);
+  const size_t blocks = (total + 255) / 256;
+  pack_phase_weights_kernel<<<static_cast<int>(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      w_iohw, packed, d.c, d.cout, (d.c + kBlockK - 1) / kBlockK * kBlockK, t);
+  count_launch();
+  return static_cast<int>(cudaGetLastError());
+}
+
+namespace mcb200 {
+namespace {
+
+// [c_in, c_out, kh, kw] -> [phase][c_out][c_in][window_h][window_w] over the union of the phases'
+// windows, zero where a phase's filter does not reach.
+__global__ void window_weights_kernel(const float* __restrict__ w, float* __restrict__ out, int c, int cout, int win_h, int win_w,
+                                      int lowest_h, int lowest_w, PhaseTable p) {
+  const size_t total = static_cast<size_t>(p.stride_h) * p.stride_w * cout * c * win_h * win_w;
+  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total;
+       i += static_cast<size_t>(gridDim.x) * blockDim.x) {
+    size_t t = i;
+    const int tx = static_cast<int>(t % win_w);
+    t /= win_w;
+    const int ty = static_cast<int>(t % win_h);
+    t /= win_h;
+    const int cc = static_cast<int>(t % c);
+    t /= c;
+    const int co = static_cast<int>(t % cout), phase = static_cast<int>(t / cout);
+    const int r = phase / p.stride_w + p.pad_h - p.stride_h * (lowest_h + ty);
+    const int q = phase % p.stride_w + p.pad_w - p.stride_w * (lowest_w + tx);
+    out[i] = r >= 0 && r < p.kh && q >= 0 && q < p.kw ? w[((static_cast<size_t>(cc) * cout + co) * p.kh + r) * p.kw + q] : 0.f;
+  }
+}
+
+// The window of an axis and whether a stride-1 convolution padded alike on both ends yields the grid.
+bool window_of(const PhaseAxis& a, int stride, int size, int* window) {
+  int highest = a.first[0];
+  for (int f = 1; f < stride; ++f) highest = a.first[f] > highest ? a.first[f] : highest;
+  *window = highest + a.taps - a.lowest;
+  return a.lowest <= 0 && size - 2 * a.lowest - *window + 1 == a.grid;
+}
+
+}  // namespace
+}  // namespace mcb200
+
+extern "C" int mcb200_deconv_as_window_conv(const mcb200_conv_shape* deconv, mcb200_conv_shape* conv) {
+  mcb200_conv_shape d;
+  PhaseAxis y, x;
+  int sh, sw, win_h, win_w;
+  if (!conv || !phase_geometry(deconv, &d, &y, &x, &sh, &sw)) return -1;
+  if (!window_of(y, sh, d.h, &win_h) || !window_of(x, sw, d.w, &win_w)) return -2;
+  *conv = d;
+  conv->cout = d.cout * sh * sw;
+  conv->kh = win_h;
+  conv->kw = win_w;
+  conv->pad_h = -y.lowest;
+  conv->pad_w = -x.lowest;
+  conv->stride_h = conv->stride_w = 1;
+  return mcb200_conv_out_shape(conv);
+}
+
+extern "C" int mcb200_deconv_window_weights(const mcb200_conv_shape* deconv, const float* w_iohw, float* w_oihw, void* stream) {
+  mcb200_conv_shape d, conv;
+  PhaseAxis y, x;
+  int sh, sw;
+  if (!w_iohw || !w_oihw || mcb200_deconv_as_window_conv(deconv, &conv) != 0 || !phase_geometry(deconv, &d, &y, &x, &sh, &sw)) return -1;
+  PhaseTable t = {};
+  t.stride_h = sh;
+  t.stride_w = sw;
+  t.pad_h = d.pad_h;
+  t.pad_w = d.pad_w;
+  t.kh = d.kh;
+  t.kw = d.kw;
+  const size_t total = static_cast<size_t>(conv.cout) * d.c * conv.kh * conv.kw;
+  const size_t blocks = (total + 255) / 256;
+  window_weights_kernel<<<static_cast<int>(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      w_iohw, w_oihw, d.c, d.cout, conv.kh, conv.kw, y.lowest, x.lowest, t);
+  count_launch();
+  return static_cast<int>(cudaGetLastError());
+}
+
+extern "C" int mcb200_deconv_tc_plan(const mcb200_conv_shape* deconv, const float* in, const float* packed_w,
+                                     mcb200_deconv_plan* plan) {
+  mcb200_conv_shape d;
+  PhaseAxis y, x;
+  int sh, sw;
+  if (!in || !packed_w || !plan) return -1;
+  if (!phase_geometry(deconv, &d, &y, &x, &sh, &sw)) return -2;
+  if ((reinterpret_cast<uintptr_t>(in) & 15) || (reinterpret_cast<uintptr_t>(packed_w) & 15)) return -3;
+  const DriverApi& api = driver_api();
+  if (!api.ok) return -5;
+  mcb200_conv_plan& conv = plan->conv;
+  conv.shape = d;
+  conv.shape.kh = y.taps;
+  conv.shape.kw = x.taps;
+  conv.shape.stride_h = conv.shape.stride_w = 1;
+  conv.shape.pad_h = -y.lowest;
+  conv.shape.pad_w = -x.lowest;
+  conv.out_ptr = nullptr;
+  conv.res_ptr = nullptr;
+  conv.out_ld = conv.res_ld = conv.cta_pair = 0;
+  conv.operand_bf16 = conv.out_bf16 = 0;
+  conv.m = d.n * y.grid * x.grid;
+  conv.m_virtual = conv.m;
+  conv.strip_rows = 0;
+  conv.c_blocks = (d.c + kBlockK - 1) / kBlockK;
+  conv.k_iters = y.taps * x.taps * conv.c_blocks;
+  conv.im2col = kModePhase;
+  plan->stride_h = sh;
+  plan->stride_w = sw;
+  plan->grid_h = y.grid;
+  plan->grid_w = x.grid;
+  plan->out_h = d.ho;
+  plan->out_w = d.wo;
+  for (int f = 0; f < kMaxPhase; ++f) {
+    plan->off_h[f] = static_cast<unsigned char>(f < sh ? y.first[f] - y.lowest : 0);
+    plan->off_w[f] = static_cast<unsigned char>(f < sw ? x.first[f] - x.lowest : 0);
+  }
+  // The phases multiply the tiles like so many more output pixels.
+  conv.block_n = pick_block_n(d.cout, static_cast<long long>(conv.m) * sh * sw, conv.k_iters);
+  CUtensorMap* ma = reinterpret_cast<CUtensorMap*>(conv.tma_a);
+  CUtensorMap* mb = reinterpret_cast<CUtensorMap*>(conv.tma_b);
+  const cuuint64_t pix = static_cast<cuuint64_t>(d.c_stride) * 4;
+  {
+    const cuuint64_t dims[4] = {static_cast<cuuint64_t>(d.c), static_cast<cuuint64_t>(d.w), static_cast<cuuint64_t>(d.h),
+                                static_cast<cuuint64_t>(d.n)};
+    const cuuint64_t strides[3] = {pix, pix * d.w, pix * d.w * d.h};
+    // Base pixels: as many positions per row and image as the grid has, from the lowest window start on.
+    const int lower[2] = {x.lowest, y.lowest};
+    const int upper[2] = {x.grid - d.w + x.lowest, y.grid - d.h + y.lowest};
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    CUresult r = api.im2col(ma, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float*>(in), dims, strides, lower, upper, kBlockK,
+                            kBlockM, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return -100 - static_cast<int>(r);
+    clear_small_tensor_flag(ma, pix * d.w * d.h * d.n);
+  }
+  {
+    const cuuint64_t kp = static_cast<cuuint64_t>(conv.k_iters) * kBlockK;
+    const cuuint64_t dims[2] = {kp, static_cast<cuuint64_t>(d.cout) * sh * sw};
+    const cuuint64_t strides[1] = {kp * 4};
+    const cuuint32_t box[2] = {kBlockK, static_cast<cuuint32_t>(conv.block_n)};
+    const cuuint32_t estr[2] = {1, 1};
+    CUresult r = api.tiled(mb, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(packed_w), dims, strides, box, estr,
+                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return -200 - static_cast<int>(r);
+  }
+  return 0;
+}
+
+extern "C" int mcb200_deconv_tc_launch(mcb200_deconv_plan* plan, float* out, int out_ld, const mcb200_epilogue* ep, int* status,
+                                       void* stream) {
+  if (!plan || plan->conv.im2col != kModePhase || (ep && ep->residual)) return -1;
+  return launch_core(&plan->conv, out, false, out_ld, ep, status, stream, plan);
+}
 
 // ------------------------------------------------------------------ row mode (few input channels)
 

@@ -177,6 +177,128 @@ channel_batch_stats_kernel(const float* __restrict__ x, long long per_channel, i
   }
 }
 
+// The same for channels-last data.  A block takes a run of pixels; its threads are 4-channel groups x
+// pixel lanes, so that a warp reads whole rows.  Sums of x - x0 and (x - x0)^2, x0 being the channel's
+// value at the first pixel, lose nothing to the mean's size; a thread's fp32 sums run over a few
+// dozen values, everything above them is added in double and in a fixed order.  The block that
+// finishes last adds the blocks' sums.  (One block per channel reading a float of every pixel: 240 us
+// for 64 channels of 65536 pixels, which are 16.8 MB.)
+constexpr int kStatsThreads = 256;
+constexpr int kStatsBlocks = 128;    // the last block adds as many sums per channel, sixteen loads in flight
+
+__global__ void __launch_bounds__(kStatsThreads, 1)
+channel_batch_stats_nhwc_kernel(const float* __restrict__ x, long long pixels, int channels, float eps,
+                                const float* __restrict__ then_scale, const float* __restrict__ then_shift,
+                                unsigned* __restrict__ arrived, double* __restrict__ partial, float* __restrict__ scale,
+                                float* __restrict__ shift) {
+  __shared__ double lanes[kStatsThreads][8];
+  __shared__ bool last;
+  const int quads = channels >> 2;
+  const long long per_block = (pixels + gridDim.x - 1) / gridDim.x;
+  const long long first = blockIdx.x * per_block, end = min(first + per_block, pixels);
+  double* mine = partial + static_cast<size_t>(blockIdx.x) * 2 * channels;
+  for (int q0 = 0; q0 < quads; q0 += kStatsThreads) {
+    const int width = min(quads - q0, kStatsThreads);       // groups handled side by side
+    const int rows = kStatsThreads / width;                 // pixel lanes
+    const int q = threadIdx.x % width, lane = threadIdx.x / width;
+    double sum[8] = {0., 0., 0., 0., 0., 0., 0., 0.};
+    if (lane < rows) {
+      const float4* column = reinterpret_cast<const float4*>(x) + q0 + q;
+      const float4 base = column[0];
+      for (long long p = first + lane; p < end;) {
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f), s2 = s;
+        for (int i = 0; i < 4 && p < end; ++i) {
+          // eight rows in flight; rows beyond the run stand in as x0, which adds nothing
+          float4 v[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u, p += rows) v[u] = p < end ? column[p * quads] : base;
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            const float a = v[u].x - base.x, b = v[u].y - base.y, c = v[u].z - base.z, d = v[u].w - base.w;
+            s.x += a;
+            s.y += b;
+            s.z += c;
+            s.w += d;
+            s2.x = fmaf(a, a, s2.x);
+            s2.y = fmaf(b, b, s2.y);
+            s2.z = fmaf(c, c, s2.z);
+            s2.w = fmaf(d, d, s2.w);
+          }
+        }
+        sum[0] += s.x;
+        sum[1] += s.y;
+        sum[2] += s.z;
+        sum[3] += s.w;
+        sum[4] += s2.x;
+        sum[5] += s2.y;
+        sum[6] += s2.z;
+        sum[7] += s2.w;
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) lanes[threadIdx.x][j] = sum[j];
+    __syncthreads();
+    for (int i = threadIdx.x; i < width * 8; i += kStatsThreads) {
+      const int group = i >> 3, j = i & 7;
+      double total = 0.;
+      for (int r = 0; r < rows; ++r) total += lanes[r * width + group][j];
+      mine[(j >> 2) * channels + (q0 + group) * 4 + (j & 3)] = total;
+    }
+    __syncthreads();
+  }
+  // (One thread's fence covers the block's writes, which the barrier orders before it; a fence by all
+  // of them costs tens of microseconds.)
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(arrived, 1u) == gridDim.x - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  if (!last) return;
+  for (int c = threadIdx.x; c < channels; c += kStatsThreads) {
+    double s = 0., s2 = 0.;
+    for (unsigned b0 = 0; b0 < gridDim.x; b0 += 16) {
+      double v[16], v2[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const bool in = b0 + j < gridDim.x;
+        v[j] = in ? __ldcg(partial + static_cast<size_t>(b0 + j) * 2 * channels + c) : 0.;
+        v2[j] = in ? __ldcg(partial + static_cast<size_t>(b0 + j) * 2 * channels + channels + c) : 0.;
+      }
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        s += v[j];
+        s2 += v2[j];
+      }
+    }
+    const double off = s / static_cast<double>(pixels);
+    const float mean = static_cast<float>(static_cast<double>(x[c]) + off);
+    const float var = static_cast<float>(fmax(s2 / static_cast<double>(pixels) - off * off, 0.));
+    const float inv_std = 1.f / sqrtf(var + eps);
+    const float ts = then_scale ? then_scale[c] : 1.f;
+    scale[c] = inv_std * ts;
+    shift[c] = fmaf(-mean * inv_std, ts, then_shift ? then_shift[c] : 0.f);
+  }
+  if (threadIdx.x == 0) *arrived = 0u;
+}
+
+// [n][grid_h][grid_w][stride_h][stride_w][c] -> [n][out_h][out_w][c], positions beyond the output dropped.
+__global__ void depth_to_space_kernel(const float* __restrict__ src, float* __restrict__ dst, int grid_h, int grid_w,
+                                      int stride_h, int stride_w, int c, int out_h, int out_w, long long pixels) {
+  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < pixels;
+       i += static_cast<long long>(gridDim.x) * blockDim.x) {
+    const int x = static_cast<int>(i % out_w);
+    const long long t = i / out_w;
+    const int y = static_cast<int>(t % out_h);
+    const long long image = t / out_h;
+    const size_t cell = (image * grid_h + y / stride_h) * grid_w + x / stride_w;
+    const float* s = src + ((cell * stride_h + y % stride_h) * stride_w + x % stride_w) * c;
+    float* d = dst + i * c;
+    for (int ch = 0; ch < c; ++ch) d[ch] = s[ch];
+  }
+}
+
 // Deconvolution as a convolution, step 1: the input's pixels spread `stride` apart over a zero
 // tensor (channels last, `c_stride` floats per pixel, zero in the pad lanes).  `src` is channels
 // last with `c` floats per pixel.  The destination was cleared beforehand.
@@ -264,6 +386,19 @@ extern "C" int mcb200_deconv_flip_weights(const mcb200_conv_shape* deconv, const
   return static_cast<int>(cudaGetLastError());
 }
 
+extern "C" int mcb200_depth_to_space(const float* src, float* dst, int n, int grid_h, int grid_w, int stride_h, int stride_w,
+                                     int c, int out_h, int out_w, void* stream) {
+  if (!src || !dst || n < 0 || c < 1 || out_h < 1 || out_w < 1 || stride_h < 1 || stride_w < 1 ||
+      static_cast<long long>(grid_h) * stride_h < out_h || static_cast<long long>(grid_w) * stride_w < out_w)
+    return -1;
+  if (n == 0) return 0;
+  const long long pixels = static_cast<long long>(n) * out_h * out_w;
+  depth_to_space_kernel<<<grid_for_items(pixels, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      src, dst, grid_h, grid_w, stride_h, stride_w, c, out_h, out_w, pixels);
+  count_launch();
+  return static_cast<int>(cudaGetLastError());
+}
+
 extern "C" int mcb200_deconv_out_shape(mcb200_conv_shape* s) {
   if (!s || s->kh < 1 || s->kw < 1 || s->stride_h < 1 || s->stride_w < 1 || s->dil_h < 1 || s->dil_w < 1) return -1;
   s->ho = s->stride_h * (s->h - 1) + s->dil_h * (s->kh - 1) + 1 - 2 * s->pad_h;
@@ -326,6 +461,27 @@ extern "C" int mcb200_channel_batch_stats(const float* x, long long count, int c
   if (count == 0) return 0;
   channel_batch_stats_kernel<<<channels, 256, 0, static_cast<cudaStream_t>(stream)>>>(x, count / channels, channels, inner,
                                                                                       eps, scale, shift);
+  count_launch();
+  return static_cast<int>(cudaGetLastError());
+}
+
+extern "C" size_t mcb200_channel_batch_stats_workspace_bytes(int channels) {
+  return 256 + static_cast<size_t>(kStatsBlocks) * 2 * channels * sizeof(double);
+}
+
+extern "C" int mcb200_channel_batch_stats_nhwc(const float* x, long long count, int channels, float eps, const float* then_scale,
+                                               const float* then_shift, void* workspace, float* scale, float* shift,
+                                               void* stream) {
+  if (!x || !scale || !shift || !workspace || channels < 4 || channels % 4 || count < 0 || count % channels) return -1;
+  if ((reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(workspace) & 15)) return -2;
+  if (count == 0) return 0;
+  const long long pixels = count / channels;
+  // Fewer blocks when a thread would not even get eight values.
+  const long long useful = (count / 4 + 8 * kStatsThreads - 1) / (8 * kStatsThreads);
+  const int blocks = static_cast<int>(useful < 1 ? 1 : useful > kStatsBlocks ? kStatsBlocks : useful);
+  channel_batch_stats_nhwc_kernel<<<blocks, kStatsThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+      x, pixels, channels, eps, then_scale, then_shift, static_cast<unsigned*>(workspace),
+      reinterpret_cast<double*>(static_cast<char*>(workspace) + 256), scale, shift);
   count_launch();
   return static_cast<int>(cudaGetLastError());
 }

@@ -87,7 +87,7 @@ struct DecodeIn {
   const float* anchors;       // [A][4]
 };
 
-__global__ void __launch_bounds__(kDecodeThreads)
+__global__ void __launch_bounds__(kDecodeThreads, 2)
 proposal_decode_kernel(DecodeIn in, mcb200_proposal_params p, Workspace ws, int turned) {
   extern __shared__ __align__(16) unsigned char decode_smem[];
   const int image = blockIdx.y;

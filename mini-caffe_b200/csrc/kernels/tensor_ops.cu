@@ -77,6 +77,30 @@ __global__ void nchw_to_nhwc4_kernel(const float* __restrict__ src, float4* __re
   }
 }
 
+// A few channels (a generated image): one thread per pixel, whose values a warp reads as one run, and
+// one coalesced write per plane.  (The 32 x 32 tiles of the general kernel are nine tenths empty
+// there: 18 us for 64 x 64 x 64 x 3.)
+constexpr int kFewChannels = 8;
+
+__global__ void nhwc_to_nchw_few_kernel(const float* __restrict__ src, float* __restrict__ dst, int c, int hw, int c_stride,
+                                        long long pixels) {
+  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < pixels;
+       i += static_cast<long long>(gridDim.x) * blockDim.x) {
+    const long long n = i / hw;
+    const int p = static_cast<int>(i - n * hw);
+    float v[kFewChannels];
+#pragma unroll
+    for (int ch = 0; ch < kFewChannels; ++ch) {
+      if (ch < c) v[ch] = src[i * c_stride + ch];
+    }
+    float* d = dst + n * c * hw + p;
+#pragma unroll
+    for (int ch = 0; ch < kFewChannels; ++ch) {
+      if (ch < c) d[ch * static_cast<size_t>(hw)] = v[ch];
+    }
+  }
+}
+
 __global__ void nhwc_to_nchw_kernel(const float* __restrict__ src, float* __restrict__ dst, int c, int hw,
                                     int c_stride) {
   __shared__ float tile[32][33];
@@ -608,6 +632,12 @@ extern "C" int mcb200_nhwc_to_nchw(const float* src, float* dst, int n, int c, i
   if (!src || !dst || n < 0 || c < 1 || h < 1 || w < 1 || c_stride < c) return -1;
   if (n == 0) return 0;
   const int hw = h * w;
+  if (c <= kFewChannels) {
+    const long long pixels = static_cast<long long>(n) * hw;
+    nhwc_to_nchw_few_kernel<<<grid_for(pixels, 256), 256, 0, as_stream(stream)>>>(src, dst, c, hw, c_stride, pixels);
+    count_launch();
+    return static_cast<int>(cudaGetLastError());
+  }
   dim3 grid((hw + 31) / 32, (c + 31) / 32, n);
   if (grid.y > 65535 || grid.z > 65535) return -2;
   nhwc_to_nchw_kernel<<<grid, dim3(32, 8), 0, as_stream(stream)>>>(src, dst, c, hw, c_stride);

@@ -93,6 +93,8 @@ class Layer {
   // Producer side: true if the layer can apply a FusedTail when it stores.
   virtual bool AcceptsFusedTail() const { return false; }
   virtual void SetFusedTail(const FusedTail& tail) {}
+  // Whether that tail may hold an Eltwise SUM partner.
+  virtual bool AcceptsFusedResidual() const { return true; }
   // Consumer side: express this layer as y = x * scale[c] + shift[c] over
   // `channels` channels of axis 1 (false: cannot be fused).  Called whenever
   // the parameters may have changed.

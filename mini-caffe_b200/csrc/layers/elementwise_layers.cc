@@ -111,13 +111,38 @@ void BatchNormLayer::Forward_gpu(const vector<Blob*>& bottom, const vector<Blob*
   CHECK_EQ(Channels(bottom[0]), channels_);
   float* scale = batch_scale_shift_.Reserve(2 * static_cast<size_t>(channels_));
   float* shift = scale + channels_;
+  const unsigned long long tv = 1 + TailVersion(tail_);
+  if (tv != tail_version_) {
+    std::vector<float> ts, tb;
+    bool has_scale = false, has_shift = false;
+    FoldTail(tail_, channels_, nullptr, &ts, &tb, &has_scale, &has_shift);
+    if (has_scale) tail_scale_.Assign(ts); else tail_scale_.Clear();
+    if (has_shift) tail_shift_.Assign(tb); else tail_shift_.Clear();
+    tail_version_ = tv;
+  }
   const bool nhwc = bottom[0]->device_is_nhwc();
   const float* x = nhwc ? bottom[0]->gpu_data_nhwc() : bottom[0]->gpu_data();
   float* y = nhwc ? top[0]->mutable_gpu_data_nhwc() : top[0]->mutable_gpu_data();
   const int inner = nhwc ? 1 : (bottom[0]->num_axes() > 2 ? bottom[0]->count(2) : 1);
-  KERNEL_CHECK(mcb200_channel_batch_stats(x, bottom[0]->count(), channels_, inner, eps_, scale, shift,
-                                          ctx.stream_ptr()));
   mcb200_epilogue ep = mcb200_epilogue();
+  FillTailEpilogue(tail_, tail_scale_, tail_shift_, kResidualNhwc, channels_, &ep);
+  if (inner == 1 && channels_ % 4 == 0) {
+    const size_t bytes = mcb200_channel_batch_stats_workspace_bytes(channels_);
+    if (!stats_workspace_) {
+      stats_workspace_.reset(new Blob(vector<int>(1, static_cast<int>(bytes / sizeof(float)))));
+      CUDA_CHECK(cudaMemsetAsync(stats_workspace_->mutable_gpu_data(), 0, sizeof(unsigned), ctx.stream()));
+    }
+    KERNEL_CHECK(mcb200_channel_batch_stats_nhwc(x, bottom[0]->count(), channels_, eps_, ep.scale, ep.shift,
+                                                 stats_workspace_->mutable_gpu_data(), scale, shift, ctx.stream_ptr()));
+  } else {
+    KERNEL_CHECK(mcb200_channel_batch_stats(x, bottom[0]->count(), channels_, inner, eps_, scale, shift, ctx.stream_ptr()));
+    if (ep.scale || ep.shift) {
+      KERNEL_CHECK(mcb200_channel_affine_act(x, y, bottom[0]->count(), channels_, inner, scale, shift, nullptr, ctx.stream_ptr()));
+      x = y;
+      scale = const_cast<float*>(ep.scale);
+      shift = const_cast<float*>(ep.shift);
+    }
+  }
   KERNEL_CHECK(mcb200_channel_affine_act(x, y, bottom[0]->count(), channels_, inner, scale, shift, &ep,
                                          ctx.stream_ptr()));
 }

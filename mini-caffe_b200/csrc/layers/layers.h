@@ -167,6 +167,11 @@ class BatchNormLayer : public ChannelwiseLayer {
   const char* type() const override { return "BatchNorm"; }
   int ExactNumBottomBlobs() const override { return 1; }
   bool AsChannelAffine(int channels, std::vector<double>* scale, std::vector<double>* shift) override;
+  // With the statistics of the current batch the layer is a pass of its own, which takes the Scale
+  // and ReLU behind it along.
+  bool AcceptsFusedTail() const override { return !use_global_stats_; }
+  bool AcceptsFusedResidual() const override { return false; }
+  void SetFusedTail(const FusedTail& tail) override { tail_ = tail; tail_version_ = 0; }
  protected:
   void Forward_gpu(const vector<Blob*>& bottom, const vector<Blob*>& top) override;
  private:
@@ -174,6 +179,10 @@ class BatchNormLayer : public ChannelwiseLayer {
   float eps_ = 1e-5f;
   bool use_global_stats_ = true;   // false: normalise with the statistics of the current batch
   DeviceScratch batch_scale_shift_;
+  FusedTail tail_;
+  unsigned long long tail_version_ = 0;
+  DeviceArray tail_scale_, tail_shift_;
+  std::unique_ptr<Blob> stats_workspace_;
 };
 
 class ScaleLayer : public ChannelwiseLayer {
@@ -474,13 +483,17 @@ class DeconvolutionLayer : public Layer {
   void Forward_gpu(const vector<Blob*>& bottom, const vector<Blob*>& top) override;
   mcb200_conv_shape shape_ = mcb200_conv_shape();
   bool bias_term_ = false;
-  // The layer runs as a convolution on the tensor cores: reversed filter, input spread `stride`
-  // apart over zeros (see mcb200_deconv_as_conv_shape); the direct kernel takes what is left
-  // (more padding than the filter reaches).
+  // The layer runs as a convolution on the tensor cores: phase by phase
+  // (mcb200_deconv_tc_plan), all phases side by side (mcb200_deconv_as_window_conv), or with a reversed
+  // filter over the input spread `stride` apart over zeros (mcb200_deconv_as_conv_shape); the direct kernel takes what is left (more padding than the filter
+  // reaches).
+  enum Form { kPhases, kWindow, kSpread };
+  Form form_ = kSpread;
   unsigned long long weight_version_ = 0;
-  DeviceScratch flipped_weights_, packed_weights_, spread_input_;
+  DeviceScratch flipped_weights_, packed_weights_, scratch_;
+  DeviceArray window_bias_;   // the bias once per phase
   struct PlanSlot {
-    mcb200_conv_plan plan;
+    mcb200_deconv_plan plan;   // phase by phase; its `conv` alone serves the spread form
     const float* in = nullptr;
     const float* weights = nullptr;
     mcb200_conv_shape shape = mcb200_conv_shape();

@@ -259,7 +259,7 @@ void Net::PlaceMemory() {
             tail.affine.push_back(next);
           } else if (bottom_id_vecs_[k].size() == 1 && next->AsActivation(&act)) {
             tail.activation = next;
-          } else if (!tail.residual && bottom_id_vecs_[k].size() == 2 && !in_place && next->AsWeightedSum(&coeffs) &&
+          } else if (producer->AcceptsFusedResidual() && !tail.residual && bottom_id_vecs_[k].size() == 2 && !in_place && next->AsWeightedSum(&coeffs) &&
                      bottom_id_vecs_[k][0] != bottom_id_vecs_[k][1]) {
             const int self_slot = bottom_id_vecs_[k][0] == cur ? 0 : 1;
             const int other = bottom_id_vecs_[k][1 - self_slot];

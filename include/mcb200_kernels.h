@@ -383,6 +383,14 @@ int mcb200_detout_max_rows_per_image(const mcb200_detout_params* p);
  * top_k (or num_priors when top_k is -1) may be at most 4096.                */
 int mcb200_detout_forward(const mcb200_detout_params* p, int batch, const float* loc, const float* conf,
                           const float* prior, void* workspace, float* out, int* total, void* stream);
+/* The same in parts, for callers whose input arrives a few images at a time: _part for images
+ * [first_image, first_image + images) of a batch (loc and conf are those images' own), _finish once all
+ * parts are queued on the stream.  `workspace` is sized for the whole batch.  out and total may be
+ * pinned host memory that the device can address.                                                */
+int mcb200_detout_part(const mcb200_detout_params* p, int batch, int first_image, int images, const float* loc, const float* conf,
+                       const float* prior, void* workspace, void* stream);
+int mcb200_detout_finish(const mcb200_detout_params* p, int batch, void* workspace, float* out, int* total, void* stream);
+
 
 /* ROIPooling: max over an adaptive pooled_h x pooled_w grid laid on each region
  * of interest (src/layers/roi_pooling_layer.cpp:37-109).  data_nchw is

@@ -1,8 +1,8 @@
 // SSD DetectionOutput on the device:
 //   A. per (image, class) block: collect priors whose class score passes the
-//      confidence threshold, take the top_k best (radix select + bitonic sort in
+//      confidence threshold, take the top_k best (histogram + bitonic sort in
 //      shared memory, ties by prior index like std::stable_sort), decode their
-//      boxes, greedy NMS (overlap bit matrix by the whole block, walk by one warp)
+//      boxes, greedy NMS (overlap bit matrix, then the kept set iterated, by the whole block)
 //   B. per image block: if more than keep_top_k detections survive, keep the
 //      keep_top_k best over all classes; lay the rows out label-ascending
 //   C. per image block: prefix sum of the per-image counts, compact the rows
@@ -162,72 +162,211 @@ __device__ __forceinline__ float jaccard(const Box& a, const Box& b) {
   return 0.f;
 }
 
+// ---------------------------------------------------------------- the k best of many keys
+
+constexpr int kBins = 2048;
+constexpr int kEdge = 1024;
+
+// Shared memory of one selection.
+struct SelectShared {
+  int bins[kBins];
+  unsigned long long edge[kEdge];   // the keys of the bin that holds the k-th
+  int warp_sum[32];
+  uint32_t low, high;               // range of the keys' upper halves
+  int bin, before, edges;
+  unsigned long long threshold;
+  int hist[256];                    // the radix walk's
+  unsigned long long bcast[2];
+};
+
+// A threshold T such that exactly k of the keys are <= T (k smaller than their number).  The upper
+// halves, which `each` hands to its callback one by one, are spread over kBins equal steps of their own
+// range [low, high] (scores of one layer share sign and most exponent bits: bins cut from the top bits
+// would hold thousands each); the keys of the bin that the k-th falls into are ranked by counting.
+// Only when that bin holds more than kEdge (ties) the radix walk over `fetch(0 .. n - 1)` decides.
+// Whole block; sh.low / sh.high are set by the caller.
+template <typename Each, typename Fetch>
+__device__ unsigned long long select_threshold(SelectShared& sh, const Each& each, const Fetch& fetch, int n, int k) {
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, threads = blockDim.x;
+  const uint32_t low = sh.low, range = sh.high - sh.low;
+  const int shift = max(0, 32 - __clz(range) - 11);       // range >> shift < kBins
+  for (int i = t; i < kBins; i += threads) sh.bins[i] = 0;
+  if (t == 0) sh.edges = 0;
+  __syncthreads();
+  each([&](unsigned long long key) { atomicAdd(&sh.bins[(static_cast<uint32_t>(key >> 32) - low) >> shift], 1); });
+  __syncthreads();
+  // First bin whose running count reaches k.
+  const int per = kBins / threads;
+  int own = 0;
+  for (int j = 0; j < per; ++j) own += sh.bins[t * per + j];
+  int incl = own;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  if (lane == 31) sh.warp_sum[warp] = incl;
+  __syncthreads();
+  int base = lane < warp ? sh.warp_sum[lane] : 0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) base += __shfl_xor_sync(0xffffffffu, base, o);
+  int before = base + incl - own;
+  if (before < k && before + own >= k) {
+    int bin = t * per;
+    while (before + sh.bins[bin] < k) before += sh.bins[bin++];
+    sh.bin = bin;
+    sh.before = before;
+  }
+  __syncthreads();
+  const uint32_t bin = sh.bin;
+  const int wanted = k - sh.before;
+  if (sh.bins[bin] > kEdge) return block_kth_smallest(fetch, n, k, sh.hist, sh.bcast);
+  each([&](unsigned long long key) {
+    if (((static_cast<uint32_t>(key >> 32) - low) >> shift) == bin) sh.edge[atomicAdd(&sh.edges, 1)] = key;
+  });
+  __syncthreads();
+  const int edges = sh.edges;
+  for (int i = t; i < edges; i += threads) {
+    const unsigned long long key = sh.edge[i];
+    int rank = 1;
+    for (int q = 0; q < edges; ++q) rank += sh.edge[q] < key ? 1 : 0;
+    if (rank == wanted) sh.threshold = key;
+  }
+  __syncthreads();
+  return sh.threshold;
+}
+
+// Range of the upper halves over the block, into sh.low / sh.high (a barrier follows before use).
+__device__ __forceinline__ void note_range(SelectShared& sh, uint32_t low, uint32_t high) {
+  low = __reduce_min_sync(0xffffffffu, low);
+  high = __reduce_max_sync(0xffffffffu, high);
+  if ((threadIdx.x & 31) == 0) {
+    atomicMin(&sh.low, low);
+    atomicMax(&sh.high, high);
+  }
+}
+
 // ---------------------------------------------------------------- A. per (image, class)
 
-// Shared memory: candidate keys [num_priors], selected keys [padded], boxes
-// [padded], kept list [padded].
-__global__ void __launch_bounds__(256)
+constexpr int kClassThreads = 512;
+constexpr uint32_t kNoKey = 0xFFFFFFFFu;   // the key of no score that passes a comparison (a NaN's)
+
+// Overlap > threshold without the division where a product decides (a float product of the threshold
+// widened by 2^-20 either way is off by 2^-24 of itself; in between, and for thresholds <= 0, the
+// quotient is compared).
+struct JaccardTest {
+  float threshold, below, above;
+  __device__ explicit JaccardTest(float thr)
+      : threshold(thr), below(thr > 0.f ? fmul(thr, 1.f - 0x1p-20f) : -1.f),
+        above(thr > 0.f ? fmul(thr, 1.f + 0x1p-20f) : __builtin_huge_valf()) {}
+  // 1: more than the threshold; 0: not; 2: only the quotient can tell.  Boxes that do not meet have an
+  // intersection of 0 here and pass no threshold >= 0, as in the CPU code.
+  __device__ __forceinline__ int quick(const float4& a, float size_a, const float4& b, float size_b) const {
+    const float iw = fmaxf(fsub(fminf(a.z, b.z), fmaxf(a.x, b.x)), 0.f);
+    const float ih = fmaxf(fsub(fminf(a.w, b.w), fmaxf(a.y, b.y)), 0.f);
+    const float isize = fmul(iw, ih);
+    const float uni = fsub(fadd(size_a, size_b), isize);
+    return isize < fmul(below, uni) ? 0 : (uni > 0.f && isize > fmul(above, uni)) ? 1 : 2;
+  }
+};
+
+// Shared memory: the selection's, selected keys [padded], boxes and sizes [padded], kept list [padded], then one
+// region for the priors' score keys (4 bytes each, kNoKey where the score does not pass) and, once the
+// selection is over, the overlap bits.
+struct ClassShared {
+  SelectShared select;
+  uint32_t keep[2][128];     // the walk's set, by the round's parity
+  int num_cand, num_sel, num_kept;
+};
+
+__host__ __device__ inline size_t class_region_bytes(int num_priors, int limit) {
+  const size_t keys = static_cast<size_t>(num_priors) * sizeof(uint32_t);
+  const size_t bits = limit <= 1024 ? static_cast<size_t>((limit + 31) / 32) * limit * sizeof(uint32_t) : 0;
+  return keys > bits ? keys : bits;
+}
+
+__global__ void __launch_bounds__(kClassThreads, 2)
 detout_class_kernel(const float* __restrict__ loc, const float* __restrict__ conf, const float* __restrict__ prior,
                     mcb200_detout_params p, Workspace ws, int padded, float eta) {
-  extern __shared__ unsigned long long smem_keys[];
-  unsigned long long* cand = smem_keys;
-  unsigned long long* sel = cand + p.num_priors;
-  Box* boxes = reinterpret_cast<Box*>(sel + padded);
-  int* kept = reinterpret_cast<int*>(boxes + padded);
-  __shared__ int hist[256];
-  __shared__ unsigned long long bcast[2];
-  __shared__ int num_cand, num_sel, num_kept;
+  extern __shared__ __align__(16) unsigned char class_smem[];
+  ClassShared& sh = *reinterpret_cast<ClassShared*>(class_smem);
+  unsigned long long* sel = reinterpret_cast<unsigned long long*>(class_smem + ((sizeof(ClassShared) + 15) & ~static_cast<size_t>(15)));
+  float4* corners = reinterpret_cast<float4*>(sel + padded);
+  float* sizes = reinterpret_cast<float*>(corners + padded);
+  int* kept = reinterpret_cast<int*>(sizes + padded);
+  auto box_at = [&](int i) {
+    const float4 c = corners[i];
+    return Box{c.x, c.y, c.z, c.w, sizes[i]};
+  };
+  uint32_t* region = reinterpret_cast<uint32_t*>(kept + padded);
 
   const int cls = blockIdx.x;
   const int image = blockIdx.y;
   const int limit = ws.per_class;
+  const int t = threadIdx.x, lane = t & 31;
   int* out_count = ws.class_count + static_cast<size_t>(image) * p.num_classes + cls;
   if (cls == p.background_label_id) {
-    if (threadIdx.x == 0) *out_count = 0;
+    if (t == 0) *out_count = 0;
     return;
   }
-  if (threadIdx.x == 0) {
-    num_cand = 0;
-    num_sel = 0;
-    num_kept = 0;
+  if (t == 0) {
+    sh.num_cand = 0;
+    sh.num_sel = 0;
+    sh.num_kept = 0;
+    sh.select.low = 0xFFFFFFFFu;
+    sh.select.high = 0u;
   }
+  for (int i = t; i < padded; i += kClassThreads) sel[i] = kPadKey;
   __syncthreads();
   const float* scores = conf + static_cast<size_t>(image) * p.num_priors * p.num_classes + cls;
-  // Append the passing priors, one shared-memory counter update per warp (with
-  // near-uniform scores nearly every prior passes, and 8732 single updates of
-  // one counter would serialise).  The order of the list does not matter.
-  for (int base = 0; base < p.num_priors; base += blockDim.x) {
-    const int i = base + threadIdx.x;
-    float s = 0.f;
-    bool pass = false;
-    if (i < p.num_priors) {
-      s = scores[static_cast<size_t>(i) * p.num_classes];
-      pass = s > p.confidence_threshold;
+  {
+    // The class's column of the score matrix: eight strided loads of a thread in flight.
+    int found = 0;
+    uint32_t low = 0xFFFFFFFFu, high = 0u;
+    constexpr int kFlight = 8;
+    for (int base = t; base < p.num_priors; base += kFlight * kClassThreads) {
+      float s[kFlight];
+#pragma unroll
+      for (int u = 0; u < kFlight; ++u) {
+        const int i = base + u * kClassThreads;
+        if (i < p.num_priors) s[u] = scores[static_cast<size_t>(i) * p.num_classes];
+      }
+#pragma unroll
+      for (int u = 0; u < kFlight; ++u) {
+        const int i = base + u * kClassThreads;
+        if (i >= p.num_priors) break;
+        const bool pass = s[u] > p.confidence_threshold;
+        const uint32_t key = pass ? descending_key(s[u]) : kNoKey;
+        region[i] = key;
+        if (pass) {
+          ++found;
+          low = min(low, key);
+          high = max(high, key);
+        }
+      }
     }
-    const unsigned passing = __ballot_sync(0xffffffffu, pass);
-    if (passing) {
-      const int lane = threadIdx.x & 31;
-      const int leader = __ffs(passing) - 1;
-      int first = 0;
-      if (lane == leader) first = atomicAdd(&num_cand, __popc(passing));
-      first = __shfl_sync(0xffffffffu, first, leader);
-      if (pass) cand[first + __popc(passing & ((1u << lane) - 1u))] = make_key(s, static_cast<uint32_t>(i));
-    }
+    note_range(sh.select, low, high);
+    found = __reduce_add_sync(0xffffffffu, found);
+    if (lane == 0 && found) atomicAdd(&sh.num_cand, found);
   }
   __syncthreads();
-  const int m = num_cand;
+  const int m = sh.num_cand;
   const int count = m < limit ? m : limit;
-  unsigned long long threshold = kPadKey;
-  if (m > limit) threshold = block_kth_smallest([&](int i) { return cand[i]; }, m, limit, hist, bcast);
-  for (int i = threadIdx.x; i < padded; i += blockDim.x) sel[i] = kPadKey;
-  __syncthreads();
-  for (int i = threadIdx.x; i < m; i += blockDim.x) {
-    const unsigned long long key = cand[i];
-    if (key <= threshold) {
-      const int slot = atomicAdd(&num_sel, 1);
-      if (slot < padded) sel[slot] = key;
+  auto each = [&](auto use) {
+    for (int i = t; i < p.num_priors; i += kClassThreads) {
+      const uint32_t key = region[i];
+      if (key != kNoKey) use((static_cast<unsigned long long>(key) << 32) | static_cast<uint32_t>(i));
     }
+  };
+  unsigned long long threshold = kPadKey;
+  if (m > limit) {
+    // (a prior that does not pass sorts behind every one that does)
+    auto fetch = [&](int i) { return (static_cast<unsigned long long>(region[i]) << 32) | static_cast<uint32_t>(i); };
+    threshold = select_threshold(sh.select, each, fetch, p.num_priors, limit);
   }
+  each([&](unsigned long long key) {
+    if (key <= threshold) sel[atomicAdd(&sh.num_sel, 1)] = key;
+  });
   __syncthreads();
   block_sort_keys(sel, padded);
 
@@ -235,174 +374,233 @@ detout_class_kernel(const float* __restrict__ loc, const float* __restrict__ con
   const int loc_classes = p.share_location ? 1 : p.num_classes;
   const int loc_cls = p.share_location ? 0 : cls;
   const float* var = prior + static_cast<size_t>(p.num_priors) * 4;
-  for (int i = threadIdx.x; i < count; i += blockDim.x) {
+  for (int i = t; i < count; i += kClassThreads) {
     const int pi = static_cast<int>(sel[i] & 0xFFFFFFFFull);
     const float* l = loc + ((static_cast<size_t>(image) * p.num_priors + pi) * loc_classes + loc_cls) * 4;
-    boxes[i] = decode_box(p, prior + static_cast<size_t>(pi) * 4, var + static_cast<size_t>(pi) * 4, l);
+    const Box box = decode_box(p, prior + static_cast<size_t>(pi) * 4, var + static_cast<size_t>(pi) * 4, l);
+    corners[i] = make_float4(box.xmin, box.ymin, box.xmax, box.ymax);
+    sizes[i] = box.size;
   }
   __syncthreads();
 
   // Greedy NMS: candidate i is kept iff its overlap with every box kept so far
   // is <= the threshold.  With a fixed threshold (eta == 1, the usual case) the
-  // overlaps do not depend on the walk: the whole block evaluates the lower
-  // triangle into a bit matrix (row i, bit j < i: box j would suppress box i),
-  // which takes the place of the candidate keys in shared memory, and one warp
-  // then walks the rows holding the kept set as one 32-bit word per lane.
+  // overlaps do not depend on the walk: the whole block evaluates them into a bit matrix (word w of
+  // column i, bit b: box 32 w + b < i would suppress box i), which takes the place of the score keys.
+  // The kept set is then iterated from "all": a box stays unless a box that stays suppresses it.  Bit i
+  // is final once those in front of it are, so this ends in the walk's own set, after as many rounds as
+  // the longest chain of suppressions is long.
   const int words = (count + 31) >> 5;
-  const bool fixed_threshold = !(eta < 1.f);
-  const bool use_matrix = fixed_threshold && words <= 32 &&
-                          static_cast<size_t>(count) * words * sizeof(uint32_t) <= static_cast<size_t>(p.num_priors) * 8;
-  if (use_matrix) {
-    uint32_t* suppress = reinterpret_cast<uint32_t*>(cand);
-    const float threshold_fixed = p.nms_threshold;
-    // Consecutive threads take consecutive rows of one word column: the boxes
-    // compared against are a broadcast, the row's own box a stride-5 access.
-    for (int t = threadIdx.x; t < count * words; t += blockDim.x) {
-      const int w = t / count;
-      const int i = t - w * count;
-      const int j0 = w << 5;
-      uint32_t bits = 0;
-      if (j0 < i) {
-        const Box cur = boxes[i];
-        const int jn = min(32, i - j0);
-        for (int b = 0; b < jn; ++b) {
-          if (jaccard(cur, boxes[j0 + b]) > threshold_fixed) bits |= 1u << b;
-        }
+  if (!(eta < 1.f) && words <= 32) {
+    uint32_t* suppress = region;
+    const JaccardTest overlaps(p.nms_threshold);
+    // A warp takes 32 rows x 32 columns at a time: lane = column, the rows are broadcasts.  (One thread
+    // per word over the whole square, with five scalar loads per test: 70 k cycles for 400 boxes.)
+    int column_block = 0, first_tile = 0;
+    for (int tile = t >> 5; tile < words * (words + 1) / 2; tile += kClassThreads / 32) {
+      while (tile > first_tile + column_block) first_tile += ++column_block;
+      const int w = tile - first_tile;
+      const int i = column_block * 32 + lane;
+      const float4 cur = corners[min(i, count - 1)];
+      const float cur_size = sizes[min(i, count - 1)];
+      const int rows = min(32, count - w * 32);
+      uint32_t bits = 0u, unsure = 0u;
+#pragma unroll 4
+      for (int r = 0; r < rows; ++r) {
+        const int verdict = overlaps.quick(corners[w * 32 + r], sizes[w * 32 + r], cur, cur_size);
+        bits |= static_cast<uint32_t>(verdict & 1) << r;
+        unsure |= static_cast<uint32_t>(verdict >> 1) << r;
       }
-      suppress[i * words + w] = bits;
+      if (w == column_block) {      // only boxes in front suppress
+        bits &= (1u << lane) - 1u;
+        unsure &= (1u << lane) - 1u;
+      }
+      for (; unsure; unsure &= unsure - 1) {
+        const int r = __ffs(unsure) - 1;
+        if (jaccard(box_at(w * 32 + r), box_at(min(i, count - 1))) > p.nms_threshold) bits |= 1u << r;
+      }
+      if (i < count) suppress[w * count + i] = bits;
     }
     __syncthreads();
-    if (threadIdx.x < 32) {
-      const int lane = threadIdx.x;
-      uint32_t kept_word = 0;   // lane w: boxes 32 w .. 32 w + 31 kept so far
-      int nk = 0;
-      for (int i = 0; i < count; ++i) {
-        const uint32_t hit = lane < words ? (suppress[i * words + lane] & kept_word) : 0u;
-        if (!__any_sync(0xffffffffu, hit != 0u)) {
-          if (lane == (i >> 5)) kept_word |= 1u << (i & 31);
-          if (lane == 0) kept[nk] = i;
-          ++nk;
-        }
+    // (count <= 1024: at most two groups of 32 columns per warp; `busy`: the words that hold anything)
+    uint32_t busy[2] = {0u, 0u};
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int g = (t >> 5) + u * (kClassThreads / 32), i = g * 32 + lane;
+      if (g < words && i < count) {
+        for (int w = 0; w <= g; ++w) busy[u] |= (suppress[w * count + i] != 0u ? 1u : 0u) << w;
       }
-      if (lane == 0) num_kept = nk;
+      const uint32_t all = __ballot_sync(0xffffffffu, i < count);
+      if (lane == 0 && g < words) sh.keep[0][g] = all;
     }
-  } else if (threadIdx.x < 32) {
+    __syncthreads();
+    for (int round = 0;; round ^= 1) {
+      bool changed = false;
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int g = (t >> 5) + u * (kClassThreads / 32), i = g * 32 + lane;
+        if (g >= words) break;
+        bool stays = i < count;
+        for (uint32_t left = busy[u]; left && stays; left &= left - 1) {
+          const int w = __ffs(left) - 1;
+          stays = !(suppress[w * count + i] & sh.keep[round][w]);
+        }
+        const uint32_t next = __ballot_sync(0xffffffffu, stays);
+        changed = changed || next != sh.keep[round][g];
+        if (lane == 0) sh.keep[round ^ 1][g] = next;
+      }
+      if (!__syncthreads_or(changed)) break;
+    }
+  } else if (t < 32) {
     // Adaptive threshold (eta < 1) or a very long candidate list: one warp
     // compares each candidate with the kept list, 32 kept boxes at a time.
-    const int lane = threadIdx.x;
     float adaptive = p.nms_threshold;
     int nk = 0;
+    for (int w = lane; w < 128; w += 32) sh.keep[0][w] = 0u;
+    __syncwarp();
     for (int i = 0; i < count; ++i) {
-      const Box cur = boxes[i];
+      const Box cur = box_at(i);
       bool reject = false;
       for (int base = 0; base < nk && !reject; base += 32) {
         const int j = base + lane;
-        const bool hit = j < nk && jaccard(cur, boxes[kept[j]]) > adaptive;
+        const bool hit = j < nk && jaccard(cur, box_at(kept[j])) > adaptive;
         reject = __any_sync(0xffffffffu, hit);
       }
       if (!reject) {
-        if (lane == 0) kept[nk] = i;
+        if (lane == 0) {
+          kept[nk] = i;
+          sh.keep[0][i >> 5] |= 1u << (i & 31);
+        }
         ++nk;
         __syncwarp();
         if (eta < 1.f && adaptive > 0.5f) adaptive = fmul(adaptive, eta);
       }
     }
-    if (lane == 0) num_kept = nk;
   }
   __syncthreads();
-  const int nk = num_kept;
   Entry* out = ws.entries + (static_cast<size_t>(image) * p.num_classes + cls) * limit;
-  for (int r = threadIdx.x; r < nk; r += blockDim.x) {
-    const int i = kept[r];
+  for (int i = t; i < count; i += kClassThreads) {
+    const uint32_t word = sh.keep[0][i >> 5];
+    if (!((word >> (i & 31)) & 1u)) continue;
+    int r = __popc(word & ((1u << (i & 31)) - 1u));
+    for (int w = 0; w < (i >> 5); ++w) r += __popc(sh.keep[0][w]);
     const int pi = static_cast<int>(sel[i] & 0xFFFFFFFFull);
     Entry e;
     e.score = scores[static_cast<size_t>(pi) * p.num_classes];
-    e.xmin = boxes[i].xmin;
-    e.ymin = boxes[i].ymin;
-    e.xmax = boxes[i].xmax;
-    e.ymax = boxes[i].ymax;
+    const float4 corner = corners[i];
+    e.xmin = corner.x;
+    e.ymin = corner.y;
+    e.xmax = corner.z;
+    e.ymax = corner.w;
     out[r] = e;
   }
-  if (threadIdx.x == 0) *out_count = nk;
+  if (t == 0) {
+    int total = 0;
+    for (int w = 0; w < words; ++w) total += __popc(sh.keep[0][w]);
+    *out_count = total;
+  }
 }
 
 // ---------------------------------------------------------------- B. per image
 
-// `staged`: the keys of all of the image's detections fit into dynamic shared
-// memory and are gathered there once (all of a thread's loads in flight
-// together); the passes of the radix select then read shared memory.
-__global__ void __launch_bounds__(256)
-detout_image_kernel(mcb200_detout_params p, Workspace ws, int staged) {
-  extern __shared__ unsigned long long image_keys[];
-  __shared__ int hist[256];
-  __shared__ unsigned long long bcast[2];
-  __shared__ int offsets[1025];   // first row of each class among the image's rows
-  __shared__ int selected[1024];  // rows kept per class
+constexpr int kImageThreads = 1024;
+
+struct ImageShared {
+  SelectShared select;
+  int offsets[1025];   // first row of each class among the image's rows
+  int selected[1024];  // rows kept per class
+  int total;
+};
+
+// Running sums of values[0 .. n) (n <= 1024) into sums[0 .. n], by the whole block of 1024 threads.
+__device__ void block_prefix_sum(SelectShared& sh, const int* values, int n, int* sums) {
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int own = t < n ? values[t] : 0;
+  int incl = own;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  if (lane == 31) sh.warp_sum[warp] = incl;
+  __syncthreads();
+  int base = lane < warp ? sh.warp_sum[lane] : 0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) base += __shfl_xor_sync(0xffffffffu, base, o);
+  if (t < n) sums[t] = base + incl - own;
+  if (t == n - 1) sums[n] = base + incl;
+  __syncthreads();
+}
+
+// `first_image`: the number of the grid's first image in the batch.
+__global__ void __launch_bounds__(kImageThreads, 1)
+detout_image_kernel(mcb200_detout_params p, Workspace ws, int first_image) {
+  extern __shared__ __align__(16) unsigned char image_smem[];
+  ImageShared& sh = *reinterpret_cast<ImageShared*>(image_smem);
   const int image = blockIdx.x;
+  const int t = threadIdx.x;
   const int classes = p.num_classes;
   const int limit = ws.per_class;
   const int* counts = ws.class_count + static_cast<size_t>(image) * classes;
   const Entry* entries = ws.entries + static_cast<size_t>(image) * classes * limit;
 
-  if (threadIdx.x == 0) {
-    int total = 0;
-    for (int c = 0; c < classes; ++c) {
-      offsets[c] = total;
-      total += counts[c];
-    }
-    offsets[classes] = total;
+  if (t == 0) {
+    sh.select.low = 0xFFFFFFFFu;
+    sh.select.high = 0u;
   }
+  if (t < classes) sh.selected[t] = counts[t];
   __syncthreads();
-  const int total = offsets[classes];
-  // Flat index e over (class, rank); key = (descending score, class * limit + rank).
-  auto load_key = [&](int e) {
-    int c = 0;
-    while (offsets[c + 1] <= e) ++c;
-    const int j = e - offsets[c];
-    return make_key(entries[static_cast<size_t>(c) * limit + j].score, static_cast<uint32_t>(c * limit + j));
-  };
-  const bool select = p.keep_top_k > -1 && total > p.keep_top_k;
-  if (staged && select) {
-    for (int e = threadIdx.x; e < total; e += blockDim.x) image_keys[e] = load_key(e);
+  block_prefix_sum(sh.select, sh.selected, classes, sh.offsets);
+  const int total = sh.offsets[classes];
+  if (p.keep_top_k > -1 && total > p.keep_top_k) {
+    // The keep_top_k best over all classes.  Key = (descending score, class * limit + rank); within a
+    // class the entries are in descending score order, so the kept ones are a prefix of it.
+    auto key_of = [&](int cell) { return make_key(entries[cell].score, static_cast<uint32_t>(cell)); };
+    auto each = [&](auto use) {
+      for (int cell = t; cell < classes * limit; cell += kImageThreads) {
+        const int c = cell / limit;
+        if (cell - c * limit < sh.offsets[c + 1] - sh.offsets[c]) use(key_of(cell));
+      }
+    };
+    uint32_t low = 0xFFFFFFFFu, high = 0u;
+    each([&](unsigned long long key) {
+      low = min(low, static_cast<uint32_t>(key >> 32));
+      high = max(high, static_cast<uint32_t>(key >> 32));
+    });
+    note_range(sh.select, low, high);
     __syncthreads();
-  }
-  auto fetch = [&](int e) { return staged ? image_keys[e] : load_key(e); };
-  unsigned long long threshold = kPadKey;
-  if (select) threshold = block_kth_smallest(fetch, total, p.keep_top_k, hist, bcast);
-  // Within a class the entries are in descending score order, so the kept ones
-  // are a prefix of it; its length is the number of the class's keys <= threshold.
-  for (int c = threadIdx.x; c < classes; c += blockDim.x) selected[c] = 0;
-  __syncthreads();
-  for (int e = threadIdx.x; e < total; e += blockDim.x) {
-    int c = 0;
-    while (offsets[c + 1] <= e) ++c;
-    // Without a selection every detection is kept (the threshold is the largest key).
-    if (!select || fetch(e) <= threshold) atomicAdd(&selected[c], 1);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int run = 0;
-    for (int c = 0; c < classes; ++c) {
-      offsets[c] = run;
-      run += selected[c];
+    auto fetch = [&](int e) {   // e-th entry over the classes
+      int c = 0;
+      while (sh.offsets[c + 1] <= e) ++c;
+      return key_of(c * limit + e - sh.offsets[c]);
+    };
+    unsigned long long threshold = 0ull;
+    if (p.keep_top_k > 0) threshold = select_threshold(sh.select, each, fetch, total, p.keep_top_k);
+    __syncthreads();
+    if (t < classes) sh.selected[t] = 0;
+    __syncthreads();
+    if (p.keep_top_k > 0) {
+      each([&](unsigned long long key) {
+        if (key <= threshold) atomicAdd(&sh.selected[static_cast<uint32_t>(key) / limit], 1);
+      });
     }
-    offsets[classes] = run;
-    ws.image_count[image] = run;
+    __syncthreads();
+    block_prefix_sum(sh.select, sh.selected, classes, sh.offsets);
   }
-  __syncthreads();
+  if (t == 0) ws.image_count[image] = sh.offsets[classes];
   float* rows = ws.rows + static_cast<size_t>(image) * ws.max_rows * 7;
-  for (int c = 0; c < classes; ++c) {
-    for (int j = threadIdx.x; j < selected[c]; j += blockDim.x) {
-      const Entry e = entries[static_cast<size_t>(c) * limit + j];
-      float* r = rows + static_cast<size_t>(offsets[c] + j) * 7;
-      r[0] = static_cast<float>(image);
-      r[1] = static_cast<float>(c);
-      r[2] = e.score;
-      r[3] = e.xmin;
-      r[4] = e.ymin;
-      r[5] = e.xmax;
-      r[6] = e.ymax;
-    }
+  for (int cell = t; cell < classes * limit; cell += kImageThreads) {
+    const int c = cell / limit, j = cell - c * limit;
+    if (j >= sh.selected[c]) continue;
+    const Entry e = entries[cell];
+    float* r = rows + static_cast<size_t>(sh.offsets[c] + j) * 7;
+    r[0] = static_cast<float>(first_image + image);
+    r[1] = static_cast<float>(c);
+    r[2] = e.score;
+    r[3] = e.xmin;
+    r[4] = e.ymin;
+    r[5] = e.xmax;
+    r[6] = e.ymax;
   }
 }
 
@@ -450,7 +648,8 @@ int validate(const mcb200_detout_params* p, int batch) {
 }
 
 size_t class_kernel_smem(const mcb200_detout_params& p, int padded) {
-  return static_cast<size_t>(p.num_priors) * 8 + static_cast<size_t>(padded) * (8 + sizeof(Box) + sizeof(int));
+  return ((sizeof(ClassShared) + 15) & ~static_cast<size_t>(15)) + static_cast<size_t>(padded) * (8 + sizeof(float4) + sizeof(float) + sizeof(int)) +
+         class_region_bytes(p.num_priors, per_class_limit(p));
 }
 
 }  // namespace
@@ -469,53 +668,62 @@ extern "C" int mcb200_detout_max_rows_per_image(const mcb200_detout_params* p) {
   return rows > 1 ? rows : 1;
 }
 
-extern "C" int mcb200_detout_forward(const mcb200_detout_params* p, int batch, const float* loc, const float* conf,
-                                     const float* prior, void* workspace, float* out, int* total, void* stream) {
+// Opts a kernel into the shared memory it needs, once per device and size.
+static cudaError_t allow_shared(const void* kernel, size_t bytes, size_t* configured) {
+  static std::mutex mu;   // nets on several host threads may make their first call together
+  std::lock_guard<std::mutex> lock(mu);
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64 || configured[dev] >= bytes) return cudaSuccess;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+  if (e == cudaSuccess) configured[dev] = bytes;
+  return e;
+}
+
+extern "C" int mcb200_detout_part(const mcb200_detout_params* p, int batch, int first_image, int images, const float* loc,
+                                  const float* conf, const float* prior, void* workspace, void* stream) {
   const int rc = validate(p, batch);
   if (rc != 0) return rc;
-  if (!loc || !conf || !prior || !workspace || !out || !total) return -5;
+  if (!loc || !conf || !prior || !workspace) return -5;
   if (reinterpret_cast<uintptr_t>(workspace) & 255) return -6;
+  if (first_image < 0 || images < 1 || first_image + images > batch) return -9;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   Workspace ws;
   carve(*p, batch, static_cast<char*>(workspace), &ws);
+  ws.entries += static_cast<size_t>(first_image) * p->num_classes * ws.per_class;
+  ws.class_count += static_cast<size_t>(first_image) * p->num_classes;
+  ws.rows += static_cast<size_t>(first_image) * ws.max_rows * 7;
+  ws.image_count += first_image;
   const int padded = det::next_pow2(ws.per_class);
   const size_t smem = class_kernel_smem(*p, padded);
-  if (smem > 200 * 1024) return -7;
-  {
-    static size_t configured[64] = {0};
-    static std::mutex configure_mu;   // nets on several host threads may make their first call together
-    std::lock_guard<std::mutex> lock(configure_mu);
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev >= 0 && dev < 64 && configured[dev] < smem) {
-      cudaError_t e = cudaFuncSetAttribute(detout_class_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           static_cast<int>(smem));
-      if (e != cudaSuccess) return static_cast<int>(e);
-      configured[dev] = smem;
-    }
-  }
-  detout_class_kernel<<<dim3(p->num_classes, batch), 256, smem, st>>>(loc, conf, prior, *p, ws, padded, p->eta);
+  if (smem > 220 * 1024) return -7;
+  static size_t class_configured[64], image_configured[64];
+  cudaError_t e = allow_shared(reinterpret_cast<const void*>(detout_class_kernel), smem, class_configured);
+  if (e != cudaSuccess) return static_cast<int>(e);
+  e = allow_shared(reinterpret_cast<const void*>(detout_image_kernel), sizeof(ImageShared), image_configured);
+  if (e != cudaSuccess) return static_cast<int>(e);
+  detout_class_kernel<<<dim3(p->num_classes, images), kClassThreads, smem, st>>>(loc, conf, prior, *p, ws, padded, p->eta);
   count_launch();
-  {
-    // Keys of one image: at most (classes x per-class limit) of 8 bytes.
-    const size_t key_bytes = static_cast<size_t>(p->num_classes) * ws.per_class * 8;
-    const size_t kImageSharedLimit = 200 * 1024;
-    const int staged = key_bytes <= kImageSharedLimit ? 1 : 0;
-    static size_t configured_image[64] = {0};
-    static std::mutex configure_mu;
-    std::lock_guard<std::mutex> lock(configure_mu);
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (staged && dev >= 0 && dev < 64 && configured_image[dev] < key_bytes) {
-      cudaError_t e = cudaFuncSetAttribute(detout_image_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           static_cast<int>(kImageSharedLimit));
-      if (e != cudaSuccess) return static_cast<int>(e);
-      configured_image[dev] = kImageSharedLimit;
-    }
-    detout_image_kernel<<<batch, 256, staged ? key_bytes : 0, st>>>(*p, ws, staged);
-  }
-  count_launch();
-  detout_compact_kernel<<<batch, 256, 0, st>>>(ws, batch, out, total);
+  detout_image_kernel<<<images, kImageThreads, sizeof(ImageShared), st>>>(*p, ws, first_image);
   count_launch();
   return static_cast<int>(cudaGetLastError());
+}
+
+extern "C" int mcb200_detout_finish(const mcb200_detout_params* p, int batch, void* workspace, float* out, int* total,
+                                    void* stream) {
+  const int rc = validate(p, batch);
+  if (rc != 0) return rc;
+  if (!workspace || !out || !total) return -5;
+  Workspace ws;
+  carve(*p, batch, static_cast<char*>(workspace), &ws);
+  detout_compact_kernel<<<batch, 256, 0, static_cast<cudaStream_t>(stream)>>>(ws, batch, out, total);
+  count_launch();
+  return static_cast<int>(cudaGetLastError());
+}
+
+extern "C" int mcb200_detout_forward(const mcb200_detout_params* p, int batch, const float* loc, const float* conf,
+                                     const float* prior, void* workspace, float* out, int* total, void* stream) {
+  if (!out || !total) return p ? -5 : -1;
+  const int rc = mcb200_detout_part(p, batch, 0, batch, loc, conf, prior, workspace, stream);
+  return rc != 0 ? rc : mcb200_detout_finish(p, batch, workspace, out, total, stream);
 }

@@ -457,7 +457,11 @@ class DetectionOutputLayer : public Layer {
   int ExactNumTopBlobs() const override { return 1; }
  protected:
   void Forward_gpu(const vector<Blob*>& bottom, const vector<Blob*>& top) override;
+  void SetTopsEndOnHost(bool on_host) override { tops_end_on_host_ = on_host; }
   mcb200_detout_params params_ = mcb200_detout_params();
+  bool tops_end_on_host_ = false;
+  HostInput host_loc_, host_conf_;
+  DeviceScratch input_copy_;
   std::unique_ptr<Blob> workspace_;
   std::unique_ptr<BlobInt> total_;
 };

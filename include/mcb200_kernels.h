@@ -111,6 +111,14 @@ int mcb200_conv_tc_plan(const mcb200_conv_shape* s, const float* in, const float
 int mcb200_conv_tc_launch(mcb200_conv_plan* plan, float* out, int out_ld,
                           const mcb200_epilogue* ep, int* status, void* stream);
 
+/* The same for fp32 and bfloat16 plans, with flags.  MCB200_CONV_CONSTANTS_SETTLED: the packed weights
+ * and the epilogue's per-channel arrays were complete before the previous kernel of the stream was
+ * launched, so the kernel may fetch them while that one still runs.  Do not set it on the launch
+ * that follows a change of any of them.                                                         */
+#define MCB200_CONV_CONSTANTS_SETTLED 1
+int mcb200_conv_tc_launch_flags(mcb200_conv_plan* plan, void* out, int out_is_bf16, int out_ld,
+                                const mcb200_epilogue* ep, int flags, int* status, void* stream);
+
 /* Every wait of the convolution kernel on a hardware barrier is bounded: after `cycles` SM clock
  * cycles (default 2e9, about a second) the CTA raises an abort flag, its roles leave their loops,
  * copies in flight get a bounded grace period, tensor memory is freed and *status is set to 1;
@@ -454,8 +462,8 @@ typedef struct mcb200_deconv_plan {
 size_t mcb200_deconv_tc_packed_weight_count(const mcb200_conv_shape* deconv);
 int mcb200_deconv_tc_pack_weights(const mcb200_conv_shape* deconv, const float* w_iohw, float* packed, void* stream);
 int mcb200_deconv_tc_plan(const mcb200_conv_shape* deconv, const float* in, const float* packed_w, mcb200_deconv_plan* plan);
-int mcb200_deconv_tc_launch(mcb200_deconv_plan* plan, float* out, int out_ld, const mcb200_epilogue* ep, int* status,
-                            void* stream);
+int mcb200_deconv_tc_launch(mcb200_deconv_plan* plan, float* out, int out_ld, const mcb200_epilogue* ep, int flags,
+                            int* status, void* stream);
 
 /* The same layer with all phases as output channels (phase-major) of one convolution over the union
  * of their windows: more zeros to multiply, but one N tile for layers whose phases together have

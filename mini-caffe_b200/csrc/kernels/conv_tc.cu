@@ -120,6 +120,8 @@ struct ConvTcArgs {
   int resident_b_bytes;          // row mode: all filter rows' weight tiles stay in shared memory (bytes; 0 = streamed
                                  // with the activations).  Every M tile of such a layer multiplies the same
                                  // weights, and a third of what its ring pulled out of L2 was this one image.
+  int constants_settled;         // weights and per-column constants were complete before the previous launch
+                                 // began: they are fetched while that launch still runs
   int drop_last_weight_load;     // test hook: the weight producer leaves out its last k-iteration (see
                                  // mcb200_conv_test_drop_weight_load): the waits on that stage run out
 };
@@ -332,10 +334,15 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   // makes the first and only allocation of its SM, which starts at column 0;
   // anything else is refused rather than computed wrongly.
   // Up to here the CTA has only set itself up, which may overlap the tail of
-  // the previous launch of the stream; from here on it touches tensors.
+  // the previous launch of the stream; from here on it touches tensors.  What the previous launch
+  // cannot have written, the weights and the per-column constants of a layer that has run before, need
+  // not wait for its end: the weight producer fills the ring and the epilogue warps their first table
+  // while the activations are still being computed.  (At batch 1 a layer is a few microseconds of
+  // latency, one of which was the weights' first trip out of DRAM and 0.4 the table's.)
   MCB200_TRACE_CTA(1);
   grid_launch_dependents();
-  grid_dependency_wait();
+  const bool early = args.constants_settled != 0;
+  if (!early || (warp != kWarpLoadB && warp < kFirstEpilogueWarp)) grid_dependency_wait();
   MCB200_TRACE_CTA(2);
   const bool usable = !kPair || tmem_base == 0u;
   if (!usable && threadIdx.x == 0) abort_flag = 1;
@@ -783,6 +790,27 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       }
     };
     const bool staged = args.tma_epilogue != 0;
+    int table_n0[2] = {-1, -1};          // first column the per-column tables were filled for
+    uint32_t table_fills[2] = {0u, 0u};
+    auto fill_table = [&](int ab, int n0) {
+      for (int c = epi_tid; c < BN; c += kEpilogueWarps * 32) {
+        const int cc = n0 + c;
+        const bool in = cc < args.cout;
+        col_scale[ab][c] = (in && ep.scale) ? __ldg(ep.scale + cc) : 1.f;
+        col_shift[ab][c] = (in && ep.shift) ? __ldg(ep.shift + cc) : 0.f;
+        col_slope[ab][c] = ep.act == 2 ? ((in && ep.prelu) ? __ldg(ep.prelu + (ep.prelu_shared ? 0 : cc)) : 0.f) : ep.slope;
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&col_bar[ab]);
+      table_n0[ab] = n0;
+    };
+    // The first tile's table, before anything else is waited for.
+    if (worker < num_tiles) {
+      int n0 = (worker % n_tiles) * BN;
+      if (kMode == kModePhase) n0 = (worker % n_tiles % args.phase_tiles) * BN;
+      fill_table(0, n0);
+    }
+    if (early) grid_dependency_wait();
     // Residual sub-tiles are requested `res_depth` chunks ahead: a request takes
     // a DRAM round trip (one to two microseconds), several times the time a warp
     // needs per chunk.  Requesting chunk g + depth reuses the slot of chunk
@@ -799,8 +827,6 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     bool alive = true;
     MCB200_TRACE_DECL;
     MCB200_TRACE_CHUNK_DECL;
-    int table_n0[2] = {-1, -1};          // first column the per-column tables were filled for
-    uint32_t table_fills[2] = {0u, 0u};
     for (int tile = worker; tile < num_tiles && alive; tile += workers, ++local) {
       const int ab = local & 1;
       const uint32_t use = static_cast<uint32_t>(local >> 1) & 1u;
@@ -850,22 +876,14 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       float* t_scale = col_scale[ab];
       float* t_shift = col_shift[ab];
       float* t_slope = col_slope[ab];
-      if (table_n0[ab] != n0) {
-        for (int c = epi_tid; c < BN; c += kEpilogueWarps * 32) {
-          const int cc = n0 + c;
-          const bool in = cc < args.cout;
-          t_scale[c] = (in && ep.scale) ? __ldg(ep.scale + cc) : 1.f;
-          t_shift[c] = (in && ep.shift) ? __ldg(ep.shift + cc) : 0.f;
-          t_slope[c] = ep.act == 2 ? ((in && ep.prelu) ? __ldg(ep.prelu + (ep.prelu_shared ? 0 : cc)) : 0.f) : ep.slope;
-        }
+      const bool refill = table_n0[ab] != n0;
+      if (refill) fill_table(ab, n0);
+      if (refill || local == 0) {
         // Rendezvous of the epilogue warps on the table (an mbarrier rather than a
         // named barrier, so that the wait is bounded like every other one).
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&col_bar[ab]);
         alive = __all_sync(0xffffffffu, mbar_wait_bounded(&col_bar[ab], table_fills[ab] & 1u, abort, wait_limit));
         if (!alive) break;
         ++table_fills[ab];
-        table_n0[ab] = n0;
       }
       const uint32_t tmem_acc = tmem_base + static_cast<uint32_t>(ab * BN) + (static_cast<uint32_t>(quad * 32) << 16);
 #pragma unroll 1
@@ -1826,7 +1844,7 @@ int plan_core(const mcb200_conv_shape* s, const void* in, const void* packed_w, 
 }
 
 int launch_core(mcb200_conv_plan* plan, void* out, bool out_half, int out_ld, const mcb200_epilogue* ep, int* status,
-                void* stream, const mcb200_deconv_plan* phases = nullptr);
+                void* stream, int flags = 0, const mcb200_deconv_plan* phases = nullptr);
 
 }  // namespace
 
@@ -1846,6 +1864,11 @@ extern "C" int mcb200_conv_tc_launch(mcb200_conv_plan* plan, float* out, int out
   return launch_core(plan, out, false, out_ld, ep, status, stream);
 }
 
+extern "C" int mcb200_conv_tc_launch_flags(mcb200_conv_plan* plan, void* out, int out_is_bf16, int out_ld,
+                                           const mcb200_epilogue* ep, int flags, int* status, void* stream) {
+  return launch_core(plan, out, out_is_bf16 != 0, out_ld, ep, status, stream, flags);
+}
+
 extern "C" int mcb200_conv_tc_launch_bf16(mcb200_conv_plan* plan, void* out, int out_is_bf16, int out_ld,
                                           const mcb200_epilogue* ep, int* status, void* stream) {
   return launch_core(plan, out, out_is_bf16 != 0, out_ld, ep, status, stream);
@@ -1854,7 +1877,7 @@ extern "C" int mcb200_conv_tc_launch_bf16(mcb200_conv_plan* plan, void* out, int
 namespace {
 
 int launch_core(mcb200_conv_plan* plan, void* out, bool out_half, int out_ld, const mcb200_epilogue* ep, int* status,
-                void* stream, const mcb200_deconv_plan* phases) {
+                void* stream, int flags, const mcb200_deconv_plan* phases) {
   if (!plan || !out || out_ld < plan->shape.cout) return -1;
   const bool half = plan->operand_bf16 != 0;
   ConvTcArgs a;
@@ -1890,6 +1913,7 @@ int launch_core(mcb200_conv_plan* plan, void* out, bool out_half, int out_ld, co
   a.vec_store = a.tma_epilogue;
   a.l2_prefetch = a.halo_staged = 0;
   a.wait_limit = g_wait_limit_cycles;
+  a.constants_settled = (flags & MCB200_CONV_CONSTANTS_SETTLED) ? 1 : 0;
   a.drop_last_weight_load = t_drop_weight_load;
   t_drop_weight_load = 0;
   a.group_cout = plan->shape.group > 1 ? plan->shape.cout / plan->shape.group : 0;
@@ -2248,10 +2272,10 @@ extern "C" int mcb200_deconv_tc_plan(const mcb200_conv_shape* deconv, const floa
   return 0;
 }
 
-extern "C" int mcb200_deconv_tc_launch(mcb200_deconv_plan* plan, float* out, int out_ld, const mcb200_epilogue* ep, int* status,
-                                       void* stream) {
+extern "C" int mcb200_deconv_tc_launch(mcb200_deconv_plan* plan, float* out, int out_ld, const mcb200_epilogue* ep, int flags,
+                                       int* status, void* stream) {
   if (!plan || plan->conv.im2col != kModePhase || (ep && ep->residual)) return -1;
-  return launch_core(&plan->conv, out, false, out_ld, ep, status, stream, plan);
+  return launch_core(&plan->conv, out, false, out_ld, ep, status, stream, flags, plan);
 }
 
 // ------------------------------------------------------------------ row mode (few input channels)

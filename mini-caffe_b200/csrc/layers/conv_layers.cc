@@ -233,12 +233,14 @@ void ConvolutionLayer::RefreshParameters() {
       KERNEL_CHECK(mcb200_dw_pack_weights(&shape_, blobs_[0]->gpu_data(), packed, ctx.stream_ptr()));
     }
     weight_version_ = wv;
+    constants_settled_ = false;
     for (auto& slot : plans_) {
       if (slot) slot->valid = false;
     }
   }
   const unsigned long long tv = 1 + TailVersion(tail_) + (bias_term_ ? blobs_[1]->host_version() : 0);
   if (tv != tail_version_) {
+    constants_settled_ = false;
     std::vector<float> scale, shift;
     bool has_scale = false, has_shift = false;
     FoldTail(tail_, shape_.cout, bias_term_ ? blobs_[1]->cpu_data() : nullptr, &scale, &shift, &has_scale,
@@ -326,12 +328,9 @@ void ConvolutionLayer::Forward_gpu(const vector<Blob*>& bottom, const vector<Blo
         slot.shape = s;
         slot.valid = true;
       }
-      if (half || half_out) {
-        KERNEL_CHECK(mcb200_conv_tc_launch_bf16(&slot.plan, out, half_out ? 1 : 0, s.cout, &ep, ctx.status_word(),
-                                                ctx.stream_ptr()));
-      } else {
-        KERNEL_CHECK(mcb200_conv_tc_launch(&slot.plan, out, s.cout, &ep, ctx.status_word(), ctx.stream_ptr()));
-      }
+      KERNEL_CHECK(mcb200_conv_tc_launch_flags(&slot.plan, out, half_out ? 1 : 0, s.cout, &ep,
+                                               constants_settled_ ? MCB200_CONV_CONSTANTS_SETTLED : 0, ctx.status_word(),
+                                               ctx.stream_ptr()));
     } else if (path_ == kDepthwise && (half || half_out)) {
       KERNEL_CHECK(mcb200_conv_depthwise_bf16(&s, in, half ? 1 : 0, packed_weights_.Reserve(0), out, half_out ? 1 : 0,
                                               &ep, ctx.stream_ptr()));
@@ -352,6 +351,7 @@ void ConvolutionLayer::Forward_gpu(const vector<Blob*>& bottom, const vector<Blo
       KERNEL_CHECK(mcb200_conv_direct(&s, in, blobs_[0]->gpu_data(), out, s.cout, &ep, ctx.stream_ptr()));
     }
   }
+  constants_settled_ = true;
 }
 
 static shared_ptr<Layer> CreateConvolution(const LayerParameter& param) {
@@ -428,9 +428,11 @@ void InnerProductLayer::Forward_gpu(const vector<Blob*>& bottom, const vector<Bl
     }
     weight_version_ = wv;
     plan_in_ = nullptr;
+    constants_settled_ = false;
   }
   const unsigned long long tv = 1 + TailVersion(tail_) + (bias_term_ ? blobs_[1]->host_version() : 0);
   if (tv != tail_version_) {
+    constants_settled_ = false;
     std::vector<float> scale, shift;
     bool has_scale = false, has_shift = false;
     FoldTail(tail_, N_, bias_term_ ? blobs_[1]->cpu_data() : nullptr, &scale, &shift, &has_scale, &has_shift);
@@ -457,7 +459,9 @@ void InnerProductLayer::Forward_gpu(const vector<Blob*>& bottom, const vector<Bl
       plan_w_ = w;
       plan_m_ = M_;
     }
-    KERNEL_CHECK(mcb200_conv_tc_launch(plan_, out, N_, &ep, ctx.status_word(), ctx.stream_ptr()));
+    KERNEL_CHECK(mcb200_conv_tc_launch_flags(plan_, out, 0, N_, &ep, constants_settled_ ? MCB200_CONV_CONSTANTS_SETTLED : 0,
+                                             ctx.status_word(), ctx.stream_ptr()));
+    constants_settled_ = true;
   } else {
     KERNEL_CHECK(mcb200_conv_direct(&s, in, w_rows, out, N_, &ep, ctx.stream_ptr()));
   }

@@ -113,6 +113,7 @@ void DeconvolutionLayer::Forward_gpu(const vector<Blob*>& bottom, const vector<B
         KERNEL_CHECK(mcb200_conv_pack_weights(&conv, flipped, packed, ctx.stream_ptr()));
       }
       weight_version_ = wv;
+      constants_settled_ = false;
       for (auto& slot : plans_) {
         if (slot) slot->valid = false;
       }
@@ -141,13 +142,14 @@ void DeconvolutionLayer::Forward_gpu(const vector<Blob*>& bottom, const vector<B
     ep.residual_coeff = 1.f;
     ep.shift = !bias_term_ ? nullptr : form == kWindow ? window_bias_.get() : blobs_[1]->gpu_data();
     float* out = top[i]->mutable_gpu_data_nhwc();
+    const int flags = constants_settled_ ? MCB200_CONV_CONSTANTS_SETTLED : 0;
     if (form == kPhases) {
-      KERNEL_CHECK(mcb200_deconv_tc_launch(&slot.plan, out, s.cout, &ep, ctx.status_word(), ctx.stream_ptr()));
+      KERNEL_CHECK(mcb200_deconv_tc_launch(&slot.plan, out, s.cout, &ep, flags, ctx.status_word(), ctx.stream_ptr()));
       continue;
     }
     float* result = out;
     if (form == kWindow) result = scratch_.Reserve(static_cast<size_t>(window.n) * window.ho * window.wo * window.cout);
-    KERNEL_CHECK(mcb200_conv_tc_launch(&slot.plan.conv, result, shape.cout, &ep, ctx.status_word(), ctx.stream_ptr()));
+    KERNEL_CHECK(mcb200_conv_tc_launch_flags(&slot.plan.conv, result, 0, shape.cout, &ep, flags, ctx.status_word(), ctx.stream_ptr()));
     if (form == kWindow) {
       const int phases_h = s.h == 1 && s.w == 1 && s.pad_h == 0 && s.pad_w == 0 ? s.kh : s.stride_h;
       const int phases_w = window.cout / s.cout / phases_h;
@@ -155,6 +157,7 @@ void DeconvolutionLayer::Forward_gpu(const vector<Blob*>& bottom, const vector<B
                                          ctx.stream_ptr()));
     }
   }
+  constants_settled_ = true;
 }
 REGISTER_LAYER_CLASS(Deconvolution);
 

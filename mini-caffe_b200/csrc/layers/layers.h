@@ -89,6 +89,7 @@ class ConvolutionLayer : public Layer {
   bool bias_term_ = false;
   FusedTail tail_;
   unsigned long long tail_version_ = 0;    // parameter versions the folded arrays were built from
+  bool constants_settled_ = false;   // weights and tail arrays are those of the launch before
   unsigned long long weight_version_ = 0;
   DeviceArray scale_, shift_;
   DeviceScratch packed_weights_, padded_input_;
@@ -122,6 +123,7 @@ class InnerProductLayer : public Layer {
   int M_ = 0, K_ = 0, N_ = 0;
   bool bias_term_ = false, transpose_ = false;
   FusedTail tail_;
+  bool constants_settled_ = false;   // weights and tail arrays are those of the launch before
   unsigned long long tail_version_ = 0, weight_version_ = 0;
   DeviceArray scale_, shift_;
   DeviceScratch packed_weights_, staged_weights_;
@@ -493,6 +495,7 @@ class DeconvolutionLayer : public Layer {
   // reaches).
   enum Form { kPhases, kWindow, kSpread };
   Form form_ = kSpread;
+  bool constants_settled_ = false;   // weights and tail arrays are those of the launch before
   unsigned long long weight_version_ = 0;
   DeviceScratch flipped_weights_, packed_weights_, scratch_;
   DeviceArray window_bias_;   // the bias once per phase

@@ -84,6 +84,9 @@ class CAFFE_API Net {
   void AppendParam(const NetParameter& param, const int layer_id, const int param_id);
   /*! \brief (re)build the execution plan: fusion, blob lifetimes, storage sharing */
   void PlaceMemory();
+  /*! \brief which steps run part by part behind the copies of a new input, and those steps of a pass */
+  void PlanParts();
+  void ForwardInParts();
 
   string name_;
   vector<shared_ptr<Layer> > layers_;

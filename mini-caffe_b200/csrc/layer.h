@@ -115,6 +115,13 @@ class Layer {
   // The net's decision.  operands: read bottoms / residual as bfloat16; top:
   // store top 0 as bfloat16.
   virtual void SetHalfStorage(bool operands, bool top) {}
+  // ---- running a pass in parts of its batch ----
+  // PartSeconds: as shaped and fused now, about how long the layer takes for the whole batch, or 0 if
+  // it cannot run for some of the images only (first_of_net: it reads the net's input, of which no
+  // more than these images may have arrived).  ForwardImages runs images [first, first + count) as
+  // the part-th piece of a pass; the pieces of a pass cover the batch in order.
+  virtual double PartSeconds(const vector<Blob*>& bottom, const vector<Blob*>& top, bool first_of_net) const { return 0; }
+  inline void ForwardImages(const vector<Blob*>& bottom, const vector<Blob*>& top, int first, int count, int part);
   // The net's word that no later layer of the pass reads this layer's tops: the pass ends by
   // bringing them to the host, so the layer may as well write them there.
   virtual void SetTopsEndOnHost(bool on_host) {}
@@ -133,6 +140,10 @@ class Layer {
     LOG(FATAL) << type() << " layer: this engine has no CPU compute path";
   }
   virtual void Forward_gpu(const vector<Blob*>& bottom, const vector<Blob*>& top) { Forward_cpu(bottom, top); }
+
+  virtual void ForwardImages_gpu(const vector<Blob*>& bottom, const vector<Blob*>& top, int first, int count, int part) {
+    LOG(FATAL) << type() << " layer: does not run for some of the images only";
+  }
 
   virtual void CheckBlobCounts(const vector<Blob*>& bottom, const vector<Blob*>& top) {
     const int nb = static_cast<int>(bottom.size());
@@ -174,6 +185,11 @@ inline void Layer::Forward(const vector<Blob*>& bottom, const vector<Blob*>& top
   // Raises caffe::Error in CPU mode or without a device: there is no CPU path.
   Context::Get().Activate();
   Forward_gpu(bottom, top);
+}
+
+inline void Layer::ForwardImages(const vector<Blob*>& bottom, const vector<Blob*>& top, int first, int count, int part) {
+  Context::Get().Activate();
+  ForwardImages_gpu(bottom, top, first, count, part);
 }
 
 inline void Layer::ToProto(LayerParameter* param) {

@@ -1,6 +1,7 @@
 // Convolution and InnerProduct: parameter handling on the host, tensor-core /
 // depthwise / direct kernels on the device, fused tails folded into
 // per-channel scale and shift arrays.
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 
@@ -40,6 +41,7 @@ const float* HostInput::Take(const Blob& blob) {
 unsigned long long TailVersion(const FusedTail& tail) {
   unsigned long long v = 0;
   for (Layer* l : tail.affine) v += l->ParamVersion();
+  if (tail.activation) v += tail.activation->ParamVersion();
   return v;
 }
 
@@ -251,107 +253,141 @@ void ConvolutionLayer::RefreshParameters() {
   }
 }
 
+double ConvolutionLayer::PartSeconds(const vector<Blob*>& bottom, const vector<Blob*>& top, bool first_of_net) const {
+  const mcb200_conv_shape& s = shape_;
+  if (bottom.size() != 1 || path_ == kDirect || s.cout % 8 != 0) return 0;
+  // Of the net's input only a layer that reads (N, C, H, W) rows itself may take a part.
+  if (first_of_net ? !use_rows_ || s.c % 4 == 0 : s.c % 8 != 0) return 0;
+  const double in_cell = half_operands_ && HalfOperandsCapable() ? 2.0 : 4.0;
+  const double out_cell = half_top_ && HalfTopCapable() ? 2.0 : 4.0;
+  double bytes = in_cell * bottom[0]->count() + out_cell * top[0]->count();
+  if (tail_.residual) bytes += in_cell * top[0]->count();
+  const double flops = 2.0 * top[0]->count() * (s.c / s.group) * s.kh * s.kw;
+  const double rate = path_ == kDepthwise ? 20e12 : in_cell == 2.0 ? 1.1e15 : 0.6e15;
+  return std::max(bytes / kPartBytesPerSecond, flops / rate);
+}
+
 void ConvolutionLayer::Forward_gpu(const vector<Blob*>& bottom, const vector<Blob*>& top) {
-  Context& ctx = Context::Get();
   RefreshParameters();
-  if (plans_.size() < bottom.size()) plans_.resize(bottom.size());
-  for (size_t i = 0; i < bottom.size(); ++i) {
-    mcb200_conv_shape s = shape_;
-    const float* in = nullptr;
-    const bool half = half_operands_ && HalfOperandsCapable();
-    if (half) {
-      s.c_stride = s.c;
-      in = static_cast<const float*>(bottom[i]->gpu_data_nhwc_bf16());   // 16-bit cells
-    } else if (path_ == kTensorCore && use_rows_) {
-      int hp = 0, wp = 0;
-      CHECK_EQ(mcb200_conv_rows_padded_dims(&s, &hp, &wp), 0);
-      s.c_stride = 4;
-      float* padded = padded_input_.Reserve(static_cast<size_t>(s.n) * hp * wp * 4);
-      KERNEL_CHECK(mcb200_conv_rows_pad_input(&s, bottom[i]->gpu_data(), padded, ctx.stream_ptr()));
-      in = padded;
-    } else if (shape_.c % 4 == 0) {
-      s.c_stride = s.c;
-      in = bottom[i]->gpu_data_nhwc();
-    } else {
-      // Pad the channels to a multiple of four (16-byte pixels) in a private
-      // channels-last copy, e.g. the three colour planes of the first layer.
-      s.c_stride = (s.c + 3) / 4 * 4;
-      float* padded = padded_input_.Reserve(static_cast<size_t>(s.n) * s.h * s.w * s.c_stride);
-      if (bottom[i]->device_is_nhwc()) {
-        // The pad lanes meet zero weights but still have to be finite.
-        CUDA_CHECK(cudaMemsetAsync(padded, 0, static_cast<size_t>(s.n) * s.h * s.w * s.c_stride * sizeof(float),
-                                   ctx.stream()));
-        KERNEL_CHECK(mcb200_copy_2d(bottom[i]->gpu_data_nhwc(), s.c, padded, s.c_stride,
-                                    static_cast<long long>(s.n) * s.h * s.w, s.c, ctx.stream_ptr()));
-      } else {
-        KERNEL_CHECK(mcb200_nchw_to_nhwc(bottom[i]->gpu_data(), padded, s.n, s.c, s.h, s.w, s.c_stride,
-                                         ctx.stream_ptr()));
-      }
-      in = padded;
-    }
-    mcb200_epilogue ep;
-    FillTailEpilogue(i == 0 ? tail_ : FusedTail(), scale_, shift_, half ? kResidualNhwcHalf : kResidualNhwc, s.cout,
-                     &ep);
-    const bool half_out = half_top_ && HalfTopCapable();
-    float* out = half_out ? static_cast<float*>(top[i]->mutable_gpu_data_nhwc_bf16()) : top[i]->mutable_gpu_data_nhwc();
-    if (path_ == kTensorCore) {
-      if (!plans_[i]) plans_[i].reset(new PlanSlot);
-      PlanSlot& slot = *plans_[i];
-      const float* w = packed_weights_.Reserve(0);
-      if (!slot.valid || slot.in != in || slot.weights != w || std::memcmp(&slot.shape, &s, sizeof(s)) != 0) {
-        int rc = half ? mcb200_conv_tc_plan_bf16(&s, reinterpret_cast<const uint16_t*>(in),
-                                                 reinterpret_cast<const uint16_t*>(w), &slot.plan)
-                 : use_rows_ ? mcb200_conv_rows_plan(&s, in, w, &slot.plan)
-                             : mcb200_conv_tc_plan(&s, in, w, &slot.plan);
-        if (rc != 0 && use_rows_) {
-          // The driver refused the row-mode tensor map: use the general path from now on.
-          LOG(WARNING) << "layer " << layer_param_.name() << ": row-mode plan rejected (" << rc
-                       << "), using the im2col path";
-          rows_rejected_ = true;
-          use_rows_ = false;
-          weight_version_ = 0;
-          Forward_gpu(bottom, top);
-          return;
-        }
-        if (rc != 0 && !half && !half_out) {
-          // A shape the tensor maps cannot express (for instance a stride above 8, which the
-          // im2col map refuses as traversal stride): the plain kernel runs it from now on.
-          LOG(WARNING) << "layer " << layer_param_.name() << ": tensor-core plan rejected (" << rc
-                       << "), using the direct kernel";
-          path_ = kDirect;
-          Forward_gpu(bottom, top);
-          return;
-        }
-        CHECK_EQ(rc, 0) << "cannot build the tensor-core plan for layer " << layer_param_.name();
-        slot.in = in;
-        slot.weights = w;
-        slot.shape = s;
-        slot.valid = true;
-      }
-      KERNEL_CHECK(mcb200_conv_tc_launch_flags(&slot.plan, out, half_out ? 1 : 0, s.cout, &ep,
-                                               constants_settled_ ? MCB200_CONV_CONSTANTS_SETTLED : 0, ctx.status_word(),
-                                               ctx.stream_ptr()));
-    } else if (path_ == kDepthwise && (half || half_out)) {
-      KERNEL_CHECK(mcb200_conv_depthwise_bf16(&s, in, half ? 1 : 0, packed_weights_.Reserve(0), out, half_out ? 1 : 0,
-                                              &ep, ctx.stream_ptr()));
-    } else if (path_ == kDepthwise) {
-      const char* dw_tma = getenv("MCB200_DW_TMA");   // "0": the register-window kernel, for comparisons
-      // Outputs of 8 x 8 pixels and more: the TMA-staged kernel's 8 x 16 tiles; on smaller maps
-      // (the 7 x 7 end of MobileNet) most of a tile is outside the image and the register-window
-      // kernel is quicker (11 / 14 us against 15 / 18 us at batch 64).  The rule looks at the
-      // layer's geometry only, never at the batch.
-      const bool roomy = s.ho >= 8 && s.wo >= 8;
-      if (!ep.residual && roomy && mcb200_conv_depthwise_tma_supported(&s) && !(dw_tma && dw_tma[0] == '0')) {
-        KERNEL_CHECK(mcb200_conv_depthwise_tma(&s, in, packed_weights_.Reserve(0), out, &ep, ctx.status_word(),
-                                               ctx.stream_ptr()));
-      } else {
-        KERNEL_CHECK(mcb200_conv_depthwise(&s, in, packed_weights_.Reserve(0), out, &ep, ctx.stream_ptr()));
-      }
-    } else {
-      KERNEL_CHECK(mcb200_conv_direct(&s, in, blobs_[0]->gpu_data(), out, s.cout, &ep, ctx.stream_ptr()));
-    }
-  }
+  for (size_t i = 0; i < bottom.size(); ++i) RunImages(bottom[i], top[i], i, 0, shape_.n, i);
   constants_settled_ = true;
+}
+
+void ConvolutionLayer::ForwardImages_gpu(const vector<Blob*>& bottom, const vector<Blob*>& top, int first, int count,
+                                         int part) {
+  if (first == 0) RefreshParameters();
+  RunImages(bottom[0], top[0], 0, first, count, part);
+  if (first + count == shape_.n) constants_settled_ = true;
+}
+
+void ConvolutionLayer::RunImages(Blob* bottom, Blob* top, size_t i, int first, int count, size_t slot_index) {
+  Context& ctx = Context::Get();
+  mcb200_conv_shape s = shape_;
+  s.n = count;
+  const size_t in_at = static_cast<size_t>(first) * s.c * s.h * s.w;
+  const size_t out_at = static_cast<size_t>(first) * s.cout * s.ho * s.wo;
+  const float* in = nullptr;
+  const bool half = half_operands_ && HalfOperandsCapable();
+  if (half) {
+    s.c_stride = s.c;
+    in = reinterpret_cast<const float*>(static_cast<const uint16_t*>(bottom->gpu_data_nhwc_bf16()) + in_at);
+  } else if (path_ == kTensorCore && use_rows_) {
+    int hp = 0, wp = 0;
+    CHECK_EQ(mcb200_conv_rows_padded_dims(&s, &hp, &wp), 0);
+    s.c_stride = 4;
+    const size_t image = static_cast<size_t>(hp) * wp * 4;
+    float* padded = padded_input_.Reserve(shape_.n * image) + first * image;
+    KERNEL_CHECK(mcb200_conv_rows_pad_input(&s, bottom->gpu_data() + in_at, padded, ctx.stream_ptr()));
+    in = padded;
+  } else if (shape_.c % 4 == 0) {
+    s.c_stride = s.c;
+    in = bottom->gpu_data_nhwc() + in_at;
+  } else {
+    // Pad the channels to a multiple of four (16-byte pixels) in a private
+    // channels-last copy, e.g. the three colour planes of the first layer.
+    s.c_stride = (s.c + 3) / 4 * 4;
+    const size_t image = static_cast<size_t>(s.h) * s.w * s.c_stride;
+    float* padded = padded_input_.Reserve(shape_.n * image) + first * image;
+    if (bottom->device_is_nhwc()) {
+      // The pad lanes meet zero weights but still have to be finite.
+      CUDA_CHECK(cudaMemsetAsync(padded, 0, static_cast<size_t>(s.n) * s.h * s.w * s.c_stride * sizeof(float),
+                                 ctx.stream()));
+      KERNEL_CHECK(mcb200_copy_2d(bottom->gpu_data_nhwc() + in_at, s.c, padded, s.c_stride,
+                                  static_cast<long long>(s.n) * s.h * s.w, s.c, ctx.stream_ptr()));
+    } else {
+      KERNEL_CHECK(mcb200_nchw_to_nhwc(bottom->gpu_data() + in_at, padded, s.n, s.c, s.h, s.w, s.c_stride,
+                                       ctx.stream_ptr()));
+    }
+    in = padded;
+  }
+  mcb200_epilogue ep;
+  FillTailEpilogue(i == 0 ? tail_ : FusedTail(), scale_, shift_, half ? kResidualNhwcHalf : kResidualNhwc, s.cout,
+                   &ep);
+  if (ep.residual) {
+    ep.residual = half ? reinterpret_cast<const float*>(reinterpret_cast<const uint16_t*>(ep.residual) + out_at)
+                       : ep.residual + out_at;
+  }
+  const bool half_out = half_top_ && HalfTopCapable();
+  float* out = half_out ? reinterpret_cast<float*>(static_cast<uint16_t*>(top->mutable_gpu_data_nhwc_bf16()) + out_at)
+                        : top->mutable_gpu_data_nhwc() + out_at;
+  if (path_ == kTensorCore) {
+    if (plans_.size() <= slot_index) plans_.resize(slot_index + 1);
+    if (!plans_[slot_index]) plans_[slot_index].reset(new PlanSlot);
+    PlanSlot& slot = *plans_[slot_index];
+    const float* w = packed_weights_.Reserve(0);
+    if (!slot.valid || slot.in != in || slot.weights != w || std::memcmp(&slot.shape, &s, sizeof(s)) != 0) {
+      int rc = half ? mcb200_conv_tc_plan_bf16(&s, reinterpret_cast<const uint16_t*>(in),
+                                               reinterpret_cast<const uint16_t*>(w), &slot.plan)
+               : use_rows_ ? mcb200_conv_rows_plan(&s, in, w, &slot.plan)
+                           : mcb200_conv_tc_plan(&s, in, w, &slot.plan);
+      if (rc != 0 && use_rows_) {
+        // The driver refused the row-mode tensor map: use the general path from now on.
+        LOG(WARNING) << "layer " << layer_param_.name() << ": row-mode plan rejected (" << rc
+                     << "), using the im2col path";
+        rows_rejected_ = true;
+        use_rows_ = false;
+        weight_version_ = 0;
+        RefreshParameters();
+        RunImages(bottom, top, i, first, count, slot_index);
+        return;
+      }
+      if (rc != 0 && !half && !half_out) {
+        // A shape the tensor maps cannot express (for instance a stride above 8, which the
+        // im2col map refuses as traversal stride): the plain kernel runs it from now on.
+        LOG(WARNING) << "layer " << layer_param_.name() << ": tensor-core plan rejected (" << rc
+                     << "), using the direct kernel";
+        path_ = kDirect;
+        RunImages(bottom, top, i, first, count, slot_index);
+        return;
+      }
+      CHECK_EQ(rc, 0) << "cannot build the tensor-core plan for layer " << layer_param_.name();
+      slot.in = in;
+      slot.weights = w;
+      slot.shape = s;
+      slot.valid = true;
+    }
+    KERNEL_CHECK(mcb200_conv_tc_launch_flags(&slot.plan, out, half_out ? 1 : 0, s.cout, &ep,
+                                             constants_settled_ ? MCB200_CONV_CONSTANTS_SETTLED : 0, ctx.status_word(),
+                                             ctx.stream_ptr()));
+  } else if (path_ == kDepthwise && (half || half_out)) {
+    KERNEL_CHECK(mcb200_conv_depthwise_bf16(&s, in, half ? 1 : 0, packed_weights_.Reserve(0), out, half_out ? 1 : 0,
+                                            &ep, ctx.stream_ptr()));
+  } else if (path_ == kDepthwise) {
+    const char* dw_tma = getenv("MCB200_DW_TMA");   // "0": the register-window kernel, for comparisons
+    // Outputs of 8 x 8 pixels and more: the TMA-staged kernel's 8 x 16 tiles; on smaller maps
+    // (the 7 x 7 end of MobileNet) most of a tile is outside the image and the register-window
+    // kernel is quicker (11 / 14 us against 15 / 18 us at batch 64).  The rule looks at the
+    // layer's geometry only, never at the batch.
+    const bool roomy = s.ho >= 8 && s.wo >= 8;
+    if (!ep.residual && roomy && mcb200_conv_depthwise_tma_supported(&s) && !(dw_tma && dw_tma[0] == '0')) {
+      KERNEL_CHECK(mcb200_conv_depthwise_tma(&s, in, packed_weights_.Reserve(0), out, &ep, ctx.status_word(),
+                                             ctx.stream_ptr()));
+    } else {
+      KERNEL_CHECK(mcb200_conv_depthwise(&s, in, packed_weights_.Reserve(0), out, &ep, ctx.stream_ptr()));
+    }
+  } else {
+    KERNEL_CHECK(mcb200_conv_direct(&s, in, blobs_[0]->gpu_data(), out, s.cout, &ep, ctx.stream_ptr()));
+  }
 }
 
 static shared_ptr<Layer> CreateConvolution(const LayerParameter& param) {

@@ -78,19 +78,31 @@ void PoolingLayer::Reshape(const vector<Blob*>& bottom, const vector<Blob*>& top
   channels_ = bottom[0]->channels();
 }
 
+double PoolingLayer::PartSeconds(const vector<Blob*>& bottom, const vector<Blob*>& top, bool first_of_net) const {
+  if (first_of_net || channels_ % 8 != 0) return 0;
+  const double cell = half_ && HalfOperandsCapable() ? 2.0 : 4.0;
+  return cell * (static_cast<double>(bottom[0]->count()) + top[0]->count()) / kPartBytesPerSecond;
+}
+
 void PoolingLayer::Forward_gpu(const vector<Blob*>& bottom, const vector<Blob*>& top) {
+  ForwardImages_gpu(bottom, top, 0, bottom[0]->num(), 0);
+}
+
+void PoolingLayer::ForwardImages_gpu(const vector<Blob*>& bottom, const vector<Blob*>& top, int first, int count, int part) {
   Context& ctx = Context::Get();
+  const size_t in_at = static_cast<size_t>(first) * channels_ * bottom[0]->height() * bottom[0]->width();
+  const size_t out_at = static_cast<size_t>(first) * channels_ * pooled_h_ * pooled_w_;
   if (half_ && HalfOperandsCapable()) {
-    const uint16_t* in16 = static_cast<const uint16_t*>(bottom[0]->gpu_data_nhwc_bf16());
-    uint16_t* out16 = static_cast<uint16_t*>(top[0]->mutable_gpu_data_nhwc_bf16());
-    KERNEL_CHECK(mcb200_pool_max_nhwc_bf16(in16, out16, bottom[0]->num(), bottom[0]->height(), bottom[0]->width(),
+    const uint16_t* in16 = static_cast<const uint16_t*>(bottom[0]->gpu_data_nhwc_bf16()) + in_at;
+    uint16_t* out16 = static_cast<uint16_t*>(top[0]->mutable_gpu_data_nhwc_bf16()) + out_at;
+    KERNEL_CHECK(mcb200_pool_max_nhwc_bf16(in16, out16, count, bottom[0]->height(), bottom[0]->width(),
                                            bottom[0]->channels(), kernel_h_, kernel_w_, stride_h_, stride_w_, pad_h_,
                                            pad_w_, pooled_h_, pooled_w_, ctx.stream_ptr()));
     return;
   }
-  const float* in = bottom[0]->gpu_data_nhwc();
-  float* out = top[0]->mutable_gpu_data_nhwc();
-  KERNEL_CHECK(mcb200_pool_nhwc(in, out, bottom[0]->num(), bottom[0]->height(), bottom[0]->width(),
+  const float* in = bottom[0]->gpu_data_nhwc() + in_at;
+  float* out = top[0]->mutable_gpu_data_nhwc() + out_at;
+  KERNEL_CHECK(mcb200_pool_nhwc(in, out, count, bottom[0]->height(), bottom[0]->width(),
                                 bottom[0]->channels(), kernel_h_, kernel_w_, stride_h_, stride_w_, pad_h_, pad_w_,
                                 pooled_h_, pooled_w_, method_, ctx.stream_ptr()));
 }

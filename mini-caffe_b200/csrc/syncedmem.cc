@@ -327,6 +327,13 @@ void* SyncedMemory::overwrite_on_host() {
   return host_.ptr;
 }
 
+void* SyncedMemory::device_to_fill() {
+  EnsureDevice();
+  nhwc_aliases_dev_ = false;
+  valid_ |= kDevice;
+  return dev_.ptr;
+}
+
 void SyncedMemory::EndHostCopy() { valid_ |= kHost; }
 
 void* SyncedMemory::mutable_cpu_data() {

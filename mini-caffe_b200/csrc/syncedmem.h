@@ -89,6 +89,9 @@ class SyncedMemory {
   // stream before anything reads it (as the end of a forward pass does).
   const void* host_only() const { return valid_ == kHost ? host_.ptr : nullptr; }
   void* overwrite_on_host();
+  // The device buffer for the caller to fill with the host copy's values, which counts as current at
+  // once: the caller orders every reader behind its copies.
+  void* device_to_fill();
   // Channels-last copy of the (n, c, h, w) tensor stored here.  When the two
   // orders coincide (c == 1 or h*w == 1) it is the plain device copy.
   const void* gpu_data_nhwc(int n, int c, int h, int w);

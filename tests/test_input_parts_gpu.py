@@ -1,0 +1,73 @@
+"""A pass whose first layers run part by part behind the copies of a new input gives the bits of the pass
+that copies first: every kernel's result for an image is independent of the images beside it."""
+import numpy as np
+import pytest
+
+from conftest import pkg
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def gpu_engine(engine):
+    engine.set_mode(True, 0)
+    return engine
+
+
+def _net(wl, batch, size):
+    """Image -> row-mode convolution, pooling, a residual block, depthwise, PReLU, then a layer that ends the
+    part-wise steps (12 output channels)."""
+    b = wl.NetBuilder("parts")
+    b.input([("data", (batch, 3, size, size))])
+    b.conv("conv1", "data", "conv1", 3, 32, 5, stride=2, pad=2)
+    b.relu("conv1_relu", "conv1")
+    b.pool("pool1", "conv1", "pool1", "MAX", k=3, stride=2)
+    b.conv_bn("wide", "pool1", "wide", 32, 64, 1, relu=False)
+    b.conv_bn("a", "pool1", "a", 32, 32, 3, pad=1)
+    b.conv_bn("z", "a", "z", 32, 64, 1, relu=False)
+    b.eltwise_sum("sum", ["wide", "z"], "sum")
+    b.relu("sum_relu", "sum")
+    b.conv("dw", "sum", "dw", 64, 64, 3, stride=2, pad=1, group=64)
+    b.raw("dw_prelu", "PReLU", ["dw"], ["dw"])
+    b.params.append(("dw_prelu_0", (64,), "one", 0))
+    b.conv("point", "dw", "point", 64, 40, 1)
+    b.conv("odd", "point", "odd", 40, 12, 3, pad=1)
+    b.pool("pool5", "odd", "pool5", "AVE", global_pooling=True)
+    return b
+
+
+@pytest.mark.parametrize("precision", ["fp32", "bf16"])
+@pytest.mark.parametrize("batch,parts,size", [(2, 2, 33), (5, 3, 40), (8, 8, 64), (13, 4, 57)])
+def test_parts_give_the_bits_of_the_whole(monkeypatch, capi, gpu_engine, batch, parts, size, precision):
+    wl = pkg("workloads")
+    b = _net(wl, batch, size)
+    weights = wl.init_params(b.params, seed=batch, bn_identity=False)
+    rng = np.random.default_rng(size)
+    inputs = [rng.standard_normal((batch, 3, size, size)).astype(np.float32) for _ in range(2)]
+    inputs.append(inputs[1].copy())
+    inputs.append(inputs[0][:max(1, batch // 2)])          # the plan is made again for another batch
+    monkeypatch.setenv("MINICAFFE_PRECISION", precision)
+
+    def run(value):
+        monkeypatch.setenv("MCB200_INPUT_PARTS", str(value))
+        net = capi.Net(gpu_engine, b.text(), None, from_buffer=True)
+        net.set_params(weights)
+        net.mark_output("pool1")
+        got = []
+        for i, x in enumerate(inputs):
+            if i == 2:                                      # new slopes reach the launch that follows them
+                net.set_params({"dw_prelu_0": np.full(64, 0.25, np.float32)})
+            net.forward(data=x)
+            got += [net.blob("pool1").data.copy(), net.blob("pool5").data.copy()]
+            net.forward()                                   # the same input once more
+            got.append(net.blob("pool5").data.copy())
+        net.close()
+        return got
+
+    whole, pieces = run(1), run(parts)
+    for w, p in zip(whole, pieces):
+        assert w.shape == p.shape and np.isfinite(w).all()
+        assert (w == p).all()
+    assert (whole[4] != whole[7]).any()                     # the slopes alone
+    for i in range(0, len(whole), 3):
+        assert (whole[i + 1] == whole[i + 2]).all()

@@ -86,6 +86,8 @@ class CAFFE_API Net {
   void PlaceMemory();
   /*! \brief which steps run part by part behind the copies of a new input, and those steps of a pass */
   void PlanParts();
+  /*! \brief steps that only rename axes in front of a Concat are left out */
+  void AbsorbViews();
   void ForwardInParts();
 
   string name_;

@@ -254,6 +254,18 @@ int mcb200_softmax(const float* in, float* out, int outer, int channels, int inn
  * in floats).  Concat / Slice style block copies (src/layers/concat_layer.cpp:53-70). */
 int mcb200_copy_2d(const float* src, long long src_pitch, float* dst, long long dst_pitch, long long rows,
                    long long cols, void* stream);
+/* dst[rows][sum of cols] from up to MCB200_CONCAT_SOURCES dense sources [rows][cols[i]], side by side, in one
+ * launch.  -2: a form it does not take (the caller copies source by source).                    */
+#define MCB200_CONCAT_SOURCES 16
+int mcb200_concat_rows(int sources, const float* const* src, const long long* cols, long long rows, float* dst, void* stream);
+/* SSD's prior boxes of a layer_h x layer_w map: `boxes` pairs (width, height) per cell, around cell centres
+ * ((w + offset) * step_w, (h + offset) * step_h), as fractions of the image, then the variances (1 or 4) in
+ * the second half of out[2][layer_h * layer_w * boxes * 4].  float centres, double arithmetic around them, one rounding
+ * per coordinate (src/layers/prior_box_layer.cpp:79-164).                                       */
+#define MCB200_PRIOR_BOXES 64
+int mcb200_prior_box(int layer_h, int layer_w, int img_h, int img_w, float step_h, float step_w, float offset, int boxes,
+                     const float* box_w, const float* box_h, const float* variance, int variances, int clip, float* out,
+                     void* stream);
 /* out[permuted index] = in[index] for up to 6 axes; order[i] is the input axis
  * that becomes output axis i (src/layers/permute_layer.cpp:8-22).           */
 int mcb200_permute(const float* in, float* out, int num_axes, const int* in_shape, const int* order, void* stream);

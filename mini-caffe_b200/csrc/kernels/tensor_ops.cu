@@ -565,6 +565,63 @@ __global__ void copy_2d_vec4_kernel(const float4* __restrict__ src, long long sr
   }
 }
 
+struct ConcatArgs {
+  const float* src[MCB200_CONCAT_SOURCES];
+  unsigned cols[MCB200_CONCAT_SOURCES];     // in cells of V floats
+  unsigned offset[MCB200_CONCAT_SOURCES];
+  unsigned rows, pitch;
+};
+
+// blockIdx.y is the source.  Bound by its bytes for a batch and by the launch for one image: SSD300's six
+// confidence heads were a permutation, a flattening and a block copy each, 18 launches of about 4 us apart
+// (and three times the bytes); they are one.
+template <typename Cell>
+__global__ void __launch_bounds__(256) concat_rows_kernel(const ConcatArgs a, Cell* __restrict__ dst) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const unsigned cols = a.cols[blockIdx.y];
+  const Cell* __restrict__ src = reinterpret_cast<const Cell*>(a.src[blockIdx.y]);
+  dst += a.offset[blockIdx.y];
+  const unsigned total = a.rows * cols;
+  for (unsigned i = blockIdx.x * 256u + threadIdx.x; i < total; i += gridDim.x * 256u) {
+    const unsigned r = i / cols;
+    dst[static_cast<size_t>(r) * a.pitch + (i - r * cols)] = src[i];
+  }
+}
+
+struct PriorBoxArgs {
+  int layer_h, layer_w, boxes, variances, clip;
+  double img_h, img_w;
+  float step_h, step_w, offset;
+  float box_w[MCB200_PRIOR_BOXES], box_h[MCB200_PRIOR_BOXES];
+  float variance[4];
+};
+
+// A thread per box and half.  Every operation is a correctly rounded one of its own (no contraction), in
+// the order of the host expression: the same bits.
+__global__ void __launch_bounds__(128) prior_box_kernel(const PriorBoxArgs a, float4* __restrict__ out) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int count = a.layer_h * a.layer_w * a.boxes;
+  const int i = blockIdx.x * 128 + threadIdx.x;
+  if (i >= count) return;
+  const int cell = i / a.boxes, box = i - cell * a.boxes;
+  const int h = cell / a.layer_w, w = cell - h * a.layer_w;
+  const double cx = __fmul_rn(__fadd_rn(static_cast<float>(w), a.offset), a.step_w);
+  const double cy = __fmul_rn(__fadd_rn(static_cast<float>(h), a.offset), a.step_h);
+  const double hw = __ddiv_rn(a.box_w[box], 2.0), hh = __ddiv_rn(a.box_h[box], 2.0);
+  float v[4] = {static_cast<float>(__ddiv_rn(__dsub_rn(cx, hw), a.img_w)), static_cast<float>(__ddiv_rn(__dsub_rn(cy, hh), a.img_h)),
+                static_cast<float>(__ddiv_rn(__dadd_rn(cx, hw), a.img_w)), static_cast<float>(__ddiv_rn(__dadd_rn(cy, hh), a.img_h))};
+  if (a.clip) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float low = v[j] < 0.f ? 0.f : v[j];   // std::max, then std::min: their operand order
+      v[j] = 1.f < low ? 1.f : low;
+    }
+  }
+  out[i] = make_float4(v[0], v[1], v[2], v[3]);
+  out[count + i] = a.variances == 1 ? make_float4(a.variance[0], a.variance[0], a.variance[0], a.variance[0])
+                                    : make_float4(a.variance[0], a.variance[1], a.variance[2], a.variance[3]);
+}
+
 struct PermuteArgs {
   int num_axes;
   int out_shape[6];
@@ -863,6 +920,76 @@ extern "C" int mcb200_copy_2d(const float* src, long long src_pitch, float* dst,
     copy_2d_kernel<<<grid_for(rows * cols, threads), threads, 0, as_stream(stream)>>>(src, src_pitch, dst, dst_pitch,
                                                                                      rows, cols);
   }
+  count_launch();
+  return static_cast<int>(cudaGetLastError());
+}
+
+extern "C" int mcb200_concat_rows(int sources, const float* const* src, const long long* cols, long long rows, float* dst,
+                                  void* stream) {
+  if (sources < 1 || !src || !cols || rows < 0 || !dst) return -1;
+  if (sources > MCB200_CONCAT_SOURCES) return -2;
+  long long pitch = 0, widest = 0;
+  uintptr_t bits = reinterpret_cast<uintptr_t>(dst);
+  for (int i = 0; i < sources; ++i) {
+    if (!src[i] || cols[i] < 0) return -1;
+    bits |= reinterpret_cast<uintptr_t>(src[i]) | static_cast<uintptr_t>(cols[i]) * sizeof(float);
+    pitch += cols[i];
+    if (cols[i] > widest) widest = cols[i];
+  }
+  // (the grid's last step may carry the 32-bit index past the end of a source)
+  if (rows > 0x3fffffffLL || pitch > 0x3fffffffLL || rows * widest > 0x7fffffffLL) return -2;
+  if (rows == 0 || widest == 0) return 0;
+  // The widest cell that every source's row and address is a multiple of.
+  const int v = (bits & 15) == 0 ? 4 : (bits & 7) == 0 ? 2 : 1;
+  ConcatArgs a = {};
+  unsigned at = 0;
+  for (int i = 0; i < sources; ++i) {
+    a.src[i] = src[i];
+    a.cols[i] = static_cast<unsigned>(cols[i] / v);
+    a.offset[i] = at;
+    at += a.cols[i];
+  }
+  a.rows = static_cast<unsigned>(rows);
+  a.pitch = at;
+  const dim3 grid(grid_for(rows * widest / v, 256), sources);
+  cudaStream_t st = as_stream(stream);
+  if (v == 4) {
+    concat_rows_kernel<<<grid, 256, 0, st>>>(a, reinterpret_cast<float4*>(dst));
+  } else if (v == 2) {
+    concat_rows_kernel<<<grid, 256, 0, st>>>(a, reinterpret_cast<float2*>(dst));
+  } else {
+    concat_rows_kernel<<<grid, 256, 0, st>>>(a, dst);
+  }
+  count_launch();
+  return static_cast<int>(cudaGetLastError());
+}
+
+extern "C" int mcb200_prior_box(int layer_h, int layer_w, int img_h, int img_w, float step_h, float step_w, float offset,
+                                int boxes, const float* box_w, const float* box_h, const float* variance, int variances,
+                                int clip, float* out, void* stream) {
+  if (layer_h < 1 || layer_w < 1 || boxes < 1 || !box_w || !box_h || !variance || (variances != 1 && variances != 4) || !out)
+    return -1;
+  if (boxes > MCB200_PRIOR_BOXES || (reinterpret_cast<uintptr_t>(out) & 15) ||
+      static_cast<long long>(layer_h) * layer_w * boxes > 0x0fffffffLL)
+    return -2;
+  PriorBoxArgs a = {};
+  a.layer_h = layer_h;
+  a.layer_w = layer_w;
+  a.boxes = boxes;
+  a.variances = variances;
+  a.clip = clip;
+  a.img_h = img_h;
+  a.img_w = img_w;
+  a.step_h = step_h;
+  a.step_w = step_w;
+  a.offset = offset;
+  for (int i = 0; i < boxes; ++i) {
+    a.box_w[i] = box_w[i];
+    a.box_h[i] = box_h[i];
+  }
+  for (int i = 0; i < variances; ++i) a.variance[i] = variance[i];
+  const int blocks = (layer_h * layer_w * boxes + 127) / 128;
+  prior_box_kernel<<<blocks, 128, 0, as_stream(stream)>>>(a, reinterpret_cast<float4*>(out));
   count_launch();
   return static_cast<int>(cudaGetLastError());
 }

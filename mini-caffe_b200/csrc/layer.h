@@ -115,6 +115,15 @@ class Layer {
   // The net's decision.  operands: read bottoms / residual as bfloat16; top:
   // store top 0 as bfloat16.
   virtual void SetHalfStorage(bool operands, bool top) {}
+  // ---- views: layers that only rename the axes of their bottom ----
+  // kSameOrder: the top is the bottom's (N, C, H, W) order under another shape.  kChannelsLast: it is the
+  // order of a 4-axis bottom's channels-last copy.  As shaped now.
+  enum View { kNotAView, kSameOrder, kChannelsLast };
+  virtual View AsView() const { return kNotAView; }
+  // A layer that can read its bottoms from in front of views: SetViews says per bottom whether it is
+  // now handed a blob whose channels-last copy holds the values in the order it expects.
+  virtual bool AcceptsViews() const { return false; }
+  virtual void SetViews(const std::vector<bool>& channels_last) {}
   // ---- running a pass in parts of its batch ----
   // PartSeconds: as shaped and fused now, about how long the layer takes for the whole batch, or 0 if
   // it cannot run for some of the images only (first_of_net: it reads the net's input, of which no

@@ -80,9 +80,15 @@ void PriorBoxLayer::Reshape(const vector<Blob*>& bottom, const vector<Blob*>& to
   top[0]->Reshape(vector<int>{1, 2, dim});
 }
 
-// Same expression shapes as the reference (float centre, int-truncated sizes,
-// `/ 2.` in double, one rounding to float per coordinate).
-void PriorBoxLayer::Compute(int layer_h, int layer_w, int img_h, int img_w, float* out) const {
+// Same expression shapes as the reference (float centre, int-truncated sizes, `/ 2.` in double, one rounding
+// to float per coordinate).  The boxes are written by the device: computed on the host they had to be uploaded per
+// layer, and where the storage had held a device blob before, its old values came down first (SSD300, one
+// image: four such round trips and six uploads, about 170 of 1020 us per pass).
+void PriorBoxLayer::Forward_gpu(const vector<Blob*>& bottom, const vector<Blob*>& top) {
+  Context& ctx = Context::Get();
+  const int layer_w = bottom[0]->width(), layer_h = bottom[0]->height();
+  const int img_w = (img_h_ == 0 || img_w_ == 0) ? bottom[1]->width() : img_w_;
+  const int img_h = (img_h_ == 0 || img_w_ == 0) ? bottom[1]->height() : img_h_;
   float step_w, step_h;
   if (step_w_ == 0 || step_h_ == 0) {
     step_w = static_cast<float>(img_w) / layer_w;
@@ -91,62 +97,49 @@ void PriorBoxLayer::Compute(int layer_h, int layer_w, int img_h, int img_w, floa
     step_w = step_w_;
     step_h = step_h_;
   }
-  const int dim = layer_h * layer_w * num_priors_ * 4;
-  int idx = 0;
-  auto emit = [&](float cx, float cy, float bw, float bh) {
-    out[idx++] = (cx - bw / 2.) / img_w;
-    out[idx++] = (cy - bh / 2.) / img_h;
-    out[idx++] = (cx + bw / 2.) / img_w;
-    out[idx++] = (cy + bh / 2.) / img_h;
-  };
-  for (int h = 0; h < layer_h; ++h) {
-    for (int w = 0; w < layer_w; ++w) {
-      const float cx = (w + offset_) * step_w;
-      const float cy = (h + offset_) * step_h;
-      for (size_t s = 0; s < min_sizes_.size(); ++s) {
-        const int min_size = static_cast<int>(min_sizes_[s]);
-        float bw, bh;
-        bw = bh = min_size;
-        emit(cx, cy, bw, bh);
-        if (!max_sizes_.empty()) {
-          const int max_size = static_cast<int>(max_sizes_[s]);
-          bw = bh = std::sqrt(static_cast<double>(min_size * max_size));
-          emit(cx, cy, bw, bh);
-        }
-        for (float ar : aspect_ratios_) {
-          if (std::fabs(ar - 1.) < 1e-6) continue;
-          bw = min_size * std::sqrt(ar);
-          bh = min_size / std::sqrt(ar);
-          emit(cx, cy, bw, bh);
-        }
-      }
+  std::vector<float> box_w, box_h;
+  for (size_t s = 0; s < min_sizes_.size(); ++s) {
+    const int min_size = static_cast<int>(min_sizes_[s]);
+    box_w.push_back(min_size);
+    box_h.push_back(min_size);
+    if (!max_sizes_.empty()) {
+      const int max_size = static_cast<int>(max_sizes_[s]);
+      box_w.push_back(std::sqrt(static_cast<double>(min_size * max_size)));
+      box_h.push_back(box_w.back());
+    }
+    for (float ar : aspect_ratios_) {
+      if (std::fabs(ar - 1.) < 1e-6) continue;
+      box_w.push_back(min_size * std::sqrt(ar));
+      box_h.push_back(min_size / std::sqrt(ar));
     }
   }
-  CHECK_EQ(idx, dim);
+  const int boxes = static_cast<int>(box_w.size());
+  const int dim = layer_h * layer_w * boxes * 4;
+  CHECK_EQ(2 * dim, top[0]->count());
+  const int rc = mcb200_prior_box(layer_h, layer_w, img_h, img_w, step_h, step_w, offset_, boxes, box_w.data(), box_h.data(),
+                                  variance_.data(), static_cast<int>(variance_.size()), clip_ ? 1 : 0,
+                                  top[0]->mutable_gpu_data(), ctx.stream_ptr());
+  if (rc != -2) {
+    KERNEL_CHECK(rc);
+    return;
+  }
+  // More boxes per cell than the kernel takes as arguments: on the host.
+  float* out = top[0]->mutable_cpu_data();
+  int idx = 0;
+  for (int cell = 0; cell < layer_h * layer_w; ++cell) {
+    const float cx = (cell % layer_w + offset_) * step_w;
+    const float cy = (cell / layer_w + offset_) * step_h;
+    for (int i = 0; i < boxes; ++i) {
+      out[idx++] = (cx - box_w[i] / 2.) / img_w;
+      out[idx++] = (cy - box_h[i] / 2.) / img_h;
+      out[idx++] = (cx + box_w[i] / 2.) / img_w;
+      out[idx++] = (cy + box_h[i] / 2.) / img_h;
+    }
+  }
   if (clip_) {
     for (int d = 0; d < dim; ++d) out[d] = std::min<float>(std::max<float>(out[d], 0.), 1.);
   }
-  float* var = out + dim;
-  if (variance_.size() == 1) {
-    for (int d = 0; d < dim; ++d) var[d] = variance_[0];
-  } else {
-    for (int d = 0; d < dim; ++d) var[d] = variance_[d % 4];
-  }
-}
-
-void PriorBoxLayer::Forward_gpu(const vector<Blob*>& bottom, const vector<Blob*>& top) {
-  const int layer_w = bottom[0]->width(), layer_h = bottom[0]->height();
-  const int img_w = (img_h_ == 0 || img_w_ == 0) ? bottom[1]->width() : img_w_;
-  const int img_h = (img_h_ == 0 || img_w_ == 0) ? bottom[1]->height() : img_h_;
-  const int key[4] = {layer_h, layer_w, img_h, img_w};
-  if (std::memcmp(key, cached_key_, sizeof(key)) != 0) {
-    cached_.resize(top[0]->count());
-    Compute(layer_h, layer_w, img_h, img_w, cached_.data());
-    std::memcpy(cached_key_, key, sizeof(key));
-  }
-  // The storage may be shared with other blobs between passes, so the values
-  // are written every time (a few hundred KB at most).
-  std::memcpy(top[0]->mutable_cpu_data(), cached_.data(), cached_.size() * sizeof(float));
+  for (int d = 0; d < dim; ++d) out[dim + d] = variance_[variance_.size() == 1 ? 0 : d % 4];
 }
 REGISTER_LAYER_CLASS(PriorBox);
 

@@ -361,6 +361,7 @@ class FlattenLayer : public Layer {
   const char* type() const override { return "Flatten"; }
   int ExactNumBottomBlobs() const override { return 1; }
   int ExactNumTopBlobs() const override { return 1; }
+  View AsView() const override { return kSameOrder; }
  protected:
   void Forward_gpu(const vector<Blob*>& bottom, const vector<Blob*>& top) override;
 };
@@ -373,6 +374,7 @@ class ReshapeLayer : public Layer {
   const char* type() const override { return "Reshape"; }
   int ExactNumBottomBlobs() const override { return 1; }
   int ExactNumTopBlobs() const override { return 1; }
+  View AsView() const override { return kSameOrder; }
  protected:
   void Forward_gpu(const vector<Blob*>& bottom, const vector<Blob*>& top) override;
   std::vector<int> copy_axes_;
@@ -388,8 +390,12 @@ class PermuteLayer : public Layer {
   const char* type() const override { return "Permute"; }
   int ExactNumBottomBlobs() const override { return 1; }
   int ExactNumTopBlobs() const override { return 1; }
+  View AsView() const override { return !need_permute_ ? kSameOrder : to_channels_last() ? kChannelsLast : kNotAView; }
  protected:
   void Forward_gpu(const vector<Blob*>& bottom, const vector<Blob*>& top) override;
+  bool to_channels_last() const {
+    return order_.size() == 4 && order_[0] == 0 && order_[1] == 2 && order_[2] == 3 && order_[3] == 1;
+  }
   std::vector<int> order_;
   bool need_permute_ = false;
 };
@@ -402,9 +408,13 @@ class ConcatLayer : public Layer {
   const char* type() const override { return "Concat"; }
   int MinBottomBlobs() const override { return 1; }
   int ExactNumTopBlobs() const override { return 1; }
+  bool AcceptsViews() const override { return rows_; }
+  void SetViews(const std::vector<bool>& channels_last) override { channels_last_ = channels_last; }
  protected:
   void Forward_gpu(const vector<Blob*>& bottom, const vector<Blob*>& top) override;
   int axis_ = 1;
+  bool rows_ = false;                  // fewer than four axes: always concatenated in (N, C, H, W) order
+  std::vector<bool> channels_last_;    // per bottom, see SetViews
 };
 
 // ---------------------------------------------------------------- detection
@@ -422,13 +432,10 @@ class PriorBoxLayer : public Layer {
   int ExactNumTopBlobs() const override { return 1; }
  protected:
   void Forward_gpu(const vector<Blob*>& bottom, const vector<Blob*>& top) override;
-  void Compute(int layer_h, int layer_w, int img_h, int img_w, float* out) const;
   std::vector<float> min_sizes_, max_sizes_, aspect_ratios_, variance_;
   bool flip_ = true, clip_ = false;
   int num_priors_ = 0, img_h_ = 0, img_w_ = 0;
   float step_h_ = 0, step_w_ = 0, offset_ = 0.5f;
-  std::vector<float> cached_;
-  int cached_key_[4] = {-1, -1, -1, -1};
 };
 
 // RPN proposals (src/layers/proposal_layer.cpp).  The reference accepts one

@@ -11,6 +11,13 @@ static void DeviceCopy(const float* src, float* dst, size_t count) {
   CUDA_CHECK(cudaMemcpyAsync(dst, src, count * sizeof(float), cudaMemcpyDeviceToDevice, Context::Get().stream()));
 }
 
+// The net may have given the top its bottom's storage: then the bottom's (N, C, H, W) copy is made current
+// before the top's becomes the only one, and nothing moves.
+static void CopyThrough(Blob* bottom, Blob* top) {
+  const float* src = bottom->gpu_data();
+  DeviceCopy(src, top->mutable_gpu_data(), bottom->count());
+}
+
 // ---------------------------------------------------------------- Input
 
 void InputLayer::LayerSetUp(const vector<Blob*>& bottom, const vector<Blob*>& top) {
@@ -61,7 +68,7 @@ void FlattenLayer::Reshape(const vector<Blob*>& bottom, const vector<Blob*>& top
 
 void FlattenLayer::Forward_gpu(const vector<Blob*>& bottom, const vector<Blob*>& top) {
   // The flattened order is the (N, C, H, W) order.
-  if (bottom[0] != top[0]) DeviceCopy(bottom[0]->gpu_data(), top[0]->mutable_gpu_data(), bottom[0]->count());
+  if (bottom[0] != top[0]) CopyThrough(bottom[0], top[0]);
 }
 REGISTER_LAYER_CLASS(Flatten);
 
@@ -121,7 +128,7 @@ void ReshapeLayer::Reshape(const vector<Blob*>& bottom, const vector<Blob*>& top
 }
 
 void ReshapeLayer::Forward_gpu(const vector<Blob*>& bottom, const vector<Blob*>& top) {
-  DeviceCopy(bottom[0]->gpu_data(), top[0]->mutable_gpu_data(), bottom[0]->count());
+  CopyThrough(bottom[0], top[0]);
 }
 REGISTER_LAYER_CLASS(Reshape);
 
@@ -155,10 +162,10 @@ void PermuteLayer::Reshape(const vector<Blob*>& bottom, const vector<Blob*>& top
 void PermuteLayer::Forward_gpu(const vector<Blob*>& bottom, const vector<Blob*>& top) {
   Context& ctx = Context::Get();
   if (!need_permute_) {
-    DeviceCopy(bottom[0]->gpu_data(), top[0]->mutable_gpu_data(), bottom[0]->count());
+    CopyThrough(bottom[0], top[0]);
     return;
   }
-  if (order_.size() == 4 && order_[0] == 0 && order_[1] == 2 && order_[2] == 3 && order_[3] == 1) {
+  if (to_channels_last()) {
     // (N, C, H, W) -> (N, H, W, C) is exactly the channels-last copy the
     // producing convolution already wrote.
     DeviceCopy(bottom[0]->gpu_data_nhwc(), top[0]->mutable_gpu_data(), bottom[0]->count());
@@ -200,6 +207,7 @@ void ConcatLayer::Reshape(const vector<Blob*>& bottom, const vector<Blob*>& top)
   }
   top[0]->Reshape(shape);
   CHECK_EQ(total, static_cast<long long>(top[0]->count()));
+  rows_ = num_axes < 4;
 }
 
 void ConcatLayer::Forward_gpu(const vector<Blob*>& bottom, const vector<Blob*>& top) {
@@ -227,11 +235,22 @@ void ConcatLayer::Forward_gpu(const vector<Blob*>& bottom, const vector<Blob*>& 
   const long long outer = top[0]->count(0, axis_);
   const long long inner = top[0]->count(axis_ + 1);
   const long long top_row = static_cast<long long>(top[0]->shape(axis_)) * inner;
+  std::vector<const float*> src;
+  std::vector<long long> cols;
+  for (size_t i = 0; i < bottom.size(); ++i) {
+    const bool last = i < channels_last_.size() && channels_last_[i];
+    src.push_back(last ? bottom[i]->gpu_data_nhwc() : bottom[i]->gpu_data());
+    cols.push_back(outer ? bottom[i]->count() / outer : 0);
+  }
+  const int rc = mcb200_concat_rows(static_cast<int>(src.size()), src.data(), cols.data(), outer, out, ctx.stream_ptr());
+  if (rc != -2) {
+    KERNEL_CHECK(rc);
+    return;
+  }
   long long offset = 0;
-  for (Blob* b : bottom) {
-    const long long cols = static_cast<long long>(b->shape(axis_)) * inner;
-    KERNEL_CHECK(mcb200_copy_2d(b->gpu_data(), cols, out + offset, top_row, outer, cols, ctx.stream_ptr()));
-    offset += cols;
+  for (size_t i = 0; i < src.size(); ++i) {
+    KERNEL_CHECK(mcb200_copy_2d(src[i], cols[i], out + offset, top_row, outer, cols[i], ctx.stream_ptr()));
+    offset += cols[i];
   }
 }
 REGISTER_LAYER_CLASS(Concat);

@@ -94,7 +94,8 @@ typedef struct mcb200_conv_plan {
   const float* res_ptr;
   int m_virtual;            /* halo mode: positions of the virtual output grid (rows widened by
                                (kw - 1) * dil_w); else m                            */
-  int strip_rows;           /* halo mode: pixels per activation load (128 + (kw - 1) * dil_w) */
+  int strip_rows;           /* pixels per activation load where they are not 128: halo mode's M tile (128 or 64)
+                               + (kw - 1) * dil_w, or the 64 of a 64-row M tile; else 0 */
 } __attribute__((aligned(64))) mcb200_conv_plan;
 
 /* Implicit-GEMM convolution on the tensor cores (tcgen05.mma kind::tf32,

@@ -48,6 +48,7 @@ namespace {
 using namespace sm100;
 
 constexpr int kBlockM = 128;
+constexpr int kSmallM = 64;                            // M tile of a launch too small for the chip, see small_tiles
 constexpr int kBlockK = 32;                            // fp32 elements = one 128-byte swizzle row
 constexpr int kBlockKHalf = 64;                        // bfloat16 elements of the same 128 bytes
 constexpr int kMmaPerBlock = 4;                        // 32-byte K steps of a swizzle row (K = 8 tf32 / 16 bf16)
@@ -84,7 +85,7 @@ struct ConvTcArgs {
   mcb200_epilogue ep;
   int* status;
   int tma_epilogue;  // output (and residual) meet the 16-byte rules of TMA tiles
-  int tile_rows;     // rows of an M tile: 128, or in row mode min(output width, 128)
+  int tile_rows;     // rows of an M tile: 128 or 64, in row mode min(output width, 128)
   int row_segments;  // row mode: M tiles per output row of an image (ceil(output width / tile_rows))
   int a_bytes;       // bytes one activation tile load delivers
   int stages;        // depth of the operand ring (2 .. kMaxStages)
@@ -277,8 +278,13 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   const int lane = threadIdx.x & 31;
   const int n_tiles = kMode == kModePhase ? args.phase_tiles * args.phase_stride_h * args.phase_stride_w
                                           : (args.cout + BN - 1) / BN;
+  // Rows of an M tile: with 64, tcgen05.mma runs at M = 64 and its accumulator lies in the first 16 lanes of
+  // each tensor-memory quadrant (row 16 * quadrant + lane).
+  constexpr bool kShortTiles = !kPair && (kMode == kModeMatrix || kMode == kModeIm2col || kMode == kModeHalo);
+  const int tile_m = kShortTiles ? args.tile_rows : kBlockM;
+  const int warp_rows = kShortTiles ? args.tile_rows >> 2 : 32;   // rows an epilogue warp owns: one quadrant's
   // Row mode: an M tile is (a segment of at most 128 pixels of) one output row of one image.
-  const int m_tiles = kMode == kModeRows ? (args.m / args.wo) * args.row_segments : (args.m + kBlockM - 1) / kBlockM;
+  const int m_tiles = kMode == kModeRows ? (args.m / args.wo) * args.row_segments : (args.m + tile_m - 1) / tile_m;
   // Row mode helpers: image row (n * ho + p) and first pixel of the segment of M tile mt.
   auto row_of = [&](int mt) { return mt / args.row_segments; };
   auto seg_start = [&](int mt) { return (mt % args.row_segments) * args.tile_rows; };
@@ -375,7 +381,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       const uint32_t a_bytes = static_cast<uint32_t>(args.a_bytes);
       for (int tile = worker; tile < num_tiles && alive; tile += workers) {
         const int mt = unit_to_mt(tile / n_tiles);
-        const int m0 = mt * kBlockM;
+        const int m0 = mt * tile_m;
         // The odd M tile out at the end of a paired launch has no pixels: its
         // CTA loads nothing, and the MMA computes rows nobody stores.
         const bool live = !kPair || mt < m_tiles;
@@ -426,7 +432,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             const int origin2 = args.group_cout > 0
                                     ? (((n_index * BN) / args.group_cout) * args.group_cin) & ~((kHalf ? 8 : 4) - 1)
                                     : 0;
-            const int v2 = mt2 * kBlockM;
+            const int v2 = mt2 * tile_m;
             if (kMode == kModeMatrix) {
               for (int cb = 0; cb < args.c_blocks; ++cb) tma_prefetch_2d(&map_a, origin2 + cb * kElemsK, v2);
             } else {
@@ -621,8 +627,10 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   } else if (warp == kWarpMma) {
     // ------------------------------------------------------------ MMA issuer
     if ((!kPair || rank == 0u) && elect_one()) {
-      constexpr uint32_t idesc = kHalf ? umma_idesc_bf16(kPair ? 2 * kBlockM : kBlockM, BN)
-                                       : umma_idesc_tf32(kPair ? 2 * kBlockM : kBlockM, BN);
+      constexpr uint32_t idesc_full = kHalf ? umma_idesc_bf16(kPair ? 2 * kBlockM : kBlockM, BN)
+                                            : umma_idesc_tf32(kPair ? 2 * kBlockM : kBlockM, BN);
+      constexpr uint32_t idesc_small = kHalf ? umma_idesc_bf16(kSmallM, BN) : umma_idesc_tf32(kSmallM, BN);
+      const uint32_t idesc = kShortTiles && tile_m == kSmallM ? idesc_small : idesc_full;
       RingPos pos;
       int local = 0;   // tiles done by this CTA
       bool alive = true;
@@ -782,11 +790,11 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       if (!cursor_next(ld, mt, col)) return;
       const int slot = ld_slot;
       if (++ld_slot == slots) ld_slot = 0;
-      mbar_expect_tx(&res_bar[ew][slot], kHalf ? 2048 : 4096);   // 32 x 32 bfloat16 or fp32
+      mbar_expect_tx(&res_bar[ew][slot], static_cast<uint32_t>(warp_rows) * (kHalf ? 64u : 128u));   // rows of 32 bfloat16 or fp32
       if (kMode == kModeRows) {
         tma_load_3d(&map_res, &res_bar[ew][slot], slot_ptr(slot), col, seg_start(mt) + quad * 32, row_of(mt));
       } else {
-        tma_load_3d(&map_res, &res_bar[ew][slot], slot_ptr(slot), col, mt * kBlockM + quad * 32, 0);
+        tma_load_3d(&map_res, &res_bar[ew][slot], slot_ptr(slot), col, mt * tile_m + quad * warp_rows, 0);
       }
     };
     const bool staged = args.tma_epilogue != 0;
@@ -841,9 +849,10 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         phase_y = phase / args.phase_stride_w;
         phase_x = phase - phase_y * args.phase_stride_w;
       }
-      // First output row (pixel) of this warp's 32-row slice, and how many of the 32 exist.
-      const int row0 = (kMode == kModeRows ? row_of(mt) * args.wo + seg_start(mt) : mt * kBlockM) + quad * 32;
-      const int rows_here = kMode == kModeRows ? min(args.tile_rows, args.wo - seg_start(mt)) - quad * 32 : args.m - row0;
+      // First output row (pixel) of this warp's slice of the tile, and how many of its rows exist.
+      const int row0 = (kMode == kModeRows ? row_of(mt) * args.wo + seg_start(mt) : mt * tile_m) + quad * warp_rows;
+      const int rows_here = kMode == kModeRows ? min(args.tile_rows, args.wo - seg_start(mt)) - quad * 32
+                                               : min(args.m - row0, warp_rows);
       // Row of the output matrix this lane stores in the plain-store epilogue, and whether it exists.
       int out_row = row0 + lane;
       bool row_ok = lane < rows_here;
@@ -1446,20 +1455,66 @@ int pick_cta_pair(int block_n, long long m, int k_iters) {
   return (block_n >= 128 && m > kBlockM && k_iters >= (block_n == 256 ? 16 : 17)) ? 1 : 0;
 }
 
+// Layers of a single image (or a few) have fewer tiles than the chip has SMs, and the time of one is the chain of its
+// k-iterations.  A K step of 128 x 64 costs the chain about 65 cycles at 256 -> 256 channels, 3 x 3, 14 x 14
+// (operand reads and the copies' writes share the shared-memory port), one of 64 x 32 about 52.  So where the tiles
+// all run at once anyway, cut them to 64 pixels and 64 or 32 columns: more SMs, each with a half or a third of the
+// bytes per iteration and half the epilogue.  The sums over K keep their order: the results are the same bits.
+// Returns whether the layer runs in 64-row tiles, with *block_n (and *pair = 0) set to match.
+// The cost model, in cycles: per K step (M + N) / 4, four steps per tap; the copies at 128 bytes per cycle, 0.4 of
+// them not hidden; 1500 per epilogue chunk of a warp.  Only up to one tile per SM: with more, ordinary tiles
+// fill the chip; and only for a tenth less by the model, which is no better than that.
+// Measured, one image: 3 x 3 at 256 channels on 14 x 14 17.3 -> 14.0 us, at 512 on 7 x 7 27.7 -> 21.9, 512 -> 512
+// on 19 x 19 in bfloat16 15.6 -> 13; per pass ResNet-50 629 -> 552, SSD300 in bfloat16 771 -> 687, MobileNet-v1
+// 216 -> 199; ResNet-50 at batch 16 in bfloat16 803 -> 788.
+bool small_tiles(int cout, long long m, int k_iters, int taps, int halo_rows, int* block_n, int* pair) {
+  const char* force = getenv("MCB200_BLOCK_M");   // "64" / "128": override for experiments and tests
+  const bool forced = force && atoi(force) == kSmallM;
+  const char* width = getenv("MCB200_BLOCK_N");
+  if (forced) {
+    *block_n = width && atoi(width) == 32 ? 32 : 64;
+    *pair = 0;
+    return true;
+  }
+  if (force || width || getenv("MCB200_CTA_PAIR")) return false;
+  auto tiles_of = [&](int bm, int bn) { return ((m + bm - 1) / bm) * ((cout + bn - 1) / bn); };
+  auto cost = [&](int bm, int bn, bool paired) {
+    const int b_rows = paired ? bn / 2 : bn;
+    double steps = taps * static_cast<double>(bm + b_rows);
+    if (bn > 64) steps = steps > 2.0 * taps * bn ? steps : 2.0 * taps * bn;   // the tensor pipe itself
+    return k_iters * (steps + 0.4 * (bm + halo_rows + taps * b_rows)) + 1500.0 * ((bn + 63) / 64);
+  };
+  if (tiles_of(kBlockM, *block_n) > 148) return false;
+  const double now = cost(kBlockM, *block_n, *pair != 0);
+  double best = 0.9 * now;
+  bool found = false;
+  for (int bn = 64; bn >= 32; bn /= 2) {
+    if (tiles_of(kSmallM, bn) > 148) break;
+    const double c = cost(kSmallM, bn, false);
+    if (c < best) {
+      best = c;
+      *block_n = bn;
+      *pair = 0;
+      found = true;
+    }
+  }
+  return found;
+}
+
 // Tile map for the staged epilogue over a row-major matrix with row pitch `ld`
-// (elements), 32 x 32 boxes: fp32 with the 128-byte swizzle, or bfloat16 (64-byte
+// (elements), boxes of 32 columns and an epilogue warp's rows (32 or 16): fp32 with the 128-byte swizzle, or bfloat16 (64-byte
 // box rows) with the 64-byte swizzle.  The rows are split as (group, row in
 // group): ordinary tiles use one group of all rows; row mode uses one group per
 // output row of an image so that a tile never spills into the next row.
 CUresult encode_tile_map(CUtensorMap* map, const void* base, bool half, int cols, int ld, long long rows_per_group,
-                         long long groups) {
+                         long long groups, int box_rows) {
   const DriverApi& api = driver_api();
   const cuuint64_t es = half ? 2 : 4;
   const cuuint64_t dims[3] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows_per_group),
                               static_cast<cuuint64_t>(groups)};
   const cuuint64_t strides[2] = {static_cast<cuuint64_t>(ld) * es,
                                  static_cast<cuuint64_t>(ld) * es * static_cast<cuuint64_t>(rows_per_group)};
-  const cuuint32_t box[3] = {32, 32, 1};
+  const cuuint32_t box[3] = {32, static_cast<cuuint32_t>(box_rows), 1};
   const cuuint32_t estr[3] = {1, 1, 1};
   return api.tiled(map, half ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
                    const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -1499,7 +1554,7 @@ cudaError_t launch_variant(const mcb200_conv_plan* plan, ConvTcArgs args, cudaSt
   }
   const long long m_tiles = kMode == kModeRows
                                 ? static_cast<long long>(plan->shape.n) * plan->shape.ho * args.row_segments
-                                : (static_cast<long long>(args.m) + kBlockM - 1) / kBlockM;   // halo: virtual positions
+                                : (static_cast<long long>(args.m) + args.tile_rows - 1) / args.tile_rows;   // halo: virtual positions
   const long long m_units = kPair ? (m_tiles + 1) / 2 : m_tiles;
   const long long n_tiles = kMode == kModePhase
                                 ? static_cast<long long>(args.phase_tiles) * args.phase_stride_h * args.phase_stride_w
@@ -1796,6 +1851,9 @@ int plan_core(const mcb200_conv_shape* s, const void* in, const void* packed_w, 
     }
   }
   const bool halo = plan->im2col == kModeHalo;
+  const bool small = !grouped && small_tiles(s->cout, plan->m_virtual, plan->k_iters, halo ? s->kw : 1, halo ? halo_w : 0,
+                                             &plan->block_n, &plan->cta_pair);
+  if (small) plan->strip_rows = kSmallM + (halo ? halo_w : 0);
 
   CUtensorMap* ma = reinterpret_cast<CUtensorMap*>(plan->tma_a);
   CUtensorMap* mb = reinterpret_cast<CUtensorMap*>(plan->tma_b);
@@ -1804,7 +1862,7 @@ int plan_core(const mcb200_conv_shape* s, const void* in, const void* packed_w, 
     // Plain row-major matrix [m, c] with row pitch c_stride.
     const cuuint64_t dims[2] = {static_cast<cuuint64_t>(s->c), static_cast<cuuint64_t>(plan->m)};
     const cuuint64_t strides[1] = {static_cast<cuuint64_t>(s->c_stride) * es};
-    const cuuint32_t box[2] = {static_cast<cuuint32_t>(kelems), kBlockM};
+    const cuuint32_t box[2] = {static_cast<cuuint32_t>(kelems), static_cast<cuuint32_t>(small ? kSmallM : kBlockM)};
     const cuuint32_t estr[2] = {1, 1};
     r = api.tiled(ma, dtype, 2, const_cast<void*>(in), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -1822,7 +1880,7 @@ int plan_core(const mcb200_conv_shape* s, const void* in, const void* packed_w, 
     const int upper[2] = {halo ? s->pad_w : s->pad_w - (s->kw - 1) * s->dil_w, s->pad_h - (s->kh - 1) * s->dil_h};
     const cuuint32_t estr[4] = {1, static_cast<cuuint32_t>(s->stride_w), static_cast<cuuint32_t>(s->stride_h), 1};
     r = api.im2col(ma, dtype, 4, const_cast<void*>(in), dims, strides, lower, upper,
-                   static_cast<cuuint32_t>(kelems), halo ? static_cast<cuuint32_t>(plan->strip_rows) : kBlockM, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                   static_cast<cuuint32_t>(kelems), static_cast<cuuint32_t>(plan->strip_rows ? plan->strip_rows : kBlockM), estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                    CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r == CUDA_SUCCESS) clear_small_tensor_flag(ma, pix * s->w * s->h * s->n);
   }
@@ -1941,13 +1999,17 @@ int launch_core(mcb200_conv_plan* plan, void* out, bool out_half, int out_ld, co
     a.ho = phases->grid_h;
     a.wo = phases->grid_w;
   }
+  const int halo_rows = plan->im2col == kModeHalo ? (plan->shape.kw - 1) * plan->shape.dil_w : 0;
+  const bool cut = plan->im2col == kModeMatrix || plan->im2col == kModeIm2col || plan->im2col == kModeHalo;
+  const bool small = cut && plan->strip_rows - halo_rows == kSmallM;
+  const int warp_rows = small ? kSmallM / 4 : kBlockM / 4;
   if (a.tma_epilogue) {
     const bool rows = plan->im2col == kModeRows;
     const long long per_group = rows ? plan->shape.wo : plan->m;
     const long long groups = rows ? static_cast<long long>(plan->shape.n) * plan->shape.ho : 1;
     if (plan->out_ptr != out || plan->out_ld != out_ld || plan->out_bf16 != a.out_half) {
       if (encode_tile_map(reinterpret_cast<CUtensorMap*>(plan->tma_out), out, out_half, plan->shape.cout, out_ld,
-                          per_group, groups) != CUDA_SUCCESS)
+                          per_group, groups, warp_rows) != CUDA_SUCCESS)
         return -4;
       plan->out_ptr = static_cast<const float*>(out);
       plan->out_ld = out_ld;
@@ -1955,14 +2017,14 @@ int launch_core(mcb200_conv_plan* plan, void* out, bool out_half, int out_ld, co
     }
     if (a.ep.residual && (plan->res_ptr != a.ep.residual || plan->res_ld != a.ep.residual_ld)) {
       if (encode_tile_map(reinterpret_cast<CUtensorMap*>(plan->tma_res), a.ep.residual, half, plan->shape.cout,
-                          a.ep.residual_ld, per_group, groups) != CUDA_SUCCESS)
+                          a.ep.residual_ld, per_group, groups, warp_rows) != CUDA_SUCCESS)
         return -5;
       plan->res_ptr = a.ep.residual;
       plan->res_ld = a.ep.residual_ld;
     }
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  a.tile_rows = plan->im2col == kModeRows ? (plan->shape.wo < kBlockM ? plan->shape.wo : kBlockM) : kBlockM;
+  a.tile_rows = plan->im2col == kModeRows ? (plan->shape.wo < kBlockM ? plan->shape.wo : kBlockM) : small ? kSmallM : kBlockM;
   a.row_segments = plan->im2col == kModeRows ? (plan->shape.wo + a.tile_rows - 1) / a.tile_rows : 1;
   a.a_bytes = (plan->im2col == kModeHalo ? plan->strip_rows : a.tile_rows) * kBlockK * 4;
   cudaError_t e = cudaErrorInvalidValue;
@@ -1977,6 +2039,11 @@ int launch_core(mcb200_conv_plan* plan, void* out, bool out_half, int out_ld, co
   e = mode == kModeIm2col ? launch_variant<BN, kModeIm2col, true, false>(plan, a, st)     \
       : mode == kModeHalo ? launch_variant<BN, kModeHalo, true, false>(plan, a, st)       \
                           : launch_variant<BN, kModeMatrix, true, false>(plan, a, st)
+#define MCB200_DISPATCH_NARROW(HALF)                                                      \
+  e = mode == kModeIm2col   ? launch_variant<32, kModeIm2col, false, HALF>(plan, a, st)   \
+      : mode == kModeHalo   ? launch_variant<32, kModeHalo, false, HALF>(plan, a, st)     \
+      : mode == kModeMatrix ? launch_variant<32, kModeMatrix, false, HALF>(plan, a, st)   \
+                            : cudaErrorInvalidValue
 #define MCB200_DISPATCH_HALF(BN, PAIR)                                                    \
   e = mode == kModeIm2col ? launch_variant<BN, kModeIm2col, PAIR, true>(plan, a, st)      \
       : mode == kModeHalo ? launch_variant<BN, kModeHalo, PAIR, true>(plan, a, st)        \
@@ -1991,6 +2058,7 @@ int launch_core(mcb200_conv_plan* plan, void* out, bool out_half, int out_ld, co
       }
     } else {
       switch (plan->block_n) {
+        case 32: MCB200_DISPATCH_NARROW(true); break;
         case 64: MCB200_DISPATCH_HALF(64, false); break;
         case 128: MCB200_DISPATCH_HALF(128, false); break;
         case 256: MCB200_DISPATCH_HALF(256, false); break;
@@ -2009,11 +2077,13 @@ int launch_core(mcb200_conv_plan* plan, void* out, bool out_half, int out_ld, co
     return static_cast<int>(e);
   }
   switch (plan->block_n) {
+    case 32: MCB200_DISPATCH_NARROW(false); break;
     case 64: MCB200_DISPATCH(64); break;
     case 128: MCB200_DISPATCH(128); break;
     case 256: MCB200_DISPATCH(256); break;
     default: return -3;
   }
+#undef MCB200_DISPATCH_NARROW
 #undef MCB200_DISPATCH_HALF
 #undef MCB200_DISPATCH_PAIR
 #undef MCB200_DISPATCH

@@ -390,8 +390,11 @@ detout_class_kernel(const float* __restrict__ loc, const float* __restrict__ con
   // The kept set is then iterated from "all": a box stays unless a box that stays suppresses it.  Bit i
   // is final once those in front of it are, so this ends in the walk's own set, after as many rounds as
   // the longest chain of suppressions is long.
+  // The bits of a list of up to 1024 have their place in the region if the limit is not above that; beyond it
+  // the region was sized for the keys, which a short list's bits may still fit in.
   const int words = (count + 31) >> 5;
-  if (!(eta < 1.f) && words <= 32) {
+  const bool bits_fit = static_cast<size_t>(words) * count * sizeof(uint32_t) <= class_region_bytes(p.num_priors, limit);
+  if (!(eta < 1.f) && words <= 32 && bits_fit) {
     uint32_t* suppress = region;
     const JaccardTest overlaps(p.nms_threshold);
     // A warp takes 32 rows x 32 columns at a time: lane = column, the rows are broadcasts.  (One thread

@@ -47,3 +47,37 @@ def test_selection_against_the_restatement(capi, gpu_engine, case):
         got = net.blob("detection_out").data.copy().reshape(-1, 7)
         assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
     net.close()
+
+
+def _against_the_restatement(capi, gpu_engine, feed, images, priors, classes, conf_thr, top_k, keep, nms_thr=0.45):
+    wl, port = pkg("workloads"), importlib.import_module("oracle.port")
+    b = wl.detection_head(batch=images, num_priors=priors, num_classes=classes, conf_thr=conf_thr, nms_thr=nms_thr, top_k=top_k,
+                          keep_top_k=keep)
+    want = port.detection_output(feed["loc"], feed["conf"], feed["prior"], classes, confidence_threshold=conf_thr,
+                                 nms_threshold=nms_thr, top_k=top_k, keep_top_k=keep)
+    net = capi.Net(gpu_engine, b.text(), None, from_buffer=True)
+    net.forward(**feed)
+    got = net.blob("detection_out").data.copy().reshape(-1, 7)
+    net.close()
+    assert got.shape == want.shape and np.array_equal(got.view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.parametrize("priors,top_k,passing", [
+    (3000, 2000, 900),       # bits of 104 KB, a region of 12 KB of keys: the warp's walk
+    (3000, 2000, 300),       # 12 000 bytes of bits in 12 000 bytes: the matrix, to the last byte
+    (3000, 2000, 301),
+    (1500, -1, 600),
+    (4096, -1, 1024),
+    (8732, 1100, 513),       # either side of the region of a full SSD head
+    (8732, 1100, 514),
+])
+def test_short_lists_under_a_long_limit(capi, gpu_engine, priors, top_k, passing):
+    """Beyond 1024 candidates per class no room for their overlap bits is set aside: a list that turns out short
+    takes the bit matrix only where its bits fit into the keys' place."""
+    feed = pkg("workloads").detection_head_input(1, priors, 2, seed=priors, peaked=True)
+    rng = np.random.default_rng(passing)
+    scores = 0.4 * rng.permutation(priors) / priors
+    pick = rng.permutation(priors)[:passing]
+    scores[pick] = 0.5 + 0.4 * np.arange(passing) / passing
+    feed["conf"].reshape(priors, 2)[:, 1] = scores
+    _against_the_restatement(capi, gpu_engine, feed, 1, priors, 2, 0.45, top_k, 200)

@@ -697,7 +697,8 @@ extern "C" int mcb200_detout_part(const mcb200_detout_params* p, int batch, int 
   ws.class_count += static_cast<size_t>(first_image) * p->num_classes;
   ws.rows += static_cast<size_t>(first_image) * ws.max_rows * 7;
   ws.image_count += first_image;
-  const int padded = det::next_pow2(ws.per_class);
+  // (Two keys at least: the boxes behind them are read 16 bytes at a time.)
+  const int padded = ws.per_class > 1 ? det::next_pow2(ws.per_class) : 2;
   const size_t smem = class_kernel_smem(*p, padded);
   if (smem > 220 * 1024) return -7;
   static size_t class_configured[64], image_configured[64];

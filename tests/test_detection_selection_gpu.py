@@ -81,3 +81,10 @@ def test_short_lists_under_a_long_limit(capi, gpu_engine, priors, top_k, passing
     scores[pick] = 0.5 + 0.4 * np.arange(passing) / passing
     feed["conf"].reshape(priors, 2)[:, 1] = scores
     _against_the_restatement(capi, gpu_engine, feed, 1, priors, 2, 0.45, top_k, 200)
+
+
+@pytest.mark.parametrize("images,priors,classes,top_k,keep", [(2, 40, 3, 1, 5), (1, 1, 2, 400, 200), (1, 1, 21, -1, -1), (3, 300, 2, 1, 1)])
+def test_a_single_candidate_per_class(capi, gpu_engine, images, priors, classes, top_k, keep):
+    """The smallest list: one key, behind which the boxes still start on 16 bytes."""
+    feed = pkg("workloads").detection_head_input(images, priors, classes, seed=top_k + priors, peaked=True)
+    _against_the_restatement(capi, gpu_engine, feed, images, priors, classes, 0.01, top_k, keep)

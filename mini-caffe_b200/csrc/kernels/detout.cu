@@ -305,7 +305,7 @@ detout_class_kernel(const float* __restrict__ loc, const float* __restrict__ con
   const int limit = ws.per_class;
   const int t = threadIdx.x, lane = t & 31;
   int* out_count = ws.class_count + static_cast<size_t>(image) * p.num_classes + cls;
-  if (cls == p.background_label_id) {
+  if (cls == p.background_label_id || limit == 0) {   // top_k 0 keeps nothing: there is no key to cut at
     if (t == 0) *out_count = 0;
     return;
   }

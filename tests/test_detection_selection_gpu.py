@@ -88,3 +88,10 @@ def test_a_single_candidate_per_class(capi, gpu_engine, images, priors, classes,
     """The smallest list: one key, behind which the boxes still start on 16 bytes."""
     feed = pkg("workloads").detection_head_input(images, priors, classes, seed=top_k + priors, peaked=True)
     _against_the_restatement(capi, gpu_engine, feed, images, priors, classes, 0.01, top_k, keep)
+
+
+@pytest.mark.parametrize("images,top_k,keep", [(1, 0, 200), (3, 0, -1), (2, 0, 0), (2, 400, 0), (9, 1, 0)])
+def test_limits_of_nothing(capi, gpu_engine, images, top_k, keep):
+    """top_k 0 (no candidate of any class) and keep_top_k 0 (no detection of any image): a placeholder row per image."""
+    feed = pkg("workloads").detection_head_input(images, 700, 4, seed=images, peaked=True)
+    _against_the_restatement(capi, gpu_engine, feed, images, 700, 4, 0.01, top_k, keep)

@@ -221,14 +221,15 @@ void ProposalLayer::Forward_gpu(const vector<Blob*>& bottom, const vector<Blob*>
   const long long image_bytes = 4 * n * static_cast<long long>(sizeof(float));
   const int per_part = from_host ? static_cast<int>(std::min<long long>(batch, (4 << 20) / image_bytes + 1)) : batch;
   const bool in_parts = per_part < batch;
+  // (The buffer first: a new one is cleared on the compute stream, and the copies wait for what is queued there.)
+  float* copied_deltas = from_host ? input_copy_.Reserve(static_cast<size_t>(batch) * (5 * n + 3)) : nullptr;
   cudaStream_t copies = in_parts ? ctx.CopiesBegin() : ctx.stream();
   const float* info = nullptr;
   const float* deltas = nullptr;
   const float* scores = nullptr;
   long long score_stride = 2 * n;
-  float* copied_deltas = nullptr;
   if (from_host) {
-    deltas = copied_deltas = input_copy_.Reserve(static_cast<size_t>(batch) * (5 * n + 3));
+    deltas = copied_deltas;
     info = info_on_host;
     scores = scores_on_host + n;
     if (batch > 1) {
@@ -340,8 +341,9 @@ void DetectionOutputLayer::Forward_gpu(const vector<Blob*>& bottom, const vector
   const size_t image_bytes = (loc_floats + conf_floats) * sizeof(float);
   const int small_part = static_cast<int>(std::min<size_t>(batch, (3 << 20) / image_bytes + 1));
   const bool in_parts = from_host && small_part < batch;
-  cudaStream_t copies = in_parts ? ctx.CopiesBegin() : ctx.stream();
+  // (The buffer first, see Proposal.)
   float* copied = from_host ? input_copy_.Reserve(batch * (loc_floats + conf_floats + 4)) : nullptr;
+  cudaStream_t copies = in_parts ? ctx.CopiesBegin() : ctx.stream();
   float* copied_conf = copied + (batch * loc_floats + 3) / 4 * 4;
   const float* loc = from_host ? copied : bottom[0]->gpu_data();
   const float* conf = from_host ? copied_conf : bottom[1]->gpu_data();

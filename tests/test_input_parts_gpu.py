@@ -71,3 +71,26 @@ def test_parts_give_the_bits_of_the_whole(monkeypatch, capi, gpu_engine, batch, 
     assert (whole[4] != whole[7]).any()                     # the slopes alone
     for i in range(0, len(whole), 3):
         assert (whole[i + 1] == whole[i + 2]).all()
+
+
+@pytest.mark.parametrize("kind", ["proposal", "detection_output"])
+def test_detection_layers_whose_buffers_grow(capi, gpu_engine, kind):
+    """Input in parts into a buffer that is new in the same pass (the first pass, and each larger batch): its zero
+    fill comes before the copies.  The pass that follows reads the same input from the device."""
+    wl = pkg("workloads")
+    if kind == "proposal":
+        b, top = wl.proposal(), "rois"
+        images = [wl.proposal_input(seed=i)[0] for i in range(40)]
+        feeds = {k: np.concatenate([f[k] for f in images]) for k in images[0]}
+    else:
+        b, top = wl.detection_head(1, 8732, 21, 0.01, 0.45, 400, 200), "detection_out"
+        feeds = wl.detection_head_input(40, 8732, 21, 0, peaked=True)
+    net = capi.Net(gpu_engine, b.text(), None, from_buffer=True)
+    for batch in (10, 22, 40):
+        net.forward(**{k: v if k == "prior" else v[:batch] for k, v in feeds.items()})
+        first = net.blob(top).data.copy()
+        net.forward()
+        again = net.blob(top).data.copy()
+        assert first.shape == again.shape and np.array_equal(first.view(np.uint32), again.view(np.uint32))
+        assert set(first.reshape(first.shape[0], -1)[:, 0]) == set(range(batch))
+    net.close()

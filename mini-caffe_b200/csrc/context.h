@@ -10,6 +10,8 @@
 
 #include <cuda_runtime.h>
 
+#include <exception>
+
 #include "caffe/base.hpp"
 
 #define CUDA_CHECK(expr)                                                            \
@@ -71,6 +73,23 @@ class Context {
   int* status_dev_;
   int* status_host_;
   void Release();
+};
+
+// For a scope that queues work on blobs' host memory itself.  A blob that only its host copy is current of is
+// released without a wait, so when an exception leaves the scope that work ends before it does.
+class DrainOnError {
+ public:
+  explicit DrainOnError(Context& ctx) : ctx_(ctx), before_(std::uncaught_exceptions()) {}
+  ~DrainOnError() {
+    if (std::uncaught_exceptions() == before_) return;
+    try { ctx_.Sync(); } catch (...) {}
+  }
+  DrainOnError(const DrainOnError&) = delete;
+  DrainOnError& operator=(const DrainOnError&) = delete;
+
+ private:
+  Context& ctx_;
+  const int before_;
 };
 
 // Number of usable CUDA devices (0 without a driver); cached.

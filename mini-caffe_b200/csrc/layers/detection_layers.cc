@@ -214,6 +214,7 @@ void ProposalLayer::Forward_gpu(const vector<Blob*>& bottom, const vector<Blob*>
   // and its three numbers the decode kernel reads in place (32 images of 63 x 38 cells and 15 anchors:
   // 18 MB + 5 MB over PCIe, 430 us of the call's time).
   const long long n = static_cast<long long>(num_anchors_) * params_.height * params_.width;
+  const DrainOnError drain(ctx);
   const float* scores_on_host = host_scores_.Take(*bottom[0]);
   const float* deltas_on_host = host_deltas_.Take(*bottom[1]);
   const float* info_on_host = host_info_.Take(*bottom[2]);
@@ -334,6 +335,7 @@ void DetectionOutputLayer::Forward_gpu(const vector<Blob*>& bottom, const vector
   // New scores and locations are copied in parts of some images on the copy stream, each part's
   // kernels running while the next is on its way (32 images of 8732 priors and 21 classes: 28 MB, 510 us
   // of PCIe transfer).
+  const DrainOnError drain(ctx);
   const float* loc_on_host = host_loc_.Take(*bottom[0]);
   const float* conf_on_host = host_conf_.Take(*bottom[1]);
   const bool from_host = loc_on_host && conf_on_host;

@@ -94,3 +94,22 @@ def test_detection_layers_whose_buffers_grow(capi, gpu_engine, kind):
         assert first.shape == again.shape and np.array_equal(first.view(np.uint32), again.view(np.uint32))
         assert set(first.reshape(first.shape[0], -1)[:, 0]) == set(range(batch))
     net.close()
+
+
+def test_input_is_released_after_a_refusal(capi, gpu_engine):
+    """A head that the kernels refuse (its keys and boxes need more shared memory than an SM has) when its input is
+    on the way already: the error comes back, the copies have ended, and the memory serves the next net."""
+    wl = pkg("workloads")
+    for _ in range(3):
+        feed = wl.detection_head_input(12, 26000, 2, 1, peaked=True)
+        net = capi.Net(gpu_engine, wl.detection_head(12, 26000, 2, 0.01, 0.45, 4000, 200).text(), None, from_buffer=True)
+        with pytest.raises(capi.CaffeError):
+            net.forward(**feed)
+        net.close()
+        feed = wl.detection_head_input(12, 26000, 2, 2, peaked=True)
+        net = capi.Net(gpu_engine, wl.detection_head(12, 26000, 2, 0.01, 0.45, 400, 200).text(), None, from_buffer=True)
+        net.forward(**feed)
+        first = net.blob("detection_out").data.copy()
+        net.forward()
+        assert np.array_equal(first.view(np.uint32), net.blob("detection_out").data.view(np.uint32))
+        net.close()

@@ -91,8 +91,11 @@ void DeconvolutionLayer::Forward_gpu(const vector<Blob*>& bottom, const vector<B
     const bool few = phase_weights != 0 && mcb200_deconv_as_window_conv(&s, &window) == 0 && window.cout <= 64;
     const Form form = few ? kWindow : phase_weights != 0 ? kPhases : kSpread;
     const unsigned long long wv = blobs_[0]->host_version() + (bias_term_ ? blobs_[1]->host_version() : 0);
-    if (wv != weight_version_ || form != form_) {
+    // (A single input pixel has a phase per tap, a larger input one per step of the stride: another set of rows.)
+    const bool pixel = s.h == 1 && s.w == 1 && s.pad_h == 0 && s.pad_w == 0;
+    if (wv != weight_version_ || form != form_ || pixel != packed_for_pixel_) {
       form_ = form;
+      packed_for_pixel_ = pixel;
       if (form == kPhases) {
         float* packed = packed_weights_.Reserve(phase_weights);
         KERNEL_CHECK(mcb200_deconv_tc_pack_weights(&s, blobs_[0]->gpu_data(), packed, ctx.stream_ptr()));
@@ -151,7 +154,7 @@ void DeconvolutionLayer::Forward_gpu(const vector<Blob*>& bottom, const vector<B
     if (form == kWindow) result = scratch_.Reserve(static_cast<size_t>(window.n) * window.ho * window.wo * window.cout);
     KERNEL_CHECK(mcb200_conv_tc_launch_flags(&slot.plan.conv, result, 0, shape.cout, &ep, flags, ctx.status_word(), ctx.stream_ptr()));
     if (form == kWindow) {
-      const int phases_h = s.h == 1 && s.w == 1 && s.pad_h == 0 && s.pad_w == 0 ? s.kh : s.stride_h;
+      const int phases_h = pixel ? s.kh : s.stride_h;
       const int phases_w = window.cout / s.cout / phases_h;
       KERNEL_CHECK(mcb200_depth_to_space(result, out, s.n, window.ho, window.wo, phases_h, phases_w, s.cout, s.ho, s.wo,
                                          ctx.stream_ptr()));

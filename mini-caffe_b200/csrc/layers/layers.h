@@ -509,7 +509,8 @@ class DeconvolutionLayer : public Layer {
   // filter over the input spread `stride` apart over zeros (mcb200_deconv_as_conv_shape); the direct kernel takes what is left (more padding than the filter
   // reaches).
   enum Form { kPhases, kWindow, kSpread };
-  Form form_ = kSpread;
+  Form form_ = kSpread;              // what the packed weights are laid out for
+  bool packed_for_pixel_ = false;
   bool constants_settled_ = false;   // weights and tail arrays are those of the launch before
   unsigned long long weight_version_ = 0;
   DeviceScratch flipped_weights_, packed_weights_, scratch_;

@@ -80,3 +80,32 @@ def test_batch_statistics_with_scale_and_relu_behind(capi, gpu_engine, shape):
         scale = np.abs(mean) / np.sqrt(var + 1e-5) * gamma.reshape(1, -1, 1, 1) + 1.0
         assert (np.abs(got - want) <= 1e-5 * np.abs(want) + 4 * 2.0 ** -24 * scale).all(), float(np.abs(got - want).max())
     net.close()
+
+
+@pytest.mark.parametrize("cout", [68, 3], ids=["phases", "window"])
+@pytest.mark.parametrize("k,stride", [(4, 1), (3, 2), (4, 4), (2, 1)])
+def test_one_net_from_a_pixel_to_a_map_and_back(capi, gpu_engine, cout, k, stride):
+    """A single input pixel runs with a phase per tap, a larger input with one per step of the stride: the weights
+    packed for the one do not serve the other.  Nor do they for two inputs of one layer."""
+    wl = pkg("workloads")
+    rng = np.random.default_rng(k)
+    weight = (rng.standard_normal((12, cout, k, k)) / np.sqrt(12)).astype(np.float32)
+    bias = rng.standard_normal(cout).astype(np.float32)
+    b = wl.NetBuilder("deconv")
+    b.input([("data", (2, 12, 1, 1)), ("more", (2, 12, 1, 1))])
+    b.raw("up", "Deconvolution", ["data", "more"], ["up", "up_more"],
+          "convolution_param { num_output: %d kernel_size: %d stride: %d }" % (cout, k, stride))
+    net = capi.Net(gpu_engine, b.text(), None, from_buffer=True)
+    net.set_params({"up_0": weight, "up_1": bias})
+    for (h, w), (h2, w2) in (((1, 1), (1, 1)), ((2, 2), (2, 2)), ((1, 1), (1, 1)), ((1, 1), (3, 2)), ((3, 2), (1, 1))):
+        feed = {"data": rng.standard_normal((2, 12, h, w)).astype(np.float32),
+                "more": rng.standard_normal((2, 12, h2, w2)).astype(np.float32)}
+        for _ in range(2):
+            net.forward(**feed)
+            for x, top in (("data", "up"), ("more", "up_more")):
+                got = net.blob(top).data.copy()
+                want = torch.nn.functional.conv_transpose2d(torch.from_numpy(feed[x]).double(), torch.from_numpy(weight).double(),
+                                                            torch.from_numpy(bias).double(), stride).numpy()
+                assert got.shape == want.shape
+                assert (np.abs(got - want) <= 2e-2 + 1e-2 * np.abs(want)).all(), (h, w, h2, w2, top)
+    net.close()

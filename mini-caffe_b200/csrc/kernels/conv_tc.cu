@@ -134,19 +134,15 @@ struct ConvTcArgs {
 // full, MMAs issued and committed); 3: epilogue warp 0 (per tile: accumulator ready, tile stored);
 // 4: the same warp inside its chunk loop, five stamps per 32 x 32 chunk of a launch with the staged
 // epilogue (chunk begins, accumulator in registers, slot free / residual there, tail computed and
-// written to the slot, store issued); 5: the CTA (entered, set up, previous launch complete, roles done, left).
+// written to the slot, store issued).  A reader's buffer holds these five rows and no more.
 #ifdef MCB200_CONV_TRACE
 constexpr int kTraceSlots = 2048;
-constexpr int kTraceRoles = 6;
+constexpr int kTraceRoles = 5;
 __device__ long long g_conv_trace[kTraceRoles * kTraceSlots];
 #define MCB200_TRACE_DECL int trace_n = 0
 #define MCB200_TRACE(role)                                                                         \
   do {                                                                                             \
     if (blockIdx.x == 0 && trace_n < kTraceSlots) g_conv_trace[(role) * kTraceSlots + trace_n++] = clock64(); \
-  } while (0)
-#define MCB200_TRACE_CTA(i)                                                                        \
-  do {                                                                                             \
-    if (blockIdx.x == 0 && threadIdx.x == 0) g_conv_trace[5 * kTraceSlots + (i)] = clock64();      \
   } while (0)
 #define MCB200_TRACE_CHUNK_DECL int trace_c = 0
 #define MCB200_TRACE_CHUNK()                                                                       \
@@ -157,7 +153,6 @@ __device__ long long g_conv_trace[kTraceRoles * kTraceSlots];
 #else
 #define MCB200_TRACE_DECL
 #define MCB200_TRACE(role)
-#define MCB200_TRACE_CTA(i)
 #define MCB200_TRACE_CHUNK_DECL
 #define MCB200_TRACE_CHUNK()
 #endif
@@ -246,7 +241,6 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   constexpr bool kScatter = kMode == kModeHalo || kMode == kModePhase;      // output rows are not one box
   using Plan = SmemPlan<BN, kMode, kPair>;
   constexpr int kElemsK = kHalf ? kBlockKHalf : kBlockK;   // channels per k-iteration
-  MCB200_TRACE_CTA(0);
   const int stages = args.stages;
   const int slots = args.slots;
   const long long wait_limit = args.wait_limit;   // SM cycles a barrier wait may take before the CTA gives up
@@ -345,11 +339,9 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   // not wait for its end: the weight producer fills the ring and the epilogue warps their first table
   // while the activations are still being computed.  (At batch 1 a layer is a few microseconds of
   // latency, one of which was the weights' first trip out of DRAM and 0.4 the table's.)
-  MCB200_TRACE_CTA(1);
   grid_launch_dependents();
   const bool early = args.constants_settled != 0;
   if (!early || (warp != kWarpLoadB && warp < kFirstEpilogueWarp)) grid_dependency_wait();
-  MCB200_TRACE_CTA(2);
   const bool usable = !kPair || tmem_base == 0u;
   if (!usable && threadIdx.x == 0) abort_flag = 1;
   // Cluster-window addresses of rank 0's shared barriers.
@@ -1211,7 +1203,6 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   } else {
     __syncthreads();
   }
-  MCB200_TRACE_CTA(3);
   if (warp == kWarpMma) {
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, 2 * BN);
@@ -2499,7 +2490,7 @@ extern "C" int mcb200_conv_rows_plan(const mcb200_conv_shape* s, const float* pa
   return 0;
 }
 
-// With -DMCB200_CONV_TRACE: copies the cycle stamps of the last traced launches' CTA 0 (6 roles x
+// With -DMCB200_CONV_TRACE: copies the cycle stamps of the last traced launches' CTA 0 (5 roles x
 // 2048 slots, see MCB200_TRACE above) to `out` and clears the device array; returns the number
 // of values per role, or 0 when the library was built without the trace.
 extern "C" int mcb200_conv_trace_read(long long* out) {

@@ -178,9 +178,12 @@ channel_batch_stats_kernel(const float* __restrict__ x, long long per_channel, i
 }
 
 // The same for channels-last data.  A block takes a run of pixels; its threads are 4-channel groups x
-// pixel lanes, so that a warp reads whole rows.  Sums of x - x0 and (x - x0)^2, x0 being the channel's
-// value at the first pixel, lose nothing to the mean's size; a thread's fp32 sums run over a few
-// dozen values, everything above them is added in double and in a fixed order.  The block that
+// pixel lanes, so that a warp reads whole rows.  Eight values at a time, still in registers, give their mean and the sum of
+// squared deviations from it in fp32, which loses nothing to the mean's size; these are merged in double and in a fixed order, relative
+// to the channel's value at the first pixel: (x0 - mean)^2 is at most the number of values times the variance, so
+// that however far x0 lies off, the subtraction at the end costs that number of units of 2^-53.  (Sums of x - x0 and
+// (x - x0)^2 in fp32 were off by 1e-4 of the variance with x0 200 standard deviations from the mean, as a
+// corner pixel under zero padding may be.)  The block that
 // finishes last adds the blocks' sums.  (One block per channel reading a float of every pixel: 240 us
 // for 64 channels of 65536 pixels, which are 16.8 MB.)
 constexpr int kStatsThreads = 256;
@@ -206,33 +209,33 @@ channel_batch_stats_nhwc_kernel(const float* __restrict__ x, long long pixels, i
       const float4* column = reinterpret_cast<const float4*>(x) + q0 + q;
       const float4 base = column[0];
       for (long long p = first + lane; p < end;) {
-        float4 s = make_float4(0.f, 0.f, 0.f, 0.f), s2 = s;
-        for (int i = 0; i < 4 && p < end; ++i) {
-          // eight rows in flight; rows beyond the run stand in as x0, which adds nothing
-          float4 v[8];
+        // eight rows in flight
+        float4 v[8];
+        const long long left = (end - p + rows - 1) / rows;
+        const int count = left < 8 ? static_cast<int>(left) : 8;
 #pragma unroll
-          for (int u = 0; u < 8; ++u, p += rows) v[u] = p < end ? column[p * quads] : base;
+        for (int u = 0; u < 8; ++u, p += rows) v[u] = u < count ? column[p * quads] : base;
+        auto merge = [&](auto value, float x0, int j) {
+          float total = 0.f;
+#pragma unroll
+          for (int u = 0; u < 8; ++u) total += u < count ? value(u) : 0.f;
+          const float mean = total / static_cast<float>(count);
+          float rest = 0.f, squares = 0.f;       // of the deviations; `rest` is what the rounding of `mean` left
 #pragma unroll
           for (int u = 0; u < 8; ++u) {
-            const float a = v[u].x - base.x, b = v[u].y - base.y, c = v[u].z - base.z, d = v[u].w - base.w;
-            s.x += a;
-            s.y += b;
-            s.z += c;
-            s.w += d;
-            s2.x = fmaf(a, a, s2.x);
-            s2.y = fmaf(b, b, s2.y);
-            s2.z = fmaf(c, c, s2.z);
-            s2.w = fmaf(d, d, s2.w);
+            const float d = u < count ? value(u) - mean : 0.f;
+            rest += d;
+            squares = fmaf(d, d, squares);
           }
-        }
-        sum[0] += s.x;
-        sum[1] += s.y;
-        sum[2] += s.z;
-        sum[3] += s.w;
-        sum[4] += s2.x;
-        sum[5] += s2.y;
-        sum[6] += s2.z;
-        sum[7] += s2.w;
+          const double off = static_cast<double>(mean) - static_cast<double>(x0);
+          // sum of (x - x0) and of (x - x0)^2 = squares + 2 off rest + count off^2
+          sum[j] += static_cast<double>(rest) + count * off;
+          sum[4 + j] += static_cast<double>(squares) + off * (2. * static_cast<double>(rest) + count * off);
+        };
+        merge([&](int u) { return v[u].x; }, base.x, 0);
+        merge([&](int u) { return v[u].y; }, base.y, 1);
+        merge([&](int u) { return v[u].z; }, base.z, 2);
+        merge([&](int u) { return v[u].w; }, base.w, 3);
       }
     }
 #pragma unroll

@@ -109,3 +109,31 @@ def test_one_net_from_a_pixel_to_a_map_and_back(capi, gpu_engine, cout, k, strid
                 assert got.shape == want.shape
                 assert (np.abs(got - want) <= 2e-2 + 1e-2 * np.abs(want)).all(), (h, w, h2, w2, top)
     net.close()
+
+
+@pytest.mark.parametrize("shape,outlier,mean", [
+    ((16, 8, 64, 64), 60.0, 0.0), ((16, 8, 64, 64), -200.0, 0.0), ((16, 8, 64, 64), 200.0, 1000.0),
+    ((2, 1032, 9, 7), 50.0, -30.0), ((3, 4, 5, 5), 5.0, 0.0), ((1, 4, 1, 2), 1.0, 7.0), ((7, 12, 11, 13), 0.0, 4096.0),
+], ids=str)
+def test_batch_statistics_behind_a_first_pixel_far_from_the_mean(capi, gpu_engine, shape, outlier, mean):
+    """Every channel's first value lies `outlier` standard deviations from the others' mean, as under a zero border.
+    The bound is that of y = x * scale + shift alone, with exact statistics: four roundings in the layer's scale, six
+    in its shift, one in the result, each 2^-24 of its value."""
+    wl = pkg("workloads")
+    rng = np.random.default_rng(shape[1])
+    x = (rng.standard_normal(shape) + mean).astype(np.float32)
+    x[0, :, 0, 0] = mean + outlier
+    b = wl.NetBuilder("bn")
+    b.input([("data", shape)])
+    b.raw("pool", "Pooling", ["data"], ["x"], "pooling_param { pool: MAX kernel_size: 1 stride: 1 }")     # channels last from here
+    b.raw("bn", "BatchNorm", ["x"], ["x"], "batch_norm_param { use_global_stats: false }")
+    net = capi.Net(gpu_engine, b.text(), None, from_buffer=True)
+    net.forward(data=x)
+    got = net.blob("x").data.copy()
+    net.close()
+    d = x.astype(np.float64)
+    centre, var = d.mean(axis=(0, 2, 3), keepdims=True), d.var(axis=(0, 2, 3), keepdims=True)
+    std = np.sqrt(var + 1e-5)
+    want = (d - centre) / std
+    bound = 2.0 ** -24 * (4 * np.abs(d) / std + 6 * np.abs(centre) / std + np.abs(want) + 1)
+    assert (np.abs(got - want) <= bound).all(), float((np.abs(got - want) / bound).max())

@@ -372,14 +372,14 @@ void Net::PlaceMemory() {
   for (int b = 0; b < num_blobs; ++b) {
     if (plan.visible[b]) last_use[b] = num_steps;
   }
-  // Steps that run part by part come back to their blobs for every part: none of these hands its
-  // storage to a later step of the same group.
-  std::vector<int> held;
+  // Steps that run part by part hand storage on among themselves like any others: a blob that only they read is
+  // done with, image by image, before the next part writes there again.  A blob that a later step or the caller
+  // reads collects its images over all parts: it takes nobody's storage inside the group.  (With every blob of the
+  // group on storage of its own, MobileNet-v1 at batch 64 held 1105 MB, so 614, run whole 606; ResNet-50 1447, 1084 and
+  // 877.)
+  std::vector<bool> collects(num_blobs, false);
   for (int s = 1; s < plan.parts_end; ++s) {
-    for (int b : plan.steps[s].top_ids) {
-      last_use[b] = std::max(last_use[b], plan.parts_end - 1);
-      held.push_back(b);
-    }
+    for (int b : plan.steps[s].top_ids) collects[b] = last_use[b] >= plan.parts_end;
   }
 
   // ---- greedy storage sharing ----
@@ -407,10 +407,11 @@ void Net::PlaceMemory() {
         continue;
       }
     }
-    for (Blob* t : step.tops) {
+    for (size_t i = 0; i < step.tops.size(); ++i) {
+      Blob* t = step.tops[i];
       if (std::find(step.bottoms.begin(), step.bottoms.end(), t) != step.bottoms.end()) continue;  // in place
       t->ResetMemory();
-      need.push_back(std::make_pair(static_cast<size_t>(t->count()), t));
+      if (!collects[step.top_ids[i]]) need.push_back(std::make_pair(static_cast<size_t>(t->count()), t));
     }
     std::sort(need.begin(), need.end(),
               [](const std::pair<size_t, Blob*>& a, const std::pair<size_t, Blob*>& b) { return a.first > b.first; });
@@ -421,9 +422,7 @@ void Net::PlaceMemory() {
         retired.erase(it);
       }
     }
-    std::vector<int> done = step.bottom_ids;
-    if (s == plan.parts_end - 1) done.insert(done.end(), held.begin(), held.end());
-    for (int b : done) {
+    for (int b : step.bottom_ids) {
       if (!released[b] && last_use[b] <= s) {
         released[b] = true;
         retired.insert(std::make_pair(static_cast<size_t>(blobs_[b]->capacity()), blobs_[b].get()));

@@ -113,3 +113,26 @@ def test_input_is_released_after_a_refusal(capi, gpu_engine):
         net.forward()
         assert np.array_equal(first.view(np.uint32), net.blob("detection_out").data.view(np.uint32))
         net.close()
+
+
+def test_parts_share_storage(monkeypatch, capi, gpu_engine):
+    """A chain run part by part takes the storage of the same chain run whole, and at most one more of its largest
+    blob: the one that collects the parts' results."""
+    torch = pytest.importorskip("torch")
+    wl = pkg("workloads")
+    b = wl.mobilenet_v1(64)
+    weights, feed = wl.init_params(b.params, 0), wl.normal_image_input(64, 224, 0)
+    used = {}
+    for parts in (1, 8):
+        monkeypatch.setenv("MCB200_INPUT_PARTS", str(parts))
+        gpu_engine.memory_pool_clear()
+        before = torch.cuda.mem_get_info()[0]
+        net = capi.Net(gpu_engine, b.text(), None, from_buffer=True)
+        net.set_params(weights)
+        net.forward(**feed)
+        used[parts] = before - torch.cuda.mem_get_info()[0]
+        largest = max(blob.count for _, blob in net.blobs()) * 4
+        net.close()
+    gpu_engine.memory_pool_clear()
+    assert largest < used[1]
+    assert used[8] <= used[1] + largest + (4 << 20), used

@@ -82,17 +82,21 @@ void DeconvolutionLayer::Forward_gpu(const vector<Blob*>& bottom, const vector<B
                                         ctx.stream_ptr()));
       continue;
     }
-    // Phase by phase where the kernel takes the shape (strides up to 4, no groups, no dilation, a
+    // (A single input pixel has a phase per tap, a larger input one per step of the stride: another set of rows.)
+    const bool pixel = s.h == 1 && s.w == 1 && s.pad_h == 0 && s.pad_w == 0;
+    // Stride 1 is a convolution as it stands: nothing to spread, one phase, and the convolution's own tile modes are
+    // quicker than phase mode (256 -> 256 channels, 4 x 4, on 8 x 38 x 38 pixels: 86 and 76 us per pass) and need
+    // no pass behind them (64 -> 64, 3 x 3, on 8 x 64 x 64: 60 us with all phases in one tile, 37 so).
+    const bool plain = s.stride_h == 1 && s.stride_w == 1 && !pixel;
+    // Else phase by phase where the kernel takes the shape (strides up to 4, no groups, no dilation, a
     // channel count that is a multiple of four), all phases in one N tile when they have few channels
     // between them (64 -> 3 channels on 64 x 32 x 32 pixels: 57 us by phases of three columns each, 20 us
     // so); else as the convolution of the spread input.
     const size_t phase_weights = mcb200_deconv_tc_packed_weight_count(&s);
     mcb200_conv_shape window;
     const bool few = phase_weights != 0 && mcb200_deconv_as_window_conv(&s, &window) == 0 && window.cout <= 64;
-    const Form form = few ? kWindow : phase_weights != 0 ? kPhases : kSpread;
+    const Form form = plain ? kSpread : few ? kWindow : phase_weights != 0 ? kPhases : kSpread;
     const unsigned long long wv = blobs_[0]->host_version() + (bias_term_ ? blobs_[1]->host_version() : 0);
-    // (A single input pixel has a phase per tap, a larger input one per step of the stride: another set of rows.)
-    const bool pixel = s.h == 1 && s.w == 1 && s.pad_h == 0 && s.pad_w == 0;
     if (wv != weight_version_ || form != form_ || pixel != packed_for_pixel_) {
       form_ = form;
       packed_for_pixel_ = pixel;

@@ -137,3 +137,23 @@ def test_batch_statistics_behind_a_first_pixel_far_from_the_mean(capi, gpu_engin
     want = (d - centre) / std
     bound = 2.0 ** -24 * (4 * np.abs(d) / std + 6 * np.abs(centre) / std + np.abs(want) + 1)
     assert (np.abs(got - want) <= bound).all(), float((np.abs(got - want) / bound).max())
+
+
+@pytest.mark.parametrize("c,hw,cout,k,pad", [(64, 18, 68, 3, 1), (64, 18, 8, 3, 1), (40, 14, 12, 4, 0), (12, 9, 72, 2, 1), (36, 17, 5, 5, 2)])
+def test_stride_one_is_the_convolution(capi, gpu_engine, c, hw, cout, k, pad):
+    """A deconvolution of stride 1 runs as the convolution with the reversed filter: the same bits."""
+    wl = pkg("workloads")
+    rng = np.random.default_rng(c)
+    x = rng.standard_normal((2, c, hw, hw)).astype(np.float32)
+    weight = (rng.standard_normal((c, cout, k, k)) / np.sqrt(c)).astype(np.float32)
+    got = []
+    for kind, w, p in (("Deconvolution", weight, pad), ("Convolution", weight.transpose(1, 0, 2, 3)[:, :, ::-1, ::-1], k - 1 - pad)):
+        b = wl.NetBuilder("stride_one")
+        b.input([("data", x.shape)])
+        b.raw("up", kind, ["data"], ["up"], "convolution_param { num_output: %d kernel_size: %d pad: %d bias_term: false }" % (cout, k, p))
+        net = capi.Net(gpu_engine, b.text(), None, from_buffer=True)
+        net.set_params({"up_0": np.ascontiguousarray(w)})
+        net.forward(data=x)
+        got.append(net.blob("up").data.copy())
+        net.close()
+    assert got[0].shape == got[1].shape and np.array_equal(got[0].view(np.uint32), got[1].view(np.uint32))

@@ -177,113 +177,155 @@ channel_batch_stats_kernel(const float* __restrict__ x, long long per_channel, i
   }
 }
 
-// The same for channels-last data.  A block takes a run of pixels; its threads are 4-channel groups x
-// pixel lanes, so that a warp reads whole rows.  Eight values at a time, still in registers, give their mean and the sum of
-// squared deviations from it in fp32, which loses nothing to the mean's size; these are merged in double and in a fixed order, relative
-// to the channel's value at the first pixel: (x0 - mean)^2 is at most the number of values times the variance, so
-// that however far x0 lies off, the subtraction at the end costs that number of units of 2^-53.  (Sums of x - x0 and
-// (x - x0)^2 in fp32 were off by 1e-4 of the variance with x0 200 standard deviations from the mean, as a
-// corner pixel under zero padding may be.)  The block that
-// finishes last adds the blocks' sums.  (One block per channel reading a float of every pixel: 240 us
-// for 64 channels of 65536 pixels, which are 16.8 MB.)
+// The same for channels-last data.  A block takes a run of pixels; its threads are 4-channel groups x pixel lanes, so
+// that a warp reads whole rows.  Eight values at a time, still in registers, give their mean and the sum of squared
+// deviations from it in fp32, which loses nothing to the mean's size; these are merged in double and in a fixed order,
+// relative to the channel's value x0 at the first pixel.  (x0 - mean)^2 is at most the number of values times the
+// variance, so however far x0 lies off, the subtraction at the end costs that number of units of 2^-53.  (Sums of
+// x - x0 and (x - x0)^2 in fp32 were off by 1e-4 of the variance with x0 200 standard deviations from the mean, as a
+// corner pixel under zero padding may be.)  The block that finishes last adds the runs' sums.  (One block per channel
+// reading a float of every pixel: 240 us for 64 channels of 65536 pixels, which are 16.8 MB.)
 constexpr int kStatsThreads = 256;
-constexpr int kStatsBlocks = 128;    // the last block adds as many sums per channel, sixteen loads in flight
+constexpr int kStatsBlocks = 128;    // runs of pixels; as many sums per channel are added, sixteen loads in flight
+// Channels side by side in a block (in groups of 4).  More are spread over blocks of their own (blockIdx.x), and their
+// sums added by a launch of its own unless there is one run only.  (Added by the block that finishes last: 2048
+// channels on 16 x 7 x 7 pixels 97 us per pass where it is 57, 4096 on 2 x 14 x 14 127 and 47; a block per channel took 92 and 85.)
+constexpr int kStatsQuads = 64;
+
+struct StatsResult {
+  float eps;
+  const float* then_scale;
+  const float* then_shift;
+  float* scale;
+  float* shift;
+};
+
+// The layer's scale and shift from the sums of x - x0 and (x - x0)^2 over `pixels` values.
+__device__ __forceinline__ void store_batch_stats(const StatsResult& r, int c, float x0, double s, double s2, long long pixels) {
+  const double off = s / static_cast<double>(pixels);
+  const float mean = static_cast<float>(static_cast<double>(x0) + off);
+  const float var = static_cast<float>(fmax(s2 / static_cast<double>(pixels) - off * off, 0.));
+  const float inv_std = 1.f / sqrtf(var + r.eps);
+  const float ts = r.then_scale ? r.then_scale[c] : 1.f;
+  r.scale[c] = inv_std * ts;
+  r.shift[c] = fmaf(-mean * inv_std, ts, r.then_shift ? r.then_shift[c] : 0.f);
+}
+
+// Sixteen runs' sums of a channel, from run b0 on.
+__device__ __forceinline__ void add_runs(const double* partial, int b0, int runs, int channels, int c, double* s, double* s2) {
+  double v[16], v2[16];
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    const bool in = b0 + j < runs;
+    v[j] = in ? __ldcg(partial + static_cast<size_t>(b0 + j) * 2 * channels + c) : 0.;
+    v2[j] = in ? __ldcg(partial + static_cast<size_t>(b0 + j) * 2 * channels + channels + c) : 0.;
+  }
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    *s += v[j];
+    *s2 += v2[j];
+  }
+}
 
 __global__ void __launch_bounds__(kStatsThreads, 1)
-channel_batch_stats_nhwc_kernel(const float* __restrict__ x, long long pixels, int channels, float eps,
-                                const float* __restrict__ then_scale, const float* __restrict__ then_shift,
-                                unsigned* __restrict__ arrived, double* __restrict__ partial, float* __restrict__ scale,
-                                float* __restrict__ shift) {
+channel_batch_stats_nhwc_kernel(const float* __restrict__ x, long long pixels, int channels, unsigned* __restrict__ arrived,
+                                double* __restrict__ partial, const StatsResult result) {
   __shared__ double lanes[kStatsThreads][8];
   __shared__ bool last;
   const int quads = channels >> 2;
-  const long long per_block = (pixels + gridDim.x - 1) / gridDim.x;
-  const long long first = blockIdx.x * per_block, end = min(first + per_block, pixels);
-  double* mine = partial + static_cast<size_t>(blockIdx.x) * 2 * channels;
-  for (int q0 = 0; q0 < quads; q0 += kStatsThreads) {
-    const int width = min(quads - q0, kStatsThreads);       // groups handled side by side
-    const int rows = kStatsThreads / width;                 // pixel lanes
-    const int q = threadIdx.x % width, lane = threadIdx.x / width;
-    double sum[8] = {0., 0., 0., 0., 0., 0., 0., 0.};
-    if (lane < rows) {
-      const float4* column = reinterpret_cast<const float4*>(x) + q0 + q;
-      const float4 base = column[0];
-      for (long long p = first + lane; p < end;) {
-        // eight rows in flight
-        float4 v[8];
-        const long long left = (end - p + rows - 1) / rows;
-        const int count = left < 8 ? static_cast<int>(left) : 8;
+  const int q0 = blockIdx.x * kStatsQuads;
+  const int width = min(quads - q0, kStatsQuads);         // groups handled side by side
+  const int rows = kStatsThreads / width;                 // pixel lanes
+  const int q = threadIdx.x % width, lane = threadIdx.x / width;
+  const long long per_block = (pixels + gridDim.y - 1) / gridDim.y;
+  const long long first = blockIdx.y * per_block, end = min(first + per_block, pixels);
+  double sum[8] = {0., 0., 0., 0., 0., 0., 0., 0.};
+  if (lane < rows && first + lane < end) {
+    const float4* column = reinterpret_cast<const float4*>(x) + q0 + q;
+    const float4 base = column[0];
+    const float4* row = column + (first + lane) * quads;
+    const long long step = static_cast<long long>(rows) * quads;
+    auto merge = [&](auto value, int count, float part, float x0, int j) {
+      float total = 0.f;
 #pragma unroll
-        for (int u = 0; u < 8; ++u, p += rows) v[u] = u < count ? column[p * quads] : base;
-        auto merge = [&](auto value, float x0, int j) {
-          float total = 0.f;
+      for (int u = 0; u < 8; ++u) total += u < count ? value(u) : 0.f;
+      const float mean = total * part;
+      float rest = 0.f, squares = 0.f;       // of the deviations; `rest` is what the rounding of `mean` left
 #pragma unroll
-          for (int u = 0; u < 8; ++u) total += u < count ? value(u) : 0.f;
-          const float mean = total / static_cast<float>(count);
-          float rest = 0.f, squares = 0.f;       // of the deviations; `rest` is what the rounding of `mean` left
-#pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            const float d = u < count ? value(u) - mean : 0.f;
-            rest += d;
-            squares = fmaf(d, d, squares);
-          }
-          const double off = static_cast<double>(mean) - static_cast<double>(x0);
-          // sum of (x - x0) and of (x - x0)^2 = squares + 2 off rest + count off^2
-          sum[j] += static_cast<double>(rest) + count * off;
-          sum[4 + j] += static_cast<double>(squares) + off * (2. * static_cast<double>(rest) + count * off);
-        };
-        merge([&](int u) { return v[u].x; }, base.x, 0);
-        merge([&](int u) { return v[u].y; }, base.y, 1);
-        merge([&](int u) { return v[u].z; }, base.z, 2);
-        merge([&](int u) { return v[u].w; }, base.w, 3);
+      for (int u = 0; u < 8; ++u) {
+        const float d = u < count ? value(u) - mean : 0.f;
+        rest += d;
+        squares = fmaf(d, d, squares);
       }
-    }
+      const double off = static_cast<double>(mean) - static_cast<double>(x0);
+      const double moved = count * off;
+      // sums of (x - x0) and of (x - x0)^2 = squares + 2 off rest + count off^2
+      sum[j] += static_cast<double>(rest) + moved;
+      sum[4 + j] += fma(off, fma(2., static_cast<double>(rest), moved), static_cast<double>(squares));
+    };
+    auto take = [&](int count, float part) {
+      float4 v[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) lanes[threadIdx.x][j] = sum[j];
-    __syncthreads();
-    for (int i = threadIdx.x; i < width * 8; i += kStatsThreads) {
-      const int group = i >> 3, j = i & 7;
-      double total = 0.;
-      for (int r = 0; r < rows; ++r) total += lanes[r * width + group][j];
-      mine[(j >> 2) * channels + (q0 + group) * 4 + (j & 3)] = total;
+      for (int u = 0; u < 8; ++u) v[u] = u < count ? row[u * step] : base;
+      merge([&](int u) { return v[u].x; }, count, part, base.x, 0);
+      merge([&](int u) { return v[u].y; }, count, part, base.y, 1);
+      merge([&](int u) { return v[u].z; }, count, part, base.z, 2);
+      merge([&](int u) { return v[u].w; }, count, part, base.w, 3);
+      row += 8 * step;
+    };
+    long long left = (end - first - lane + rows - 1) / rows;
+    for (; left >= 8; left -= 8) take(8, 0.125f);          // eight rows in flight
+    if (left > 0) take(static_cast<int>(left), 1.f / static_cast<float>(left));
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) lanes[threadIdx.x][j] = sum[j];
+  __syncthreads();
+  double* mine = partial + static_cast<size_t>(blockIdx.y) * 2 * channels;
+  for (int i = threadIdx.x; i < width * 8; i += kStatsThreads) {
+    const int group = i >> 3, j = i & 7;
+    double total = 0.;
+    for (int r = 0; r < rows; ++r) total += lanes[r * width + group][j];
+    mine[(j >> 2) * channels + (q0 + group) * 4 + (j & 3)] = total;
+  }
+  const bool one_run = gridDim.y == 1;      // each block has its channels' sums already
+  if (gridDim.x > 1 && !one_run) return;
+  __syncthreads();
+  if (!one_run) {
+    // (One thread's fence covers the block's writes, which the barrier orders before it; a fence by all
+    // of them costs tens of microseconds.)
+    if (threadIdx.x == 0) {
+      __threadfence();
+      last = atomicAdd(arrived, 1u) == gridDim.y - 1;
+      __threadfence();
     }
     __syncthreads();
+    if (!last) return;
   }
-  // (One thread's fence covers the block's writes, which the barrier orders before it; a fence by all
-  // of them costs tens of microseconds.)
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    last = atomicAdd(arrived, 1u) == gridDim.x - 1;
-    __threadfence();
-  }
-  __syncthreads();
-  if (!last) return;
-  for (int c = threadIdx.x; c < channels; c += kStatsThreads) {
+  for (int c = q0 * 4 + threadIdx.x; c < (q0 + width) * 4; c += kStatsThreads) {
     double s = 0., s2 = 0.;
-    for (unsigned b0 = 0; b0 < gridDim.x; b0 += 16) {
-      double v[16], v2[16];
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const bool in = b0 + j < gridDim.x;
-        v[j] = in ? __ldcg(partial + static_cast<size_t>(b0 + j) * 2 * channels + c) : 0.;
-        v2[j] = in ? __ldcg(partial + static_cast<size_t>(b0 + j) * 2 * channels + channels + c) : 0.;
-      }
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        s += v[j];
-        s2 += v2[j];
-      }
-    }
-    const double off = s / static_cast<double>(pixels);
-    const float mean = static_cast<float>(static_cast<double>(x[c]) + off);
-    const float var = static_cast<float>(fmax(s2 / static_cast<double>(pixels) - off * off, 0.));
-    const float inv_std = 1.f / sqrtf(var + eps);
-    const float ts = then_scale ? then_scale[c] : 1.f;
-    scale[c] = inv_std * ts;
-    shift[c] = fmaf(-mean * inv_std, ts, then_shift ? then_shift[c] : 0.f);
+    for (int b0 = 0; b0 < static_cast<int>(gridDim.y); b0 += 16) add_runs(partial, b0, gridDim.y, channels, c, &s, &s2);
+    store_batch_stats(result, c, x[c], s, s2, pixels);
   }
-  if (threadIdx.x == 0) *arrived = 0u;
+  if (threadIdx.x == 0 && !one_run) *arrived = 0u;
+}
+
+// The runs' sums of many channels: a thread takes sixteen runs of a channel, a block 32 channels.
+__global__ void __launch_bounds__(kStatsThreads)
+add_batch_stats_kernel(const float* __restrict__ x, long long pixels, int channels, const double* __restrict__ partial, int runs,
+                       const StatsResult result) {
+  __shared__ double sums[2][kStatsBlocks / 16][32];
+  const int c = blockIdx.x * 32 + (threadIdx.x & 31), slice = threadIdx.x >> 5;
+  double s = 0., s2 = 0.;
+  if (c < channels && slice * 16 < runs) add_runs(partial, slice * 16, runs, channels, c, &s, &s2);
+  sums[0][slice][threadIdx.x & 31] = s;
+  sums[1][slice][threadIdx.x & 31] = s2;
+  __syncthreads();
+  if (slice > 0 || c >= channels) return;
+  for (int j = 1; j < kStatsBlocks / 16; ++j) {
+    s += sums[0][j][threadIdx.x];
+    s2 += sums[1][j][threadIdx.x];
+  }
+  store_batch_stats(result, c, x[c], s, s2, pixels);
 }
 
 // [n][grid_h][grid_w][stride_h][stride_w][c] -> [n][out_h][out_w][c], positions beyond the output dropped.
@@ -479,13 +521,21 @@ extern "C" int mcb200_channel_batch_stats_nhwc(const float* x, long long count, 
   if ((reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(workspace) & 15)) return -2;
   if (count == 0) return 0;
   const long long pixels = count / channels;
-  // Fewer blocks when a thread would not even get eight values.
+  const int groups = (channels / 4 + kStatsQuads - 1) / kStatsQuads;
+  // Fewer runs when a thread would not even get eight values, or the groups of channels fill the chip by themselves.
   const long long useful = (count / 4 + 8 * kStatsThreads - 1) / (8 * kStatsThreads);
-  const int blocks = static_cast<int>(useful < 1 ? 1 : useful > kStatsBlocks ? kStatsBlocks : useful);
-  channel_batch_stats_nhwc_kernel<<<blocks, kStatsThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-      x, pixels, channels, eps, then_scale, then_shift, static_cast<unsigned*>(workspace),
-      reinterpret_cast<double*>(static_cast<char*>(workspace) + 256), scale, shift);
+  const long long most = useful < kStatsBlocks ? useful : kStatsBlocks;
+  const int runs = static_cast<int>(most <= groups ? 1 : most / groups);
+  double* partial = reinterpret_cast<double*>(static_cast<char*>(workspace) + 256);
+  const StatsResult result = {eps, then_scale, then_shift, scale, shift};
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  channel_batch_stats_nhwc_kernel<<<dim3(groups, runs), kStatsThreads, 0, st>>>(x, pixels, channels, static_cast<unsigned*>(workspace),
+                                                                               partial, result);
   count_launch();
+  if (groups > 1 && runs > 1) {
+    add_batch_stats_kernel<<<(channels + 31) / 32, kStatsThreads, 0, st>>>(x, pixels, channels, partial, runs, result);
+    count_launch();
+  }
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -113,7 +113,8 @@ def test_one_net_from_a_pixel_to_a_map_and_back(capi, gpu_engine, cout, k, strid
 
 @pytest.mark.parametrize("shape,outlier,mean", [
     ((16, 8, 64, 64), 60.0, 0.0), ((16, 8, 64, 64), -200.0, 0.0), ((16, 8, 64, 64), 200.0, 1000.0),
-    ((2, 1032, 9, 7), 50.0, -30.0), ((3, 4, 5, 5), 5.0, 0.0), ((1, 4, 1, 2), 1.0, 7.0), ((7, 12, 11, 13), 0.0, 4096.0),
+    ((2, 1032, 9, 7), 50.0, -30.0), ((3, 260, 41, 40), 30.0, 0.0), ((9, 2048, 7, 7), 20.0, 3.0), ((64, 4096, 1, 1), 7.0, 0.0),
+    ((2, 512, 1, 1), 1.0, 0.0), ((3, 4, 5, 5), 5.0, 0.0), ((1, 4, 1, 2), 1.0, 7.0), ((7, 12, 11, 13), 0.0, 4096.0),
 ], ids=str)
 def test_batch_statistics_behind_a_first_pixel_far_from_the_mean(capi, gpu_engine, shape, outlier, mean):
     """Every channel's first value lies `outlier` standard deviations from the others' mean, as under a zero border.

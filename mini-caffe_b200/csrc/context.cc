@@ -1,5 +1,6 @@
 #include "context.h"
 
+#include <atomic>
 #include <mutex>
 
 namespace caffe {
@@ -82,6 +83,21 @@ cudaStream_t Context::CopiesBegin() {
 void Context::CopiesArrived() {
   CUDA_CHECK(cudaEventRecord(event_, copy_stream_));
   CUDA_CHECK(cudaStreamWaitEvent(stream_, event_, 0));
+}
+
+static const int kMaxDevices = 64;
+static std::atomic<int> g_passes[kMaxDevices];
+
+int Context::passes_in_flight() const {
+  return device_ >= 0 && device_ < kMaxDevices ? g_passes[device_].load(std::memory_order_relaxed) : 1;
+}
+
+PassInFlight::PassInFlight(int device) : device_(device) {
+  if (device_ >= 0 && device_ < kMaxDevices) g_passes[device_].fetch_add(1, std::memory_order_relaxed);
+}
+
+PassInFlight::~PassInFlight() {
+  if (device_ >= 0 && device_ < kMaxDevices) g_passes[device_].fetch_sub(1, std::memory_order_relaxed);
 }
 
 void Context::Sync() {

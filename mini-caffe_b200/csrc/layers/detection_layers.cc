@@ -220,7 +220,7 @@ void ProposalLayer::Forward_gpu(const vector<Blob*>& bottom, const vector<Blob*>
   const float* info_on_host = host_info_.Take(*bottom[2]);
   const bool from_host = scores_on_host && deltas_on_host && info_on_host;
   const long long image_bytes = 4 * n * static_cast<long long>(sizeof(float));
-  const int per_part = from_host ? static_cast<int>(std::min<long long>(batch, (4 << 20) / image_bytes + 1)) : batch;
+  const int per_part = from_host && ctx.passes_in_flight() == 1 ? static_cast<int>(std::min<long long>(batch, (4 << 20) / image_bytes + 1)) : batch;
   const bool in_parts = per_part < batch;
   // (The buffer first: a new one is cleared on the compute stream, and the copies wait for what is queued there.)
   float* copied_deltas = from_host ? input_copy_.Reserve(static_cast<size_t>(batch) * (5 * n + 3)) : nullptr;
@@ -342,7 +342,7 @@ void DetectionOutputLayer::Forward_gpu(const vector<Blob*>& bottom, const vector
   const size_t loc_floats = bottom[0]->count() / batch, conf_floats = bottom[1]->count() / batch;
   const size_t image_bytes = (loc_floats + conf_floats) * sizeof(float);
   const int small_part = static_cast<int>(std::min<size_t>(batch, (3 << 20) / image_bytes + 1));
-  const bool in_parts = from_host && small_part < batch;
+  const bool in_parts = from_host && small_part < batch && ctx.passes_in_flight() == 1;
   // (The buffer first, see Proposal.)
   float* copied = from_host ? input_copy_.Reserve(batch * (loc_floats + conf_floats + 4)) : nullptr;
   cudaStream_t copies = in_parts ? ctx.CopiesBegin() : ctx.stream();

@@ -587,13 +587,15 @@ void Net::Forward(bool reshape) {
   }
   Context& ctx = Context::Get();
   ctx.Activate();
+  const PassInFlight in_flight(ctx.device());
   Profiler* profiler = Profiler::Get();
   const bool profiling = profiler->running();
   // A plan's first pass is bound by the host, which allocates, packs weights and builds each launch's descriptors
   // (a set per part): the input arrives long before the kernels that read it are queued.  It runs whole.  First passes
   // of a MobileNet-v1 in parts and whole, blocks from the pool: batch 64 2.79 and 2.57 ms, batch 128 4.20 and 3.91.
-  const bool in_parts = plan.parts > 1 && plan.ran && !profiling && plan.parts_input->shape() == plan.parts_shape &&
-                        plan.parts_input->data() && plan.parts_input->data()->host_only();
+  const bool in_parts = plan.parts > 1 && plan.ran && ctx.passes_in_flight() == 1 && !profiling &&
+                        plan.parts_input->shape() == plan.parts_shape && plan.parts_input->data() &&
+                        plan.parts_input->data()->host_only();
   for (size_t s = 0; s < plan.steps.size(); ++s) {
     NetStep& step = plan.steps[s];
     if (in_parts && s == 1) {

@@ -136,3 +136,43 @@ def test_parts_share_storage(monkeypatch, capi, gpu_engine):
     gpu_engine.memory_pool_clear()
     assert largest < used[1]
     assert used[8] <= used[1] + largest + (4 << 20), used
+
+
+def test_nets_on_several_threads(monkeypatch, capi, gpu_engine):
+    """Passes that meet on the device copy their input whole, one that is alone in parts: the same bits, whichever a
+    pass happens to be."""
+    import threading
+    wl = pkg("workloads")
+    b = _net(wl, 24, 48)
+    weights = wl.init_params(b.params, seed=3, bn_identity=False)
+    monkeypatch.setenv("MCB200_INPUT_PARTS", "4")
+    d = wl.detection_head(24, 4000, 9, 0.01, 0.45, 200, 100)
+    feeds = [{"data": np.random.default_rng(i).standard_normal((24, 3, 48, 48)).astype(np.float32)} for i in range(3)]
+    heads = [wl.detection_head_input(24, 4000, 9, i, peaked=True) for i in range(3)]
+
+    def passes(seed, rounds, out):
+        gpu_engine.set_mode(True, 0)
+        net, head = (capi.Net(gpu_engine, x.text(), None, from_buffer=True) for x in (b, d))
+        net.set_params(weights)
+        for i in range(rounds):
+            k = (seed + i) % 3
+            net.forward(**feeds[k])
+            head.forward(**heads[k])
+            out.append((k, net.blob("pool5").data.copy(), head.blob("detection_out").data.copy()))
+        net.close()
+        head.close()
+
+    alone = []
+    passes(0, 3, alone)
+    want = {k: (p, q) for k, p, q in alone}
+    results = [[] for _ in range(3)]
+    threads = [threading.Thread(target=passes, args=(i, 12, results[i])) for i in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for got in results:
+        assert len(got) == 12
+        for k, p, q in got:
+            assert np.array_equal(p.view(np.uint32), want[k][0].view(np.uint32))
+            assert np.array_equal(q.view(np.uint32), want[k][1].view(np.uint32))

@@ -37,16 +37,17 @@ struct Workspace {
   float4* boxes;                 // [batch][n]     decoded boxes, proposal order
   float* scores;                 // [batch][score_ld]
   uint32_t* score_keys;          // [batch][score_ld]   ascending keys of the descending scores
-  float4* kept_boxes;            // [batch][post], then the areas; used when they do not fit in shared memory
+  float4* kept_boxes;            // [batch][kept], then the areas; used when they do not fit in shared memory
   int n, k;
+  int kept;                      // boxes an image can keep: the smaller of post_nms_topn and k
   int score_ld;                  // floats between two images' scores: rows start on 16 bytes
 };
 
 size_t align_up(size_t v) { return (v + 255) & ~static_cast<size_t>(255); }
 
 // Bytes of one image's kept list: boxes, then areas.
-__host__ __device__ inline size_t kept_bytes(int post_nms_topn) {
-  return (static_cast<size_t>(post_nms_topn) * (sizeof(float4) + sizeof(float)) + 15) & ~static_cast<size_t>(15);
+__host__ __device__ inline size_t kept_bytes(int kept) {
+  return (static_cast<size_t>(kept) * (sizeof(float4) + sizeof(float)) + 15) & ~static_cast<size_t>(15);
 }
 
 size_t carve(const mcb200_proposal_params& p, int batch, char* base, Workspace* ws) {
@@ -60,11 +61,12 @@ size_t carve(const mcb200_proposal_params& p, int batch, char* base, Workspace* 
   Workspace w;
   w.n = n;
   w.k = n < p.pre_nms_topn ? n : p.pre_nms_topn;
+  w.kept = w.k < p.post_nms_topn ? w.k : p.post_nms_topn;
   w.score_ld = (n + 3) & ~3;
   w.boxes = reinterpret_cast<float4*>(take(sizeof(float4) * n * static_cast<size_t>(batch)));
   w.scores = reinterpret_cast<float*>(take(sizeof(float) * w.score_ld * static_cast<size_t>(batch)));
   w.score_keys = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * w.score_ld * static_cast<size_t>(batch)));
-  w.kept_boxes = reinterpret_cast<float4*>(take(kept_bytes(p.post_nms_topn) * batch));
+  w.kept_boxes = reinterpret_cast<float4*>(take(kept_bytes(w.kept) * batch));
   if (ws) *ws = w;
   return off;
 }
@@ -389,8 +391,8 @@ proposal_rank_nms_kernel(Workspace ws, float threshold, int post_nms_topn, int k
   // The kept list: a copy per CTA in shared memory or, when it is too long for that, one in the workspace.
   float4* kept_box = reinterpret_cast<float4*>(
       kept_in_smem ? rank_smem + ((sizeof(RankShared) + 15) & ~static_cast<size_t>(15))
-                   : reinterpret_cast<unsigned char*>(ws.kept_boxes) + image * kept_bytes(post_nms_topn));
-  float* kept_area = reinterpret_cast<float*>(kept_box + post_nms_topn);
+                   : reinterpret_cast<unsigned char*>(ws.kept_boxes) + image * kept_bytes(ws.kept));
+  float* kept_area = reinterpret_cast<float*>(kept_box + ws.kept);
   const float4* boxes = ws.boxes + static_cast<size_t>(image) * n;
   const float* scores = ws.scores + static_cast<size_t>(image) * ws.score_ld;
   const uint32_t* keys = ws.score_keys + static_cast<size_t>(image) * ws.score_ld;
@@ -758,8 +760,8 @@ extern "C" int mcb200_proposal_forward_from(const mcb200_proposal_params* p, int
   }
   // The kept list goes to shared memory where it fits beside the fixed part.
   size_t smem = (sizeof(RankShared) + 15) & ~static_cast<size_t>(15);
-  const int kept_in_smem = smem + kept_bytes(p->post_nms_topn) <= kRankSharedLimit ? 1 : 0;
-  if (kept_in_smem) smem += kept_bytes(p->post_nms_topn);
+  const int kept_in_smem = smem + kept_bytes(ws.kept) <= kRankSharedLimit ? 1 : 0;
+  if (kept_in_smem) smem += kept_bytes(ws.kept);
   // Eight CTAs per image while all of them find an SM of their own, else four.
   const int parts = batch * 8 <= 148 ? 8 : 4;
   cudaLaunchConfig_t cfg = {};

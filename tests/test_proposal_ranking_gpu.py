@@ -70,3 +70,11 @@ def test_ranking_against_the_restatement(capi, gpu_engine, case):
         if not levels:
             assert np.array_equal(kept.view(np.uint32), np.concatenate(want_scores).view(np.uint32))
     net.close()
+
+
+@pytest.mark.parametrize("case", [
+    (9, 6, 5, 6000, 5000, 0.7, 16, 3, 0),       # 270 proposals, room asked for 5000
+    (9, 24, 25, 900, 16000, 0.9, 0, 2, 0),      # the cut at pre_nms_topn below it
+], ids=lambda c: "x".join(str(v) for v in c))
+def test_more_asked_for_than_there_is(capi, gpu_engine, case):
+    test_ranking_against_the_restatement(capi, gpu_engine, case)

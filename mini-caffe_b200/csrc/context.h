@@ -93,7 +93,7 @@ class PassInFlight {
   const int device_;
 };
 
-// For a scope that queues work on blobs' host memory itself.  A blob that only its host copy is current of is
+// For a scope that queues work on blobs' host memory itself.  A blob whose host copy is the only current one is
 // released without a wait, so when an exception leaves the scope that work ends before it does.
 class DrainOnError {
  public:

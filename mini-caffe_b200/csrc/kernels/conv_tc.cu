@@ -1457,7 +1457,8 @@ int pick_cta_pair(int block_n, long long m, int k_iters) {
 // fill the chip; and only for a tenth less by the model, which is no better than that.
 // Measured, one image: 3 x 3 at 256 channels on 14 x 14 17.3 -> 14.0 us, at 512 on 7 x 7 27.7 -> 21.9, 512 -> 512
 // on 19 x 19 in bfloat16 15.6 -> 13; per pass ResNet-50 629 -> 552, SSD300 in bfloat16 771 -> 687, MobileNet-v1
-// 216 -> 199; ResNet-50 at batch 16 in bfloat16 803 -> 788.
+// 216 -> 199; ResNet-50 at batch 16 in bfloat16 803 -> 788.  (A chip that other nets keep busy has no SMs to give: three
+// threads with a ResNet-50 at batch 16 each make 22 400 images/s so and 22 900 without.)
 bool small_tiles(int cout, long long m, int k_iters, int taps, int halo_rows, int* block_n, int* pair) {
   const char* force = getenv("MCB200_BLOCK_M");   // "64" / "128": override for experiments and tests
   const bool forced = force && atoi(force) == kSmallM;

@@ -276,7 +276,7 @@ struct JaccardTest {
 struct ClassShared {
   SelectShared select;
   uint32_t keep[2][128];     // the walk's set, by the round's parity
-  int num_cand, num_sel, num_kept;
+  int num_cand, num_sel;
 };
 
 __host__ __device__ inline size_t class_region_bytes(int num_priors, int limit) {
@@ -312,7 +312,6 @@ detout_class_kernel(const float* __restrict__ loc, const float* __restrict__ con
   if (t == 0) {
     sh.num_cand = 0;
     sh.num_sel = 0;
-    sh.num_kept = 0;
     sh.select.low = 0xFFFFFFFFu;
     sh.select.high = 0u;
   }

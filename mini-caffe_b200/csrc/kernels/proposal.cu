@@ -1,7 +1,8 @@
 // RPN ProposalLayer on the device, batched over images:
 //   1. decode      anchor + deltas -> clipped box, score (0 for boxes below the minimum size)
 //   2. rank + NMS  a cluster of CTAs per image: takes the best boxes a segment of at most 1024 at a
-//                  time, walks each segment 64 boxes at a time against the kept ones, stops at
+//                  time, marks in a bit matrix which boxes of the segment suppress which, and which the
+//                  boxes kept earlier do, iterates the kept set to its fixed point, stops at
 //                  post_nms_topn; writes rois (+ scores) and the count
 // The host only needs the per-image counts.
 //

@@ -142,10 +142,10 @@ class InnerProductLayer : public Layer {
 unsigned long long TailVersion(const FusedTail& tail);
 void FoldTail(const FusedTail& tail, int channels, const float* bias, std::vector<float>* scale,
               std::vector<float>* shift, bool* has_scale, bool* has_shift);
-// Which device copy of the residual blob the kernel reads.
 // What Layer::PartSeconds takes a pass over an activation to run at: half-filled layers of ResNet-50,
 // MobileNet-v1 and SSD300 move 3 to 5.5 TB/s.
 const double kPartBytesPerSecond = 4e12;
+// Which device copy of the residual blob the kernel reads.
 enum ResidualCopy { kResidualNchw, kResidualNhwc, kResidualNhwcHalf };
 void FillTailEpilogue(const FusedTail& tail, const DeviceArray& scale, const DeviceArray& shift,
                       ResidualCopy residual_copy, int channels, mcb200_epilogue* ep);
@@ -504,10 +504,10 @@ class DeconvolutionLayer : public Layer {
   void Forward_gpu(const vector<Blob*>& bottom, const vector<Blob*>& top) override;
   mcb200_conv_shape shape_ = mcb200_conv_shape();
   bool bias_term_ = false;
-  // The layer runs as a convolution on the tensor cores: phase by phase
-  // (mcb200_deconv_tc_plan), all phases side by side (mcb200_deconv_as_window_conv), or with a reversed
-  // filter over the input spread `stride` apart over zeros (mcb200_deconv_as_conv_shape); the direct kernel takes what is left (more padding than the filter
-  // reaches).
+  // The layer runs as a convolution on the tensor cores: phase by phase (mcb200_deconv_tc_plan), all phases
+  // side by side (mcb200_deconv_as_window_conv), or with a reversed filter over the input, spread `stride` apart
+  // over zeros (mcb200_deconv_as_conv_shape; at stride 1 the input as it is); the direct kernel takes what is left
+  // (more padding than the filter reaches).
   enum Form { kPhases, kWindow, kSpread };
   Form form_ = kSpread;              // what the packed weights are laid out for
   bool packed_for_pixel_ = false;

@@ -53,8 +53,8 @@ BATCH_PER_GPU = 64
 def _e2e_threads():
     """Host threads per GPU in the end-to-end leg, each with its own Net and stream.  Three where the
     host has the cores for it: the third net's kernels run on the SMs that the under-filled launches
-    of the other two leave idle (measured on one B200: 31 500 images/s with two threads, 35 200 with
-    three or four); two when eight ranks share sixteen cores."""
+    of the other two leave idle (measured on one B200: 32 000 images/s with two threads, 34 900 with
+    three); two when eight ranks share sixteen cores."""
     forced = os.environ.get("MCB200_E2E_THREADS")
     if forced:
         return max(1, int(forced))
@@ -67,7 +67,7 @@ E2E_THREADS = _e2e_threads()
 # the 54 launches of one pass at batch 64) from one ncu launch-list capture of this workload, and
 # the hash of the kernel sources the capture was made with.  A different hash means the figure is
 # stale: the line then carries null until the capture is repeated.
-CONV_TRAFFIC = {"bytes_per_launch": 87.96e6, "kernel_sha16": "fb7a1d4658a37bed"}
+CONV_TRAFFIC = {"bytes_per_launch": 87.95e6, "kernel_sha16": "ec836a5e68acd6a0"}
 METRIC = "resnet50_images_per_sec"
 UNIT = "images/s"
 

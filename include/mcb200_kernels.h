@@ -80,8 +80,8 @@ int mcb200_conv_pack_weights(const mcb200_conv_shape* s, const float* w_oihw, fl
 typedef struct mcb200_conv_plan {
   uint64_t tma_a[16];
   uint64_t tma_b[16];
-  uint64_t tma_out[16];     /* output / residual tile maps, built on first launch  */
-  uint64_t tma_res[16];     /* and rebuilt when the pointers below change          */
+  uint64_t tma_out[16];     /* not used (callers rely on the layout)               */
+  uint64_t tma_res[16];     /* not used                                            */
   mcb200_conv_shape shape;
   int m, k_iters, c_blocks, block_n;
   int im2col;               /* 0 matrix rows, 1 im2col tensor map, 2 row mode, 3 halo mode (the taps
@@ -89,7 +89,7 @@ typedef struct mcb200_conv_plan {
   int out_ld, res_ld;
   int cta_pair;             /* 1: launched as two-CTA clusters (tcgen05 cta_group::2) */
   int operand_bf16;         /* 1: built by mcb200_conv_tc_plan_bf16                 */
-  int out_bf16;             /* element type the cached output tile map was built for */
+  int out_bf16;             /* not used, nor are out_ld, res_ld and the two pointers */
   const float* out_ptr;
   const float* res_ptr;
   int m_virtual;            /* halo mode: positions of the virtual output grid (rows widened by
@@ -107,8 +107,6 @@ typedef struct mcb200_conv_plan {
  * (src/layers/inner_product_layer.cpp:80-93).                                */
 int mcb200_conv_tc_plan(const mcb200_conv_shape* s, const float* in, const float* packed_w,
                         mcb200_conv_plan* plan);
-/* The plan is updated in place when `out` / the residual pointer differ from
- * the previous launch (their tile maps are cached in it).                     */
 int mcb200_conv_tc_launch(mcb200_conv_plan* plan, float* out, int out_ld,
                           const mcb200_epilogue* ep, int* status, void* stream);
 

@@ -149,9 +149,9 @@ def main():
     c = t[4][t[4] > 0]
     c = c[: len(c) // 5 * 5].reshape(-1, 5)
     if len(c) >= 2:
-        print("epilogue warp 0, per 32 x 32 chunk (staged epilogue), %d chunks:" % len(c))
-        for name, col in (("  accumulator -> registers (tcgen05.ld)", 1), ("  wait for the slot / the residual", 2),
-                          ("  tail arithmetic + write to the slot", 3), ("  fence + store issue", 4)):
+        print("epilogue warp 0, per chunk (staged / from registers), %d chunks:" % len(c))
+        for name, col in (("  accumulator -> registers (tcgen05.ld)", 1), ("  slot, residual wait / tail", 2),
+                          ("  tail, write to slot / next residual", 3), ("  store issue", 4)):
             print(summary(name, (c[:, col] - c[:, col - 1]).tolist()))
         print(summary("  from store issue to the next chunk", (c[1:, 0] - c[:-1, 4]).tolist()))
     if args.dump:

@@ -19,11 +19,10 @@
 //   warps 3-10 read the accumulator out of tensor memory (tcgen05.ld), apply
 //            the fused tail (per-channel scale/shift, residual add, ReLU or
 //            PReLU) and store channels-last.  Two warps share each 32-lane
-//            quadrant of tensor memory and take alternate 32-column chunks.
-//            Each warp stages its 32 x 32 sub-tiles in shared memory (128-byte
-//            swizzled) so that the residual comes in and the result goes out as
-//            whole 128-byte rows through TMA tile loads / stores, double
-//            buffered per warp.
+//            quadrant of tensor memory and take alternate chunks of columns.  Results go
+//            straight from registers to memory, or, where many tiles keep HBM busy, through
+//            swizzled 32 x 32 sub-tiles in shared memory and out as TMA tile stores, a
+//            residual the same way in (see staged_epilogue).
 // Every barrier wait is bounded; a timed-out wait raises an abort flag, the
 // roles drain, tensor memory is freed and *status is set.
 //
@@ -84,22 +83,21 @@ struct ConvTcArgs {
   int stride_h, stride_w, pad_h, pad_w, dil_h, dil_w;
   mcb200_epilogue ep;
   int* status;
-  int tma_epilogue;  // output (and residual) meet the 16-byte rules of TMA tiles
   int tile_rows;     // rows of an M tile: 128 or 64, in row mode min(output width, 128)
   int row_segments;  // row mode: M tiles per output row of an image (ceil(output width / tile_rows))
   int a_bytes;       // bytes one activation tile load delivers
   int stages;        // depth of the operand ring (2 .. kMaxStages)
-  int slots;         // staging slots per epilogue warp: 1 or 2; 2 .. kMaxSlots when a residual is added
-  int res_depth;     // residual sub-tiles a warp requests ahead of the one it works on (1 .. slots - 1)
   int out_half;      // the output is stored as bfloat16 (else fp32), whatever the operands are
   // Halo mode.  The M index runs over a virtual output grid whose rows are `wp` = wo + (kw - 1) *
   // dil_w positions wide (the last wp - wo positions of a row are computed and never stored), so
   // that the taps s = 0 .. kw-1 of a filter row are the same strip of `128 + wp - wo` input
   // pixels read at row offsets s * dil_w.  `m` then counts virtual positions.
   int wp;
-  int stage_bytes;     // strip slot + kw weight tiles
+  int stage_bytes;     // activation tiles (halo mode: a strip) + weight tiles
   int stage_b_offset;  // where the weight tiles start inside a stage
-  int vec_store;       // plain-store epilogue: rows are 16-byte aligned, use 128-bit accesses
+  int slots;           // staged epilogue: staging slots per warp, 1 or 2; 2 .. kMaxSlots when a residual is added
+  int res_depth;       // and residual sub-tiles a warp requests ahead of the one it works on (1 .. slots - 1)
+  int vec_store;       // the rows of output and residual can be accessed two fp32 (eight bfloat16) columns at a time
   // Grouped convolution (group_cout > 0): output columns [g * group_cout, (g + 1) * group_cout)
   // read input channels [g * group_cin, (g + 1) * group_cin).  An N tile multiplies the channels
   // its groups span (from `c_origin`, rounded down to 16 bytes) by a block-diagonal weight tile:
@@ -115,8 +113,6 @@ struct ConvTcArgs {
   unsigned char phase_off_h[kMaxPhase], phase_off_w[kMaxPhase];
   int out_h, out_w;              // the output image, which may cut the last row and column of the grid short
   int l2_prefetch;               // ask L2 for the next tile's activations a tile ahead
-  int halo_staged;               // halo mode: results pass through a shared-memory slot so that the stores are
-                                 // whole 128-byte rows (fp32 output with 16-byte aligned rows)
   long long wait_limit;          // bound of every barrier wait, in SM cycles
   int resident_b_bytes;          // row mode: all filter rows' weight tiles stay in shared memory (bytes; 0 = streamed
                                  // with the activations).  Every M tile of such a layer multiplies the same
@@ -132,9 +128,9 @@ struct ConvTcArgs {
 // array that mcb200_conv_trace_read copies out.  Role 0: activation producer (per k-iteration:
 // stage free, loads issued); 1: weight producer (same); 2: MMA issuer (per k-iteration: stage
 // full, MMAs issued and committed); 3: epilogue warp 0 (per tile: accumulator ready, tile stored);
-// 4: the same warp inside its chunk loop, five stamps per 32 x 32 chunk of a launch with the staged
-// epilogue (chunk begins, accumulator in registers, slot free / residual there, tail computed and
-// written to the slot, store issued).  A reader's buffer holds these five rows and no more.
+// 4: the same warp inside its chunk loop, five stamps per chunk (chunk begins, accumulator in registers, then staged:
+// slot free / residual there, tail computed and written to the slot, store issued; from registers: tail computed, next
+// residual asked for, stores issued).  A reader's buffer holds these five rows and no more.
 #ifdef MCB200_CONV_TRACE
 constexpr int kTraceSlots = 2048;
 constexpr int kTraceRoles = 5;
@@ -157,18 +153,13 @@ __device__ long long g_conv_trace[kTraceRoles * kTraceSlots];
 #define MCB200_TRACE_CHUNK()
 #endif
 
-constexpr int kMaxStages = 8;
+constexpr int kMaxStages = 10;
 constexpr int kMaxSlots = 4;     // every barrier here is static shared memory that the operand ring cannot use
 constexpr int kSharedLimit = 232448;   // 227 KiB: the most one CTA can have on sm_100
 
-// Shared memory of one persistent CTA = operand ring (`stages` x (A tile + B
-// tile)) + epilogue staging (`slots` x 4 KiB for each of the eight warps; 2 KiB
-// when residual and result are both bfloat16).  The
-// copies in flight are what hides the round trip of a stage (L2 -> shared
-// memory, barrier hop, MMA completion, barrier hop: about a microsecond), so
-// the ring takes every byte the epilogue can spare: launches that add a
-// residual, or whose tiles are short (few k-iterations per epilogue), double
-// buffer the staging; all others give that memory to the ring.
+// Shared memory of one persistent CTA is the operand ring, `stages` x (A tiles + B tiles): the copies in
+// flight are what hides the round trip of a stage (L2 -> shared memory, barrier hop, MMA completion,
+// barrier hop: about a microsecond).
 template <int BN, int kMode, bool kPair>
 struct SmemPlan {
   static constexpr int kTileBRows = kPair ? BN / 2 : BN;   // a CTA of a pair holds half of the weight tile
@@ -181,19 +172,32 @@ struct SmemPlan {
   // Halo mode: a stage is one pixel strip plus the weight tiles of a whole filter row (sized at run time).
   static constexpr int kSub =
       (kMode != kModeRows && kMode != kModeHalo && kTileABytes + kTileBBytes <= 24 * 1024) ? 2 : 1;
-  static constexpr int kStageBytes = kSub * (kTileABytes + kTileBBytes);
-  static constexpr int kStageBOffset = kSub * kTileABytes;   // [A sub-tiles][B sub-tiles]
-  static constexpr int staging_bytes(int slots, int slot_bytes) { return kEpilogueWarps * slots * slot_bytes; }
-  static constexpr int dynamic_bytes(int stages, int slots, int slot_bytes) {
-    return stages * kStageBytes + staging_bytes(slots, slot_bytes) + 1024;   // + alignment slack
-  }
 };
 
-// Compile-time tag for the activation of the fused tail (0 none, 1 ReLU, 2 per-column negative slope).
-template <int kAct>
-struct ActTag {
-  static constexpr int value = kAct;
+// Compile-time tag, for the activation of the fused tail (0 none, 1 ReLU, 2 per-column negative slope) and
+// whether a residual is added.
+template <int kValue>
+struct Tag {
+  static constexpr int value = kValue;
 };
+
+// w[k] of lane q of a quad becomes word q of the quad's lane k.
+__device__ __forceinline__ void quad_transpose(uint32_t (&w)[4], int q) {
+#pragma unroll
+  for (int step = 1; step <= 2; step *= 2) {
+    const bool upper = (q & step) != 0;
+    const int lo0 = 0, hi0 = step, lo1 = step == 1 ? 2 : 1, hi1 = 3;
+    const uint32_t x = __shfl_xor_sync(0xffffffffu, upper ? w[lo0] : w[hi0], step);
+    const uint32_t y = __shfl_xor_sync(0xffffffffu, upper ? w[lo1] : w[hi1], step);
+    if (upper) {
+      w[lo0] = x;
+      w[lo1] = y;
+    } else {
+      w[hi0] = x;
+      w[hi1] = y;
+    }
+  }
+}
 
 // Ring position of a k-iteration: stage index and the parity of its use.
 // Advancing it costs an increment and a compare; the single-thread loops
@@ -229,11 +233,12 @@ struct RingPos {
 // kind::f16, fp32 accumulation); a k-iteration then covers 64 channels in the
 // same 128-byte rows.  Independently of that, the output is stored as fp32 or
 // as bfloat16 (args.out_half).
-template <int BN, int kMode, bool kPair, bool kHalf>
+template <int BN, int kMode, bool kPair, bool kHalf, bool kStaged>
 __global__ void __launch_bounds__(kThreads, 1)
 conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const __grid_constant__ CUtensorMap map_out, const __grid_constant__ CUtensorMap map_res,
                const ConvTcArgs args) {
+  static_assert(!(kStaged && (BN < 64 || kMode == kModeHalo || kMode == kModePhase)), "a staged tile is one box of the output");
   static_assert(!(kPair && kMode == kModeRows), "row mode runs unpaired");
   static_assert(!(kHalf && kMode == kModeRows), "row mode takes fp32 images");
   static_assert(!((kPair || kHalf) && kMode == kModePhase), "phase mode runs unpaired on fp32 operands");
@@ -242,7 +247,6 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   using Plan = SmemPlan<BN, kMode, kPair>;
   constexpr int kElemsK = kHalf ? kBlockKHalf : kBlockK;   // channels per k-iteration
   const int stages = args.stages;
-  const int slots = args.slots;
   const long long wait_limit = args.wait_limit;   // SM cycles a barrier wait may take before the CTA gives up
 
   extern __shared__ uint8_t smem_raw[];
@@ -250,7 +254,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   __shared__ uint64_t empty_bar[kMaxStages];   // the MMAs reading a stage have retired
   __shared__ uint64_t tmem_full_bar[2];
   __shared__ uint64_t tmem_empty_bar[2];
-  __shared__ uint64_t res_bar[kEpilogueWarps][kMaxSlots];   // per epilogue warp, per staging slot
+  __shared__ uint64_t res_bar[kStaged ? kEpilogueWarps : 1][kMaxSlots];   // per epilogue warp, per staging slot
   __shared__ uint64_t col_bar[2];              // per-column table of a tile is complete
   __shared__ uint64_t wres_bar;                // row mode: the resident weight tiles have landed
   __shared__ uint32_t tmem_base_slot;
@@ -262,8 +266,9 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   // 128-byte swizzled tiles must start on a 1024-byte boundary.
   const uint32_t raw_addr = smem_addr(smem_raw);
   uint8_t* tiles = smem_raw + ((1024u - (raw_addr & 1023u)) & 1023u);
-  const int stage_bytes = (kMode == kModeHalo || kMode == kModeRows) ? args.stage_bytes : Plan::kStageBytes;
-  const int stage_b_offset = (kMode == kModeHalo || kMode == kModeRows) ? args.stage_b_offset : Plan::kStageBOffset;
+  const int stage_bytes = args.stage_bytes;
+  const int stage_b_offset = args.stage_b_offset;
+  const int a_sub_bytes = stage_b_offset / Plan::kSub;   // sub-tiles of a stage: [A ...][B ...]
   const bool resident_b = kMode == kModeRows && args.resident_b_bytes > 0;
   uint8_t* resident = tiles + stages * stage_bytes;   // stages are multiples of 1024 bytes: so is this address
   uint8_t* staging_base = resident + (kMode == kModeRows ? args.resident_b_bytes : 0);
@@ -274,7 +279,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                                           : (args.cout + BN - 1) / BN;
   // Rows of an M tile: with 64, tcgen05.mma runs at M = 64 and its accumulator lies in the first 16 lanes of
   // each tensor-memory quadrant (row 16 * quadrant + lane).
-  constexpr bool kShortTiles = !kPair && (kMode == kModeMatrix || kMode == kModeIm2col || kMode == kModeHalo);
+  constexpr bool kShortTiles = !kPair && !kStaged && (kMode == kModeMatrix || kMode == kModeIm2col || kMode == kModeHalo);
   const int tile_m = kShortTiles ? args.tile_rows : kBlockM;
   const int warp_rows = kShortTiles ? args.tile_rows >> 2 : 32;   // rows an epilogue warp owns: one quadrant's
   // Row mode: an M tile is (a segment of at most 128 pixels of) one output row of one image.
@@ -291,7 +296,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   const int num_tiles = n_tiles * m_units;
   auto unit_to_mt = [&](int unit) { return kPair ? 2 * unit + static_cast<int>(rank) : unit; };
 
-  // Some fifty barriers: a thread each (one thread doing them all costs every launch most of a
+  // Some twenty barriers: a thread each (one thread doing them all costs every launch most of a
   // microsecond before its first load can go out).
   {
     const int t = static_cast<int>(threadIdx.x);
@@ -306,7 +311,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       mbar_init(&tmem_empty_bar[b], kPair ? 2 * kEpilogueWarps : kEpilogueWarps);   // one arrival per epilogue warp
       mbar_init(&col_bar[b], kEpilogueWarps);
       fence_barrier_init();
-    } else if (t >= 64 && t < 64 + kEpilogueWarps * kMaxSlots) {
+    } else if (kStaged && t >= 64 && t < 64 + kEpilogueWarps * kMaxSlots) {
       mbar_init(&res_bar[(t - 64) / kMaxSlots][(t - 64) % kMaxSlots], 1);
       fence_barrier_init();
     } else if (t == 34) {
@@ -520,7 +525,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
               }
               c0 += kElemsK;
             }
-            a_dst += kTileABytes;
+            a_dst += a_sub_bytes;
           }
           MCB200_TRACE(0);
           ++issued;
@@ -701,7 +706,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
               }
               accumulate = 1u;
             }
-            desc_a += kTileABytes >> 4;            // next sub-tile (start address is in 16-byte units)
+            desc_a += a_sub_bytes >> 4;            // next sub-tile (start address is in 16-byte units)
             desc_b += Plan::kTileBBytes >> 4;
           }
           if (kPair) {
@@ -723,20 +728,128 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     }
   } else {
     // ------------------------------------------------------------ epilogue
-    const int ew = warp - kFirstEpilogueWarp;   // 0..7: staging ring and barriers of this warp
+    const int ew = warp - kFirstEpilogueWarp;   // 0..7
     const int quad = warp & 3;                  // tensor-memory lanes [32*quad, 32*quad+32)
     const int half = ew >> 2;                   // chunks half, half + 2, ... of every tile
     const mcb200_epilogue& ep = args.ep;
     const bool has_res = ep.residual != nullptr;
-    // A slot holds a 32 x 32 sub-tile: 4 KiB, or 2 KiB when residual and result are both bfloat16.
-    const int slot_bytes = (kHalf && args.out_half) ? 2048 : 4096;
-    uint8_t* staging = staging_base + ew * (slots * slot_bytes);
-    auto slot_ptr = [&](int slot) { return reinterpret_cast<float*>(staging + slot * slot_bytes); };
-    const int chunks_full = BN / 32;
+    constexpr int kChunk = BN >= 64 ? 32 : 16;  // columns of a chunk: both warps of a quadrant have one
+    constexpr int kChunks = BN / kChunk;
+    constexpr int kGroups = kChunk / 8;         // a chunk comes out of tensor memory in groups of eight columns
+    // Of group j a lane holds columns 8 j + col_in and the next, of rows row_in + 8 i (i < row_sets).
+    const int col_in = 2 * (lane & 3);
+    const int row_in = lane >> 2;
+    const int row_sets = kShortTiles ? warp_rows >> 3 : 4;
+    const bool vec = args.vec_store != 0;
     const int epi_tid = threadIdx.x - kFirstEpilogueWarp * 32;   // 0..255 over the epilogue warps
     // 0: no activation, 1: plain ReLU, 2: per-column negative slope (leaky ReLU / PReLU)
     const int act_mode = ep.act == 0 ? 0 : ((ep.act == 1 && ep.slope == 0.f) ? 1 : 2);
 
+    // First column of a tile, and the output rows (-1: none) of this lane's row sets.
+    auto tile_n0 = [&](int tile) {
+      const int nt = tile % n_tiles;
+      return (kMode == kModePhase ? nt % args.phase_tiles : nt) * BN;
+    };
+    auto tile_rows = [&](int tile, int (&rows)[4]) {
+      const int unit = tile / n_tiles;
+      const int mt = unit_to_mt(unit);
+      // First output row (pixel) of this warp's slice of the tile, and how many of its rows exist.
+      const int row0 = (kMode == kModeRows ? row_of(mt) * args.wo + seg_start(mt) : mt * tile_m) + quad * warp_rows;
+      const int rows_here = kMode == kModeRows ? min(args.tile_rows, args.wo - seg_start(mt)) - quad * 32
+                                               : min(args.m - row0, warp_rows);
+      if (!kScatter) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) rows[i] = row_in + 8 * i < rows_here ? row0 + row_in + 8 * i : -1;
+        return;
+      }
+      // A division or two per tile and lane: lane r works out row r and hands it to the lanes that store it.
+      int mine = row0 + lane;
+      bool ok = lane < rows_here;
+      if (kMode == kModeHalo) {
+        const int t = mine / args.wp;              // (image, output row); `mine` counts virtual positions
+        const int j = mine - t * args.wp;
+        ok = ok && j < args.wo;
+        mine = t * args.wo + j;
+      }
+      if (kMode == kModePhase) {
+        const int phase = (tile - unit * n_tiles) / args.phase_tiles;
+        const int phase_y = phase / args.phase_stride_w;
+        const int t = mine / args.wo;              // (image, grid row)
+        const int image = t / args.ho;
+        const int y = (t - image * args.ho) * args.phase_stride_h + phase_y;
+        const int x = (mine - t * args.wo) * args.phase_stride_w + (phase - phase_y * args.phase_stride_w);
+        ok = ok && y < args.out_h && x < args.out_w;
+        mine = (image * args.out_h + y) * args.out_w + x;
+      }
+      if (!ok) mine = -1;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) rows[i] = __shfl_sync(0xffffffffu, mine, (row_in + 8 * i) & 31);
+    };
+    // The residual of the chunk at col0, asked for a chunk ahead: a DRAM round trip (one to two microseconds)
+    // that the chunk before it, or the main loop of a first chunk, hides.
+    float res[4][kGroups][2];
+    auto fetch_residual = [&](const int (&rows)[4], int col0) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (i >= row_sets) break;
+        const size_t at = static_cast<size_t>(rows[i] < 0 ? 0 : rows[i]) * ep.residual_ld + col0 + col_in;
+#pragma unroll
+        for (int j = 0; j < kGroups; ++j) {
+          const int c = col0 + 8 * j + col_in;
+          float2 r = make_float2(0.f, 0.f);
+          if (rows[i] >= 0 && c < args.cout) {
+            if (kHalf) {
+              const uint16_t* src = reinterpret_cast<const uint16_t*>(ep.residual) + at + 8 * j;
+              if (vec) {
+                const uint32_t w = *reinterpret_cast<const uint32_t*>(src);
+                r = make_float2(bf16_lo(w), bf16_hi(w));
+              } else {
+                r.x = bf16_lo(src[0]);
+                if (c + 1 < args.cout) r.y = bf16_lo(src[1]);
+              }
+            } else {
+              const float* src = ep.residual + at + 8 * j;
+              if (vec) {
+                r = *reinterpret_cast<const float2*>(src);
+              } else {
+                r.x = src[0];
+                if (c + 1 < args.cout) r.y = src[1];
+              }
+            }
+          }
+          res[i][j][0] = r.x;
+          res[i][j][1] = r.y;
+        }
+      }
+    };
+    int table_n0[2] = {-1, -1};          // first column the per-column tables were filled for
+    uint32_t table_fills[2] = {0u, 0u};
+    auto fill_table = [&](int ab, int n0) {
+      for (int c = epi_tid; c < BN; c += kEpilogueWarps * 32) {
+        const int cc = n0 + c;
+        const bool in = cc < args.cout;
+        col_scale[ab][c] = (in && ep.scale) ? __ldg(ep.scale + cc) : 1.f;
+        col_shift[ab][c] = (in && ep.shift) ? __ldg(ep.shift + cc) : 0.f;
+        col_slope[ab][c] = ep.act == 2 ? ((in && ep.prelu) ? __ldg(ep.prelu + (ep.prelu_shared ? 0 : cc)) : 0.f) : ep.slope;
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&col_bar[ab]);
+      table_n0[ab] = n0;
+    };
+    // The first tile's table, before anything else is waited for.
+    if (worker < num_tiles) fill_table(0, tile_n0(worker));
+    if (early) grid_dependency_wait();
+    int rows[4] = {-1, -1, -1, -1};
+    if (!kStaged && worker < num_tiles) {
+      tile_rows(worker, rows);
+      if (has_res) fetch_residual(rows, tile_n0(worker) + half * kChunk);
+    }
+
+    // Staged form.  A slot holds a 32 x 32 sub-tile: 4 KiB, or 2 KiB when residual and result are both bfloat16.
+    const int slots = args.slots;
+    const int slot_bytes = (kHalf && args.out_half) ? 2048 : 4096;
+    uint8_t* staging = staging_base + ew * (slots * slot_bytes);
+    auto slot_ptr = [&](int slot) { return reinterpret_cast<float*>(staging + slot * slot_bytes); };
     // Chunk sequence of this warp: for each of its CTA's tiles, the 32-column
     // chunks it owns that exist (the last n-tile may have fewer), left to right.
     // `seq` numbers them.  With a residual the warp cycles through its staging
@@ -762,7 +875,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           cur.n0 = (tile - unit * n_tiles) * BN;
         }
         col = cur.n0 + cur.chunk * 32;
-        if (cur.chunk >= chunks_full || col >= args.cout) {   // this warp's chunks of the tile are done
+        if (cur.chunk >= kChunks || col >= args.cout) {   // this warp's chunks of the tile are done
           cur.chunk = half;
           ++cur.local;
           cur.mt = -1;
@@ -782,35 +895,13 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       if (!cursor_next(ld, mt, col)) return;
       const int slot = ld_slot;
       if (++ld_slot == slots) ld_slot = 0;
-      mbar_expect_tx(&res_bar[ew][slot], static_cast<uint32_t>(warp_rows) * (kHalf ? 64u : 128u));   // rows of 32 bfloat16 or fp32
+      mbar_expect_tx(&res_bar[ew][slot], 32u * (kHalf ? 64u : 128u));   // rows of 32 bfloat16 or fp32
       if (kMode == kModeRows) {
         tma_load_3d(&map_res, &res_bar[ew][slot], slot_ptr(slot), col, seg_start(mt) + quad * 32, row_of(mt));
       } else {
-        tma_load_3d(&map_res, &res_bar[ew][slot], slot_ptr(slot), col, mt * tile_m + quad * warp_rows, 0);
+        tma_load_3d(&map_res, &res_bar[ew][slot], slot_ptr(slot), col, mt * kBlockM + quad * 32, 0);
       }
     };
-    const bool staged = args.tma_epilogue != 0;
-    int table_n0[2] = {-1, -1};          // first column the per-column tables were filled for
-    uint32_t table_fills[2] = {0u, 0u};
-    auto fill_table = [&](int ab, int n0) {
-      for (int c = epi_tid; c < BN; c += kEpilogueWarps * 32) {
-        const int cc = n0 + c;
-        const bool in = cc < args.cout;
-        col_scale[ab][c] = (in && ep.scale) ? __ldg(ep.scale + cc) : 1.f;
-        col_shift[ab][c] = (in && ep.shift) ? __ldg(ep.shift + cc) : 0.f;
-        col_slope[ab][c] = ep.act == 2 ? ((in && ep.prelu) ? __ldg(ep.prelu + (ep.prelu_shared ? 0 : cc)) : 0.f) : ep.slope;
-      }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&col_bar[ab]);
-      table_n0[ab] = n0;
-    };
-    // The first tile's table, before anything else is waited for.
-    if (worker < num_tiles) {
-      int n0 = (worker % n_tiles) * BN;
-      if (kMode == kModePhase) n0 = (worker % n_tiles % args.phase_tiles) * BN;
-      fill_table(0, n0);
-    }
-    if (early) grid_dependency_wait();
     // Residual sub-tiles are requested `res_depth` chunks ahead: a request takes
     // a DRAM round trip (one to two microseconds), several times the time a warp
     // needs per chunk.  Requesting chunk g + depth reuses the slot of chunk
@@ -818,11 +909,12 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     // still be reading shared memory at that point.
     const int res_depth = args.res_depth;
     const int stores_in_flight = slots - res_depth - 1;
-    if (staged && has_res && lane == 0) {
+    if (kStaged && has_res && lane == 0) {
       for (int d = 0; d < res_depth; ++d) issue_residual();
     }
 
-    int seq = 0;
+
+    int seq = 0;                         // chunks this warp has finished
     int local = 0;
     bool alive = true;
     MCB200_TRACE_DECL;
@@ -830,53 +922,30 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     for (int tile = worker; tile < num_tiles && alive; tile += workers, ++local) {
       const int ab = local & 1;
       const uint32_t use = static_cast<uint32_t>(local >> 1) & 1u;
+      // Where the tile lies, before the wait: the divisions cost a few hundred cycles.
       const int unit = tile / n_tiles;
-      const int mt = unit_to_mt(unit);
-      int n0 = (tile - unit * n_tiles) * BN;
-      int phase_y = 0, phase_x = 0;
-      if (kMode == kModePhase) {
-        const int nt = tile - unit * n_tiles;
-        const int phase = nt / args.phase_tiles;
-        n0 = (nt - phase * args.phase_tiles) * BN;
-        phase_y = phase / args.phase_stride_w;
-        phase_x = phase - phase_y * args.phase_stride_w;
-      }
-      // First output row (pixel) of this warp's slice of the tile, and how many of its rows exist.
-      const int row0 = (kMode == kModeRows ? row_of(mt) * args.wo + seg_start(mt) : mt * tile_m) + quad * warp_rows;
-      const int rows_here = kMode == kModeRows ? min(args.tile_rows, args.wo - seg_start(mt)) - quad * 32
-                                               : min(args.m - row0, warp_rows);
-      // Row of the output matrix this lane stores in the plain-store epilogue, and whether it exists.
-      int out_row = row0 + lane;
-      bool row_ok = lane < rows_here;
-      if (kMode == kModeHalo) {
-        const int t = out_row / args.wp;           // (image, output row); out_row counts virtual positions
-        const int j = out_row - t * args.wp;
-        row_ok = row_ok && j < args.wo;
-        out_row = t * args.wo + j;
-      }
-      if (kMode == kModePhase) {
-        const int t = out_row / args.wo;           // (image, grid row)
-        const int image = t / args.ho;
-        const int y = (t - image * args.ho) * args.phase_stride_h + phase_y;
-        const int x = (out_row - t * args.wo) * args.phase_stride_w + phase_x;
-        row_ok = row_ok && y < args.out_h && x < args.out_w;
-        out_row = (image * args.out_h + y) * args.out_w + x;
+      const int n0 = kMode == kModePhase ? tile_n0(tile) : (tile - unit * n_tiles) * BN;
+      int box_row = unit_to_mt(unit), box_image = 0;   // staged form: first output row of this warp's boxes
+      if (kMode == kModeRows) {
+        box_image = row_of(box_row);
+        box_row = (box_row - box_image * args.row_segments) * args.tile_rows + quad * 32;
+      } else {
+        box_row = box_row * kBlockM + quad * 32;
       }
       // tcgen05.ld is warp-collective: the whole warp takes the same branch.
       alive = __all_sync(0xffffffffu, mbar_wait_bounded(&tmem_full_bar[ab], use, abort, wait_limit));
       if (!alive) break;
       tc_fence_after_sync();
       if (ew == 0 && lane == 0) MCB200_TRACE(3);
-      // Per-column constants of the tile's columns go to shared memory, so that the
-      // inner loops are a broadcast 16-byte load and fused multiply-adds.  Two
+      // Per-column constants of the tile's columns go to shared memory.  Two
       // copies (tile parity), each kept while the CTA's tiles of that parity stay
       // in the same column range (always, when the layer has one N tile or the
       // grid is a multiple of the N tiles).  A copy may be overwritten here: the
-      // accumulator of this parity is full again, so every warp has finished
-      // the tile that last used the copy.
-      float* t_scale = col_scale[ab];
-      float* t_shift = col_shift[ab];
-      float* t_slope = col_slope[ab];
+      // accumulator of this parity is full again, so every warp has read what it
+      // needed for the tile that last used the copy.
+      const float* t_scale = col_scale[ab];
+      const float* t_shift = col_shift[ab];
+      const float* t_slope = col_slope[ab];
       const bool refill = table_n0[ab] != n0;
       if (refill) fill_table(ab, n0);
       if (refill || local == 0) {
@@ -887,8 +956,29 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         ++table_fills[ab];
       }
       const uint32_t tmem_acc = tmem_base + static_cast<uint32_t>(ab * BN) + (static_cast<uint32_t>(quad * 32) << 16);
+      const int next = tile + workers;
+      int next_rows[4] = {-1, -1, -1, -1};
+      // After the last read of this accumulator (and of the per-column tables) it goes back to the MMA
+      // issuer, and the next tile's first residual is asked for.
+      auto hand_back = [&]() {
+        if (ew == 0 && lane == 0) MCB200_TRACE(3);
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) {
+          if (kPair) {
+            mbar_arrive_cluster(tmem_empty_leader + static_cast<uint32_t>(ab) * 8u);
+          } else {
+            mbar_arrive(&tmem_empty_bar[ab]);
+          }
+        }
+        if (!kStaged && next < num_tiles) {
+          tile_rows(next, next_rows);
+          if (has_res) fetch_residual(next_rows, tile_n0(next) + half * kChunk);
+        }
+      };
+      bool handed = false;
 #pragma unroll 1
-      for (int chunk = half; chunk < chunks_full; chunk += 2) {
+      for (int chunk = half; kStaged && chunk < kChunks; chunk += 2) {
         const int col0 = n0 + chunk * 32;
         if (col0 >= args.cout) break;          // uniform across the warp
         const int g = seq++;
@@ -940,256 +1030,247 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           v.z = round_to_tf32(v.z);
           v.w = round_to_tf32(v.w);
         };
-        if (staged) {
-          const int slot = has_res ? cur_slot : (slots == 2 ? (g & 1) : 0);
-          float* buf = slot_ptr(slot) + lane * 32;
-          if (has_res) {
-            if (lane == 0) {
-              switch (stores_in_flight) {
-                case 0: tma_store_wait_read<0>(); break;
-                case 1: tma_store_wait_read<1>(); break;
-                case 2: tma_store_wait_read<2>(); break;
-                default: tma_store_wait_read<3>(); break;
-              }
-              issue_residual();
+        const int slot = has_res ? cur_slot : (slots == 2 ? (g & 1) : 0);
+        float* buf = slot_ptr(slot) + lane * 32;
+        if (has_res) {
+          if (lane == 0) {
+            switch (stores_in_flight) {
+              case 0: tma_store_wait_read<0>(); break;
+              case 1: tma_store_wait_read<1>(); break;
+              case 2: tma_store_wait_read<2>(); break;
+              default: tma_store_wait_read<3>(); break;
             }
-            alive = __all_sync(0xffffffffu,
-                               mbar_wait_bounded(&res_bar[ew][slot], cur_parity, abort, wait_limit));
-            if (!alive) break;
-            if (++cur_slot == slots) {
-              cur_slot = 0;
-              cur_parity ^= 1u;
-            }
+            issue_residual();
           }
-          MCB200_TRACE_CHUNK();
-          // Row `lane` of the 32 x 32 tile is 128 bytes: eight 16-byte pieces,
-          // piece j stored at position j ^ (row & 7) (the 128-byte swizzle).
-          // The result overwrites the residual in place.
-          const int swz = lane & 7;
-          // All reads of the chunk (residual cells, per-column tables) come
-          // before its first write: the loads are then independent of each other
-          // and overlap, where a read-modify-write per cell would expose one
-          // shared-memory round trip after the other (long ones while the
-          // tensor core and the TMA keep shared memory busy).
-          float4 v[8];
-          // bfloat16 rows are 64 bytes: four 16-byte pieces, piece q stored at
-          // position q ^ ((row >> 1) & 3) (the 64-byte swizzle).
-          uint8_t* hrow = reinterpret_cast<uint8_t*>(slot_ptr(slot)) + lane * 64;
-          const int hswz = (lane >> 1) & 3;
-          auto fill = [&](auto act_tag) {
-            if (!has_res) {
-#pragma unroll
-              for (int j = 0; j < 8; ++j) v[j] = finish4(act_tag, j, make_float4(0.f, 0.f, 0.f, 0.f), false);
-            } else if (kHalf) {
-              uint4 w[4];
-#pragma unroll
-              for (int q = 0; q < 4; ++q) w[q] = *reinterpret_cast<const uint4*>(hrow + ((q ^ hswz) << 4));
-#pragma unroll
-              for (int q = 0; q < 4; ++q) {
-                v[2 * q] = finish4(act_tag, 2 * q,
-                                   make_float4(bf16_lo(w[q].x), bf16_hi(w[q].x), bf16_lo(w[q].y), bf16_hi(w[q].y)), true);
-                v[2 * q + 1] = finish4(act_tag, 2 * q + 1,
-                                       make_float4(bf16_lo(w[q].z), bf16_hi(w[q].z), bf16_lo(w[q].w), bf16_hi(w[q].w)),
-                                       true);
-              }
-            } else {
-              float4 r[8];
-#pragma unroll
-              for (int j = 0; j < 8; ++j) r[j] = *reinterpret_cast<const float4*>(buf + ((j ^ swz) << 2));
-#pragma unroll
-              for (int j = 0; j < 8; ++j) v[j] = finish4(act_tag, j, r[j], true);
-            }
-          };
-          if (act_mode == 1) {
-            fill(ActTag<1>());
-          } else if (act_mode == 0) {
-            fill(ActTag<0>());
-          } else {
-            fill(ActTag<2>());
+          alive = __all_sync(0xffffffffu,
+                             mbar_wait_bounded(&res_bar[ew][slot], cur_parity, abort, wait_limit));
+          if (!alive) break;
+          if (++cur_slot == slots) {
+            cur_slot = 0;
+            cur_parity ^= 1u;
           }
-          if (ep.round_tf32) {
+        }
+        MCB200_TRACE_CHUNK();
+        // Row `lane` of the 32 x 32 tile is 128 bytes: eight 16-byte pieces,
+        // piece j stored at position j ^ (row & 7) (the 128-byte swizzle).
+        // The result overwrites the residual in place.
+        const int swz = lane & 7;
+        // All reads of the chunk (residual cells, per-column tables) come
+        // before its first write: the loads are then independent of each other
+        // and overlap, where a read-modify-write per cell would expose one
+        // shared-memory round trip after the other (long ones while the
+        // tensor core and the TMA keep shared memory busy).
+        float4 v[8];
+        // bfloat16 rows are 64 bytes: four 16-byte pieces, piece q stored at
+        // position q ^ ((row >> 1) & 3) (the 64-byte swizzle).
+        uint8_t* hrow = reinterpret_cast<uint8_t*>(slot_ptr(slot)) + lane * 64;
+        const int hswz = (lane >> 1) & 3;
+        auto fill = [&](auto act_tag) {
+          if (!has_res) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) round4(v[j]);
-          }
-          if (!has_res && g >= slots) {
-            // The store that last used this slot must have finished reading it.  Asked only now,
-            // with the chunk's values in registers: the query costs its thread some 200 cycles
-            // whatever the answer, which the table loads above spend in flight.
-            if (lane == 0) {
-              if (slots == 2) {
-                tma_store_wait_read<1>();
-              } else {
-                tma_store_wait_read<0>();
-              }
-            }
-            __syncwarp();
-          }
-          // Residual and result rows of different widths overlap other lanes' rows.
-          if (has_res && (args.out_half != 0) != kHalf) __syncwarp();
-          if (args.out_half) {
+            for (int j = 0; j < 8; ++j) v[j] = finish4(act_tag, j, make_float4(0.f, 0.f, 0.f, 0.f), false);
+          } else if (kHalf) {
+            uint4 w[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) w[q] = *reinterpret_cast<const uint4*>(hrow + ((q ^ hswz) << 4));
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-              uint4 w;
-              w.x = pack_bf16x2(v[2 * q].x, v[2 * q].y);
-              w.y = pack_bf16x2(v[2 * q].z, v[2 * q].w);
-              w.z = pack_bf16x2(v[2 * q + 1].x, v[2 * q + 1].y);
-              w.w = pack_bf16x2(v[2 * q + 1].z, v[2 * q + 1].w);
-              *reinterpret_cast<uint4*>(hrow + ((q ^ hswz) << 4)) = w;
+              v[2 * q] = finish4(act_tag, 2 * q,
+                                 make_float4(bf16_lo(w[q].x), bf16_hi(w[q].x), bf16_lo(w[q].y), bf16_hi(w[q].y)), true);
+              v[2 * q + 1] = finish4(act_tag, 2 * q + 1,
+                                     make_float4(bf16_lo(w[q].z), bf16_hi(w[q].z), bf16_lo(w[q].w), bf16_hi(w[q].w)),
+                                     true);
             }
           } else {
+            float4 r[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) *reinterpret_cast<float4*>(buf + ((j ^ swz) << 2)) = v[j];
+            for (int j = 0; j < 8; ++j) r[j] = *reinterpret_cast<const float4*>(buf + ((j ^ swz) << 2));
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = finish4(act_tag, j, r[j], true);
           }
-          MCB200_TRACE_CHUNK();
-          fence_proxy_async_smem();
-          __syncwarp();
+        };
+        if (act_mode == 1) {
+          fill(Tag<1>());
+        } else if (act_mode == 0) {
+          fill(Tag<0>());
+        } else {
+          fill(Tag<2>());
+        }
+        if (ep.round_tf32) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) round4(v[j]);
+        }
+        if (chunk + 2 >= kChunks || col0 + 64 >= args.cout) {
+          hand_back();
+          handed = true;
+        }
+        if (!has_res && g >= slots) {
+          // The store that last used this slot must have finished reading it.  Asked only now,
+          // with the chunk's values in registers: the query costs its thread some 200 cycles
+          // whatever the answer, which the table loads above spend in flight.
           if (lane == 0) {
-            if (kMode == kModeRows) {
-              tma_store_3d(&map_out, slot_ptr(slot), col0, seg_start(mt) + quad * 32, row_of(mt));   // clipped at the row's end
+            if (slots == 2) {
+              tma_store_wait_read<1>();
             } else {
-              tma_store_3d(&map_out, slot_ptr(slot), col0, row0, 0);
+              tma_store_wait_read<0>();
             }
-            tma_store_commit();
           }
-          MCB200_TRACE_CHUNK();
+          __syncwarp();
+        }
+        // Residual and result rows of different widths overlap other lanes' rows.
+        if (has_res && (args.out_half != 0) != kHalf) __syncwarp();
+        if (args.out_half) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            uint4 w;
+            w.x = pack_bf16x2(v[2 * q].x, v[2 * q].y);
+            w.y = pack_bf16x2(v[2 * q].z, v[2 * q].w);
+            w.z = pack_bf16x2(v[2 * q + 1].x, v[2 * q + 1].y);
+            w.w = pack_bf16x2(v[2 * q + 1].z, v[2 * q + 1].w);
+            *reinterpret_cast<uint4*>(hrow + ((q ^ hswz) << 4)) = w;
+          }
         } else {
-          // ---- plain stores: rows that are not 16-byte aligned, and halo mode, whose tiles are
-          // pieces of the virtual output grid (a lane's row may be one of the positions that are
-          // computed and dropped) ----
-          const size_t out_off = static_cast<size_t>(row_ok ? out_row : 0) * args.out_ld;
-          const size_t res_off = static_cast<size_t>(row_ok ? out_row : 0) * ep.residual_ld;
-          const bool whole_chunk = args.vec_store && col0 + 32 <= args.cout;
-          // The lane's 32 outputs of its row (128 bytes, 64 as bfloat16), fused tail applied.
-          float4 v[8];
-          if (whole_chunk && (row_ok || (kScatter && args.halo_staged))) {
-            const bool add_res = has_res && row_ok;
-            auto fill = [&](auto act_tag) {
-              if (!add_res) {
 #pragma unroll
-                for (int j = 0; j < 8; ++j) v[j] = finish4(act_tag, j, make_float4(0.f, 0.f, 0.f, 0.f), false);
-              } else if (kHalf) {
-                const uint4* rp = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(ep.residual) + res_off + col0);
-                uint4 w[4];
+          for (int j = 0; j < 8; ++j) *reinterpret_cast<float4*>(buf + ((j ^ swz) << 2)) = v[j];
+        }
+        MCB200_TRACE_CHUNK();
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          tma_store_3d(&map_out, slot_ptr(slot), col0, box_row, box_image);   // clipped at the row's (the matrix's) end
+          tma_store_commit();
+        }
+        MCB200_TRACE_CHUNK();
+      }
+#pragma unroll 1
+      for (int chunk = half; !kStaged && chunk < kChunks; chunk += 2) {
+        const int col0 = n0 + chunk * kChunk;
+        if (col0 >= args.cout) break;          // uniform across the warp
+        uint32_t acc[2][4 * kGroups];          // lanes 0-15 and 16-31 of the quadrant
+        MCB200_TRACE_CHUNK();
+        tmem_load_16x256<kGroups>(tmem_acc + static_cast<uint32_t>(chunk * kChunk), acc[0]);
+        if (row_sets > 2) tmem_load_16x256<kGroups>(tmem_acc + (16u << 16) + static_cast<uint32_t>(chunk * kChunk), acc[1]);
+        tmem_load_wait();
+        MCB200_TRACE_CHUNK();
+        // v = acc * scale + shift (+ coeff * residual), then the activation, in place.  Activation and
+        // residual are compile-time tags: with run-time tests inside, every value became its own chain of
+        // small basic blocks, each exposing its latencies; as straight-line code the chains overlap.
+        auto finish = [&](auto act_tag, auto res_tag) {
+          constexpr int kAct = decltype(act_tag)::value;
+          constexpr bool kRes = decltype(res_tag)::value != 0;
 #pragma unroll
-                for (int q = 0; q < 4; ++q) w[q] = rp[q];
+          for (int j = 0; j < kGroups; ++j) {
+            const int at = chunk * kChunk + 8 * j + col_in;
+            const float2 sc = *reinterpret_cast<const float2*>(t_scale + at);
+            const float2 sh = *reinterpret_cast<const float2*>(t_shift + at);
+            float2 sl = make_float2(0.f, 0.f);
+            if (kAct == 2) sl = *reinterpret_cast<const float2*>(t_slope + at);
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                  v[2 * q] = finish4(act_tag, 2 * q,
-                                     make_float4(bf16_lo(w[q].x), bf16_hi(w[q].x), bf16_lo(w[q].y), bf16_hi(w[q].y)), true);
-                  v[2 * q + 1] = finish4(act_tag, 2 * q + 1,
-                                         make_float4(bf16_lo(w[q].z), bf16_hi(w[q].z), bf16_lo(w[q].w), bf16_hi(w[q].w)),
-                                         true);
-                }
-              } else {
-                const float4* rp = reinterpret_cast<const float4*>(ep.residual + res_off + col0);
-                float4 r[8];
+            for (int i = 0; i < 4; ++i) {
+              if (i >= row_sets) break;
 #pragma unroll
-                for (int j = 0; j < 8; ++j) r[j] = rp[j];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) v[j] = finish4(act_tag, j, r[j], true);
+              for (int e = 0; e < 2; ++e) {
+                uint32_t& cell = acc[i >> 1][4 * j + 2 * (i & 1) + e];
+                float v = fmaf(__uint_as_float(cell), e ? sc.y : sc.x, e ? sh.y : sh.x);
+                if (kRes) v = fmaf(ep.residual_coeff, res[i][j][e], v);
+                if (kAct == 1) v = fmaxf(v, 0.f);
+                if (kAct == 2) v = v > 0.f ? v : v * (e ? sl.y : sl.x);
+                cell = __float_as_uint(v);
               }
-            };
-            if (act_mode == 1) {
-              fill(ActTag<1>());
-            } else if (act_mode == 0) {
-              fill(ActTag<0>());
-            } else {
-              fill(ActTag<2>());
-            }
-            if (ep.round_tf32) {
-#pragma unroll
-              for (int j = 0; j < 8; ++j) round4(v[j]);
             }
           }
-          if (kScatter && args.halo_staged && whole_chunk) {
-            // Through the warp's shared-memory slot, so that a store instruction writes four whole
-            // 128-byte rows (eight lanes each) instead of 16 bytes of 32 different rows: a lane's
-            // own row may be a dropped position, its neighbours' rows are not.
-            float* slot = slot_ptr(0);
-            const int swz = lane & 7;
+        };
+        if (has_res) {
+          if (act_mode == 1) {
+            finish(Tag<1>(), Tag<1>());
+          } else if (act_mode == 0) {
+            finish(Tag<0>(), Tag<1>());
+          } else {
+            finish(Tag<2>(), Tag<1>());
+          }
+        } else if (act_mode == 1) {
+          finish(Tag<1>(), Tag<0>());
+        } else if (act_mode == 0) {
+          finish(Tag<0>(), Tag<0>());
+        } else {
+          finish(Tag<2>(), Tag<0>());
+        }
+        if (ep.round_tf32) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) *reinterpret_cast<float4*>(slot + lane * 32 + ((j ^ swz) << 2)) = v[j];
-            __syncwarp();
-            const int piece = lane & 7;
+          for (int h = 0; h < 2; ++h)
 #pragma unroll
-            for (int p = 0; p < 8; ++p) {
-              const int r = 4 * p + (lane >> 3);
-              const int orow = __shfl_sync(0xffffffffu, out_row, r);
-              const int ok = __shfl_sync(0xffffffffu, row_ok ? 1 : 0, r);
-              const float4 val = *reinterpret_cast<const float4*>(slot + r * 32 + ((piece ^ (r & 7)) << 2));
-              if (ok) *reinterpret_cast<float4*>(args.out + static_cast<size_t>(orow) * args.out_ld + col0 + piece * 4) = val;
+            for (int k = 0; k < 4 * kGroups; ++k) acc[h][k] = __float_as_uint(round_to_tf32(__uint_as_float(acc[h][k])));
+        }
+        MCB200_TRACE_CHUNK();
+        if (chunk + 2 >= kChunks || col0 + 2 * kChunk >= args.cout) {
+          hand_back();
+          handed = true;
+        } else if (has_res) {
+          fetch_residual(rows, col0 + 2 * kChunk);
+        }
+        MCB200_TRACE_CHUNK();
+        if (vec && !args.out_half) {
+          // Four lanes hold 32 bytes of a row: a store instruction writes eight whole sectors.
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            if (i >= row_sets || rows[i] < 0) continue;
+            float* dst = args.out + static_cast<size_t>(rows[i]) * args.out_ld + col0 + col_in;
+#pragma unroll
+            for (int j = 0; j < kGroups; ++j) {
+              if (col0 + 8 * j + col_in < args.cout)
+                *reinterpret_cast<float2*>(dst + 8 * j) =
+                    make_float2(__uint_as_float(acc[i >> 1][4 * j + 2 * (i & 1)]), __uint_as_float(acc[i >> 1][4 * j + 2 * (i & 1) + 1]));
             }
-            __syncwarp();   // the slot is rewritten by the next chunk
-          } else if (row_ok) {
-            if (whole_chunk) {
+          }
+        } else if (vec) {
+          // As bfloat16 a lane's two columns are one word; the four lanes of a row exchange theirs (a 4 x 4
+          // transpose) so that each stores eight columns, 16 bytes.  Word k of a block is group k of one
+          // row set, or with two groups per chunk, group k & 1 of two row sets.
+          constexpr int kSets = 4 / kGroups;   // row sets in a block
+          const int q = lane & 3;
+#pragma unroll
+          for (int b = 0; b < 4 / kSets; ++b) {
+            if (b * kSets >= row_sets) break;
+            uint32_t w[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              const int i = b * kSets + k / kGroups, j = k % kGroups;
+              w[k] = pack_bf16x2(__uint_as_float(acc[i >> 1][4 * j + 2 * (i & 1)]), __uint_as_float(acc[i >> 1][4 * j + 2 * (i & 1) + 1]));
+            }
+            quad_transpose(w, q);
+            int row = rows[b * kSets];
+            if (kSets == 2 && q >= 2) row = rows[b * kSets + kSets - 1];
+            const int c = col0 + 8 * (q % kGroups);
+            if (row >= 0 && c < args.cout)
+              *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(args.out) + static_cast<size_t>(row) * args.out_ld + c) =
+                  make_uint4(w[0], w[1], w[2], w[3]);
+          }
+        } else {
+          // Rows whose pitch or start rules wide accesses out, element by element.
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            if (i >= row_sets || rows[i] < 0) continue;
+            const size_t at = static_cast<size_t>(rows[i]) * args.out_ld + col0 + col_in;
+#pragma unroll
+            for (int k = 0; k < 2 * kGroups; ++k) {
+              const int j = k >> 1, e = k & 1;
+              if (col0 + 8 * j + col_in + e >= args.cout) continue;
+              const float v = __uint_as_float(acc[i >> 1][4 * j + 2 * (i & 1) + e]);
               if (args.out_half) {
-                uint4* op = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(args.out) + out_off + col0);
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                  uint4 w;
-                  w.x = pack_bf16x2(v[2 * q].x, v[2 * q].y);
-                  w.y = pack_bf16x2(v[2 * q].z, v[2 * q].w);
-                  w.z = pack_bf16x2(v[2 * q + 1].x, v[2 * q + 1].y);
-                  w.w = pack_bf16x2(v[2 * q + 1].z, v[2 * q + 1].w);
-                  op[q] = w;
-                }
+                reinterpret_cast<uint16_t*>(args.out)[at + 8 * j + e] = static_cast<uint16_t>(pack_bf16x2(v, 0.f));
               } else {
-                float4* op = reinterpret_cast<float4*>(args.out + out_off + col0);
-#pragma unroll
-                for (int j = 0; j < 8; ++j) op[j] = v[j];
-              }
-            } else {
-              auto residual_at = [&](int c) {
-                if (kHalf) {
-                  return __uint_as_float(static_cast<uint32_t>(reinterpret_cast<const uint16_t*>(ep.residual)[res_off + c])
-                                         << 16);
-                }
-                return ep.residual[res_off + c];
-              };
-              auto store_at = [&](int c, float value) {
-                if (args.out_half) {
-                  reinterpret_cast<uint16_t*>(args.out)[out_off + c] = static_cast<uint16_t>(pack_bf16x2(value, 0.f));
-                } else {
-                  args.out[out_off + c] = value;
-                }
-              };
-#pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                const int c = col0 + j * 4;
-                if (c >= args.cout) break;
-                float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (has_res) {
-                  r.x = residual_at(c);
-                  if (c + 1 < args.cout) r.y = residual_at(c + 1);
-                  if (c + 2 < args.cout) r.z = residual_at(c + 2);
-                  if (c + 3 < args.cout) r.w = residual_at(c + 3);
-                }
-                float4 v = act_mode == 1   ? finish4(ActTag<1>(), j, r, has_res)
-                           : act_mode == 0 ? finish4(ActTag<0>(), j, r, has_res)
-                                           : finish4(ActTag<2>(), j, r, has_res);
-                if (ep.round_tf32) round4(v);
-                store_at(c, v.x);
-                if (c + 1 < args.cout) store_at(c + 1, v.y);
-                if (c + 2 < args.cout) store_at(c + 2, v.z);
-                if (c + 3 < args.cout) store_at(c + 3, v.w);
+                args.out[at + 8 * j + e] = v;
               }
             }
           }
         }
+        MCB200_TRACE_CHUNK();
       }
-      // All of this warp's reads of the accumulator are complete: hand it back.
-      if (ew == 0 && lane == 0) MCB200_TRACE(3);
-      tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) {
-        if (kPair) {
-          mbar_arrive_cluster(tmem_empty_leader + static_cast<uint32_t>(ab) * 8u);
-        } else {
-          mbar_arrive(&tmem_empty_bar[ab]);
-        }
-      }
+      if (!handed) hand_back();
+#pragma unroll
+      for (int i = 0; i < 4; ++i) rows[i] = next_rows[i];
     }
-    if (staged && lane == 0) tma_store_wait_read<0>();
+    if (kStaged && lane == 0) tma_store_wait_read<0>();
     __syncwarp();
   }
 
@@ -1494,19 +1575,19 @@ bool small_tiles(int cout, long long m, int k_iters, int taps, int halo_rows, in
 }
 
 // Tile map for the staged epilogue over a row-major matrix with row pitch `ld`
-// (elements), boxes of 32 columns and an epilogue warp's rows (32 or 16): fp32 with the 128-byte swizzle, or bfloat16 (64-byte
+// (elements), boxes of 32 rows x 32 columns: fp32 with the 128-byte swizzle, or bfloat16 (64-byte
 // box rows) with the 64-byte swizzle.  The rows are split as (group, row in
 // group): ordinary tiles use one group of all rows; row mode uses one group per
 // output row of an image so that a tile never spills into the next row.
 CUresult encode_tile_map(CUtensorMap* map, const void* base, bool half, int cols, int ld, long long rows_per_group,
-                         long long groups, int box_rows) {
+                         long long groups) {
   const DriverApi& api = driver_api();
   const cuuint64_t es = half ? 2 : 4;
   const cuuint64_t dims[3] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows_per_group),
                               static_cast<cuuint64_t>(groups)};
   const cuuint64_t strides[2] = {static_cast<cuuint64_t>(ld) * es,
                                  static_cast<cuuint64_t>(ld) * es * static_cast<cuuint64_t>(rows_per_group)};
-  const cuuint32_t box[3] = {32, static_cast<cuuint32_t>(box_rows), 1};
+  const cuuint32_t box[3] = {32, 32, 1};
   const cuuint32_t estr[3] = {1, 1, 1};
   return api.tiled(map, half ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
                    const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -1514,10 +1595,10 @@ CUresult encode_tile_map(CUtensorMap* map, const void* base, bool half, int cols
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
 }
 
-template <int BN, int kMode, bool kPair, bool kHalf>
+template <int BN, int kMode, bool kPair, bool kHalf, bool kStaged = false>
 cudaError_t launch_variant(const mcb200_conv_plan* plan, ConvTcArgs args, cudaStream_t stream) {
   using Plan = SmemPlan<BN, kMode, kPair>;
-  auto kernel = conv_tc_kernel<BN, kMode, kPair, kHalf>;
+  auto kernel = conv_tc_kernel<BN, kMode, kPair, kHalf, kStaged>;
   // The large-shared-memory opt-in is per device: do it once for each device
   // this process launches on.  What the ring may use is the CTA limit minus the
   // kernel's static shared memory (barriers, per-column tables).
@@ -1558,28 +1639,9 @@ cudaError_t launch_variant(const mcb200_conv_plan* plan, ConvTcArgs args, cudaSt
   const int sms = (dev >= 0 && dev < 64 && sm_count[dev] > 0) ? sm_count[dev] : 148;
   const long long workers_max = kPair ? sms / 2 : sms;
   const unsigned workers = static_cast<unsigned>(tiles < workers_max ? tiles : workers_max);
-  // Staging slots per epilogue warp.  With a residual: three where tiles are so short that the
-  // ring needs little (load, work and store of consecutive chunks overlap), else two.  Without:
-  // one, and the ring takes the rest.  (Two slots for short or single tiles were the rule until
-  // interleaved runs on one GPU showed one slot to be as quick or quicker on every layer of the
-  // three benchmark networks: ResNet-50 1.963 -> 1.946 ms per pass, MobileNet-v1 0.778 -> 0.776,
-  // SSD300 5.00 -> 4.98; a 7 x 7 first layer keeps eight activation tiles in flight instead of six.)
-  const int k_units = args.k_iters * (kHalf ? 2 : 1);   // in 32-channel steps, the unit the rules were measured in
-  args.slots = args.ep.residual != nullptr ? (k_units <= 4 ? 3 : 2) : 1;
-  args.res_depth = 1;
-  if (args.ep.residual == nullptr) {
-    const char* force = getenv("MCB200_SLOTS");   // experiments: "1" / "2"
-    if (force && (force[0] == '1' || force[0] == '2')) args.slots = force[0] - '0';
-  } else {
-    const char* force_slots = getenv("MCB200_RES_SLOTS");   // experiments: "2" .. "8"
-    const char* force_depth = getenv("MCB200_RES_DEPTH");   // experiments: "1" .. slots - 1
-    if (force_slots && atoi(force_slots) >= 2 && atoi(force_slots) <= kMaxSlots) args.slots = atoi(force_slots);
-    if (force_depth && atoi(force_depth) >= 1) args.res_depth = atoi(force_depth);
-    if (args.res_depth > args.slots - 1) args.res_depth = args.slots - 1;
-  }
-  const int slot_bytes = (kHalf && args.out_half) ? 2048 : 4096;
-  int stage_bytes = Plan::kStageBytes;
-  int staging_bytes = Plan::staging_bytes(args.slots, slot_bytes);
+  // A stage: sub-tiles of activations, then of weights.
+  args.stage_b_offset = Plan::kSub * (args.tile_rows == kSmallM && kMode != kModeRows ? kSmallM : kBlockM) * kBlockK * 4;
+  args.stage_bytes = args.stage_b_offset + Plan::kSub * Plan::kTileBBytes;
   int resident_bytes = 0;
   if (kMode == kModeRows) {
     // One N tile: every M tile multiplies the same kh weight tiles; they stay in shared memory
@@ -1588,25 +1650,13 @@ cudaError_t launch_variant(const mcb200_conv_plan* plan, ConvTcArgs args, cudaSt
     const char* off = getenv("MCB200_ROWS_RESIDENT");   // "0": stream the weights with the activations (experiments)
     if (plan->shape.cout <= BN && all_rows <= 56 * 1024 && !(off && off[0] == '0')) resident_bytes = static_cast<int>(all_rows);
     args.resident_b_bytes = resident_bytes;
-    args.stage_b_offset = kTileABytes;
-    args.stage_bytes = resident_bytes ? kTileABytes : kTileABytes + Plan::kTileBBytes;
-    stage_bytes = args.stage_bytes;
+    if (resident_bytes) args.stage_bytes = args.stage_b_offset;
   }
   if (kMode == kModeHalo) {
-    // A stage = the pixel strip (rounded up to the 1024-byte swizzle period) + the weight tiles of
-    // the kw taps of one filter row.  The epilogue stores from registers: no staging.
+    // The pixel strip (rounded up to the 1024-byte swizzle period) + the weight tiles of the kw taps of
+    // one filter row.
     args.stage_b_offset = (args.a_bytes + 1023) / 1024 * 1024;
     args.stage_bytes = args.stage_b_offset + plan->shape.kw * Plan::kTileBBytes;
-    stage_bytes = args.stage_bytes;
-    args.halo_staged = (args.vec_store && !args.out_half && !getenv("MCB200_HALO_DIRECT_STORES")) ? 1 : 0;
-    args.slots = 1;
-    staging_bytes = args.halo_staged ? Plan::staging_bytes(1, 4096) : 0;
-  }
-  if (kMode == kModePhase) {
-    // Results pass through one slot per warp, as in halo mode.
-    args.halo_staged = args.vec_store ? 1 : 0;
-    args.slots = 1;
-    staging_bytes = args.halo_staged ? Plan::staging_bytes(1, 4096) : 0;
   }
   {
     // At most 64 prefetch instructions per tile (long-K tiles take long enough for the ring).
@@ -1618,15 +1668,23 @@ cudaError_t launch_variant(const mcb200_conv_plan* plan, ConvTcArgs args, cudaSt
     const char* pf = getenv("MCB200_L2_PREFETCH");
     args.l2_prefetch = (kMode != kModeRows && kMode != kModePhase && count <= 64 && pf && pf[0] == '1') ? 1 : 0;
   }
-  int stages = (dynamic_limit - 1024 - staging_bytes - resident_bytes) / stage_bytes;
+  int staging_bytes = 0;
+  args.slots = args.res_depth = 1;
+  if (kStaged) {
+    // Slots per epilogue warp.  With a residual three where tiles are so short that the ring needs little (load,
+    // work and store of consecutive chunks overlap), else two.  Without: one, and the ring takes the rest.
+    if (args.ep.residual != nullptr) args.slots = args.k_iters * (kHalf ? 2 : 1) <= 4 ? 3 : 2;
+    staging_bytes = kEpilogueWarps * args.slots * ((kHalf && args.out_half) ? 2048 : 4096);
+  }
+  int stages = (dynamic_limit - 1024 - resident_bytes - staging_bytes) / args.stage_bytes;
   if (stages > kMaxStages) stages = kMaxStages;
   if (stages < 2) return cudaErrorInvalidConfiguration;
   args.stages = stages;
-  const int dynamic_bytes = stages * stage_bytes + staging_bytes + resident_bytes + 1024;
+  const int dynamic_bytes = stages * args.stage_bytes + resident_bytes + staging_bytes + 1024;   // + alignment slack
   const CUtensorMap* ma = reinterpret_cast<const CUtensorMap*>(plan->tma_a);
   const CUtensorMap* mb = reinterpret_cast<const CUtensorMap*>(plan->tma_b);
-  const CUtensorMap* mo = reinterpret_cast<const CUtensorMap*>(plan->tma_out);
-  const CUtensorMap* mr = reinterpret_cast<const CUtensorMap*>(plan->tma_res);
+  const CUtensorMap* mo = kStaged ? reinterpret_cast<const CUtensorMap*>(plan->tma_out) : ma;
+  const CUtensorMap* mr = kStaged && args.ep.residual ? reinterpret_cast<const CUtensorMap*>(plan->tma_res) : ma;
   cudaError_t launched;
   {
     TimedLaunch timed(stream);
@@ -1650,6 +1708,24 @@ cudaError_t launch_variant(const mcb200_conv_plan* plan, ConvTcArgs args, cudaSt
   }
   count_launch();
   return launched;
+}
+
+// Whether results leave through shared memory as TMA tiles rather than straight from registers.  Registers are
+// the shorter way (a chunk of 32 x 32 takes its warp 1100 cycles, 1400 through shared memory, and the ring gets the
+// staging's bytes), which counts where a CTA has one tile whose end nothing overlaps.  But a store
+// instruction then writes 32 bytes of eight rows each, and with many tiles in flight that, not HBM, is the limit
+// (64 -> 256 columns and a residual on 56 x 56 maps, batch 64: 107 us against 80; 32 -> 64 on 112 x 112, no residual: 71
+// against 59), as 16 bytes of a bfloat16 row are.  Per launch in fp32 without a residual and with one tile per
+// CTA: 1024 -> 2048 at 14 x 14, stride 2, batch 64 37 -> 33 us, 2048 -> 512 on 7 x 7 27 -> 23.
+bool staged_epilogue(const mcb200_conv_plan* plan, bool residual) {
+  const char* force = getenv("MCB200_STAGED");   // "0" / "1": override for experiments and tests
+  if (force && (force[0] == '0' || force[0] == '1')) return force[0] == '1';
+  const long long m_tiles = plan->im2col == kModeRows
+                                ? static_cast<long long>(plan->shape.n) * plan->shape.ho * ((plan->shape.wo + kBlockM - 1) / kBlockM)
+                                : (static_cast<long long>(plan->m) + kBlockM - 1) / kBlockM;
+  const long long tiles = m_tiles * ((plan->shape.cout + plan->block_n - 1) / plan->block_n);
+  const long long workers = plan->cta_pair ? 74 : 148, units = plan->cta_pair ? (tiles + 1) / 2 : tiles;
+  return residual || plan->operand_bf16 || units > 3 * workers || plan->k_iters < 16;
 }
 
 }  // namespace
@@ -1955,13 +2031,14 @@ int launch_core(mcb200_conv_plan* plan, void* out, bool out_half, int out_ld, co
   }
   if (a.ep.act == 2 && !a.ep.prelu) return -2;
   a.status = status;
-  // The staged epilogue needs 16-byte aligned rows; otherwise plain stores are used.
-  const bool out_ok = (out_ld % (out_half ? 8 : 4) == 0) && ((reinterpret_cast<uintptr_t>(out) & 15) == 0);
-  const bool res_ok = !a.ep.residual || ((a.ep.residual_ld % (half ? 8 : 4) == 0) && a.ep.residual_ld >= plan->shape.cout &&
-                                         ((reinterpret_cast<uintptr_t>(a.ep.residual) & 15) == 0));
-  a.tma_epilogue = (out_ok && res_ok) ? 1 : 0;
-  a.vec_store = a.tma_epilogue;
-  a.l2_prefetch = a.halo_staged = 0;
+  // Wide accesses of the epilogue: pairs of fp32 columns, eight bfloat16 columns of the output, pairs of the residual.
+  const int wide = out_half ? 8 : 2;
+  const bool out_ok = out_ld % wide == 0 && a.cout % wide == 0 &&
+                      (reinterpret_cast<uintptr_t>(out) & (out_half ? 15 : 7)) == 0;
+  const bool res_ok = !a.ep.residual || (a.ep.residual_ld % 2 == 0 && a.cout % 2 == 0 &&
+                                         (reinterpret_cast<uintptr_t>(a.ep.residual) & (half ? 3 : 7)) == 0);
+  a.vec_store = out_ok && res_ok ? 1 : 0;
+  a.l2_prefetch = 0;
   a.wait_limit = g_wait_limit_cycles;
   a.constants_settled = (flags & MCB200_CONV_CONSTANTS_SETTLED) ? 1 : 0;
   a.drop_last_weight_load = t_drop_weight_load;
@@ -1971,14 +2048,11 @@ int launch_core(mcb200_conv_plan* plan, void* out, bool out_half, int out_ld, co
   a.wp = plan->shape.wo;
   a.stage_bytes = a.stage_b_offset = a.resident_b_bytes = 0;
   if (plan->im2col == kModeHalo) {
-    // Tiles are pieces of the virtual output grid: results leave through plain (128-bit) stores.
-    a.tma_epilogue = 0;
     a.m = plan->m_virtual;
     a.wp = plan->m_virtual / (plan->shape.n * plan->shape.ho);
   }
   a.phase_tiles = 0;
   if (phases) {
-    a.tma_epilogue = 0;
     a.phase_tiles = (a.cout + plan->block_n - 1) / plan->block_n;
     a.phase_stride_h = phases->stride_h;
     a.phase_stride_w = phases->stride_w;
@@ -1994,14 +2068,19 @@ int launch_core(mcb200_conv_plan* plan, void* out, bool out_half, int out_ld, co
   const int halo_rows = plan->im2col == kModeHalo ? (plan->shape.kw - 1) * plan->shape.dil_w : 0;
   const bool cut = plan->im2col == kModeMatrix || plan->im2col == kModeIm2col || plan->im2col == kModeHalo;
   const bool small = cut && plan->strip_rows - halo_rows == kSmallM;
-  const int warp_rows = small ? kSmallM / 4 : kBlockM / 4;
-  if (a.tma_epilogue) {
+  // Tile maps of output and residual: rows of 16-byte cells, one box per sub-tile.
+  const bool tma_ok = out_ld % (out_half ? 8 : 4) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0 &&
+                      (!a.ep.residual || (a.ep.residual_ld % (half ? 8 : 4) == 0 && a.ep.residual_ld >= a.cout &&
+                                          (reinterpret_cast<uintptr_t>(a.ep.residual) & 15) == 0));
+  const bool cut_or_rows = plan->im2col == kModeMatrix || plan->im2col == kModeIm2col || plan->im2col == kModeRows;
+  const bool staged = cut_or_rows && !small && tma_ok && staged_epilogue(plan, a.ep.residual != nullptr);
+  if (staged) {
     const bool rows = plan->im2col == kModeRows;
     const long long per_group = rows ? plan->shape.wo : plan->m;
     const long long groups = rows ? static_cast<long long>(plan->shape.n) * plan->shape.ho : 1;
     if (plan->out_ptr != out || plan->out_ld != out_ld || plan->out_bf16 != a.out_half) {
       if (encode_tile_map(reinterpret_cast<CUtensorMap*>(plan->tma_out), out, out_half, plan->shape.cout, out_ld,
-                          per_group, groups, warp_rows) != CUDA_SUCCESS)
+                          per_group, groups) != CUDA_SUCCESS)
         return -4;
       plan->out_ptr = static_cast<const float*>(out);
       plan->out_ld = out_ld;
@@ -2009,7 +2088,7 @@ int launch_core(mcb200_conv_plan* plan, void* out, bool out_half, int out_ld, co
     }
     if (a.ep.residual && (plan->res_ptr != a.ep.residual || plan->res_ld != a.ep.residual_ld)) {
       if (encode_tile_map(reinterpret_cast<CUtensorMap*>(plan->tma_res), a.ep.residual, half, plan->shape.cout,
-                          a.ep.residual_ld, per_group, groups, warp_rows) != CUDA_SUCCESS)
+                          a.ep.residual_ld, per_group, groups) != CUDA_SUCCESS)
         return -5;
       plan->res_ptr = a.ep.residual;
       plan->res_ld = a.ep.residual_ld;
@@ -2021,25 +2100,27 @@ int launch_core(mcb200_conv_plan* plan, void* out, bool out_half, int out_ld, co
   a.a_bytes = (plan->im2col == kModeHalo ? plan->strip_rows : a.tile_rows) * kBlockK * 4;
   cudaError_t e = cudaErrorInvalidValue;
   const int mode = plan->im2col;
+#define MCB200_STAGED(BN, MODE, PAIR, HALF)                                               \
+  (staged ? launch_variant<BN, MODE, PAIR, HALF, true>(plan, a, st) : launch_variant<BN, MODE, PAIR, HALF>(plan, a, st))
 #define MCB200_DISPATCH(BN)                                                               \
-  e = mode == kModeRows     ? launch_variant<BN, kModeRows, false, false>(plan, a, st)    \
-      : mode == kModeIm2col ? launch_variant<BN, kModeIm2col, false, false>(plan, a, st)  \
+  e = mode == kModeRows     ? MCB200_STAGED(BN, kModeRows, false, false)                  \
+      : mode == kModeIm2col ? MCB200_STAGED(BN, kModeIm2col, false, false)                \
       : mode == kModeHalo   ? launch_variant<BN, kModeHalo, false, false>(plan, a, st)    \
       : mode == kModePhase  ? launch_variant<BN, kModePhase, false, false>(plan, a, st)   \
-                            : launch_variant<BN, kModeMatrix, false, false>(plan, a, st)
+                            : MCB200_STAGED(BN, kModeMatrix, false, false)
 #define MCB200_DISPATCH_PAIR(BN)                                                          \
-  e = mode == kModeIm2col ? launch_variant<BN, kModeIm2col, true, false>(plan, a, st)     \
+  e = mode == kModeIm2col ? MCB200_STAGED(BN, kModeIm2col, true, false)                   \
       : mode == kModeHalo ? launch_variant<BN, kModeHalo, true, false>(plan, a, st)       \
-                          : launch_variant<BN, kModeMatrix, true, false>(plan, a, st)
+                          : MCB200_STAGED(BN, kModeMatrix, true, false)
 #define MCB200_DISPATCH_NARROW(HALF)                                                      \
   e = mode == kModeIm2col   ? launch_variant<32, kModeIm2col, false, HALF>(plan, a, st)   \
       : mode == kModeHalo   ? launch_variant<32, kModeHalo, false, HALF>(plan, a, st)     \
       : mode == kModeMatrix ? launch_variant<32, kModeMatrix, false, HALF>(plan, a, st)   \
                             : cudaErrorInvalidValue
 #define MCB200_DISPATCH_HALF(BN, PAIR)                                                    \
-  e = mode == kModeIm2col ? launch_variant<BN, kModeIm2col, PAIR, true>(plan, a, st)      \
+  e = mode == kModeIm2col ? MCB200_STAGED(BN, kModeIm2col, PAIR, true)                    \
       : mode == kModeHalo ? launch_variant<BN, kModeHalo, PAIR, true>(plan, a, st)        \
-                          : launch_variant<BN, kModeMatrix, PAIR, true>(plan, a, st)
+                          : MCB200_STAGED(BN, kModeMatrix, PAIR, true)
   if (half) {
     if (mode == kModeRows) return -3;
     if (plan->cta_pair) {
@@ -2079,6 +2160,7 @@ int launch_core(mcb200_conv_plan* plan, void* out, bool out_half, int out_ld, co
 #undef MCB200_DISPATCH_HALF
 #undef MCB200_DISPATCH_PAIR
 #undef MCB200_DISPATCH
+#undef MCB200_STAGED
   return static_cast<int>(e);
 }
 

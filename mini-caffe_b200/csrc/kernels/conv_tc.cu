@@ -69,6 +69,9 @@ constexpr int kModeRows = 2;     // <= 4 channels: one filter row of 8 pixels x 
 constexpr int kModeHalo = 3;     // stride-1 filters wider than one tap: the taps of a filter row share one pixel strip
 constexpr int kModePhase = 4;    // deconvolution: one im2col convolution per phase of the output grid
 constexpr int kMaxPhase = 4;      // largest deconvolution stride that phase mode takes
+constexpr int kOutDirect = 0;     // how results leave: from registers,
+constexpr int kOutStaged = 1;     // through shared memory as TMA tiles,
+constexpr int kOutSplit = 2;      // or after a cluster's CTAs have added up their segments of the sum over K
 constexpr int kMaxHaloRows = 16; // extra strip rows ((kw - 1) * dilation) the halo mode takes
 
 struct ConvTcArgs {
@@ -95,6 +98,7 @@ struct ConvTcArgs {
   int wp;
   int stage_bytes;     // activation tiles (halo mode: a strip) + weight tiles
   int stage_b_offset;  // where the weight tiles start inside a stage
+  int segment_shift;   // the sum over K is made in 1, 2 or 4 segments (log2), then added up: see segment_shift_of
   int slots;           // staged epilogue: staging slots per warp, 1 or 2; 2 .. kMaxSlots when a residual is added
   int res_depth;       // and residual sub-tiles a warp requests ahead of the one it works on (1 .. slots - 1)
   int vec_store;       // the rows of output and residual can be accessed two fp32 (eight bfloat16) columns at a time
@@ -233,11 +237,15 @@ struct RingPos {
 // kind::f16, fp32 accumulation); a k-iteration then covers 64 channels in the
 // same 128-byte rows.  Independently of that, the output is stored as fp32 or
 // as bfloat16 (args.out_half).
-template <int BN, int kMode, bool kPair, bool kHalf, bool kStaged>
+template <int BN, int kMode, bool kPair, bool kHalf, int kOut>
 __global__ void __launch_bounds__(kThreads, 1)
 conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const __grid_constant__ CUtensorMap map_out, const __grid_constant__ CUtensorMap map_res,
                const ConvTcArgs args) {
+  constexpr bool kStaged = kOut == kOutStaged, kSplit = kOut == kOutSplit;
+  // Layers whose sum over K is cut into segments (segment_shift_of): these modes.
+  constexpr bool kSegments = !kStaged && (kMode == kModeMatrix || kMode == kModeIm2col || kMode == kModeHalo);
+  static_assert(!kSplit || (kSegments && !kPair), "a split tile belongs to one CTA per segment");
   static_assert(!(kStaged && (BN < 64 || kMode == kModeHalo || kMode == kModePhase)), "a staged tile is one box of the output");
   static_assert(!(kPair && kMode == kModeRows), "row mode runs unpaired");
   static_assert(!(kHalf && kMode == kModeRows), "row mode takes fp32 images");
@@ -272,6 +280,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   const bool resident_b = kMode == kModeRows && args.resident_b_bytes > 0;
   uint8_t* resident = tiles + stages * stage_bytes;   // stages are multiples of 1024 bytes: so is this address
   uint8_t* staging_base = resident + (kMode == kModeRows ? args.resident_b_bytes : 0);
+  uint8_t* exchange = staging_base;                   // split form: the cluster's partial sums of what this CTA finishes
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -290,8 +299,19 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   // A work unit is an M tile (or a pair of neighbouring M tiles) x an N tile;
   // `worker` is the CTA (or pair) index among `workers`.
   const uint32_t rank = kPair ? cluster_cta_rank() : 0u;
-  const int worker = kPair ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
-  const int workers = kPair ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
+  // A cluster of 2 or 4 CTAs splits a tile's sum over K, a segment each.
+  const uint32_t split_rank = kSplit ? cluster_cta_rank() : 0u;
+  const int cluster_shift = kPair ? 1 : kSplit ? args.segment_shift : 0;
+  const int worker = static_cast<int>(blockIdx.x) >> cluster_shift;
+  const int workers = static_cast<int>(gridDim.x) >> cluster_shift;
+  // This CTA's k-iterations, and the first of segment i.
+  const int segments = kSegments ? 1 << args.segment_shift : 1;
+  auto segment_begin = [&](int i) { return kSegments ? (args.k_iters * i) >> args.segment_shift : i * args.k_iters; };
+  const int first_segment = kSplit ? static_cast<int>(split_rank) : 0;
+  const int k_begin = segment_begin(first_segment), k_end = kSplit ? segment_begin(first_segment + 1) : args.k_iters;
+  // Tensor memory: an accumulator per segment, twice where that fits (one is then drained while the other fills).
+  const int accumulators = kSegments && !kSplit && segments * BN > 256 ? 1 : 2;
+  const int acc_columns = kSplit ? BN : segments * BN;
   const int m_units = kPair ? (m_tiles + 1) >> 1 : m_tiles;
   const int num_tiles = n_tiles * m_units;
   auto unit_to_mt = [&](int unit) { return kPair ? 2 * unit + static_cast<int>(rank) : unit; };
@@ -323,12 +343,12 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     }
   }
   if (warp == kWarpMma) {
-    tmem_alloc(&tmem_base_slot, 2 * BN);
+    tmem_alloc(&tmem_base_slot, static_cast<uint32_t>(accumulators * acc_columns));
     tmem_relinquish();
   }
   tc_fence_before_sync();
-  if (kPair) {
-    cluster_sync_all();   // the peer's barriers are initialised before anything signals them
+  if (kPair || kSplit) {
+    cluster_sync_all();   // the peers run, and their barriers are initialised before anything signals them
   } else {
     __syncthreads();
   }
@@ -470,13 +490,25 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
         uint16_t off_w = off_w0;
         int row_h = base_h;
-        for (int k = 0; k < args.k_iters; k += Plan::kSub) {
+        if (kSplit && k_begin > 0) {   // the segment's first position inside the filter
+          const int tap = k_begin / args.c_blocks;
+          c0 = (k_begin - tap * args.c_blocks) * kElemsK;
+          if (kMode == kModeHalo) off_h = static_cast<uint16_t>(tap * args.dil_h);
+          if (kMode == kModeIm2col) {
+            off_h = static_cast<uint16_t>(tap / args.kw * args.dil_h);
+            sx = tap % args.kw;
+            off_w = static_cast<uint16_t>(sx * args.dil_w);
+          }
+        }
+        int segment = first_segment, segment_end = segment_begin(first_segment + 1), nsub = 0;
+        for (int k = k_begin; k < k_end; k += nsub) {
           if (!mbar_wait_bounded(&empty_bar[pos.stage], pos.parity ^ 1u, abort, wait_limit)) {
             alive = false;
             break;
           }
           MCB200_TRACE(0);
-          const int nsub = args.k_iters - k < Plan::kSub ? args.k_iters - k : Plan::kSub;
+          nsub = Plan::kSub == 1 ? 1 : min(segment_end - k, Plan::kSub);   // (a constant step keeps the loop short)
+          if (kSegments && k + nsub == segment_end) segment_end = segment_begin(++segment + 1);
           uint8_t* a_dst = tiles + pos.stage * stage_bytes;
           uint64_t* bar = &full_bar[pos.stage];
           const uint32_t bar_leader = full_bar_leader + static_cast<uint32_t>(pos.stage) * 8u;
@@ -563,17 +595,26 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
         int k0 = 0;
         int halo_cb = 0, halo_row_k0 = 0;   // halo mode: channel block and first packed-weight column of the filter row
-        for (int k = 0; k < args.k_iters; k += Plan::kSub) {
+        if (kSplit && kMode == kModeHalo) {
+          const int row = k_begin / args.c_blocks;
+          halo_cb = k_begin - row * args.c_blocks;
+          halo_row_k0 = row * args.kw * args.c_blocks * kElemsK;
+        } else if (kSplit) {
+          k0 = k_begin * kElemsK;
+        }
+        int segment = first_segment, segment_end = segment_begin(first_segment + 1), nsub = 0;
+        for (int k = k_begin; k < k_end; k += nsub) {
           if (!mbar_wait_bounded(&empty_bar[pos.stage], pos.parity ^ 1u, abort, wait_limit)) {
             alive = false;
             break;
           }
           MCB200_TRACE(1);
-          if (args.drop_last_weight_load && tile + workers >= num_tiles && k + Plan::kSub >= args.k_iters) {
+          nsub = Plan::kSub == 1 ? 1 : min(segment_end - k, Plan::kSub);   // (a constant step keeps the loop short)
+          if (kSegments && k + nsub == segment_end) segment_end = segment_begin(++segment + 1);
+          if (args.drop_last_weight_load && tile + workers >= num_tiles && k + nsub >= k_end) {
             alive = false;   // nothing arrives on this stage's barrier: every role's wait on it is bounded
             break;
           }
-          const int nsub = args.k_iters - k < Plan::kSub ? args.k_iters - k : Plan::kSub;
           uint8_t* b_dst = tiles + pos.stage * stage_bytes + stage_b_offset;
           uint64_t* bar = &full_bar[pos.stage];
           const uint32_t bar_leader = full_bar_leader + static_cast<uint32_t>(pos.stage) * 8u;
@@ -638,21 +679,22 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         tc_fence_after_sync();
       }
       for (int tile = worker; tile < num_tiles && alive; tile += workers, ++local) {
-        const int ab = local & 1;
-        const uint32_t use = static_cast<uint32_t>(local >> 1) & 1u;
+        const int ab = accumulators == 2 ? local & 1 : 0;
+        const uint32_t use = static_cast<uint32_t>(accumulators == 2 ? local >> 1 : local) & 1u;
         // The epilogue must have drained this accumulator (first use passes).
         if (!mbar_wait_bounded(&tmem_empty_bar[ab], use ^ 1u, abort, wait_limit)) break;
         tc_fence_after_sync();
-        const uint32_t tmem_acc = tmem_base + static_cast<uint32_t>(ab * BN);
+        uint32_t tmem_acc = tmem_base + static_cast<uint32_t>(ab * acc_columns);
         uint32_t accumulate = 0;
-        for (int k = 0; k < args.k_iters; k += Plan::kSub) {
+        int segment = first_segment, segment_end = segment_begin(first_segment + 1), nsub = 0;
+        for (int k = k_begin; k < k_end; k += nsub) {
           if (!mbar_wait_bounded(&full_bar[pos.stage], pos.parity, abort, wait_limit)) {
             alive = false;
             break;
           }
           tc_fence_after_sync();
           MCB200_TRACE(2);
-          const int nsub = args.k_iters - k < Plan::kSub ? args.k_iters - k : Plan::kSub;
+          nsub = Plan::kSub == 1 ? 1 : min(segment_end - k, Plan::kSub);   // (a constant step keeps the loop short)
           const uint32_t a_addr = tiles_addr + static_cast<uint32_t>(pos.stage * stage_bytes);
           uint64_t desc_a = umma_desc_k_sw128(a_addr);
           uint64_t desc_b = umma_desc_k_sw128(
@@ -715,6 +757,11 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             umma_commit(&empty_bar[pos.stage]);
           }
           MCB200_TRACE(2);
+          if (kSegments && k + nsub == segment_end) {   // the next segment sums in an accumulator of its own
+            segment_end = segment_begin(++segment + 1);
+            tmem_acc += BN;
+            accumulate = 0;
+          }
           pos.advance(stages);
         }
         if (alive) {
@@ -842,7 +889,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     int rows[4] = {-1, -1, -1, -1};
     if (!kStaged && worker < num_tiles) {
       tile_rows(worker, rows);
-      if (has_res) fetch_residual(rows, tile_n0(worker) + half * kChunk);
+      if (!kSplit && has_res) fetch_residual(rows, tile_n0(worker) + half * kChunk);
     }
 
     // Staged form.  A slot holds a 32 x 32 sub-tile: 4 KiB, or 2 KiB when residual and result are both bfloat16.
@@ -919,9 +966,9 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     bool alive = true;
     MCB200_TRACE_DECL;
     MCB200_TRACE_CHUNK_DECL;
-    for (int tile = worker; tile < num_tiles && alive; tile += workers, ++local) {
-      const int ab = local & 1;
-      const uint32_t use = static_cast<uint32_t>(local >> 1) & 1u;
+    for (int tile = worker; !kSplit && tile < num_tiles && alive; tile += workers, ++local) {
+      const int ab = accumulators == 2 ? local & 1 : 0;
+      const uint32_t use = static_cast<uint32_t>(accumulators == 2 ? local >> 1 : local) & 1u;
       // Where the tile lies, before the wait: the divisions cost a few hundred cycles.
       const int unit = tile / n_tiles;
       const int n0 = kMode == kModePhase ? tile_n0(tile) : (tile - unit * n_tiles) * BN;
@@ -955,7 +1002,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         if (!alive) break;
         ++table_fills[ab];
       }
-      const uint32_t tmem_acc = tmem_base + static_cast<uint32_t>(ab * BN) + (static_cast<uint32_t>(quad * 32) << 16);
+      const uint32_t tmem_acc = tmem_base + static_cast<uint32_t>(ab * acc_columns) + (static_cast<uint32_t>(quad * 32) << 16);
       const int next = tile + workers;
       int next_rows[4] = {-1, -1, -1, -1};
       // After the last read of this accumulator (and of the per-column tables) it goes back to the MMA
@@ -1151,6 +1198,20 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         tmem_load_16x256<kGroups>(tmem_acc + static_cast<uint32_t>(chunk * kChunk), acc[0]);
         if (row_sets > 2) tmem_load_16x256<kGroups>(tmem_acc + (16u << 16) + static_cast<uint32_t>(chunk * kChunk), acc[1]);
         tmem_load_wait();
+        // The segments' sums, first to last: the order in which a cluster that splits the tile adds them.
+#pragma unroll 1
+        for (int i = 1; kSegments && i < segments; ++i) {
+          uint32_t more[2][4 * kGroups];
+          const uint32_t at = tmem_acc + static_cast<uint32_t>(i * BN + chunk * kChunk);
+          tmem_load_16x256<kGroups>(at, more[0]);
+          if (row_sets > 2) tmem_load_16x256<kGroups>(at + (16u << 16), more[1]);
+          tmem_load_wait();
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int k = 0; k < 4 * kGroups; ++k)
+              acc[h][k] = __float_as_uint(__fadd_rn(__uint_as_float(acc[h][k]), __uint_as_float(more[h][k])));
+        }
         MCB200_TRACE_CHUNK();
         // v = acc * scale + shift (+ coeff * residual), then the activation, in place.  Activation and
         // residual are compile-time tags: with run-time tests inside, every value became its own chain of
@@ -1271,7 +1332,123 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       for (int i = 0; i < 4; ++i) rows[i] = next_rows[i];
     }
     if (kStaged && lane == 0) tma_store_wait_read<0>();
+    if (kSplit) {
+      // A cluster has one tile.  Each CTA sends every partial sum to the CTA that finishes it: of a chunk's four
+      // pieces (its groups of eight columns, or with two groups the upper and lower rows of each) CTA r of the
+      // cluster finishes pieces [r, r + 1) * 4 / segments.
+      constexpr int kOwn = kChunks > 1 ? kChunks / 2 : 1;   // chunks of a warp
+      const int n0 = tile_n0(worker);
+      const int pieces = 4 >> args.segment_shift;           // per CTA and chunk
+      const int words = kGroups == 4 ? row_sets : row_sets >> 1;   // row sets of a piece
+      // Place of a partial sum: [chunk][piece][source][row set][warp][lane], two floats each.
+      auto place = [&](int own, int piece, int source, int word) {
+        return smem_addr(exchange) +
+               8u * static_cast<uint32_t>((((((own * pieces + piece) << args.segment_shift) + source) * words + word) * kEpilogueWarps + ew) * 32 + lane);
+      };
+      alive = worker < num_tiles && __all_sync(0xffffffffu, mbar_wait_bounded(&tmem_full_bar[0], 0u, abort, wait_limit));
+      if (alive) alive = __all_sync(0xffffffffu, mbar_wait_bounded(&col_bar[0], 0u, abort, wait_limit));
+      if (alive) {
+        tc_fence_after_sync();
+#pragma unroll
+        for (int own = 0; own < kOwn; ++own) {
+          const int chunk = half + 2 * own;
+          if (chunk >= kChunks || n0 + chunk * kChunk >= args.cout) break;   // uniform across the warp
+          uint32_t acc[2][4 * kGroups];
+          const uint32_t at = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + static_cast<uint32_t>(chunk * kChunk);
+          tmem_load_16x256<kGroups>(at, acc[0]);
+          if (row_sets > 2) tmem_load_16x256<kGroups>(at + (16u << 16), acc[1]);
+          tmem_load_wait();
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            if (i >= row_sets) break;
+#pragma unroll
+            for (int j = 0; j < kGroups; ++j) {
+              const int lower = kGroups == 2 && i >= words ? 1 : 0;
+              const int piece = kGroups == 4 ? j : 2 * j + lower;
+              const int owner = piece >> (2 - args.segment_shift);
+              cluster_store(cluster_map(place(own, piece - owner * pieces, static_cast<int>(split_rank), i - lower * words),
+                                        static_cast<uint32_t>(owner)),
+                            __uint_as_float(acc[i >> 1][4 * j + 2 * (i & 1)]), __uint_as_float(acc[i >> 1][4 * j + 2 * (i & 1) + 1]));
+            }
+          }
+        }
+      }
+      // The partial sums are where they are finished (a CTA that gave up is here too: its status says so).
+      __syncwarp();
+      cluster_sync_all();
+#pragma unroll 1
+      for (int own = 0; alive && own < kOwn; ++own) {
+        const int chunk = half + 2 * own;
+        const int col0 = n0 + chunk * kChunk;
+        if (chunk >= kChunks || col0 >= args.cout) break;
+#pragma unroll 1
+        for (int piece = 0; piece < pieces; ++piece) {
+          const int which = static_cast<int>(split_rank) * pieces + piece;
+          const int lower = kGroups == 2 ? which & 1 : 0;
+          const int in_chunk = 8 * (kGroups == 4 ? which : which >> 1) + col_in;
+          const int c = col0 + in_chunk;
+          const float2 sc = *reinterpret_cast<const float2*>(&col_scale[0][chunk * kChunk + in_chunk]);
+          const float2 sh = *reinterpret_cast<const float2*>(&col_shift[0][chunk * kChunk + in_chunk]);
+          const float2 sl = *reinterpret_cast<const float2*>(&col_slope[0][chunk * kChunk + in_chunk]);
+#pragma unroll
+          for (int word = 0; word < 4; ++word) {
+            if (word >= words) break;
+            const int row = kGroups == 4 ? rows[word] : lower == 0 ? rows[word & 1] : rows[(word + words) & 3];
+            float v[2] = {0.f, 0.f};
+#pragma unroll
+            for (int source = 0; source < 4; ++source) {
+              if (source >= segments) break;
+              const float2 part = *reinterpret_cast<const float2*>(exchange + (place(own, piece, source, word) - smem_addr(exchange)));
+              v[0] = source == 0 ? part.x : __fadd_rn(v[0], part.x);
+              v[1] = source == 0 ? part.y : __fadd_rn(v[1], part.y);
+            }
+            if (row < 0 || c >= args.cout) continue;
+            const bool second = c + 1 < args.cout;
+            const size_t at = static_cast<size_t>(row) * args.out_ld + c;
+            v[0] = fmaf(v[0], sc.x, sh.x);
+            v[1] = fmaf(v[1], sc.y, sh.y);
+            if (has_res) {
+              const size_t r = static_cast<size_t>(row) * ep.residual_ld + c;
+              const uint16_t* narrow = reinterpret_cast<const uint16_t*>(ep.residual);
+              v[0] = fmaf(ep.residual_coeff, kHalf ? bf16_lo(narrow[r]) : ep.residual[r], v[0]);
+              if (second) v[1] = fmaf(ep.residual_coeff, kHalf ? bf16_lo(narrow[r + 1]) : ep.residual[r + 1], v[1]);
+            }
+            if (act_mode == 1) {
+              v[0] = fmaxf(v[0], 0.f);
+              v[1] = fmaxf(v[1], 0.f);
+            } else if (act_mode == 2) {
+              v[0] = v[0] > 0.f ? v[0] : v[0] * sl.x;
+              v[1] = v[1] > 0.f ? v[1] : v[1] * sl.y;
+            }
+            if (ep.round_tf32) {
+              v[0] = round_to_tf32(v[0]);
+              v[1] = round_to_tf32(v[1]);
+            }
+            if (args.out_half) {
+              uint16_t* dst = reinterpret_cast<uint16_t*>(args.out) + at;
+              const uint32_t w = pack_bf16x2(v[0], v[1]);
+              if (vec) {
+                *reinterpret_cast<uint32_t*>(dst) = w;
+              } else {
+                dst[0] = static_cast<uint16_t>(w);
+                if (second) dst[1] = static_cast<uint16_t>(w >> 16);
+              }
+            } else if (vec) {
+              *reinterpret_cast<float2*>(args.out + at) = make_float2(v[0], v[1]);
+            } else {
+              args.out[at] = v[0];
+              if (second) args.out[at + 1] = v[1];
+            }
+          }
+        }
+      }
+    }
     __syncwarp();
+  }
+
+  if (kSplit && warp < kFirstEpilogueWarp) {
+    __syncwarp();
+    cluster_sync_all();   // the other warps' is between their sending and finishing
   }
 
   // ------------------------------------------------------------ teardown
@@ -1286,7 +1463,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   }
   if (warp == kWarpMma) {
     tc_fence_after_sync();
-    tmem_dealloc(tmem_base, 2 * BN);
+    tmem_dealloc(tmem_base, static_cast<uint32_t>(accumulators * acc_columns));
   }
   if (threadIdx.x == 0 && abort_flag && args.status) *static_cast<volatile int*>(args.status) = 1;
 }
@@ -1435,16 +1612,16 @@ const DriverApi& driver_api() {
 // (operand bytes per iteration grow with BN) plus an epilogue proportional to BN.
 // Wide tiles re-read the activations less often, narrow tiles fill the machine
 // when there are few output pixels; take the cheapest of the three.
-int pick_block_n(int cout, long long m, int k_iters, double* cost_out = nullptr) {
+int pick_block_n(int cout, long long m, int k_iters, int widest) {
   const char* force = getenv("MCB200_BLOCK_N");   // "64" / "128" / "256": override for experiments and tests
-  if (force && !cost_out) {
+  if (force) {
     const int bn = atoi(force);
     if (bn == 64 || bn == 128 || bn == 256) return bn;
   }
   const long long m_tiles = (m + kBlockM - 1) / kBlockM;
   int best = 64;
   double best_cost = 0.0;
-  for (int bn = 64; bn <= 256; bn *= 2) {
+  for (int bn = 64; bn <= widest; bn *= 2) {
     if (bn > 64 && bn / 2 >= cout) break;   // wider than the layer: only padding
     const long long tiles = m_tiles * ((cout + bn - 1) / bn);
     const long long waves = (tiles + 147) / 148;
@@ -1460,7 +1637,6 @@ int pick_block_n(int cout, long long m, int k_iters, double* cost_out = nullptr)
       best_cost = cost;
     }
   }
-  if (cost_out) *cost_out = best_cost;
   return best;
 }
 
@@ -1527,20 +1703,60 @@ int pick_cta_pair(int block_n, long long m, int k_iters) {
   return (block_n >= 128 && m > kBlockM && k_iters >= (block_n == 256 ? 16 : 17)) ? 1 : 0;
 }
 
+// Segments of the sum over K, as a power of two: each is summed on its own and they are added first to last.  By the
+// layer's geometry alone: an image's result must not depend on the batch it runs in.
+// Worth it from 128 MMA steps per tap chain on.  Large batches pay: such a tile needs a tensor-memory accumulator per
+// segment, so with four segments it is at most 128 columns wide and the tile behind it waits until it is drained.  Hence
+// four on maps of at most 64 pixels, and up to 256 pixels from 256 steps; else two (256 columns, as without).
+// Measured, four / two / one segments: 3 x 3 at 256 channels on 14 x 14, batch 64 39.4 / 35.3 / 35.2 us, ResNet-50 with
+// one image 397 / 411 / 454 us per pass; 1024 -> 256 on 14 x 14, batch 64 29.2 / 25.1 / 25.0; 3 x 3 at 512 channels on
+// 19 x 19, batch 32 84 / 78 / 78, one image in bfloat16 18.5 / 20.4 / 28.7.
+int segment_shift_of(const mcb200_conv_shape& s, int mode, int k_iters) {
+  if (s.group != 1 || (mode != kModeMatrix && mode != kModeIm2col && mode != kModeHalo)) return 0;
+  const long long steps = static_cast<long long>(k_iters) * (mode == kModeHalo ? s.kw : 1) * kMmaPerBlock;
+  const long long positions = static_cast<long long>(s.ho) * s.wo;
+  if (positions <= 64) return steps >= 128 ? 2 : 0;
+  if (positions <= 256) return steps >= 256 ? 2 : steps >= 128 ? 1 : 0;
+  return positions <= 400 && steps >= 512 ? 1 : 0;
+}
+
+// CTAs that run at one time as clusters of 1 << shift, one tile each.
+int split_capacity(int shift) { return shift == 2 ? 128 : 144; }
+
+int m_tile_of(const mcb200_conv_plan& p) {
+  const int halo_rows = p.im2col == kModeHalo ? (p.shape.kw - 1) * p.shape.dil_w : 0;
+  const bool cut = p.im2col == kModeMatrix || p.im2col == kModeIm2col || p.im2col == kModeHalo;
+  return cut && p.strip_rows - halo_rows == kSmallM ? kSmallM : kBlockM;
+}
+
+int plan_segment_shift(const mcb200_conv_plan& p) {
+  int shift = segment_shift_of(p.shape, p.im2col, p.k_iters);
+  while ((p.block_n << shift) > 512) --shift;   // a tile width that was asked for (MCB200_BLOCK_N)
+  return shift;
+}
+
+// Whether a cluster's CTAs make a tile's segments side by side: where all tiles then still run at one time.
+bool split_launch(const mcb200_conv_plan& p, int shift) {
+  const char* off = getenv("MCB200_SPLIT");   // "0": one CTA makes all segments (experiments and tests)
+  if (off && off[0] == '0') return false;
+  const long long bm = m_tile_of(p);
+  const long long tiles = (p.m_virtual + bm - 1) / bm * ((p.shape.cout + p.block_n - 1) / p.block_n);
+  return shift > 0 && !p.cta_pair && p.block_n <= 128 && (tiles << shift) <= split_capacity(shift);
+}
+
 // Layers of a single image (or a few) have fewer tiles than the chip has SMs, and the time of one is the chain of its
-// k-iterations.  A K step of 128 x 64 costs the chain about 65 cycles at 256 -> 256 channels, 3 x 3, 14 x 14
-// (operand reads and the copies' writes share the shared-memory port), one of 64 x 32 about 52.  So where the tiles
+// k-iterations.  An MMA takes at least 41 cycles with 64 rows and 52 with 128, however few its columns, and the
+// copies' writes to shared memory get in the way of its operand reads.  So where the tiles
 // all run at once anyway, cut them to 64 pixels and 64 or 32 columns: more SMs, each with a half or a third of the
-// bytes per iteration and half the epilogue.  The sums over K keep their order: the results are the same bits.
-// Returns whether the layer runs in 64-row tiles, with *block_n (and *pair = 0) set to match.
-// The cost model, in cycles: per K step (M + N) / 4, four steps per tap; the copies at 128 bytes per cycle, 0.4 of
-// them not hidden; 1500 per epilogue chunk of a warp.  Only up to one tile per SM: with more, ordinary tiles
+// bytes per iteration and half the epilogue; and where the sum over K has segments, let a cluster make them side by side.
+// The results are the same bits.  Returns whether the layer runs in 64-row tiles, with *block_n and *pair set to match.
+// The cost model, in cycles: four MMAs per k-iteration and tap, half of the copies' bytes at 128 per cycle, 1500 per 64
+// columns of epilogue, 2000 for the exchange of a split tile.  Only up to one tile per SM: with more, ordinary tiles
 // fill the chip; and only for a tenth less by the model, which is no better than that.
-// Measured, one image: 3 x 3 at 256 channels on 14 x 14 17.3 -> 14.0 us, at 512 on 7 x 7 27.7 -> 21.9, 512 -> 512
-// on 19 x 19 in bfloat16 15.6 -> 13; per pass ResNet-50 629 -> 552, SSD300 in bfloat16 771 -> 687, MobileNet-v1
-// 216 -> 199; ResNet-50 at batch 16 in bfloat16 803 -> 788.  (A chip that other nets keep busy has no SMs to give: three
-// threads with a ResNet-50 at batch 16 each make 22 400 images/s so and 22 900 without.)
-bool small_tiles(int cout, long long m, int k_iters, int taps, int halo_rows, int* block_n, int* pair) {
+// Measured, one image (each launch on its own): 3 x 3 at 256 channels on 14 x 14 18.9 -> 12.8 us, at 512 on 7 x 7
+// 27.1 -> 14.8, 2048 -> 1000 classes 18.4 -> 12.3; per pass ResNet-50 496 -> 406, SSD300 in bfloat16 620 -> 495.  (A chip
+// that other nets keep busy has no SMs to give.)
+bool small_tiles(int cout, long long m, int k_iters, int taps, int halo_rows, int shift, int* block_n, int* pair) {
   const char* force = getenv("MCB200_BLOCK_M");   // "64" / "128": override for experiments and tests
   const bool forced = force && atoi(force) == kSmallM;
   const char* width = getenv("MCB200_BLOCK_N");
@@ -1552,26 +1768,29 @@ bool small_tiles(int cout, long long m, int k_iters, int taps, int halo_rows, in
   if (force || width || getenv("MCB200_CTA_PAIR")) return false;
   auto tiles_of = [&](int bm, int bn) { return ((m + bm - 1) / bm) * ((cout + bn - 1) / bn); };
   auto cost = [&](int bm, int bn, bool paired) {
+    const bool split = !paired && shift > 0 && bn <= 128 && (tiles_of(bm, bn) << shift) <= split_capacity(shift);
     const int b_rows = paired ? bn / 2 : bn;
-    double steps = taps * static_cast<double>(bm + b_rows);
-    if (bn > 64) steps = steps > 2.0 * taps * bn ? steps : 2.0 * taps * bn;   // the tensor pipe itself
-    return k_iters * (steps + 0.4 * (bm + halo_rows + taps * b_rows)) + 1500.0 * ((bn + 63) / 64);
+    const double floor = bm == kSmallM ? 40 : 50, pipe = bn / 2.0;
+    const double iter = taps * 4 * (pipe > floor ? pipe : floor) + 0.5 * (bm + halo_rows + taps * b_rows);
+    return (split ? k_iters >> shift : k_iters) * iter + 1500.0 * ((bn + 63) / 64) + (split ? 2000.0 : 0.0);
   };
   if (tiles_of(kBlockM, *block_n) > 148) return false;
-  const double now = cost(kBlockM, *block_n, *pair != 0);
-  double best = 0.9 * now;
-  bool found = false;
-  for (int bn = 64; bn >= 32; bn /= 2) {
-    if (tiles_of(kSmallM, bn) > 148) break;
-    const double c = cost(kSmallM, bn, false);
-    if (c < best) {
-      best = c;
-      *block_n = bn;
-      *pair = 0;
-      found = true;
+  double best = 0.9 * cost(kBlockM, *block_n, *pair != 0);
+  bool small = false;
+  for (int bm = kSmallM; bm <= kBlockM; bm *= 2) {
+    for (int bn = shift > 0 ? 128 : 64; bn >= 32; bn /= 2) {
+      if (tiles_of(bm, bn) > 148 || (bm == kBlockM && shift == 0)) break;
+      if (bn > 64 && (bm == kSmallM || bn / 2 >= cout)) continue;
+      const double c = cost(bm, bn, false);
+      if (c < best) {
+        best = c;
+        *block_n = bn;
+        *pair = 0;
+        small = bm == kSmallM;
+      }
     }
   }
-  return found;
+  return small;
 }
 
 // Tile map for the staged epilogue over a row-major matrix with row pitch `ld`
@@ -1595,10 +1814,11 @@ CUresult encode_tile_map(CUtensorMap* map, const void* base, bool half, int cols
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
 }
 
-template <int BN, int kMode, bool kPair, bool kHalf, bool kStaged = false>
+template <int BN, int kMode, bool kPair, bool kHalf, int kOut = kOutDirect>
 cudaError_t launch_variant(const mcb200_conv_plan* plan, ConvTcArgs args, cudaStream_t stream) {
+  constexpr bool kStaged = kOut == kOutStaged, kSplit = kOut == kOutSplit;
   using Plan = SmemPlan<BN, kMode, kPair>;
-  auto kernel = conv_tc_kernel<BN, kMode, kPair, kHalf, kStaged>;
+  auto kernel = conv_tc_kernel<BN, kMode, kPair, kHalf, kOut>;
   // The large-shared-memory opt-in is per device: do it once for each device
   // this process launches on.  What the ring may use is the CTA limit minus the
   // kernel's static shared memory (barriers, per-column tables).
@@ -1676,6 +1896,7 @@ cudaError_t launch_variant(const mcb200_conv_plan* plan, ConvTcArgs args, cudaSt
     if (args.ep.residual != nullptr) args.slots = args.k_iters * (kHalf ? 2 : 1) <= 4 ? 3 : 2;
     staging_bytes = kEpilogueWarps * args.slots * ((kHalf && args.out_half) ? 2048 : 4096);
   }
+  if (kSplit) staging_bytes = args.tile_rows * BN * 4;   // as many partial sums arrive at a CTA as its tile has cells
   int stages = (dynamic_limit - 1024 - resident_bytes - staging_bytes) / args.stage_bytes;
   if (stages > kMaxStages) stages = kMaxStages;
   if (stages < 2) return cudaErrorInvalidConfiguration;
@@ -1689,7 +1910,8 @@ cudaError_t launch_variant(const mcb200_conv_plan* plan, ConvTcArgs args, cudaSt
   {
     TimedLaunch timed(stream);
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(kPair ? workers * 2 : workers, 1, 1);
+    const unsigned cluster = kPair ? 2u : kSplit ? 1u << args.segment_shift : 1u;
+    cfg.gridDim = dim3((kSplit ? static_cast<unsigned>(tiles) : workers) * cluster, 1, 1);
     cfg.blockDim = dim3(kThreads, 1, 1);
     cfg.dynamicSmemBytes = static_cast<size_t>(dynamic_bytes);
     cfg.stream = stream;
@@ -1699,11 +1921,11 @@ cudaError_t launch_variant(const mcb200_conv_plan* plan, ConvTcArgs args, cudaSt
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = 2;
+    attr[1].val.clusterDim.x = cluster;
     attr[1].val.clusterDim.y = 1;
     attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = kPair ? 2 : 1;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
     launched = cudaLaunchKernelEx(&cfg, kernel, *ma, *mb, *mo, *mr, args);
   }
   count_launch();
@@ -1725,7 +1947,8 @@ bool staged_epilogue(const mcb200_conv_plan* plan, bool residual) {
                                 : (static_cast<long long>(plan->m) + kBlockM - 1) / kBlockM;
   const long long tiles = m_tiles * ((plan->shape.cout + plan->block_n - 1) / plan->block_n);
   const long long workers = plan->cta_pair ? 74 : 148, units = plan->cta_pair ? (tiles + 1) / 2 : tiles;
-  return residual || plan->operand_bf16 || units > 3 * workers || plan->k_iters < 16;
+  const bool one_column = plan->shape.cout <= plan->block_n;
+  return residual || plan->operand_bf16 || units > (one_column ? 3 : 1) * workers || plan->k_iters < 16;
 }
 
 }  // namespace
@@ -1875,11 +2098,12 @@ int plan_core(const mcb200_conv_shape* s, const void* in, const void* packed_w, 
   const bool grouped = s->group > 1;
   plan->c_blocks = grouped ? grouped_c_blocks(s, kelems, half ? 8 : 4) : (s->c + kelems - 1) / kelems;
   plan->k_iters = s->kh * s->kw * plan->c_blocks;
-  plan->block_n = grouped ? kGroupedBlockN : pick_block_n(s->cout, plan->m, plan->k_iters);
-  // The pairing rule was measured in 32-channel k-iterations; a bfloat16 k-iteration covers 64.
-  plan->cta_pair = grouped ? 0 : pick_cta_pair(plan->block_n, plan->m, plan->k_iters * (half ? 2 : 1));
   const bool pointwise = s->kh == 1 && s->kw == 1 && s->stride_h == 1 && s->stride_w == 1 && s->pad_h == 0 &&
                          s->pad_w == 0;
+  const int segments = segment_shift_of(plan->shape, pointwise ? kModeMatrix : kModeIm2col, plan->k_iters);
+  plan->block_n = grouped ? kGroupedBlockN : pick_block_n(s->cout, plan->m, plan->k_iters, segments > 1 ? 512 >> segments : 256);
+  // The pairing rule was measured in 32-channel k-iterations; a bfloat16 k-iteration covers 64.
+  plan->cta_pair = grouped ? 0 : pick_cta_pair(plan->block_n, plan->m, plan->k_iters * (half ? 2 : 1));
   plan->im2col = pointwise ? 0 : 1;
   plan->m_virtual = plan->m;
   plan->strip_rows = 0;
@@ -1920,7 +2144,7 @@ int plan_core(const mcb200_conv_shape* s, const void* in, const void* packed_w, 
   }
   const bool halo = plan->im2col == kModeHalo;
   const bool small = !grouped && small_tiles(s->cout, plan->m_virtual, plan->k_iters, halo ? s->kw : 1, halo ? halo_w : 0,
-                                             &plan->block_n, &plan->cta_pair);
+                                             segment_shift_of(plan->shape, plan->im2col, plan->k_iters), &plan->block_n, &plan->cta_pair);
   if (small) plan->strip_rows = kSmallM + (halo ? halo_w : 0);
 
   CUtensorMap* ma = reinterpret_cast<CUtensorMap*>(plan->tma_a);
@@ -2065,15 +2289,15 @@ int launch_core(mcb200_conv_plan* plan, void* out, bool out_half, int out_ld, co
     a.ho = phases->grid_h;
     a.wo = phases->grid_w;
   }
-  const int halo_rows = plan->im2col == kModeHalo ? (plan->shape.kw - 1) * plan->shape.dil_w : 0;
-  const bool cut = plan->im2col == kModeMatrix || plan->im2col == kModeIm2col || plan->im2col == kModeHalo;
-  const bool small = cut && plan->strip_rows - halo_rows == kSmallM;
+  const bool small = m_tile_of(*plan) == kSmallM;
+  a.segment_shift = plan_segment_shift(*plan);
+  const bool split = split_launch(*plan, a.segment_shift);
   // Tile maps of output and residual: rows of 16-byte cells, one box per sub-tile.
   const bool tma_ok = out_ld % (out_half ? 8 : 4) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0 &&
                       (!a.ep.residual || (a.ep.residual_ld % (half ? 8 : 4) == 0 && a.ep.residual_ld >= a.cout &&
                                           (reinterpret_cast<uintptr_t>(a.ep.residual) & 15) == 0));
   const bool cut_or_rows = plan->im2col == kModeMatrix || plan->im2col == kModeIm2col || plan->im2col == kModeRows;
-  const bool staged = cut_or_rows && !small && tma_ok && staged_epilogue(plan, a.ep.residual != nullptr);
+  const bool staged = cut_or_rows && !small && tma_ok && a.segment_shift == 0 && staged_epilogue(plan, a.ep.residual != nullptr);
   if (staged) {
     const bool rows = plan->im2col == kModeRows;
     const long long per_group = rows ? plan->shape.wo : plan->m;
@@ -2100,27 +2324,43 @@ int launch_core(mcb200_conv_plan* plan, void* out, bool out_half, int out_ld, co
   a.a_bytes = (plan->im2col == kModeHalo ? plan->strip_rows : a.tile_rows) * kBlockK * 4;
   cudaError_t e = cudaErrorInvalidValue;
   const int mode = plan->im2col;
-#define MCB200_STAGED(BN, MODE, PAIR, HALF)                                               \
-  (staged ? launch_variant<BN, MODE, PAIR, HALF, true>(plan, a, st) : launch_variant<BN, MODE, PAIR, HALF>(plan, a, st))
-#define MCB200_DISPATCH(BN)                                                               \
-  e = mode == kModeRows     ? MCB200_STAGED(BN, kModeRows, false, false)                  \
-      : mode == kModeIm2col ? MCB200_STAGED(BN, kModeIm2col, false, false)                \
-      : mode == kModeHalo   ? launch_variant<BN, kModeHalo, false, false>(plan, a, st)    \
-      : mode == kModePhase  ? launch_variant<BN, kModePhase, false, false>(plan, a, st)   \
-                            : MCB200_STAGED(BN, kModeMatrix, false, false)
-#define MCB200_DISPATCH_PAIR(BN)                                                          \
-  e = mode == kModeIm2col ? MCB200_STAGED(BN, kModeIm2col, true, false)                   \
-      : mode == kModeHalo ? launch_variant<BN, kModeHalo, true, false>(plan, a, st)       \
-                          : MCB200_STAGED(BN, kModeMatrix, true, false)
-#define MCB200_DISPATCH_NARROW(HALF)                                                      \
-  e = mode == kModeIm2col   ? launch_variant<32, kModeIm2col, false, HALF>(plan, a, st)   \
-      : mode == kModeHalo   ? launch_variant<32, kModeHalo, false, HALF>(plan, a, st)     \
-      : mode == kModeMatrix ? launch_variant<32, kModeMatrix, false, HALF>(plan, a, st)   \
+#define MCB200_OUT(BN, MODE, PAIR, HALF)                                                           \
+  (staged ? launch_variant<BN, MODE, PAIR, HALF, kOutStaged>(plan, a, st) : launch_variant<BN, MODE, PAIR, HALF>(plan, a, st))
+#define MCB200_DISPATCH(BN)                                                                        \
+  e = mode == kModeRows     ? MCB200_OUT(BN, kModeRows, false, false)                              \
+      : mode == kModeIm2col ? MCB200_OUT(BN, kModeIm2col, false, false)                            \
+      : mode == kModeHalo   ? launch_variant<BN, kModeHalo, false, false>(plan, a, st)             \
+      : mode == kModePhase  ? launch_variant<BN, kModePhase, false, false>(plan, a, st)            \
+                            : MCB200_OUT(BN, kModeMatrix, false, false)
+#define MCB200_DISPATCH_PAIR(BN)                                                                   \
+  e = mode == kModeIm2col ? MCB200_OUT(BN, kModeIm2col, true, false)                               \
+      : mode == kModeHalo ? launch_variant<BN, kModeHalo, true, false>(plan, a, st)                \
+                          : MCB200_OUT(BN, kModeMatrix, true, false)
+#define MCB200_DISPATCH_NARROW(HALF)                                                               \
+  e = mode == kModeIm2col   ? launch_variant<32, kModeIm2col, false, HALF>(plan, a, st)            \
+      : mode == kModeHalo   ? launch_variant<32, kModeHalo, false, HALF>(plan, a, st)              \
+      : mode == kModeMatrix ? launch_variant<32, kModeMatrix, false, HALF>(plan, a, st)            \
                             : cudaErrorInvalidValue
-#define MCB200_DISPATCH_HALF(BN, PAIR)                                                    \
-  e = mode == kModeIm2col ? MCB200_STAGED(BN, kModeIm2col, PAIR, true)                    \
-      : mode == kModeHalo ? launch_variant<BN, kModeHalo, PAIR, true>(plan, a, st)        \
-                          : MCB200_STAGED(BN, kModeMatrix, PAIR, true)
+#define MCB200_DISPATCH_HALF(BN, PAIR)                                                             \
+  e = mode == kModeIm2col ? MCB200_OUT(BN, kModeIm2col, PAIR, true)                                \
+      : mode == kModeHalo ? launch_variant<BN, kModeHalo, PAIR, true>(plan, a, st)                 \
+                          : MCB200_OUT(BN, kModeMatrix, PAIR, true)
+#define MCB200_DISPATCH_SPLIT(BN, HALF)                                                            \
+  e = mode == kModeIm2col ? launch_variant<BN, kModeIm2col, false, HALF, kOutSplit>(plan, a, st)   \
+      : mode == kModeHalo ? launch_variant<BN, kModeHalo, false, HALF, kOutSplit>(plan, a, st)     \
+                          : launch_variant<BN, kModeMatrix, false, HALF, kOutSplit>(plan, a, st)
+  if (split) {
+    switch (plan->block_n * 2 + (half ? 1 : 0)) {
+      case 64: MCB200_DISPATCH_SPLIT(32, false); break;
+      case 65: MCB200_DISPATCH_SPLIT(32, true); break;
+      case 128: MCB200_DISPATCH_SPLIT(64, false); break;
+      case 129: MCB200_DISPATCH_SPLIT(64, true); break;
+      case 256: MCB200_DISPATCH_SPLIT(128, false); break;
+      case 257: MCB200_DISPATCH_SPLIT(128, true); break;
+      default: return -3;
+    }
+    return static_cast<int>(e);
+  }
   if (half) {
     if (mode == kModeRows) return -3;
     if (plan->cta_pair) {
@@ -2160,7 +2400,8 @@ int launch_core(mcb200_conv_plan* plan, void* out, bool out_half, int out_ld, co
 #undef MCB200_DISPATCH_HALF
 #undef MCB200_DISPATCH_PAIR
 #undef MCB200_DISPATCH
-#undef MCB200_STAGED
+#undef MCB200_OUT
+#undef MCB200_DISPATCH_SPLIT
   return static_cast<int>(e);
 }
 
@@ -2384,7 +2625,7 @@ extern "C" int mcb200_deconv_tc_plan(const mcb200_conv_shape* deconv, const floa
     plan->off_w[f] = static_cast<unsigned char>(f < sw ? x.first[f] - x.lowest : 0);
   }
   // The phases multiply the tiles like so many more output pixels.
-  conv.block_n = pick_block_n(d.cout, static_cast<long long>(conv.m) * sh * sw, conv.k_iters);
+  conv.block_n = pick_block_n(d.cout, static_cast<long long>(conv.m) * sh * sw, conv.k_iters, 256);
   CUtensorMap* ma = reinterpret_cast<CUtensorMap*>(conv.tma_a);
   CUtensorMap* mb = reinterpret_cast<CUtensorMap*>(conv.tma_b);
   const cuuint64_t pix = static_cast<cuuint64_t>(d.c_stride) * 4;
@@ -2538,7 +2779,7 @@ extern "C" int mcb200_conv_rows_plan(const mcb200_conv_shape* s, const float* pa
   plan->strip_rows = 0;
   plan->c_blocks = 1;
   plan->k_iters = s->kh;
-  plan->block_n = pick_block_n(s->cout, plan->m, plan->k_iters);
+  plan->block_n = pick_block_n(s->cout, plan->m, plan->k_iters, 256);
   plan->im2col = kModeRows;
   // (Measured and dropped: a strip form that sorts the padded row into stride_w planes, loads a
   // filter row's pixels once (four to seven times fewer bytes out of L2) and lets the tensor core

@@ -181,8 +181,8 @@ __device__ __forceinline__ void grid_launch_dependents() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// ---------------------------------------------------------------- CTA pairs
-// Two CTAs of a cluster (ranks 0 and 1) that run one tcgen05.mma.cta_group::2
+// ---------------------------------------------------------------- clusters, CTA pairs
+// A pair are two CTAs of a cluster (ranks 0 and 1) that run one tcgen05.mma.cta_group::2
 // between them.  Rank 0 issues the MMAs; barriers that both CTAs signal live in
 // rank 0's shared memory and are addressed through the cluster window.
 
@@ -203,6 +203,12 @@ __device__ __forceinline__ uint32_t cluster_map(uint32_t local, uint32_t rank) {
   uint32_t r;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
   return r;
+}
+
+// Two floats into the shared memory of a CTA of the cluster (cluster-window address); the receiver may read them
+// after a cluster_sync_all().
+__device__ __forceinline__ void cluster_store(uint32_t cluster_addr, float a, float b) {
+  asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(cluster_addr), "f"(a), "f"(b) : "memory");
 }
 
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster_addr) {

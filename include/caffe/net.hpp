@@ -88,6 +88,8 @@ class CAFFE_API Net {
   void PlanParts();
   /*! \brief steps that only rename axes in front of a Concat are left out */
   void AbsorbViews();
+  /*! \brief two layers of one input run in one launch */
+  void MergeSiblings();
   void ForwardInParts();
 
   string name_;

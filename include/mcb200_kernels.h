@@ -118,6 +118,21 @@ int mcb200_conv_tc_launch(mcb200_conv_plan* plan, float* out, int out_ld,
 int mcb200_conv_tc_launch_flags(mcb200_conv_plan* plan, void* out, int out_is_bf16, int out_ld,
                                 const mcb200_epilogue* ep, int flags, int* status, void* stream);
 
+/* Two layers of the same input and geometry (SSD's two heads on a map, a projection beside the first layer of a
+ * bottleneck) in one launch.  The plan is that of one layer of `begin` + (the second's) output columns,
+ * whose packed weights hold the first layer's rows, zero rows up to `begin` (a multiple of 32) and the second's;
+ * ep->scale / shift run over these columns too.  ep->act (0 or 1, no slope) is the first layer's activation;
+ * no residual.  The plan's shape must not be a row-mode one.                                    */
+typedef struct mcb200_conv_second {
+  int begin;        /* first column of the second layer          */
+  int first_cout;   /* columns of the first, at most `begin`     */
+  void* out;        /* of the same element type as the first's   */
+  int out_ld;
+  int act;          /* 0 none, 1 ReLU                            */
+} mcb200_conv_second;
+int mcb200_conv_tc_launch_two(mcb200_conv_plan* plan, void* out, int out_is_bf16, int out_ld, const mcb200_epilogue* ep,
+                              const mcb200_conv_second* second, int flags, int* status, void* stream);
+
 /* Every wait of the convolution kernel on a hardware barrier is bounded: after `cycles` SM clock
  * cycles (default 2e9, about a second) the CTA raises an abort flag, its roles leave their loops,
  * copies in flight get a bounded grace period, tensor memory is freed and *status is set to 1;

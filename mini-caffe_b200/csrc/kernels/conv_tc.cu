@@ -85,6 +85,13 @@ struct ConvTcArgs {
   int ho, wo;
   int stride_h, stride_w, pad_h, pad_w, dil_h, dil_w;
   mcb200_epilogue ep;
+  // Two layers of one input in one launch: columns from second_begin on (a multiple of 32; past every column where
+  // there is one layer) are the second layer's, with an output of its own.  cout counts both.
+  int second_begin;
+  int first_cout;    // columns of the first output
+  float* second_out;
+  int second_ld;
+  int second_act;    // 0 none, 1 ReLU
   int* status;
   int tile_rows;     // rows of an M tile: 128 or 64, in row mode min(output width, 128)
   int row_segments;  // row mode: M tiles per output row of an image (ceil(output width / tile_rows))
@@ -245,6 +252,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   constexpr bool kStaged = kOut == kOutStaged, kSplit = kOut == kOutSplit;
   // Layers whose sum over K is cut into segments (segment_shift_of): these modes.
   constexpr bool kSegments = !kStaged && (kMode == kModeMatrix || kMode == kModeIm2col || kMode == kModeHalo);
+  constexpr bool kTwo = kMode == kModeMatrix || kMode == kModeIm2col || kMode == kModeHalo;   // may hold two layers
   static_assert(!kSplit || (kSegments && !kPair), "a split tile belongs to one CTA per segment");
   static_assert(!(kStaged && (BN < 64 || kMode == kModeHalo || kMode == kModePhase)), "a staged tile is one box of the output");
   static_assert(!(kPair && kMode == kModeRows), "row mode runs unpaired");
@@ -1136,9 +1144,10 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             for (int j = 0; j < 8; ++j) v[j] = finish4(act_tag, j, r[j], true);
           }
         };
-        if (act_mode == 1) {
+        const int act = (kTwo && col0 >= args.second_begin) ? args.second_act : act_mode;
+        if (act == 1) {
           fill(Tag<1>());
-        } else if (act_mode == 0) {
+        } else if (act == 0) {
           fill(Tag<0>());
         } else {
           fill(Tag<2>());
@@ -1184,7 +1193,12 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) {
-          tma_store_3d(&map_out, slot_ptr(slot), col0, box_row, box_image);   // clipped at the row's (the matrix's) end
+          // clipped at the row's (the matrix's) end; a launch of two layers has no residual
+          if ((kTwo && col0 >= args.second_begin)) {
+            tma_store_3d(&map_res, slot_ptr(slot), col0 - args.second_begin, box_row, box_image);
+          } else {
+            tma_store_3d(&map_out, slot_ptr(slot), col0, box_row, box_image);
+          }
           tma_store_commit();
         }
         MCB200_TRACE_CHUNK();
@@ -1213,6 +1227,13 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
               acc[h][k] = __float_as_uint(__fadd_rn(__uint_as_float(acc[h][k]), __uint_as_float(more[h][k])));
         }
         MCB200_TRACE_CHUNK();
+        // Which layer's columns these are.
+        const bool second = (kTwo && col0 >= args.second_begin);
+        const int act = second ? args.second_act : act_mode;
+        float* const out = second ? args.second_out : args.out;
+        const int out_ld = second ? args.second_ld : args.out_ld;
+        const int side0 = second ? col0 - args.second_begin : col0;
+        const int side_cout = second ? args.cout - args.second_begin : args.first_cout;
         // v = acc * scale + shift (+ coeff * residual), then the activation, in place.  Activation and
         // residual are compile-time tags: with run-time tests inside, every value became its own chain of
         // small basic blocks, each exposing its latencies; as straight-line code the chains overlap.
@@ -1249,9 +1270,9 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           } else {
             finish(Tag<2>(), Tag<1>());
           }
-        } else if (act_mode == 1) {
+        } else if (act == 1) {
           finish(Tag<1>(), Tag<0>());
-        } else if (act_mode == 0) {
+        } else if (act == 0) {
           finish(Tag<0>(), Tag<0>());
         } else {
           finish(Tag<2>(), Tag<0>());
@@ -1275,10 +1296,10 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             if (i >= row_sets || rows[i] < 0) continue;
-            float* dst = args.out + static_cast<size_t>(rows[i]) * args.out_ld + col0 + col_in;
+            float* dst = out + static_cast<size_t>(rows[i]) * out_ld + side0 + col_in;
 #pragma unroll
             for (int j = 0; j < kGroups; ++j) {
-              if (col0 + 8 * j + col_in < args.cout)
+              if (side0 + 8 * j + col_in < side_cout)
                 *reinterpret_cast<float2*>(dst + 8 * j) =
                     make_float2(__uint_as_float(acc[i >> 1][4 * j + 2 * (i & 1)]), __uint_as_float(acc[i >> 1][4 * j + 2 * (i & 1) + 1]));
             }
@@ -1301,9 +1322,9 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             quad_transpose(w, q);
             int row = rows[b * kSets];
             if (kSets == 2 && q >= 2) row = rows[b * kSets + kSets - 1];
-            const int c = col0 + 8 * (q % kGroups);
-            if (row >= 0 && c < args.cout)
-              *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(args.out) + static_cast<size_t>(row) * args.out_ld + c) =
+            const int c = side0 + 8 * (q % kGroups);
+            if (row >= 0 && c < side_cout)
+              *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(out) + static_cast<size_t>(row) * out_ld + c) =
                   make_uint4(w[0], w[1], w[2], w[3]);
           }
         } else {
@@ -1311,16 +1332,16 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             if (i >= row_sets || rows[i] < 0) continue;
-            const size_t at = static_cast<size_t>(rows[i]) * args.out_ld + col0 + col_in;
+            const size_t at = static_cast<size_t>(rows[i]) * out_ld + side0 + col_in;
 #pragma unroll
             for (int k = 0; k < 2 * kGroups; ++k) {
               const int j = k >> 1, e = k & 1;
-              if (col0 + 8 * j + col_in + e >= args.cout) continue;
+              if (side0 + 8 * j + col_in + e >= side_cout) continue;
               const float v = __uint_as_float(acc[i >> 1][4 * j + 2 * (i & 1) + e]);
               if (args.out_half) {
-                reinterpret_cast<uint16_t*>(args.out)[at + 8 * j + e] = static_cast<uint16_t>(pack_bf16x2(v, 0.f));
+                reinterpret_cast<uint16_t*>(out)[at + 8 * j + e] = static_cast<uint16_t>(pack_bf16x2(v, 0.f));
               } else {
-                args.out[at + 8 * j + e] = v;
+                out[at + 8 * j + e] = v;
               }
             }
           }
@@ -1386,7 +1407,12 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           const int which = static_cast<int>(split_rank) * pieces + piece;
           const int lower = kGroups == 2 ? which & 1 : 0;
           const int in_chunk = 8 * (kGroups == 4 ? which : which >> 1) + col_in;
-          const int c = col0 + in_chunk;
+          const bool second = (kTwo && col0 >= args.second_begin);
+          const int act = second ? args.second_act : act_mode;
+          float* const out = second ? args.second_out : args.out;
+          const int out_ld = second ? args.second_ld : args.out_ld;
+          const int side_cout = second ? args.cout - args.second_begin : args.first_cout;
+          const int c = (second ? col0 - args.second_begin : col0) + in_chunk;
           const float2 sc = *reinterpret_cast<const float2*>(&col_scale[0][chunk * kChunk + in_chunk]);
           const float2 sh = *reinterpret_cast<const float2*>(&col_shift[0][chunk * kChunk + in_chunk]);
           const float2 sl = *reinterpret_cast<const float2*>(&col_slope[0][chunk * kChunk + in_chunk]);
@@ -1402,9 +1428,9 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
               v[0] = source == 0 ? part.x : __fadd_rn(v[0], part.x);
               v[1] = source == 0 ? part.y : __fadd_rn(v[1], part.y);
             }
-            if (row < 0 || c >= args.cout) continue;
-            const bool second = c + 1 < args.cout;
-            const size_t at = static_cast<size_t>(row) * args.out_ld + c;
+            if (row < 0 || c >= side_cout) continue;
+            const bool second = c + 1 < side_cout;
+            const size_t at = static_cast<size_t>(row) * out_ld + c;
             v[0] = fmaf(v[0], sc.x, sh.x);
             v[1] = fmaf(v[1], sc.y, sh.y);
             if (has_res) {
@@ -1413,10 +1439,10 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
               v[0] = fmaf(ep.residual_coeff, kHalf ? bf16_lo(narrow[r]) : ep.residual[r], v[0]);
               if (second) v[1] = fmaf(ep.residual_coeff, kHalf ? bf16_lo(narrow[r + 1]) : ep.residual[r + 1], v[1]);
             }
-            if (act_mode == 1) {
+            if (act == 1) {
               v[0] = fmaxf(v[0], 0.f);
               v[1] = fmaxf(v[1], 0.f);
-            } else if (act_mode == 2) {
+            } else if (act == 2) {
               v[0] = v[0] > 0.f ? v[0] : v[0] * sl.x;
               v[1] = v[1] > 0.f ? v[1] : v[1] * sl.y;
             }
@@ -1425,7 +1451,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
               v[1] = round_to_tf32(v[1]);
             }
             if (args.out_half) {
-              uint16_t* dst = reinterpret_cast<uint16_t*>(args.out) + at;
+              uint16_t* dst = reinterpret_cast<uint16_t*>(out) + at;
               const uint32_t w = pack_bf16x2(v[0], v[1]);
               if (vec) {
                 *reinterpret_cast<uint32_t*>(dst) = w;
@@ -1434,10 +1460,10 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 if (second) dst[1] = static_cast<uint16_t>(w >> 16);
               }
             } else if (vec) {
-              *reinterpret_cast<float2*>(args.out + at) = make_float2(v[0], v[1]);
+              *reinterpret_cast<float2*>(out + at) = make_float2(v[0], v[1]);
             } else {
-              args.out[at] = v[0];
-              if (second) args.out[at + 1] = v[1];
+              out[at] = v[0];
+              if (second) out[at + 1] = v[1];
             }
           }
         }
@@ -1905,7 +1931,7 @@ cudaError_t launch_variant(const mcb200_conv_plan* plan, ConvTcArgs args, cudaSt
   const CUtensorMap* ma = reinterpret_cast<const CUtensorMap*>(plan->tma_a);
   const CUtensorMap* mb = reinterpret_cast<const CUtensorMap*>(plan->tma_b);
   const CUtensorMap* mo = kStaged ? reinterpret_cast<const CUtensorMap*>(plan->tma_out) : ma;
-  const CUtensorMap* mr = kStaged && args.ep.residual ? reinterpret_cast<const CUtensorMap*>(plan->tma_res) : ma;
+  const CUtensorMap* mr = kStaged && (args.ep.residual || args.second_out) ? reinterpret_cast<const CUtensorMap*>(plan->tma_res) : ma;
   cudaError_t launched;
   {
     TimedLaunch timed(stream);
@@ -2194,7 +2220,7 @@ int plan_core(const mcb200_conv_shape* s, const void* in, const void* packed_w, 
 }
 
 int launch_core(mcb200_conv_plan* plan, void* out, bool out_half, int out_ld, const mcb200_epilogue* ep, int* status,
-                void* stream, int flags = 0, const mcb200_deconv_plan* phases = nullptr);
+                void* stream, int flags = 0, const mcb200_deconv_plan* phases = nullptr, const mcb200_conv_second* second = nullptr);
 
 }  // namespace
 
@@ -2224,11 +2250,17 @@ extern "C" int mcb200_conv_tc_launch_bf16(mcb200_conv_plan* plan, void* out, int
   return launch_core(plan, out, out_is_bf16 != 0, out_ld, ep, status, stream);
 }
 
+extern "C" int mcb200_conv_tc_launch_two(mcb200_conv_plan* plan, void* out, int out_is_bf16, int out_ld, const mcb200_epilogue* ep,
+                                         const mcb200_conv_second* second, int flags, int* status, void* stream) {
+  if (!second) return -1;
+  return launch_core(plan, out, out_is_bf16 != 0, out_ld, ep, status, stream, flags, nullptr, second);
+}
+
 namespace {
 
 int launch_core(mcb200_conv_plan* plan, void* out, bool out_half, int out_ld, const mcb200_epilogue* ep, int* status,
-                void* stream, int flags, const mcb200_deconv_plan* phases) {
-  if (!plan || !out || out_ld < plan->shape.cout) return -1;
+                void* stream, int flags, const mcb200_deconv_plan* phases, const mcb200_conv_second* second) {
+  if (!plan || !out || out_ld < (second ? second->first_cout : plan->shape.cout)) return -1;
   const bool half = plan->operand_bf16 != 0;
   ConvTcArgs a;
   a.out = static_cast<float*>(out);
@@ -2254,11 +2286,30 @@ int launch_core(mcb200_conv_plan* plan, void* out, bool out_half, int out_ld, co
     a.ep.residual_coeff = 1.f;
   }
   if (a.ep.act == 2 && !a.ep.prelu) return -2;
+  a.second_begin = 0x7fffffff;
+  a.first_cout = a.cout;
+  a.second_out = nullptr;
+  a.second_ld = a.second_act = 0;
+  if (second) {
+    const int columns = a.cout - second->begin;
+    if (second->begin % 32 != 0 || second->first_cout < 1 || second->first_cout > second->begin || columns < 1 || !second->out ||
+        second->out_ld < columns || a.ep.residual || a.ep.act > 1 || a.ep.slope != 0.f || second->act < 0 || second->act > 1 ||
+        plan->shape.group != 1 || plan->im2col == kModeRows || phases)
+      return -9;
+    a.second_begin = second->begin;
+    a.first_cout = second->first_cout;
+    a.second_out = static_cast<float*>(second->out);
+    a.second_ld = second->out_ld;
+    a.second_act = second->act;
+  }
   a.status = status;
   // Wide accesses of the epilogue: pairs of fp32 columns, eight bfloat16 columns of the output, pairs of the residual.
   const int wide = out_half ? 8 : 2;
-  const bool out_ok = out_ld % wide == 0 && a.cout % wide == 0 &&
-                      (reinterpret_cast<uintptr_t>(out) & (out_half ? 15 : 7)) == 0;
+  auto wide_ok = [&](const void* to, int ld, int columns) {
+    return ld % wide == 0 && columns % wide == 0 && (reinterpret_cast<uintptr_t>(to) & (out_half ? 15 : 7)) == 0;
+  };
+  const bool out_ok = wide_ok(out, out_ld, a.first_cout) &&
+                      (!second || wide_ok(second->out, second->out_ld, a.cout - second->begin));
   const bool res_ok = !a.ep.residual || (a.ep.residual_ld % 2 == 0 && a.cout % 2 == 0 &&
                                          (reinterpret_cast<uintptr_t>(a.ep.residual) & (half ? 3 : 7)) == 0);
   a.vec_store = out_ok && res_ok ? 1 : 0;
@@ -2293,7 +2344,8 @@ int launch_core(mcb200_conv_plan* plan, void* out, bool out_half, int out_ld, co
   a.segment_shift = plan_segment_shift(*plan);
   const bool split = split_launch(*plan, a.segment_shift);
   // Tile maps of output and residual: rows of 16-byte cells, one box per sub-tile.
-  const bool tma_ok = out_ld % (out_half ? 8 : 4) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0 &&
+  auto cells_ok = [&](const void* to, int ld) { return ld % (out_half ? 8 : 4) == 0 && (reinterpret_cast<uintptr_t>(to) & 15) == 0; };
+  const bool tma_ok = cells_ok(out, out_ld) && (!second || cells_ok(second->out, second->out_ld)) &&
                       (!a.ep.residual || (a.ep.residual_ld % (half ? 8 : 4) == 0 && a.ep.residual_ld >= a.cout &&
                                           (reinterpret_cast<uintptr_t>(a.ep.residual) & 15) == 0));
   const bool cut_or_rows = plan->im2col == kModeMatrix || plan->im2col == kModeIm2col || plan->im2col == kModeRows;
@@ -2302,13 +2354,21 @@ int launch_core(mcb200_conv_plan* plan, void* out, bool out_half, int out_ld, co
     const bool rows = plan->im2col == kModeRows;
     const long long per_group = rows ? plan->shape.wo : plan->m;
     const long long groups = rows ? static_cast<long long>(plan->shape.n) * plan->shape.ho : 1;
-    if (plan->out_ptr != out || plan->out_ld != out_ld || plan->out_bf16 != a.out_half) {
-      if (encode_tile_map(reinterpret_cast<CUtensorMap*>(plan->tma_out), out, out_half, plan->shape.cout, out_ld,
+    const bool new_out = plan->out_ptr != out || plan->out_ld != out_ld || plan->out_bf16 != a.out_half;
+    if (new_out) {
+      if (encode_tile_map(reinterpret_cast<CUtensorMap*>(plan->tma_out), out, out_half, a.first_cout, out_ld,
                           per_group, groups) != CUDA_SUCCESS)
         return -4;
       plan->out_ptr = static_cast<const float*>(out);
       plan->out_ld = out_ld;
       plan->out_bf16 = a.out_half;
+    }
+    if (second && (plan->res_ptr != second->out || plan->res_ld != second->out_ld || plan->out_bf16 != a.out_half || new_out)) {
+      if (encode_tile_map(reinterpret_cast<CUtensorMap*>(plan->tma_res), second->out, out_half, a.cout - second->begin,
+                          second->out_ld, per_group, groups) != CUDA_SUCCESS)
+        return -5;
+      plan->res_ptr = static_cast<const float*>(second->out);
+      plan->res_ld = second->out_ld;
     }
     if (a.ep.residual && (plan->res_ptr != a.ep.residual || plan->res_ld != a.ep.residual_ld)) {
       if (encode_tile_map(reinterpret_cast<CUtensorMap*>(plan->tma_res), a.ep.residual, half, plan->shape.cout,

@@ -131,6 +131,11 @@ class Layer {
   // the part-th piece of a pass; the pieces of a pass cover the batch in order.
   virtual double PartSeconds(const vector<Blob*>& bottom, const vector<Blob*>& top, bool first_of_net) const { return 0; }
   inline void ForwardImages(const vector<Blob*>& bottom, const vector<Blob*>& top, int first, int count, int part);
+  // ---- two layers of one input in one launch ----
+  // AcceptsSibling: as shaped, fused and stored now, `other` can run with this layer, on the same bottom.  The
+  // net's decision: with a sibling, Forward gets that layer's top behind its own and fills both.
+  virtual bool AcceptsSibling(const Layer* other) const { return false; }
+  virtual void SetSibling(Layer* other) {}
   // The net's word that no later layer of the pass reads this layer's tops: the pass ends by
   // bringing them to the host, so the layer may as well write them there.
   virtual void SetTopsEndOnHost(bool on_host) {}

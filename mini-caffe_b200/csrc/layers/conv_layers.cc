@@ -216,20 +216,67 @@ void ConvolutionLayer::Reshape(const vector<Blob*>& bottom, const vector<Blob*>&
   for (size_t i = 0; i < top.size(); ++i) top[i]->Reshape(shape_.n, shape_.cout, shape_.ho, shape_.wo);
 }
 
+bool ConvolutionLayer::AcceptsSibling(const Layer* layer) const {
+  const ConvolutionLayer* other = dynamic_cast<const ConvolutionLayer*>(layer);
+  if (!other || other == this) return false;
+  auto plain = [](const ConvolutionLayer& l) {
+    ActivationSpec act;
+    if (l.tail_.activation && (!l.tail_.activation->AsActivation(&act) || act.kind != 1 || act.slope != 0.f)) return false;
+    return l.path_ == kTensorCore && !l.use_rows_ && l.shape_.group == 1 && !l.tail_.residual;
+  };
+  const mcb200_conv_shape &a = shape_, &b = other->shape_;
+  // Short sums whose results fill HBM gain little from reading their input once, and lose in narrower tiles: 64 -> 256
+  // and 64 -> 64 on 56 x 56 maps, batch 64: 84 us in one launch, 77 in two (256 -> 512 and 256 -> 128 at stride 2, 56 and 73).
+  const double cells = static_cast<double>(shape_.n) * shape_.ho * shape_.wo * (shape_.cout + other->shape_.cout);
+  if (shape_.c * shape_.kh * shape_.kw < 256 && cells > 16e6) return false;
+  return plain(*this) && plain(*other) && a.n == b.n && a.h == b.h && a.w == b.w && a.c == b.c && a.kh == b.kh && a.kw == b.kw &&
+         a.stride_h == b.stride_h && a.stride_w == b.stride_w && a.pad_h == b.pad_h && a.pad_w == b.pad_w && a.dil_h == b.dil_h &&
+         a.dil_w == b.dil_w && (half_operands_ && HalfOperandsCapable()) == (other->half_operands_ && other->HalfOperandsCapable()) &&
+         (half_top_ && HalfTopCapable()) == (other->half_top_ && other->HalfTopCapable());
+}
+
+void ConvolutionLayer::SetSibling(Layer* other) {
+  ConvolutionLayer* sibling = static_cast<ConvolutionLayer*>(other);
+  if (sibling == sibling_) return;
+  sibling_ = sibling;
+  weight_version_ = tail_version_ = 0;   // packed weights and per-column arrays hold both layers
+}
+
+// `shape`'s rows of the packed tensor-core weight image.
+void ConvolutionLayer::PackRows(const mcb200_conv_shape& shape, const float* weights, float* packed) {
+  Context& ctx = Context::Get();
+  if (half_operands_) {
+    KERNEL_CHECK(mcb200_conv_pack_weights_bf16(&shape, weights, reinterpret_cast<uint16_t*>(packed), ctx.stream_ptr()));
+  } else {
+    KERNEL_CHECK(mcb200_conv_pack_weights(&shape, weights, packed, ctx.stream_ptr()));
+  }
+}
+
+void ConvolutionLayer::FoldRows(std::vector<float>* scale, std::vector<float>* shift, bool* has_scale, bool* has_shift) {
+  FoldTail(tail_, shape_.cout, bias_term_ ? blobs_[1]->cpu_data() : nullptr, scale, shift, has_scale, has_shift);
+}
+
 void ConvolutionLayer::RefreshParameters() {
   Context& ctx = Context::Get();
-  const unsigned long long wv = blobs_[0]->host_version();
+  // (versions only grow: so does their sum)
+  const unsigned long long wv = blobs_[0]->host_version() + (sibling_ ? sibling_->blobs_[0]->host_version() : 0);
   if (wv != weight_version_) {
     if (path_ == kTensorCore && use_rows_) {
       float* packed = packed_weights_.Reserve(mcb200_conv_rows_packed_weight_count(&shape_));
       KERNEL_CHECK(mcb200_conv_rows_pack_weights(&shape_, blobs_[0]->gpu_data(), packed, ctx.stream_ptr()));
-    } else if (path_ == kTensorCore && half_operands_) {
-      float* packed = packed_weights_.Reserve((mcb200_conv_packed_weight_count_bf16(&shape_) + 1) / 2);
-      KERNEL_CHECK(mcb200_conv_pack_weights_bf16(&shape_, blobs_[0]->gpu_data(), reinterpret_cast<uint16_t*>(packed),
-                                                 ctx.stream_ptr()));
     } else if (path_ == kTensorCore) {
-      float* packed = packed_weights_.Reserve(mcb200_conv_packed_weight_count(&shape_));
-      KERNEL_CHECK(mcb200_conv_pack_weights(&shape_, blobs_[0]->gpu_data(), packed, ctx.stream_ptr()));
+      mcb200_conv_shape all = shape_;
+      all.cout = columns();
+      const size_t count = half_operands_ ? (mcb200_conv_packed_weight_count_bf16(&all) + 1) / 2
+                                          : mcb200_conv_packed_weight_count(&all);
+      float* packed = packed_weights_.Reserve(count);
+      if (sibling_) {
+        // Rows: this layer's, zeros up to the sibling's first column, the sibling's.  (A row is whole 128-byte cells.)
+        const size_t row = count / all.cout;
+        CUDA_CHECK(cudaMemsetAsync(packed + shape_.cout * row, 0, (second_begin() - shape_.cout) * row * sizeof(float), ctx.stream()));
+        PackRows(sibling_->shape_, sibling_->blobs_[0]->gpu_data(), packed + second_begin() * row);
+      }
+      PackRows(shape_, blobs_[0]->gpu_data(), packed);
     } else if (path_ == kDepthwise) {
       float* packed = packed_weights_.Reserve(static_cast<size_t>(shape_.c) * shape_.kh * shape_.kw);
       KERNEL_CHECK(mcb200_dw_pack_weights(&shape_, blobs_[0]->gpu_data(), packed, ctx.stream_ptr()));
@@ -240,13 +287,24 @@ void ConvolutionLayer::RefreshParameters() {
       if (slot) slot->valid = false;
     }
   }
-  const unsigned long long tv = 1 + TailVersion(tail_) + (bias_term_ ? blobs_[1]->host_version() : 0);
+  unsigned long long tv = 1 + TailVersion(tail_) + (bias_term_ ? blobs_[1]->host_version() : 0);
+  if (sibling_) tv += TailVersion(sibling_->tail_) + (sibling_->bias_term_ ? sibling_->blobs_[1]->host_version() : 0);
   if (tv != tail_version_) {
     constants_settled_ = false;
     std::vector<float> scale, shift;
     bool has_scale = false, has_shift = false;
-    FoldTail(tail_, shape_.cout, bias_term_ ? blobs_[1]->cpu_data() : nullptr, &scale, &shift, &has_scale,
-             &has_shift);
+    FoldRows(&scale, &shift, &has_scale, &has_shift);
+    if (sibling_) {
+      std::vector<float> scale2, shift2;
+      bool has_scale2 = false, has_shift2 = false;
+      sibling_->FoldRows(&scale2, &shift2, &has_scale2, &has_shift2);
+      scale.resize(second_begin(), 1.f);
+      shift.resize(second_begin(), 0.f);
+      scale.insert(scale.end(), scale2.begin(), scale2.end());
+      shift.insert(shift.end(), shift2.begin(), shift2.end());
+      has_scale = has_scale || has_scale2;
+      has_shift = has_shift || has_shift2;
+    }
     if (has_scale) scale_.Assign(scale); else scale_.Clear();
     if (has_shift) shift_.Assign(shift); else shift_.Clear();
     tail_version_ = tv;
@@ -262,30 +320,41 @@ double ConvolutionLayer::PartSeconds(const vector<Blob*>& bottom, const vector<B
   const double out_cell = half_top_ && HalfTopCapable() ? 2.0 : 4.0;
   double bytes = in_cell * bottom[0]->count() + out_cell * top[0]->count();
   if (tail_.residual) bytes += in_cell * top[0]->count();
-  const double flops = 2.0 * top[0]->count() * (s.c / s.group) * s.kh * s.kw;
+  double outputs = top[0]->count();
+  if (sibling_) {
+    if (sibling_->shape_.cout % 8 != 0) return 0;
+    outputs += top[1]->count();
+    bytes += out_cell * top[1]->count();
+  }
+  const double flops = 2.0 * outputs * (s.c / s.group) * s.kh * s.kw;
   const double rate = path_ == kDepthwise ? 20e12 : in_cell == 2.0 ? 1.1e15 : 0.6e15;
   return std::max(bytes / kPartBytesPerSecond, flops / rate);
 }
 
 void ConvolutionLayer::Forward_gpu(const vector<Blob*>& bottom, const vector<Blob*>& top) {
   RefreshParameters();
-  for (size_t i = 0; i < bottom.size(); ++i) RunImages(bottom[i], top[i], i, 0, shape_.n, i);
+  if (sibling_) {
+    RunImages(bottom[0], top[0], 0, 0, shape_.n, 0, top[1]);
+  } else {
+    for (size_t i = 0; i < bottom.size(); ++i) RunImages(bottom[i], top[i], i, 0, shape_.n, i);
+  }
   constants_settled_ = true;
 }
 
 void ConvolutionLayer::ForwardImages_gpu(const vector<Blob*>& bottom, const vector<Blob*>& top, int first, int count,
                                          int part) {
   if (first == 0) RefreshParameters();
-  RunImages(bottom[0], top[0], 0, first, count, part);
+  RunImages(bottom[0], top[0], 0, first, count, part, sibling_ ? top[1] : nullptr);
   if (first + count == shape_.n) constants_settled_ = true;
 }
 
-void ConvolutionLayer::RunImages(Blob* bottom, Blob* top, size_t i, int first, int count, size_t slot_index) {
+void ConvolutionLayer::RunImages(Blob* bottom, Blob* top, size_t i, int first, int count, size_t slot_index, Blob* second_top) {
   Context& ctx = Context::Get();
   mcb200_conv_shape s = shape_;
   s.n = count;
+  s.cout = columns();
   const size_t in_at = static_cast<size_t>(first) * s.c * s.h * s.w;
-  const size_t out_at = static_cast<size_t>(first) * s.cout * s.ho * s.wo;
+  const size_t out_at = static_cast<size_t>(first) * shape_.cout * s.ho * s.wo;
   const float* in = nullptr;
   const bool half = half_operands_ && HalfOperandsCapable();
   if (half) {
@@ -321,8 +390,8 @@ void ConvolutionLayer::RunImages(Blob* bottom, Blob* top, size_t i, int first, i
     in = padded;
   }
   mcb200_epilogue ep;
-  FillTailEpilogue(i == 0 ? tail_ : FusedTail(), scale_, shift_, half ? kResidualNhwcHalf : kResidualNhwc, s.cout,
-                   &ep);
+  FillTailEpilogue(i == 0 ? tail_ : FusedTail(), scale_, shift_, half ? kResidualNhwcHalf : kResidualNhwc,
+                   shape_.cout, &ep);
   if (ep.residual) {
     ep.residual = half ? reinterpret_cast<const float*>(reinterpret_cast<const uint16_t*>(ep.residual) + out_at)
                        : ep.residual + out_at;
@@ -351,6 +420,17 @@ void ConvolutionLayer::RunImages(Blob* bottom, Blob* top, size_t i, int first, i
         RunImages(bottom, top, i, first, count, slot_index);
         return;
       }
+      if (rc != 0 && sibling_) {
+        // (the shape alone decides: the sibling's own plan would be refused as well)
+        ConvolutionLayer* sibling = sibling_;
+        SetSibling(nullptr);
+        RefreshParameters();
+        RunImages(bottom, top, i, first, count, slot_index);
+        sibling->RefreshParameters();
+        sibling->RunImages(bottom, second_top, 0, first, count, slot_index);
+        sibling_ = sibling;   // the net still hands both tops over
+        return;
+      }
       if (rc != 0 && !half && !half_out) {
         // A shape the tensor maps cannot express (for instance a stride above 8, which the
         // im2col map refuses as traversal stride): the plain kernel runs it from now on.
@@ -366,9 +446,22 @@ void ConvolutionLayer::RunImages(Blob* bottom, Blob* top, size_t i, int first, i
       slot.shape = s;
       slot.valid = true;
     }
-    KERNEL_CHECK(mcb200_conv_tc_launch_flags(&slot.plan, out, half_out ? 1 : 0, s.cout, &ep,
-                                             constants_settled_ ? MCB200_CONV_CONSTANTS_SETTLED : 0, ctx.status_word(),
+    const int flags = constants_settled_ ? MCB200_CONV_CONSTANTS_SETTLED : 0;
+    if (sibling_) {
+      mcb200_conv_second second;
+      second.begin = second_begin();
+      second.first_cout = shape_.cout;
+      second.out_ld = sibling_->shape_.cout;
+      second.act = sibling_->tail_.activation ? 1 : 0;
+      const size_t second_at = static_cast<size_t>(first) * second.out_ld * s.ho * s.wo;
+      second.out = half_out ? static_cast<void*>(static_cast<uint16_t*>(second_top->mutable_gpu_data_nhwc_bf16()) + second_at)
+                            : static_cast<void*>(second_top->mutable_gpu_data_nhwc() + second_at);
+      KERNEL_CHECK(mcb200_conv_tc_launch_two(&slot.plan, out, half_out ? 1 : 0, shape_.cout, &ep, &second, flags, ctx.status_word(),
                                              ctx.stream_ptr()));
+    } else {
+      KERNEL_CHECK(mcb200_conv_tc_launch_flags(&slot.plan, out, half_out ? 1 : 0, s.cout, &ep, flags, ctx.status_word(),
+                                               ctx.stream_ptr()));
+    }
   } else if (path_ == kDepthwise && (half || half_out)) {
     KERNEL_CHECK(mcb200_conv_depthwise_bf16(&s, in, half ? 1 : 0, packed_weights_.Reserve(0), out, half_out ? 1 : 0,
                                             &ep, ctx.stream_ptr()));

@@ -73,13 +73,19 @@ class ConvolutionLayer : public Layer {
     half_top_ = top;
   }
   double PartSeconds(const vector<Blob*>& bottom, const vector<Blob*>& top, bool first_of_net) const override;
+  bool AcceptsSibling(const Layer* other) const override;
+  void SetSibling(Layer* other) override;
 
  protected:
   void Forward_gpu(const vector<Blob*>& bottom, const vector<Blob*>& top) override;
   void ForwardImages_gpu(const vector<Blob*>& bottom, const vector<Blob*>& top, int first, int count, int part) override;
-  // Images [first, first + count) of bottom i, with the plan kept in `slot`.
-  void RunImages(Blob* bottom, Blob* top, size_t i, int first, int count, size_t slot);
+  // Images [first, first + count) of bottom i, with the plan kept in `slot`; second_top: the sibling's.
+  void RunImages(Blob* bottom, Blob* top, size_t i, int first, int count, size_t slot, Blob* second_top = nullptr);
   void RefreshParameters();
+  void PackRows(const mcb200_conv_shape& shape, const float* weights, float* packed);
+  void FoldRows(std::vector<float>* scale, std::vector<float>* shift, bool* has_scale, bool* has_shift);
+  int second_begin() const { return (shape_.cout + 31) / 32 * 32; }   // first of the sibling's columns
+  int columns() const { return sibling_ ? second_begin() + sibling_->shape_.cout : shape_.cout; }
 
   // The depthwise 3x3 kernel reads and writes bfloat16 cells (fp32 weights and arithmetic).
   bool DepthwiseHalfCapable() const {
@@ -99,6 +105,7 @@ class ConvolutionLayer : public Layer {
   enum Path { kTensorCore, kDepthwise, kDirect } path_ = kDirect;
   bool use_rows_ = false;       // tensor-core row mode (at most four input channels)
   bool rows_rejected_ = false;
+  ConvolutionLayer* sibling_ = nullptr;   // its result comes out of this layer's launch
   struct PlanSlot {
     mcb200_conv_plan plan;
     const float* in = nullptr;

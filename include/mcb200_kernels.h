@@ -185,6 +185,31 @@ int mcb200_conv_rows_pad_input(const mcb200_conv_shape* s, const float* src_nchw
 int mcb200_conv_rows_plan(const mcb200_conv_shape* s, const float* padded_in, const float* packed_w,
                           mcb200_conv_plan* plan);
 
+/* 3 x 3 layers of stride 1 and padding 1 with 33 to 64 input and output channels on rows that fill slabs of 62 pixels to
+ * three quarters: every input row is loaded once and contributes to three output rows at a time.  Same
+ * operands, results and flags as mcb200_conv_tc_plan / mcb200_conv_tc_plan_bf16 and their launches, no residual;
+ * weights packed by mcb200_conv_march_pack_weights (mcb200_conv_march_packed_weight_bytes bytes).  With `pool` the output
+ * is the 2 x 2 maxima, stride 2, no padding, of what it would be (mcb200_pool_nhwc's rules).  Replaces the same
+ * reference code (src/layers/base_conv_layer.cpp:254-278).                                        */
+typedef struct mcb200_march_plan {
+  uint64_t tma_a[16];
+  uint64_t tma_b[16];
+  mcb200_conv_shape shape;
+  int operand_bf16;
+  int segments, segment_w;  /* columns of an image and outputs of a column's row */
+  int column_h, pad_top;    /* rows of a column, padding included, and those above the image */
+  int total;                /* rows of all columns                              */
+  int pool;                 /* the result is its 2 x 2 maxima                   */
+} __attribute__((aligned(64))) mcb200_march_plan;
+int mcb200_conv_march_supported(const mcb200_conv_shape* s, int operands_bf16);   /* whatever the batch */
+int mcb200_conv_march_pays(const mcb200_conv_shape* s, int operands_bf16);        /* and enough rows for all SMs */
+size_t mcb200_conv_march_packed_weight_bytes(const mcb200_conv_shape* s, int operands_bf16);
+int mcb200_conv_march_pack_weights(const mcb200_conv_shape* s, int operands_bf16, const float* w_oihw, void* packed, void* stream);
+int mcb200_conv_march_plan(const mcb200_conv_shape* s, int operands_bf16, const void* in, const void* packed_w,
+                           int pool, mcb200_march_plan* plan);
+int mcb200_conv_march_launch(const mcb200_march_plan* plan, void* out, int out_is_bf16, int out_ld, const mcb200_epilogue* ep,
+                             int flags, int* status, void* stream);
+
 /* Direct convolution, one thread per output element, any group count; the
  * fallback for shapes the tensor-core path rejects.  Weights stay in Caffe
  * order [cout, c/group, kh, kw].                                             */

@@ -192,24 +192,6 @@ struct Tag {
   static constexpr int value = kValue;
 };
 
-// w[k] of lane q of a quad becomes word q of the quad's lane k.
-__device__ __forceinline__ void quad_transpose(uint32_t (&w)[4], int q) {
-#pragma unroll
-  for (int step = 1; step <= 2; step *= 2) {
-    const bool upper = (q & step) != 0;
-    const int lo0 = 0, hi0 = step, lo1 = step == 1 ? 2 : 1, hi1 = 3;
-    const uint32_t x = __shfl_xor_sync(0xffffffffu, upper ? w[lo0] : w[hi0], step);
-    const uint32_t y = __shfl_xor_sync(0xffffffffu, upper ? w[lo1] : w[hi1], step);
-    if (upper) {
-      w[lo0] = x;
-      w[lo1] = y;
-    } else {
-      w[hi0] = x;
-      w[hi1] = y;
-    }
-  }
-}
-
 // Ring position of a k-iteration: stage index and the parity of its use.
 // Advancing it costs an increment and a compare; the single-thread loops
 // below are latency-bound on exactly this kind of scalar work.
@@ -1988,6 +1970,15 @@ long long g_wait_limit_cycles = mcb200::kDefaultWaitLimitCycles;
 thread_local int t_drop_weight_load = 0;
 }  // namespace
 
+namespace mcb200 {
+long long conv_wait_limit() { return g_wait_limit_cycles; }
+int conv_take_drop_hook() {
+  const int drop = t_drop_weight_load;
+  t_drop_weight_load = 0;
+  return drop;
+}
+}  // namespace mcb200
+
 extern "C" long long mcb200_conv_set_wait_limit(long long cycles) {
   const long long previous = g_wait_limit_cycles;
   g_wait_limit_cycles = cycles > 0 ? cycles : mcb200::kDefaultWaitLimitCycles;
@@ -2316,8 +2307,7 @@ int launch_core(mcb200_conv_plan* plan, void* out, bool out_half, int out_ld, co
   a.l2_prefetch = 0;
   a.wait_limit = g_wait_limit_cycles;
   a.constants_settled = (flags & MCB200_CONV_CONSTANTS_SETTLED) ? 1 : 0;
-  a.drop_last_weight_load = t_drop_weight_load;
-  t_drop_weight_load = 0;
+  a.drop_last_weight_load = conv_take_drop_hook();
   a.group_cout = plan->shape.group > 1 ? plan->shape.cout / plan->shape.group : 0;
   a.group_cin = plan->shape.group > 1 ? plan->shape.c / plan->shape.group : 0;
   a.wp = plan->shape.wo;

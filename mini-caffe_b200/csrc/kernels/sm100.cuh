@@ -409,6 +409,24 @@ __device__ __forceinline__ void tmem_load_32x32(uint32_t taddr, uint32_t (&r)[32
 
 __device__ __forceinline__ void tmem_load_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+// w[k] of lane q of a quad becomes word q of the quad's lane k.
+__device__ __forceinline__ void quad_transpose(uint32_t (&w)[4], int q) {
+#pragma unroll
+  for (int step = 1; step <= 2; step *= 2) {
+    const bool upper = (q & step) != 0;
+    const int lo0 = 0, hi0 = step, lo1 = step == 1 ? 2 : 1, hi1 = 3;
+    const uint32_t x = __shfl_xor_sync(0xffffffffu, upper ? w[lo0] : w[hi0], step);
+    const uint32_t y = __shfl_xor_sync(0xffffffffu, upper ? w[lo1] : w[hi1], step);
+    if (upper) {
+      w[lo0] = x;
+      w[lo1] = y;
+    } else {
+      w[hi0] = x;
+      w[hi1] = y;
+    }
+  }
+}
+
 // Two floats -> two bfloat16 (round to nearest even) in one word, `lo` in the low half.
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   uint32_t r;

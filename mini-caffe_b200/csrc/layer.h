@@ -36,7 +36,9 @@ struct FusedTail {
   float self_coeff = 1.f;
   // ReLU / PReLU applied last (nullptr: none).
   class Layer* activation = nullptr;
-  bool empty() const { return affine.empty() && !residual && !activation; }
+  // A 2 x 2 max pooling of stride 2 behind all that.
+  bool pooled = false;
+  bool empty() const { return affine.empty() && !residual && !activation && !pooled; }
 };
 
 struct ActivationSpec {
@@ -103,6 +105,10 @@ class Layer {
   }
   // Consumer side: express this layer as an activation.
   virtual bool AsActivation(ActivationSpec* spec) { return false; }
+  // Consumer side: true if the layer is 2 x 2 max pooling of stride 2 without padding, as shaped now.
+  virtual bool AsMaxPool2x2() const { return false; }
+  // Producer side: can its store take such a pooling behind the rest of `tail`?
+  virtual bool AcceptsFusedPool(const FusedTail& tail) const { return false; }
   // Consumer side: true if the layer is y = sum_i coeff[i] * bottom[i].
   virtual bool AsWeightedSum(std::vector<float>* coeffs) { return false; }
   // ---- bfloat16 storage (nets built with MINICAFFE_PRECISION=bf16) ----

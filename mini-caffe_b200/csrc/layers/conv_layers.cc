@@ -216,9 +216,23 @@ void ConvolutionLayer::Reshape(const vector<Blob*>& bottom, const vector<Blob*>&
   for (size_t i = 0; i < top.size(); ++i) top[i]->Reshape(shape_.n, shape_.cout, shape_.ho, shape_.wo);
 }
 
+bool ConvolutionLayer::AcceptsFusedPool(const FusedTail& tail) const {
+  const char* off = getenv("MCB200_MARCH");
+  const double pixels = static_cast<double>(shape_.n) * shape_.h * shape_.w;   // far from the plan's limits
+  return path_ == kTensorCore && !use_rows_ && !march_rejected_ && !tail.residual && !(off && off[0] == '0') && pixels < 1e8 &&
+         shape_.c % 8 == 0 && mcb200_conv_march_supported(&shape_, 0) != 0;
+}
+
+bool ConvolutionLayer::Marches() const {
+  if (tail_.pooled) return true;              // decided when the net was planned
+  const char* off = getenv("MCB200_MARCH");   // "0": the general kernel, for comparisons in tests
+  return path_ == kTensorCore && !use_rows_ && !march_rejected_ && !sibling_ && !tail_.residual && !(off && off[0] == '0') &&
+         mcb200_conv_march_pays(&shape_, half_operands_ ? 1 : 0) != 0;
+}
+
 bool ConvolutionLayer::AcceptsSibling(const Layer* layer) const {
   const ConvolutionLayer* other = dynamic_cast<const ConvolutionLayer*>(layer);
-  if (!other || other == this) return false;
+  if (!other || other == this || Marches()) return false;
   auto plain = [](const ConvolutionLayer& l) {
     ActivationSpec act;
     if (l.tail_.activation && (!l.tail_.activation->AsActivation(&act) || act.kind != 1 || act.slope != 0.f)) return false;
@@ -258,12 +272,20 @@ void ConvolutionLayer::FoldRows(std::vector<float>* scale, std::vector<float>* s
 
 void ConvolutionLayer::RefreshParameters() {
   Context& ctx = Context::Get();
+  if (packed_march_ != Marches()) {
+    packed_march_ = !packed_march_;
+    weight_version_ = 0;
+  }
   // (versions only grow: so does their sum)
   const unsigned long long wv = blobs_[0]->host_version() + (sibling_ ? sibling_->blobs_[0]->host_version() : 0);
   if (wv != weight_version_) {
     if (path_ == kTensorCore && use_rows_) {
       float* packed = packed_weights_.Reserve(mcb200_conv_rows_packed_weight_count(&shape_));
       KERNEL_CHECK(mcb200_conv_rows_pack_weights(&shape_, blobs_[0]->gpu_data(), packed, ctx.stream_ptr()));
+    } else if (packed_march_) {
+      const int half = half_operands_ ? 1 : 0;
+      float* packed = packed_weights_.Reserve(mcb200_conv_march_packed_weight_bytes(&shape_, half) / sizeof(float));
+      KERNEL_CHECK(mcb200_conv_march_pack_weights(&shape_, half, blobs_[0]->gpu_data(), packed, ctx.stream_ptr()));
     } else if (path_ == kTensorCore) {
       mcb200_conv_shape all = shape_;
       all.cout = columns();
@@ -320,7 +342,7 @@ double ConvolutionLayer::PartSeconds(const vector<Blob*>& bottom, const vector<B
   const double out_cell = half_top_ && HalfTopCapable() ? 2.0 : 4.0;
   double bytes = in_cell * bottom[0]->count() + out_cell * top[0]->count();
   if (tail_.residual) bytes += in_cell * top[0]->count();
-  double outputs = top[0]->count();
+  double outputs = static_cast<double>(s.n) * s.cout * s.ho * s.wo;
   if (sibling_) {
     if (sibling_->shape_.cout % 8 != 0) return 0;
     outputs += top[1]->count();
@@ -354,7 +376,7 @@ void ConvolutionLayer::RunImages(Blob* bottom, Blob* top, size_t i, int first, i
   s.n = count;
   s.cout = columns();
   const size_t in_at = static_cast<size_t>(first) * s.c * s.h * s.w;
-  const size_t out_at = static_cast<size_t>(first) * shape_.cout * s.ho * s.wo;
+  const size_t out_at = static_cast<size_t>(first) * (top->count() / shape_.n);
   const float* in = nullptr;
   const bool half = half_operands_ && HalfOperandsCapable();
   if (half) {
@@ -405,7 +427,8 @@ void ConvolutionLayer::RunImages(Blob* bottom, Blob* top, size_t i, int first, i
     PlanSlot& slot = *plans_[slot_index];
     const float* w = packed_weights_.Reserve(0);
     if (!slot.valid || slot.in != in || slot.weights != w || std::memcmp(&slot.shape, &s, sizeof(s)) != 0) {
-      int rc = half ? mcb200_conv_tc_plan_bf16(&s, reinterpret_cast<const uint16_t*>(in),
+      int rc = packed_march_ ? mcb200_conv_march_plan(&s, half ? 1 : 0, in, w, tail_.pooled ? 1 : 0, &slot.march)
+               : half ? mcb200_conv_tc_plan_bf16(&s, reinterpret_cast<const uint16_t*>(in),
                                                reinterpret_cast<const uint16_t*>(w), &slot.plan)
                : use_rows_ ? mcb200_conv_rows_plan(&s, in, w, &slot.plan)
                            : mcb200_conv_tc_plan(&s, in, w, &slot.plan);
@@ -420,6 +443,13 @@ void ConvolutionLayer::RunImages(Blob* bottom, Blob* top, size_t i, int first, i
         RunImages(bottom, top, i, first, count, slot_index);
         return;
       }
+      if (rc != 0 && packed_march_ && !tail_.pooled) {
+        march_rejected_ = true;   // the general kernel from now on
+        RefreshParameters();
+        RunImages(bottom, top, i, first, count, slot_index);
+        return;
+      }
+      CHECK(rc == 0 || !tail_.pooled) << "cannot build the plan for layer " << layer_param_.name();
       if (rc != 0 && sibling_) {
         // (the shape alone decides: the sibling's own plan would be refused as well)
         ConvolutionLayer* sibling = sibling_;
@@ -447,7 +477,9 @@ void ConvolutionLayer::RunImages(Blob* bottom, Blob* top, size_t i, int first, i
       slot.valid = true;
     }
     const int flags = constants_settled_ ? MCB200_CONV_CONSTANTS_SETTLED : 0;
-    if (sibling_) {
+    if (packed_march_) {
+      KERNEL_CHECK(mcb200_conv_march_launch(&slot.march, out, half_out ? 1 : 0, s.cout, &ep, flags, ctx.status_word(), ctx.stream_ptr()));
+    } else if (sibling_) {
       mcb200_conv_second second;
       second.begin = second_begin();
       second.first_cout = shape_.cout;

@@ -74,6 +74,7 @@ class ConvolutionLayer : public Layer {
   }
   double PartSeconds(const vector<Blob*>& bottom, const vector<Blob*>& top, bool first_of_net) const override;
   bool AcceptsSibling(const Layer* other) const override;
+  bool AcceptsFusedPool(const FusedTail& tail) const override;
   void SetSibling(Layer* other) override;
 
  protected:
@@ -82,6 +83,8 @@ class ConvolutionLayer : public Layer {
   // Images [first, first + count) of bottom i, with the plan kept in `slot`; second_top: the sibling's.
   void RunImages(Blob* bottom, Blob* top, size_t i, int first, int count, size_t slot, Blob* second_top = nullptr);
   void RefreshParameters();
+  // Whether the layer runs on conv_march.cu, as shaped, fused and stored now.
+  bool Marches() const;
   void PackRows(const mcb200_conv_shape& shape, const float* weights, float* packed);
   void FoldRows(std::vector<float>* scale, std::vector<float>* shift, bool* has_scale, bool* has_shift);
   int second_begin() const { return (shape_.cout + 31) / 32 * 32; }   // first of the sibling's columns
@@ -105,9 +108,14 @@ class ConvolutionLayer : public Layer {
   enum Path { kTensorCore, kDepthwise, kDirect } path_ = kDirect;
   bool use_rows_ = false;       // tensor-core row mode (at most four input channels)
   bool rows_rejected_ = false;
+  bool packed_march_ = false;   // form of the packed weights
+  bool march_rejected_ = false;
   ConvolutionLayer* sibling_ = nullptr;   // its result comes out of this layer's launch
   struct PlanSlot {
-    mcb200_conv_plan plan;
+    union {
+      mcb200_conv_plan plan;
+      mcb200_march_plan march;
+    };
     const float* in = nullptr;
     const float* weights = nullptr;
     mcb200_conv_shape shape = mcb200_conv_shape();
@@ -298,6 +306,10 @@ class PoolingLayer : public Layer {
   bool HalfTopCapable() const override { return HalfOperandsCapable(); }
   bool HalfNeedsBoth() const override { return true; }
   void SetHalfStorage(bool operands, bool top) override { half_ = operands && top; }
+  bool AsMaxPool2x2() const override {
+    return method_ == MCB200_POOL_MAX && !global_ && kernel_h_ == 2 && kernel_w_ == 2 && stride_h_ == 2 && stride_w_ == 2 &&
+           pad_h_ == 0 && pad_w_ == 0;
+  }
   double PartSeconds(const vector<Blob*>& bottom, const vector<Blob*>& top, bool first_of_net) const override;
  protected:
   void Forward_gpu(const vector<Blob*>& bottom, const vector<Blob*>& top) override;

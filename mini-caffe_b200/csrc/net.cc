@@ -285,6 +285,16 @@ void Net::PlaceMemory() {
           scan.absorbed[k] = true;
           cur = out;
         }
+        // A 2 x 2 max pooling that alone reads the result.
+        std::vector<int> readers = scan.Consumers(cur, i);
+        if (readers.size() == 1 && !plan.visible[cur] && layers_[readers[0]]->AsMaxPool2x2() && producer->AcceptsFusedPool(tail)) {
+          const Blob &from = *blobs_[cur], &to = *top_vecs_[readers[0]][0];
+          if (to.shape(2) == (from.shape(2) + 1) / 2 && to.shape(3) == (from.shape(3) + 1) / 2) {
+            tail.pooled = true;
+            scan.absorbed[readers[0]] = true;
+            cur = top_id_vecs_[readers[0]][0];
+          }
+        }
         step.tops[0] = blobs_[cur].get();
         step.top_ids[0] = cur;
       }

@@ -956,7 +956,12 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     bool alive = true;
     MCB200_TRACE_DECL;
     MCB200_TRACE_CHUNK_DECL;
-    for (int tile = worker; !kSplit && tile < num_tiles && alive; tile += workers, ++local) {
+    // The first chunk once over before there is anything to read (`dry`: nothing is waited for, stored or handed
+    // back): these warps have nothing else to do until the first accumulator is full, and the code they run then comes
+    // out of the instruction caches.  Per pass, ResNet-50 with one
+    // image 412 -> 407 us, batch 64 2212 -> 2200.
+    bool dry = !kStaged;
+    for (int tile = worker; !kSplit && tile < num_tiles && alive; tile += dry ? 0 : workers, local += dry ? 0 : 1, dry = false) {
       const int ab = accumulators == 2 ? local & 1 : 0;
       const uint32_t use = static_cast<uint32_t>(accumulators == 2 ? local >> 1 : local) & 1u;
       // Where the tile lies, before the wait: the divisions cost a few hundred cycles.
@@ -970,7 +975,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         box_row = box_row * kBlockM + quad * 32;
       }
       // tcgen05.ld is warp-collective: the whole warp takes the same branch.
-      alive = __all_sync(0xffffffffu, mbar_wait_bounded(&tmem_full_bar[ab], use, abort, wait_limit));
+      if (!dry) alive = __all_sync(0xffffffffu, mbar_wait_bounded(&tmem_full_bar[ab], use, abort, wait_limit));
       if (!alive) break;
       tc_fence_after_sync();
       if (ew == 0 && lane == 0) MCB200_TRACE(3);
@@ -985,7 +990,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       const float* t_slope = col_slope[ab];
       const bool refill = table_n0[ab] != n0;
       if (refill) fill_table(ab, n0);
-      if (refill || local == 0) {
+      if (!dry && (refill || local == 0)) {
         // Rendezvous of the epilogue warps on the table (an mbarrier rather than a
         // named barrier, so that the wait is bounded like every other one).
         alive = __all_sync(0xffffffffu, mbar_wait_bounded(&col_bar[ab], table_fills[ab] & 1u, abort, wait_limit));
@@ -994,10 +999,12 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       }
       const uint32_t tmem_acc = tmem_base + static_cast<uint32_t>(ab * acc_columns) + (static_cast<uint32_t>(quad * 32) << 16);
       const int next = tile + workers;
-      int next_rows[4] = {-1, -1, -1, -1};
+      int next_rows[4] = {rows[0], rows[1], rows[2], rows[3]};   // (behind the last tile they are not used)
+      if (dry) rows[0] = rows[1] = rows[2] = rows[3] = -1;
       // After the last read of this accumulator (and of the per-column tables) it goes back to the MMA
       // issuer, and the next tile's first residual is asked for.
       auto hand_back = [&]() {
+        if (dry) return;
         if (ew == 0 && lane == 0) MCB200_TRACE(3);
         tc_fence_before_sync();
         __syncwarp();
@@ -1269,7 +1276,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         if (chunk + 2 >= kChunks || col0 + 2 * kChunk >= args.cout) {
           hand_back();
           handed = true;
-        } else if (has_res) {
+        } else if (has_res && !dry) {
           fetch_residual(rows, col0 + 2 * kChunk);
         }
         MCB200_TRACE_CHUNK();
@@ -1329,6 +1336,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           }
         }
         MCB200_TRACE_CHUNK();
+        if (dry) break;
       }
       if (!handed) hand_back();
 #pragma unroll

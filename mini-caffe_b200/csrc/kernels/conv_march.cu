@@ -27,8 +27,8 @@
 //
 // The sum over K runs over filter rows, then channel blocks, then taps, whatever the batch.
 // Measured: 64 -> 64 channels at 300 x 300, batch 32, with the pooling behind it 565 + 130 -> 301 us; at 56 x 56, batch 64,
-// 49.7 -> 34.  A row takes 3400 cycles where its MMAs need 2304: their operands (107 bytes per cycle) and the arriving rows (14)
-// share a port of 128.
+// 49.7 -> 34.  A row takes 3400 cycles where its MMAs need 2304.  In a run of four rows (56 x 56, batch 16, 18 us) the tensor
+// pipe is active 57 % of an SM's cycles, 72 % on the busiest; its shared-memory reads take a third of theirs.
 // Arithmetic replaced: mini-caffe's im2col + SGEMM + bias (src/layers/base_conv_layer.cpp:254-278).
 #include <cuda.h>
 #include <cuda_runtime.h>

@@ -6,8 +6,8 @@
 // filter rows, and the loop waits for it (64 -> 64 channels at 300 x 300, batch 32: 397 TFLOP/s of the tensor
 // pipe's 1107).  Here a CTA marches down the image.  An input row contributes to three output rows, whose
 // accumulators of 64 columns lie side by side in tensor memory: with the weights of the three filter rows stacked to
-// 192 rows, one MMA of 128 x 192 x 8 adds to all three.  That is as many bytes per cycle as the shared-memory port
-// delivers (ten kilobytes in 96 cycles), and the pipe runs at its full rate.  All weights stay in shared
+// 192 rows, one MMA of 128 x 192 x 8 adds to all three.  That is ten kilobytes of operands in
+// 96 cycles, which the shared-memory port (128 bytes per cycle) delivers at the pipe's full rate.  All weights stay in shared
 // memory (147 KB in fp32); what streams are the input rows, 32 KB per 2304 cycles.
 //
 // The 128 rows of an MMA are two slabs of 64 neighbouring pixels (62 outputs and the filter's overhang).  A column is a

@@ -426,7 +426,9 @@ void ConvolutionLayer::RunImages(Blob* bottom, Blob* top, size_t i, int first, i
     if (!plans_[slot_index]) plans_[slot_index].reset(new PlanSlot);
     PlanSlot& slot = *plans_[slot_index];
     const float* w = packed_weights_.Reserve(0);
-    if (!slot.valid || slot.in != in || slot.weights != w || std::memcmp(&slot.shape, &s, sizeof(s)) != 0) {
+    if (!slot.valid || slot.in != in || slot.weights != w || slot.pooled != tail_.pooled ||
+        std::memcmp(&slot.shape, &s, sizeof(s)) != 0) {
+      slot.valid = false;   // (a plan that is refused leaves nothing behind)
       int rc = packed_march_ ? mcb200_conv_march_plan(&s, half ? 1 : 0, in, w, tail_.pooled ? 1 : 0, &slot.march)
                : half ? mcb200_conv_tc_plan_bf16(&s, reinterpret_cast<const uint16_t*>(in),
                                                reinterpret_cast<const uint16_t*>(w), &slot.plan)
@@ -474,6 +476,7 @@ void ConvolutionLayer::RunImages(Blob* bottom, Blob* top, size_t i, int first, i
       slot.in = in;
       slot.weights = w;
       slot.shape = s;
+      slot.pooled = tail_.pooled;
       slot.valid = true;
     }
     const int flags = constants_settled_ ? MCB200_CONV_CONSTANTS_SETTLED : 0;

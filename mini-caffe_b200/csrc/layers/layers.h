@@ -119,6 +119,7 @@ class ConvolutionLayer : public Layer {
     const float* in = nullptr;
     const float* weights = nullptr;
     mcb200_conv_shape shape = mcb200_conv_shape();
+    bool pooled = false;        // form of the march's plan
     bool valid = false;
   };
   std::vector<std::unique_ptr<PlanSlot> > plans_;  // one per bottom and one per further part of the batch

@@ -1,0 +1,57 @@
+"""Nets that are planned again after they have run: another set of outputs, another batch.  What the layers keep from
+pass to pass (packed weights, launch plans, merged launches) has to follow."""
+import numpy as np
+import pytest
+
+from conftest import pkg
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def gpu_engine(engine):
+    engine.set_mode(True, 0)
+    return engine
+
+
+def _equal(a, b):
+    return np.array_equal(np.ascontiguousarray(a).view(np.uint32), np.ascontiguousarray(b).view(np.uint32))
+
+
+@pytest.mark.parametrize("parts", ["1", "3"])
+@pytest.mark.parametrize("precision", ["fp32", "bf16"])
+def test_a_blob_in_front_of_a_fused_pooling_is_marked_after_a_pass(monkeypatch, capi, gpu_engine, precision, parts):
+    """Enough rows that the layer marches with its pooling and without: the first plan pools in the store, the second may
+    not, on the same input buffer, weights and shape."""
+    wl = pkg("workloads")
+    b = wl.NetBuilder("marked_later")
+    b.input([("data", (9, 3, 101, 62))])
+    b.conv("conv1", "data", "conv1", 3, 64, 3, pad=1)
+    b.relu("conv1_relu", "conv1")
+    b.conv("conv2", "conv1", "conv2", 64, 64, 3, pad=1)
+    b.relu("conv2_relu", "conv2")
+    b.pool("pool", "conv2", "pool", "MAX", k=2, stride=2)
+    b.conv("conv3", "pool", "conv3", 64, 48, 1)
+    b.pool("last", "conv3", "last", "AVE", global_pooling=True)
+    weights = wl.init_params(b.params, seed=61)
+    rng = np.random.default_rng(61)
+    images = [rng.standard_normal((9, 3, 101, 62)).astype(np.float32) for _ in range(4)]
+    monkeypatch.setenv("MINICAFFE_PRECISION", precision)
+    monkeypatch.setenv("MCB200_INPUT_PARTS", parts)
+
+    def run(marked_after):
+        net = capi.Net(gpu_engine, b.text(), None, from_buffer=True)
+        net.set_params(weights)
+        got = []
+        for i, x in enumerate(images):
+            if i == marked_after:
+                net.mark_output("conv2")
+            net.forward(data=x)
+            got.append([net.blob("last").data.copy()] + ([net.blob("conv2").data.copy()] if i >= marked_after else []))
+        net.close()
+        return got
+
+    before, after = run(0), run(2)
+    for i in (2, 3):
+        assert np.isfinite(before[i][0]).all() and np.abs(before[i][0]).max() > 0
+        assert _equal(before[i][0], after[i][0]) and _equal(before[i][1], after[i][1]), i

@@ -236,7 +236,8 @@ bool ConvolutionLayer::AcceptsSibling(const Layer* layer) const {
   auto plain = [](const ConvolutionLayer& l) {
     ActivationSpec act;
     if (l.tail_.activation && (!l.tail_.activation->AsActivation(&act) || act.kind != 1 || act.slope != 0.f)) return false;
-    return l.path_ == kTensorCore && !l.use_rows_ && l.shape_.group == 1 && !l.tail_.residual;
+    // (A pooling in the store is the march's: the launch of two writes the unpooled rows.)
+    return l.path_ == kTensorCore && !l.use_rows_ && l.shape_.group == 1 && !l.tail_.residual && !l.tail_.pooled;
   };
   const mcb200_conv_shape &a = shape_, &b = other->shape_;
   // Short sums whose results fill HBM gain little from reading their input once, and lose in narrower tiles: 64 -> 256
@@ -483,6 +484,7 @@ void ConvolutionLayer::RunImages(Blob* bottom, Blob* top, size_t i, int first, i
     if (packed_march_) {
       KERNEL_CHECK(mcb200_conv_march_launch(&slot.march, out, half_out ? 1 : 0, s.cout, &ep, flags, ctx.status_word(), ctx.stream_ptr()));
     } else if (sibling_) {
+      CHECK_EQ(second_top->count(), shape_.n * sibling_->shape_.cout * s.ho * s.wo) << "top of layer " << sibling_->layer_param_.name();
       mcb200_conv_second second;
       second.begin = second_begin();
       second.first_cout = shape_.cout;

@@ -1,5 +1,5 @@
-"""Nets that are planned again after they have run: another set of outputs, another batch.  What the layers keep from
-pass to pass (packed weights, launch plans, merged launches) has to follow."""
+"""What the net's schedule fuses and merges, and nets that are planned again after they have run (another set of
+outputs, another batch): what the layers keep from pass to pass has to follow."""
 import numpy as np
 import pytest
 
@@ -55,3 +55,52 @@ def test_a_blob_in_front_of_a_fused_pooling_is_marked_after_a_pass(monkeypatch, 
     for i in (2, 3):
         assert np.isfinite(before[i][0]).all() and np.abs(before[i][0]).max() > 0
         assert _equal(before[i][0], after[i][0]) and _equal(before[i][1], after[i][1]), i
+
+
+@pytest.mark.parametrize("pooled_first", [False, True])
+@pytest.mark.parametrize("precision", ["fp32", "bf16"])
+@pytest.mark.parametrize("batch,cout", [(1, 64), (2, 128), (16, 128), (16, 64)])
+def test_a_layer_with_a_fused_pooling_stays_out_of_its_neighbours_launch(monkeypatch, capi, gpu_engine, batch, cout, precision,
+                                                                         pooled_first):
+    """Two 3 x 3 layers of one 64-channel input, the result of one read by a pooling only: the other marches or not, by its
+    columns and the batch."""
+    wl = pkg("workloads")
+    b = wl.NetBuilder("pooled_sibling")
+    b.input([("data", (batch, 3, 56, 56))])
+    b.conv("conv1", "data", "conv1", 3, 64, 3, pad=1)
+    b.relu("conv1_relu", "conv1")
+
+    def plain():
+        b.conv("plain", "conv1", "plain", 64, cout, 3, pad=1)
+        b.relu("plain_relu", "plain")
+
+    def pooled():
+        b.conv("pooled", "conv1", "pooled", 64, 64, 3, pad=1)
+        b.relu("pooled_relu", "pooled")
+        b.pool("pool", "pooled", "pool", "MAX", k=2, stride=2)
+
+    for add in (pooled, plain) if pooled_first else (plain, pooled):
+        add()
+    b.conv("next", "pool", "next", 64, 40, 1)
+    b.pool("last", "plain", "last", "AVE", global_pooling=True)
+    weights = wl.init_params(b.params, seed=62)
+    rng = np.random.default_rng(62)
+    images = [rng.standard_normal((batch, 3, 56, 56)).astype(np.float32) for _ in range(3)]
+    monkeypatch.setenv("MINICAFFE_PRECISION", precision)
+
+    def run(siblings, march):
+        monkeypatch.setenv("MCB200_SIBLINGS", siblings)
+        monkeypatch.setenv("MCB200_MARCH", march)
+        net = capi.Net(gpu_engine, b.text(), None, from_buffer=True)
+        net.set_params(weights)
+        net.mark_output("next")
+        got = []
+        for x in images:
+            net.forward(data=x)
+            got.append([net.blob(name).data.copy() for name in ("next", "last")])
+        net.close()
+        return got
+
+    for alone, together in zip(run("0", "0"), run("1", "1")):
+        for want, got in zip(alone, together):
+            assert np.isfinite(want).all() and np.abs(want).max() > 0 and _equal(want, got)

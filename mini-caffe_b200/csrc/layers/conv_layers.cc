@@ -251,9 +251,9 @@ bool ConvolutionLayer::AcceptsSibling(const Layer* layer) const {
 }
 
 void ConvolutionLayer::SetSibling(Layer* other) {
-  ConvolutionLayer* sibling = static_cast<ConvolutionLayer*>(other);
-  if (sibling == sibling_) return;
-  sibling_ = sibling;
+  ConvolutionLayer* partner = static_cast<ConvolutionLayer*>(other);
+  if (partner == partner_) return;
+  partner_ = sibling_ = partner;
   weight_version_ = tail_version_ = 0;   // packed weights and per-column arrays hold both layers
 }
 
@@ -344,8 +344,8 @@ double ConvolutionLayer::PartSeconds(const vector<Blob*>& bottom, const vector<B
   double bytes = in_cell * bottom[0]->count() + out_cell * top[0]->count();
   if (tail_.residual) bytes += in_cell * top[0]->count();
   double outputs = static_cast<double>(s.n) * s.cout * s.ho * s.wo;
-  if (sibling_) {
-    if (sibling_->shape_.cout % 8 != 0) return 0;
+  if (partner_) {
+    if (partner_->shape_.cout % 8 != 0) return 0;
     outputs += top[1]->count();
     bytes += out_cell * top[1]->count();
   }
@@ -355,20 +355,36 @@ double ConvolutionLayer::PartSeconds(const vector<Blob*>& bottom, const vector<B
 }
 
 void ConvolutionLayer::Forward_gpu(const vector<Blob*>& bottom, const vector<Blob*>& top) {
-  RefreshParameters();
-  if (sibling_) {
-    RunImages(bottom[0], top[0], 0, 0, shape_.n, 0, top[1]);
-  } else {
-    for (size_t i = 0; i < bottom.size(); ++i) RunImages(bottom[i], top[i], i, 0, shape_.n, i);
+  if (partner_) {
+    RunTwo(bottom[0], top, 0, shape_.n, 0);
+    return;
   }
+  RefreshParameters();
+  for (size_t i = 0; i < bottom.size(); ++i) RunImages(bottom[i], top[i], i, 0, shape_.n, i);
   constants_settled_ = true;
 }
 
 void ConvolutionLayer::ForwardImages_gpu(const vector<Blob*>& bottom, const vector<Blob*>& top, int first, int count,
                                          int part) {
+  if (partner_) {
+    RunTwo(bottom[0], top, first, count, part);
+    return;
+  }
   if (first == 0) RefreshParameters();
-  RunImages(bottom[0], top[0], 0, first, count, part, sibling_ ? top[1] : nullptr);
+  RunImages(bottom[0], top[0], 0, first, count, part);
   if (first + count == shape_.n) constants_settled_ = true;
+}
+
+// This layer and the net's partner: in one launch, or, once the plan of two has been refused, one behind the other.
+void ConvolutionLayer::RunTwo(Blob* bottom, const vector<Blob*>& top, int first, int count, size_t slot) {
+  RefreshParameters();
+  RunImages(bottom, top[0], 0, first, count, slot, top[1]);
+  const bool through = first + count == shape_.n;
+  if (through) constants_settled_ = true;
+  if (sibling_) return;
+  partner_->RefreshParameters();
+  partner_->RunImages(bottom, top[1], 0, first, count, slot);
+  if (through) partner_->constants_settled_ = true;
 }
 
 void ConvolutionLayer::RunImages(Blob* bottom, Blob* top, size_t i, int first, int count, size_t slot_index, Blob* second_top) {
@@ -454,14 +470,11 @@ void ConvolutionLayer::RunImages(Blob* bottom, Blob* top, size_t i, int first, i
       }
       CHECK(rc == 0 || !tail_.pooled) << "cannot build the plan for layer " << layer_param_.name();
       if (rc != 0 && sibling_) {
-        // (the shape alone decides: the sibling's own plan would be refused as well)
-        ConvolutionLayer* sibling = sibling_;
-        SetSibling(nullptr);
+        // A geometry the tensor maps cannot express for both (and mostly for neither): two layers of their own from now on.
+        sibling_ = nullptr;
+        weight_version_ = tail_version_ = 0;
         RefreshParameters();
         RunImages(bottom, top, i, first, count, slot_index);
-        sibling->RefreshParameters();
-        sibling->RunImages(bottom, second_top, 0, first, count, slot_index);
-        sibling_ = sibling;   // the net still hands both tops over
         return;
       }
       if (rc != 0 && !half && !half_out) {

@@ -82,6 +82,7 @@ class ConvolutionLayer : public Layer {
   void ForwardImages_gpu(const vector<Blob*>& bottom, const vector<Blob*>& top, int first, int count, int part) override;
   // Images [first, first + count) of bottom i, with the plan kept in `slot`; second_top: the sibling's.
   void RunImages(Blob* bottom, Blob* top, size_t i, int first, int count, size_t slot, Blob* second_top = nullptr);
+  void RunTwo(Blob* bottom, const vector<Blob*>& top, int first, int count, size_t slot);
   void RefreshParameters();
   // Whether the layer runs on conv_march.cu, as shaped, fused and stored now.
   bool Marches() const;
@@ -110,7 +111,8 @@ class ConvolutionLayer : public Layer {
   bool rows_rejected_ = false;
   bool packed_march_ = false;   // form of the packed weights
   bool march_rejected_ = false;
-  ConvolutionLayer* sibling_ = nullptr;   // its result comes out of this layer's launch
+  ConvolutionLayer* partner_ = nullptr;   // the net's decision: this layer's Forward makes its result too
+  ConvolutionLayer* sibling_ = nullptr;   // the partner while one launch makes both (null: its plan was refused)
   struct PlanSlot {
     union {
       mcb200_conv_plan plan;

@@ -104,3 +104,41 @@ def test_a_layer_with_a_fused_pooling_stays_out_of_its_neighbours_launch(monkeyp
     for alone, together in zip(run("0", "0"), run("1", "1")):
         for want, got in zip(alone, together):
             assert np.isfinite(want).all() and np.abs(want).max() > 0 and _equal(want, got)
+
+
+@pytest.mark.parametrize("parts", ["1", "3"])
+@pytest.mark.parametrize("stride,kernel", [(9, 3), (16, 16), (2, 3)])
+def test_a_refused_launch_of_two_stays_two_layers(monkeypatch, capi, gpu_engine, stride, kernel, parts):
+    """Strides above 8 are refused by the tensor map: both layers run on the plain kernel, in this pass and in all later
+    ones, with new weights and another batch too."""
+    wl = pkg("workloads")
+    b = wl.NetBuilder("refused")
+    b.input([("data", (5, 3, 48, 48))])
+    b.conv("trunk", "data", "trunk", 3, 16, 3, pad=1)
+    b.relu("trunk_relu", "trunk")
+    b.conv("left", "trunk", "left", 16, 24, kernel, stride=stride)
+    b.relu("left_relu", "left")
+    b.conv("right", "trunk", "right", 16, 40, kernel, stride=stride)
+    b.pool("last", "left", "last", "AVE", global_pooling=True)
+    weights = wl.init_params(b.params, seed=63)
+    rng = np.random.default_rng(63)
+    images = [rng.standard_normal((n, 3, 48, 48)).astype(np.float32) for n in (5, 5, 5, 5, 3, 3)]
+    monkeypatch.setenv("MCB200_INPUT_PARTS", parts)
+
+    def run(siblings):
+        monkeypatch.setenv("MCB200_SIBLINGS", siblings)
+        net = capi.Net(gpu_engine, b.text(), None, from_buffer=True)
+        net.set_params(weights)
+        net.mark_output("right")
+        got = []
+        for i, x in enumerate(images):
+            if i == 3:
+                net.set_params({"right_0": weights["right_0"] * 0.5, "left_1": weights["left_1"] + 0.25})
+            net.forward(data=x)
+            got.append([net.blob(name).data.copy() for name in ("right", "last")])
+        net.close()
+        return got
+
+    for i, (alone, together) in enumerate(zip(run("0"), run("1"))):
+        for want, got in zip(alone, together):
+            assert np.isfinite(want).all() and np.abs(want).max() > 0 and _equal(want, got), i

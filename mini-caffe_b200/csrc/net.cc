@@ -371,8 +371,10 @@ void Net::PlaceMemory() {
 
   MergeSiblings();
 
-  // The last step's tops go to the host and nowhere else.
-  for (const NetStep& step : plan.steps) layers_[step.layer_id]->SetTopsEndOnHost(&step == &plan.steps.back());
+  // The last layer's tops, where the last step makes them, go to the host and nowhere else.
+  for (const NetStep& step : plan.steps) {
+    layers_[step.layer_id]->SetTopsEndOnHost(&step == &plan.steps.back() && step.top_ids == top_id_vecs_.back());
+  }
 
   PlanParts();
 
@@ -677,10 +679,11 @@ void Net::Forward(bool reshape) {
     }
   }
   // As in the reference: return with the last layer's tops on the host.  Marked blobs that the
-  // caller has been reading there come along, so that one wait serves them all.
+  // caller has been reading there come along, so that one wait serves them all.  (The last layer may run earlier, in
+  // another's launch: the last step's tops are then a blob that nobody has asked for.)
   if (profiling) profiler->ScopeStart("Sync");
   std::vector<SyncedMemory*> copied;
-  for (Blob* b : plan.steps.back().tops) {
+  for (Blob* b : top_vecs_.back()) {
     if (b->data()->BeginHostCopy()) copied.push_back(b->data().get());
   }
   for (Blob* b : plan.marked) {

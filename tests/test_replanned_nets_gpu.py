@@ -1,5 +1,7 @@
 """What the net's schedule fuses and merges, and nets that are planned again after they have run (another set of
 outputs, another batch): what the layers keep from pass to pass has to follow."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -12,6 +14,11 @@ pytestmark = pytest.mark.gpu
 def gpu_engine(engine):
     engine.set_mode(True, 0)
     return engine
+
+
+def _launches(engine):
+    engine.lib.mcb200_launch_count.restype = ctypes.c_longlong
+    return engine.lib.mcb200_launch_count()
 
 
 def _equal(a, b):
@@ -142,3 +149,24 @@ def test_a_refused_launch_of_two_stays_two_layers(monkeypatch, capi, gpu_engine,
     for i, (alone, together) in enumerate(zip(run("0"), run("1"))):
         for want, got in zip(alone, together):
             assert np.isfinite(want).all() and np.abs(want).max() > 0 and _equal(want, got), i
+
+
+def test_the_last_layers_top_comes_to_the_host_from_another_layers_launch(capi, gpu_engine):
+    """The last layer runs in the launch of an earlier one, and the last step is a layer that nobody asked for: a pass still
+    ends with the last layer's top on the host, so that reading it launches nothing."""
+    wl = pkg("workloads")
+    b = wl.NetBuilder("last_merged")
+    b.input([("data", (2, 8, 14, 14))])
+    b.conv("trunk", "data", "trunk", 8, 64, 3, pad=1)
+    b.relu("trunk_relu", "trunk")
+    b.conv("first", "trunk", "first", 64, 24, 3, pad=1)
+    b.pool("between", "trunk", "between", "AVE", global_pooling=True)
+    b.conv("last", "trunk", "last", 64, 40, 3, pad=1)
+    net = capi.Net(gpu_engine, b.text(), None, from_buffer=True)
+    net.set_params(wl.init_params(b.params, seed=64))
+    rng = np.random.default_rng(64)
+    for i in range(3):
+        net.forward(data=rng.standard_normal((2, 8, 14, 14)).astype(np.float32))
+        before = _launches(gpu_engine)
+        assert np.isfinite(net.blob("last").data).all()
+        assert _launches(gpu_engine) == before, i

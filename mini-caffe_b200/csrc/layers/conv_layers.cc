@@ -223,16 +223,16 @@ bool ConvolutionLayer::AcceptsFusedPool(const FusedTail& tail) const {
          shape_.c % 8 == 0 && mcb200_conv_march_supported(&shape_, 0) != 0;
 }
 
-bool ConvolutionLayer::Marches() const {
+bool ConvolutionLayer::MarchesAlone() const {
   if (tail_.pooled) return true;              // decided when the net was planned
   const char* off = getenv("MCB200_MARCH");   // "0": the general kernel, for comparisons in tests
-  return path_ == kTensorCore && !use_rows_ && !march_rejected_ && !sibling_ && !tail_.residual && !(off && off[0] == '0') &&
+  return path_ == kTensorCore && !use_rows_ && !march_rejected_ && !tail_.residual && !(off && off[0] == '0') &&
          mcb200_conv_march_pays(&shape_, half_operands_ ? 1 : 0) != 0;
 }
 
 bool ConvolutionLayer::AcceptsSibling(const Layer* layer) const {
   const ConvolutionLayer* other = dynamic_cast<const ConvolutionLayer*>(layer);
-  if (!other || other == this || Marches()) return false;
+  if (!other || other == this || MarchesAlone()) return false;   // (whatever the plan before this one merged)
   auto plain = [](const ConvolutionLayer& l) {
     ActivationSpec act;
     if (l.tail_.activation && (!l.tail_.activation->AsActivation(&act) || act.kind != 1 || act.slope != 0.f)) return false;

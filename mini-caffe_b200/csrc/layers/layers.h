@@ -84,8 +84,9 @@ class ConvolutionLayer : public Layer {
   void RunImages(Blob* bottom, Blob* top, size_t i, int first, int count, size_t slot, Blob* second_top = nullptr);
   void RunTwo(Blob* bottom, const vector<Blob*>& top, int first, int count, size_t slot);
   void RefreshParameters();
-  // Whether the layer runs on conv_march.cu, as shaped, fused and stored now.
-  bool Marches() const;
+  // Whether the layer runs on conv_march.cu, as shaped, fused and stored now; MarchesAlone: if no launch held two layers.
+  bool Marches() const { return !sibling_ && MarchesAlone(); }
+  bool MarchesAlone() const;
   void PackRows(const mcb200_conv_shape& shape, const float* weights, float* packed);
   void FoldRows(std::vector<float>* scale, std::vector<float>* shift, bool* has_scale, bool* has_shift);
   int second_begin() const { return (shape_.cout + 31) / 32 * 32; }   // first of the sibling's columns

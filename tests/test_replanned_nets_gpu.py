@@ -170,3 +170,31 @@ def test_the_last_layers_top_comes_to_the_host_from_another_layers_launch(capi, 
         before = _launches(gpu_engine)
         assert np.isfinite(net.blob("last").data).all()
         assert _launches(gpu_engine) == before, i
+
+
+def test_the_batch_before_does_not_decide_what_is_merged(capi, gpu_engine):
+    """Two 3 x 3 layers that are merged where few rows do not pay for the march, and march on their own with more images: a
+    net that was planned for one image first runs sixteen as one that was planned for sixteen."""
+    wl = pkg("workloads")
+    images = np.random.default_rng(65).standard_normal((16, 64, 56, 56)).astype(np.float32)
+    got = {}
+    for planned in (1, 16):
+        b = wl.NetBuilder("history")
+        b.input([("data", (planned, 64, 56, 56))])
+        b.conv("left", "data", "left", 64, 64, 3, pad=1)
+        b.conv("right", "data", "right", 64, 64, 3, pad=1)
+        b.pool("pool", "left", "pool", "AVE", global_pooling=True)
+        b.pool("last", "right", "last", "AVE", global_pooling=True)
+        net = capi.Net(gpu_engine, b.text(), None, from_buffer=True)
+        net.set_params(wl.init_params(b.params, seed=65))
+        net.mark_output("pool")
+        counts = []
+        for x in (images[:planned], images, images[:1], images):
+            net.forward(data=x)      # (packs weights where the form changes)
+            before = _launches(gpu_engine)
+            net.forward(data=x)
+            counts.append(_launches(gpu_engine) - before)
+        got[planned] = counts[1:], net.blob("pool").data.copy(), net.blob("last").data.copy()
+        net.close()
+    assert got[1][0] == got[16][0] and got[1][0][0] == got[1][0][2] > got[1][0][1]
+    assert _equal(got[1][1], got[16][1]) and _equal(got[1][2], got[16][2])

@@ -203,6 +203,7 @@ typedef struct mcb200_march_plan {
 } __attribute__((aligned(64))) mcb200_march_plan;
 int mcb200_conv_march_supported(const mcb200_conv_shape* s, int operands_bf16);   /* whatever the batch */
 int mcb200_conv_march_pays(const mcb200_conv_shape* s, int operands_bf16);        /* and enough rows for all SMs */
+int mcb200_conv_march_rows_per_slab(const mcb200_conv_shape* s);   /* rows of all columns for each of two slabs per SM, rounded down */
 size_t mcb200_conv_march_packed_weight_bytes(const mcb200_conv_shape* s, int operands_bf16);
 int mcb200_conv_march_pack_weights(const mcb200_conv_shape* s, int operands_bf16, const float* w_oihw, void* packed, void* stream);
 int mcb200_conv_march_plan(const mcb200_conv_shape* s, int operands_bf16, const void* in, const void* packed_w,

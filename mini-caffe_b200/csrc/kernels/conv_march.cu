@@ -523,9 +523,14 @@ extern "C" int mcb200_conv_march_supported(const mcb200_conv_shape* s, int opera
 // At 56 x 56 one image (a row per slab) takes 14.8 us here and 10.6 there; sixteen in bfloat16 (four rows) 14.8 both ways
 // in runs of one launch at a time, and 3 us less per pass here.
 extern "C" int mcb200_conv_march_pays(const mcb200_conv_shape* s, int operands_bf16) {
-  if (!mcb200_conv_march_supported(s, operands_bf16)) return 0;
+  return mcb200_conv_march_supported(s, operands_bf16) && mcb200_conv_march_rows_per_slab(s) >= kFewestRows;
+}
+
+extern "C" int mcb200_conv_march_rows_per_slab(const mcb200_conv_shape* s) {
+  if (!s || s->n < 0 || s->h < 1 || s->w < 1) return 0;
   const int segments = (s->w + kSlabOutputs - 1) / kSlabOutputs;
-  return static_cast<long long>(s->n) * segments * (s->h + 2) >= 2LL * 148 * kFewestRows;
+  const long long rows = static_cast<long long>(s->n) * segments * (s->h + 2LL) / (2 * 148);
+  return rows < 0x7fffffff ? static_cast<int>(rows) : 0x7fffffff;
 }
 
 extern "C" size_t mcb200_conv_march_packed_weight_bytes(const mcb200_conv_shape* s, int operands_bf16) {

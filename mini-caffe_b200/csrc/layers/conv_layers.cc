@@ -232,7 +232,7 @@ bool ConvolutionLayer::MarchesAlone() const {
 
 bool ConvolutionLayer::AcceptsSibling(const Layer* layer) const {
   const ConvolutionLayer* other = dynamic_cast<const ConvolutionLayer*>(layer);
-  if (!other || other == this || MarchesAlone()) return false;   // (whatever the plan before this one merged)
+  if (!other || other == this) return false;
   auto plain = [](const ConvolutionLayer& l) {
     ActivationSpec act;
     if (l.tail_.activation && (!l.tail_.activation->AsActivation(&act) || act.kind != 1 || act.slope != 0.f)) return false;
@@ -240,6 +240,13 @@ bool ConvolutionLayer::AcceptsSibling(const Layer* layer) const {
     return l.path_ == kTensorCore && !l.use_rows_ && l.shape_.group == 1 && !l.tail_.residual && !l.tail_.pooled;
   };
   const mcb200_conv_shape &a = shape_, &b = other->shape_;
+  // A layer that marches on its own (whatever the plan before this one merged) gives that up in a launch of two, which pays
+  // where runs are short: beside a layer that does not march up to four rows a slab, beside one that does up to thirteen.
+  // In one launch and alone, fp32 and bfloat16: 64 -> 128 beside 64 -> 64 at 56 x 56, 16 images (three rows) 30.0 and 32.1 us,
+  // 29.5 and 31.0, 24 images (four) 42.0 and 41.7, 32.4 and 31.9, 48 images 78 and 72, 56 and 47; 64 -> 64 twice, 64 images
+  // (twelve rows) 57.7 and 61.6, 37.0 and 36.8, 72 images (fourteen) 61.8 and 64.8, 51.6 and 44.4, 112 images 108 and 100, 69 and 63.
+  const int marching = (MarchesAlone() ? 1 : 0) + (other->MarchesAlone() ? 1 : 0);
+  if (marching > 0 && mcb200_conv_march_rows_per_slab(&shape_) >= (marching == 2 ? 13 : 4)) return false;
   // Short sums whose results fill HBM gain little from reading their input once, and lose in narrower tiles: 64 -> 256
   // and 64 -> 64 on 56 x 56 maps, batch 64: 84 us in one launch, 77 in two (256 -> 512 and 256 -> 128 at stride 2, 56 and 73).
   const double cells = static_cast<double>(shape_.n) * shape_.ho * shape_.wo * (shape_.cout + other->shape_.cout);

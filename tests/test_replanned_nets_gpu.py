@@ -173,12 +173,12 @@ def test_the_last_layers_top_comes_to_the_host_from_another_layers_launch(capi, 
 
 
 def test_the_batch_before_does_not_decide_what_is_merged(capi, gpu_engine):
-    """Two 3 x 3 layers that are merged where few rows do not pay for the march, and march on their own with more images: a
-    net that was planned for one image first runs sixteen as one that was planned for sixteen."""
+    """Two 3 x 3 layers that share a launch where few rows are left for each of the march's slabs, and march on their own
+    with more images: a net that was planned for two images first runs 72 as one that was planned for 72."""
     wl = pkg("workloads")
-    images = np.random.default_rng(65).standard_normal((16, 64, 56, 56)).astype(np.float32)
+    images = np.random.default_rng(65).standard_normal((72, 64, 56, 56)).astype(np.float32)
     got = {}
-    for planned in (1, 16):
+    for planned in (2, 72):
         b = wl.NetBuilder("history")
         b.input([("data", (planned, 64, 56, 56))])
         b.conv("left", "data", "left", 64, 64, 3, pad=1)
@@ -189,12 +189,49 @@ def test_the_batch_before_does_not_decide_what_is_merged(capi, gpu_engine):
         net.set_params(wl.init_params(b.params, seed=65))
         net.mark_output("pool")
         counts = []
-        for x in (images[:planned], images, images[:1], images):
+        for x in (images[:planned], images, images[:2], images):
             net.forward(data=x)      # (packs weights where the form changes)
             before = _launches(gpu_engine)
             net.forward(data=x)
             counts.append(_launches(gpu_engine) - before)
         got[planned] = counts[1:], net.blob("pool").data.copy(), net.blob("last").data.copy()
         net.close()
-    assert got[1][0] == got[16][0] and got[1][0][0] == got[1][0][2] > got[1][0][1]
-    assert _equal(got[1][1], got[16][1]) and _equal(got[1][2], got[16][2])
+    assert got[2][0] == got[72][0] and got[2][0][0] == got[2][0][2] > got[2][0][1]
+    assert _equal(got[2][1], got[72][1]) and _equal(got[2][2], got[72][2])
+
+
+@pytest.mark.parametrize("precision", ["fp32", "bf16"])
+@pytest.mark.parametrize("batch", [16, 24, 71])
+@pytest.mark.parametrize("couts", [(64, 64), (64, 128), (128, 64), (40, 48)], ids=str)
+def test_marching_layers_give_the_same_bits_merged_and_alone(monkeypatch, capi, gpu_engine, batch, couts, precision):
+    """Around the rows at which layers that march on their own share a launch, in either order."""
+    wl = pkg("workloads")
+    b = wl.NetBuilder("marching_siblings")
+    b.input([("data", (batch, 64, 52, 50))])
+    b.conv("trunk", "data", "trunk", 64, 64, 1)
+    b.conv("left", "trunk", "left", 64, couts[0], 3, pad=1)
+    b.relu("left_relu", "left")
+    b.conv("right", "trunk", "right", 64, couts[1], 3, pad=1)
+    b.conv("next", "left", "next", couts[0], 24, 1)
+    b.pool("pool", "next", "pool", "AVE", global_pooling=True)
+    b.pool("last", "right", "last", "AVE", global_pooling=True)
+    weights = wl.init_params(b.params, seed=66)
+    x = np.random.default_rng(66).standard_normal((batch, 64, 52, 50)).astype(np.float32)
+    monkeypatch.setenv("MINICAFFE_PRECISION", precision)
+
+    def run(siblings, march):
+        monkeypatch.setenv("MCB200_SIBLINGS", siblings)
+        monkeypatch.setenv("MCB200_MARCH", march)
+        net = capi.Net(gpu_engine, b.text(), None, from_buffer=True)
+        net.set_params(weights)
+        net.mark_output("pool")
+        for _ in range(2):
+            net.forward(data=x)
+        got = [net.blob(name).data.copy() for name in ("pool", "last")]
+        net.close()
+        return got
+
+    want = run("0", "0")
+    assert all(np.isfinite(w).all() and np.abs(w).max() > 0 for w in want)
+    for got in (run("1", "1"), run("0", "1")):
+        assert _equal(want[0], got[0]) and _equal(want[1], got[1])

@@ -107,8 +107,9 @@ class Layer {
   virtual bool AsActivation(ActivationSpec* spec) { return false; }
   // Consumer side: true if the layer is 2 x 2 max pooling of stride 2 without padding, as shaped now.
   virtual bool AsMaxPool2x2() const { return false; }
-  // Producer side: can its store take such a pooling behind the rest of `tail`?
-  virtual bool AcceptsFusedPool(const FusedTail& tail) const { return false; }
+  // Producer side: can its store take such a pooling behind the rest of `tail`, and is it the quicker way (half_net: in a
+  // net that stores bfloat16)?
+  virtual bool AcceptsFusedPool(const FusedTail& tail, bool half_net) const { return false; }
   // Consumer side: true if the layer is y = sum_i coeff[i] * bottom[i].
   virtual bool AsWeightedSum(std::vector<float>* coeffs) { return false; }
   // ---- bfloat16 storage (nets built with MINICAFFE_PRECISION=bf16) ----

@@ -74,7 +74,7 @@ class ConvolutionLayer : public Layer {
   }
   double PartSeconds(const vector<Blob*>& bottom, const vector<Blob*>& top, bool first_of_net) const override;
   bool AcceptsSibling(const Layer* other) const override;
-  bool AcceptsFusedPool(const FusedTail& tail) const override;
+  bool AcceptsFusedPool(const FusedTail& tail, bool half_net) const override;
   void SetSibling(Layer* other) override;
 
  protected:

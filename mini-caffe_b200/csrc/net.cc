@@ -288,7 +288,7 @@ void Net::PlaceMemory() {
         }
         // A 2 x 2 max pooling that alone reads the result.
         std::vector<int> readers = scan.Consumers(cur, i);
-        if (readers.size() == 1 && !plan.visible[cur] && layers_[readers[0]]->AsMaxPool2x2() && producer->AcceptsFusedPool(tail)) {
+        if (readers.size() == 1 && !plan.visible[cur] && layers_[readers[0]]->AsMaxPool2x2() && producer->AcceptsFusedPool(tail, plan.half_storage)) {
           const Blob &from = *blobs_[cur], &to = *top_vecs_[readers[0]][0];
           if (to.shape(2) == (from.shape(2) + 1) / 2 && to.shape(3) == (from.shape(3) + 1) / 2) {
             tail.pooled = true;

@@ -235,3 +235,40 @@ def test_marching_layers_give_the_same_bits_merged_and_alone(monkeypatch, capi, 
     assert all(np.isfinite(w).all() and np.abs(w).max() > 0 for w in want)
     for got in (run("1", "1"), run("0", "1")):
         assert _equal(want[0], got[0]) and _equal(want[1], got[1])
+
+
+@pytest.mark.parametrize("precision", ["fp32", "bf16"])
+def test_a_pooling_is_taken_in_the_store_where_that_pays(monkeypatch, capi, gpu_engine, precision):
+    """5 images of 58 rows are fewer than 296 slabs, 6 are more: in fp32 the pooling keeps its launch with five, with the same
+    bits as everywhere."""
+    wl = pkg("workloads")
+    b = wl.NetBuilder("pool_pays")
+    b.input([("data", (6, 64, 56, 56))])
+    b.conv("trunk", "data", "trunk", 64, 64, 1)
+    b.conv("conv", "trunk", "conv", 64, 64, 3, pad=1)
+    b.relu("conv_relu", "conv")
+    b.pool("pool", "conv", "pool", "MAX", k=2, stride=2)
+    b.conv("next", "pool", "next", 64, 24, 1)
+    b.pool("last", "next", "last", "AVE", global_pooling=True)
+    weights = wl.init_params(b.params, seed=67)
+    images = np.random.default_rng(67).standard_normal((6, 64, 56, 56)).astype(np.float32)
+    monkeypatch.setenv("MINICAFFE_PRECISION", precision)
+
+    def run(march):
+        monkeypatch.setenv("MCB200_MARCH", march)
+        net = capi.Net(gpu_engine, b.text(), None, from_buffer=True)
+        net.set_params(weights)
+        got = []
+        for n in (6, 5, 6, 1):
+            net.forward(data=images[:n])
+            before = _launches(gpu_engine)
+            net.forward(data=images[:n])
+            got.append((_launches(gpu_engine) - before, net.blob("last").data.copy()))
+        net.close()
+        return got
+
+    alone, fused = run("0"), run("1")
+    saved = [a[0] - f[0] for a, f in zip(alone, fused)]
+    assert saved == ([1, 0, 1, 0] if precision == "fp32" else [1, 1, 1, 1])
+    for a, f in zip(alone, fused):
+        assert np.isfinite(a[1]).all() and np.abs(a[1]).max() > 0 and _equal(a[1], f[1])

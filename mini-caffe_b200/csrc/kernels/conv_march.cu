@@ -388,16 +388,21 @@ conv_march_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       // 2 x 2 maxima: runs begin at even rows and segments at even pixels, so a window is two rows of one
       // run and two neighbouring pixels, four lanes apart.  Windows at the last row or pixel may be cut.
       finish(below);
+      // Cells that a cut window lacks count as the lowest value of the result's type, whole windows as they are
+      // (all -infinity, all NaN): the pooling kernels' rules, whose general one, for columns that are no multiple of four,
+      // starts every window at the lowest value.  (fmaxf with NaN is its other operand.)
       const bool two_rows = y + 1 < args.h;
+      const float lowest = args.out_half ? __uint_as_float(0xff7f0000u) : -3.402823466e+38f;
       const size_t row = (static_cast<size_t>(n) * ((args.h + 1) >> 1) + (y >> 1)) * ((args.w + 1) >> 1);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int pixel = pixel0 + 8 * i;
         const bool two_pixels = (pixel & 1) != 0 || pixel + 1 < pixels;
+        const float least = two_rows && two_pixels && (args.cout & 3) == 0 ? __uint_as_float(0x7fffffffu) : lowest;
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           uint32_t& cell = acc[i >> 1][4 * (k >> 1) + 2 * (i & 1) + (k & 1)];
-          float v = fmaxf(-3.402823466e+38f, __uint_as_float(cell));
+          float v = fmaxf(least, __uint_as_float(cell));
           if (two_rows) v = fmaxf(v, __uint_as_float(below[i >> 1][4 * (k >> 1) + 2 * (i & 1) + (k & 1)]));
           const float beside = __shfl_xor_sync(0xffffffffu, v, 4);
           cell = __float_as_uint(two_pixels ? fmaxf(v, beside) : v);

@@ -401,13 +401,20 @@ void ConvolutionLayer::RunTwo(Blob* bottom, const vector<Blob*>& top, int first,
 
 void ConvolutionLayer::RunImages(Blob* bottom, Blob* top, size_t i, int first, int count, size_t slot_index, Blob* second_top) {
   Context& ctx = Context::Get();
+  const bool half_out = half_top_ && HalfTopCapable();
+  const bool half = half_operands_ && HalfOperandsCapable();
+  if (count == 0 && path_ == kTensorCore) {   // a batch of no images: the tops are there and hold nothing
+    CHECK(!half && !half_out) << "cannot build the tensor-core plan for layer " << layer_param_.name() << " (no images)";
+    top->mutable_gpu_data_nhwc();
+    if (second_top) second_top->mutable_gpu_data_nhwc();
+    return;
+  }
   mcb200_conv_shape s = shape_;
   s.n = count;
   s.cout = columns();
   const size_t in_at = static_cast<size_t>(first) * s.c * s.h * s.w;
-  const size_t out_at = static_cast<size_t>(first) * (top->count() / shape_.n);
+  const size_t out_at = first == 0 ? 0 : static_cast<size_t>(first) * (top->count() / shape_.n);
   const float* in = nullptr;
-  const bool half = half_operands_ && HalfOperandsCapable();
   if (half) {
     s.c_stride = s.c;
     in = reinterpret_cast<const float*>(static_cast<const uint16_t*>(bottom->gpu_data_nhwc_bf16()) + in_at);
@@ -447,7 +454,6 @@ void ConvolutionLayer::RunImages(Blob* bottom, Blob* top, size_t i, int first, i
     ep.residual = half ? reinterpret_cast<const float*>(reinterpret_cast<const uint16_t*>(ep.residual) + out_at)
                        : ep.residual + out_at;
   }
-  const bool half_out = half_top_ && HalfTopCapable();
   float* out = half_out ? reinterpret_cast<float*>(static_cast<uint16_t*>(top->mutable_gpu_data_nhwc_bf16()) + out_at)
                         : top->mutable_gpu_data_nhwc() + out_at;
   if (path_ == kTensorCore) {

@@ -272,3 +272,39 @@ def test_a_pooling_is_taken_in_the_store_where_that_pays(monkeypatch, capi, gpu_
     assert saved == ([1, 0, 1, 0] if precision == "fp32" else [1, 1, 1, 1])
     for a, f in zip(alone, fused):
         assert np.isfinite(a[1]).all() and np.abs(a[1]).max() > 0 and _equal(a[1], f[1])
+
+
+@pytest.mark.parametrize("first_channels", [3, 8])
+@pytest.mark.parametrize("precision", ["fp32", "bf16"])
+def test_a_batch_of_no_images(monkeypatch, capi, gpu_engine, precision, first_channels):
+    """Between ordinary batches, through layers of all forms: an empty result in fp32, an error in bfloat16, and the next
+    batch is what it was."""
+    wl = pkg("workloads")
+    b = wl.NetBuilder("empty")
+    b.input([("data", (16, first_channels, 56, 56))])
+    b.conv("conv1", "data", "conv1", first_channels, 64, 3, pad=1)
+    b.relu("conv1_relu", "conv1")
+    b.conv("conv2", "conv1", "conv2", 64, 64, 3, pad=1)
+    b.pool("pool", "conv2", "pool", "MAX", k=2, stride=2)
+    b.conv("left", "pool", "left", 64, 40, 1)
+    b.conv("right", "pool", "right", 64, 24, 1)
+    b.pool("last", "right", "last", "AVE", global_pooling=True)
+    x = np.random.default_rng(68).standard_normal((16, first_channels, 56, 56)).astype(np.float32)
+    monkeypatch.setenv("MINICAFFE_PRECISION", precision)
+    net = capi.Net(gpu_engine, b.text(), None, from_buffer=True)
+    net.set_params(wl.init_params(b.params, seed=68))
+    net.mark_output("left")
+    names = ("left", "last")
+    net.forward(data=x)
+    want = [net.blob(name).data.copy() for name in names]
+    for _ in range(2):
+        if precision == "bf16":
+            with pytest.raises(capi.CaffeError):
+                net.forward(data=x[:0])
+        else:
+            net.forward(data=x[:0])
+            assert net.blob("left").shape == (0, 40, 28, 28) and net.blob("last").shape == (0, 24, 1, 1)
+            assert net.blob("left").data.size == 0
+        net.forward(data=x)
+        for name, value in zip(names, want):
+            assert np.isfinite(value).all() and _equal(net.blob(name).data, value), name

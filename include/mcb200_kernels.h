@@ -80,8 +80,8 @@ int mcb200_conv_pack_weights(const mcb200_conv_shape* s, const float* w_oihw, fl
 typedef struct mcb200_conv_plan {
   uint64_t tma_a[16];
   uint64_t tma_b[16];
-  uint64_t tma_out[16];     /* not used (callers rely on the layout)               */
-  uint64_t tma_res[16];     /* not used                                            */
+  uint64_t tma_out[16];     /* tile maps of the output and of the residual or the second layer's output, built by a */
+  uint64_t tma_res[16];     /* launch that stores through shared memory and rebuilt when what they were built for changes */
   mcb200_conv_shape shape;
   int m, k_iters, c_blocks, block_n;
   int im2col;               /* 0 matrix rows, 1 im2col tensor map, 2 row mode, 3 halo mode (the taps
@@ -89,7 +89,8 @@ typedef struct mcb200_conv_plan {
   int out_ld, res_ld;
   int cta_pair;             /* 1: launched as two-CTA clusters (tcgen05 cta_group::2) */
   int operand_bf16;         /* 1: built by mcb200_conv_tc_plan_bf16                 */
-  int out_bf16;             /* not used, nor are out_ld, res_ld and the two pointers */
+  int out_bf16;             /* what the cached maps were built for, with out_ld, res_ld and the pointers: element type
+                               of the output + 2 x columns of the first of two layers (0: one layer) */
   const float* out_ptr;
   const float* res_ptr;
   int m_virtual;            /* halo mode: positions of the virtual output grid (rows widened by
@@ -107,6 +108,8 @@ typedef struct mcb200_conv_plan {
  * (src/layers/inner_product_layer.cpp:80-93).                                */
 int mcb200_conv_tc_plan(const mcb200_conv_shape* s, const float* in, const float* packed_w,
                         mcb200_conv_plan* plan);
+/* Launches update the plan in place (the tile maps cached in it): one plan is not launched from two host threads
+ * at a time.                                                                                    */
 int mcb200_conv_tc_launch(mcb200_conv_plan* plan, float* out, int out_ld,
                           const mcb200_epilogue* ep, int* status, void* stream);
 

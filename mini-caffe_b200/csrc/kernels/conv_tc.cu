@@ -2352,23 +2352,25 @@ int launch_core(mcb200_conv_plan* plan, void* out, bool out_half, int out_ld, co
     const bool rows = plan->im2col == kModeRows;
     const long long per_group = rows ? plan->shape.wo : plan->m;
     const long long groups = rows ? static_cast<long long>(plan->shape.n) * plan->shape.ho : 1;
-    const bool new_out = plan->out_ptr != out || plan->out_ld != out_ld || plan->out_bf16 != a.out_half;
+    // The maps are kept for the next launch to the same places, of as many layers.
+    const int kind = a.out_half | (second ? 2 * a.first_cout : 0);
+    const bool new_out = plan->out_ptr != out || plan->out_ld != out_ld || plan->out_bf16 != kind;
     if (new_out) {
       if (encode_tile_map(reinterpret_cast<CUtensorMap*>(plan->tma_out), out, out_half, a.first_cout, out_ld,
                           per_group, groups) != CUDA_SUCCESS)
         return -4;
       plan->out_ptr = static_cast<const float*>(out);
       plan->out_ld = out_ld;
-      plan->out_bf16 = a.out_half;
+      plan->out_bf16 = kind;
     }
-    if (second && (plan->res_ptr != second->out || plan->res_ld != second->out_ld || plan->out_bf16 != a.out_half || new_out)) {
+    if (second && (plan->res_ptr != second->out || plan->res_ld != second->out_ld || new_out)) {
       if (encode_tile_map(reinterpret_cast<CUtensorMap*>(plan->tma_res), second->out, out_half, a.cout - second->begin,
                           second->out_ld, per_group, groups) != CUDA_SUCCESS)
         return -5;
       plan->res_ptr = static_cast<const float*>(second->out);
       plan->res_ld = second->out_ld;
     }
-    if (a.ep.residual && (plan->res_ptr != a.ep.residual || plan->res_ld != a.ep.residual_ld)) {
+    if (a.ep.residual && (plan->res_ptr != a.ep.residual || plan->res_ld != a.ep.residual_ld || new_out)) {
       if (encode_tile_map(reinterpret_cast<CUtensorMap*>(plan->tma_res), a.ep.residual, half, plan->shape.cout,
                           a.ep.residual_ld, per_group, groups) != CUDA_SUCCESS)
         return -5;

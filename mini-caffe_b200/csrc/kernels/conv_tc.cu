@@ -34,6 +34,7 @@
 
 #include <stdlib.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "../../../include/mcb200_kernels.h"
@@ -1736,8 +1737,44 @@ int segment_shift_of(const mcb200_conv_shape& s, int mode, int k_iters) {
   return positions <= 400 && steps >= 512 ? 1 : 0;
 }
 
-// CTAs that run at one time as clusters of 1 << shift, one tile each.
-int split_capacity(int shift) { return shift == 2 ? 128 : 144; }
+// CTAs that run at one time as clusters of 1 << shift, one tile each: asked of the device, as a cluster keeps to one GPC and
+// how many SMs a GPC has differs from chip to chip (one B200: 74 clusters of two, all 148 SMs, but 33 of four, 132).
+// No more than 128 and 144, though: with the thirty-third cluster of four 512 -> 672 channels, 3 x 3, three images of 7 x 7
+// gain (11.5 -> 10.2 us) and 2048 -> 1056 on one pixel, which small_tiles then cuts to 32 columns, loses (6.5 -> 7.2).
+int split_capacity(int shift) {
+  static std::mutex mu;
+  static int ctas[64][3] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
+  std::lock_guard<std::mutex> lock(mu);
+  int& known = ctas[dev][shift];
+  if (known == 0) {
+    auto kernel = conv_tc_kernel<64, kModeMatrix, false, false, kOutSplit>;   // (all forms: one CTA per SM, most of its memory)
+    cudaFuncAttributes func;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1u << shift;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(1u << shift, 1, 1);
+    cfg.blockDim = dim3(kThreads, 1, 1);
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaFuncGetAttributes(&func, kernel) == cudaSuccess) {
+      cfg.dynamicSmemBytes = static_cast<size_t>(kSharedLimit) - func.sharedSizeBytes;
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(cfg.dynamicSmemBytes)) != cudaSuccess ||
+          cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess)
+        clusters = 0;
+    }
+    if (clusters < 1) {
+      (void)cudaGetLastError();
+      clusters = 128 >> shift;
+    }
+    known = std::min(clusters << shift, shift == 2 ? 128 : 144);
+  }
+  return known;
+}
 
 int m_tile_of(const mcb200_conv_plan& p) {
   const int halo_rows = p.im2col == kModeHalo ? (p.shape.kw - 1) * p.shape.dil_w : 0;

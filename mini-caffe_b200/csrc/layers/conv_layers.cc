@@ -252,10 +252,16 @@ bool ConvolutionLayer::AcceptsSibling(const Layer* layer) const {
   // (twelve rows) 57.7 and 61.6, 37.0 and 36.8, 72 images (fourteen) 61.8 and 64.8, 51.6 and 44.4, 112 images 108 and 100, 69 and 63.
   const int marching = (MarchesAlone() ? 1 : 0) + (other->MarchesAlone() ? 1 : 0);
   if (marching > 0 && mcb200_conv_march_rows_per_slab(&shape_) >= (marching == 2 ? 13 : 4)) return false;
-  // Short sums whose results fill HBM gain little from reading their input once, and lose in narrower tiles: 64 -> 256
-  // and 64 -> 64 on 56 x 56 maps, batch 64: 84 us in one launch, 77 in two (256 -> 512 and 256 -> 128 at stride 2, 56 and 73).
-  const double cells = static_cast<double>(shape_.n) * shape_.ho * shape_.wo * (shape_.cout + other->shape_.cout);
-  if (shape_.c * shape_.kh * shape_.kw < 256 && cells > 16e6) return false;
+  // Short sums whose results fill HBM take as long as their stores, which are quickest from tiles of 256 columns.  A layer whose
+  // columns divide by 256 keeps its launch there if the two together do not.  In one launch and in two, 1 x 1 at 56 x 56, fp32
+  // and bfloat16: 64 -> 256 and 64 at 8 images (8 million cells) 14.3 and 17.5 us, 12.0 and 14.0, at 16 images 25.4 and
+  // 23.5, 20.8 and 21.4, at 64 images 80 and 69, 71 and 58; 128 -> 512 and 128 (640 columns still run in tiles of 128)
+  // at 32 million cells 45.2 and 48.3, 31.9 and 33.0, at 64 million 77.9 and 75.8, 58.9 and 57.5.  Others gain: 96 -> 384 and 96 at
+  // 64 images 90 and 122, 83 and 92; 256 -> 512 and 128 at stride 2, longer sums, 52 and 62, 34 and 37.
+  const int both = shape_.cout + other->shape_.cout;
+  const double cells = static_cast<double>(shape_.n) * shape_.ho * shape_.wo * both;
+  const bool splits_wide = (shape_.cout % 256 == 0 || other->shape_.cout % 256 == 0) && both % 256 != 0;
+  if (shape_.c * shape_.kh * shape_.kw < 256 && splits_wide && cells > (both % 128 == 0 ? 60e6 : 16e6)) return false;
   return plain(*this) && plain(*other) && a.n == b.n && a.h == b.h && a.w == b.w && a.c == b.c && a.kh == b.kh && a.kw == b.kw &&
          a.stride_h == b.stride_h && a.stride_w == b.stride_w && a.pad_h == b.pad_h && a.pad_w == b.pad_w && a.dil_h == b.dil_h &&
          a.dil_w == b.dil_w && (half_operands_ && HalfOperandsCapable()) == (other->half_operands_ && other->HalfOperandsCapable()) &&

@@ -308,3 +308,38 @@ def test_a_batch_of_no_images(monkeypatch, capi, gpu_engine, precision, first_ch
         net.forward(data=x)
         for name, value in zip(names, want):
             assert np.isfinite(value).all() and _equal(net.blob(name).data, value), name
+
+
+@pytest.mark.parametrize("columns,merged", [((256, 64), False), ((96, 384), True), ((256, 128), True), ((512, 128), True)], ids=str)
+def test_short_sums_share_a_launch_where_that_pays(monkeypatch, capi, gpu_engine, columns, merged):
+    """Some 17 million results of 64 channels: 256 and 64 columns stay two launches, and all give the same bits."""
+    wl = pkg("workloads")
+    side = 56
+    batch = int(17.5e6 / (side * side * sum(columns)))
+    b = wl.NetBuilder("short_sums")
+    b.input([("data", (batch, 64, side, side))])
+    b.conv("left", "data", "left", 64, columns[0], 1)
+    b.relu("left_relu", "left")
+    b.conv("right", "data", "right", 64, columns[1], 1)
+    b.pool("pool", "left", "pool", "MAX", k=3, stride=2)
+    b.conv("next", "pool", "next", columns[0], 16, 1, stride=4)
+    b.pool("last", "right", "last", "AVE", global_pooling=True)
+    weights = wl.init_params(b.params, seed=69)
+    x = np.random.default_rng(69).standard_normal((batch, 64, side, side)).astype(np.float32)
+
+    def run(siblings):
+        monkeypatch.setenv("MCB200_SIBLINGS", siblings)
+        net = capi.Net(gpu_engine, b.text(), None, from_buffer=True)
+        net.set_params(weights)
+        net.mark_output("next")
+        net.forward(data=x)
+        before = _launches(gpu_engine)
+        net.forward(data=x)
+        got = _launches(gpu_engine) - before, net.blob("next").data.copy(), net.blob("last").data.copy()
+        net.close()
+        return got
+
+    alone, together = run("0"), run("1")
+    assert alone[0] - together[0] == int(merged)
+    for want, got in zip(alone[1:], together[1:]):
+        assert np.isfinite(want).all() and np.abs(want).max() > 0 and _equal(want, got)

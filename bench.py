@@ -855,9 +855,12 @@ def main():
         "share_of_step_note": "sum of the kernel's own launch durations / time of a step; launches overlap by "
                               "their set-up (programmatic dependent launch), so the ratio is capped at 1",
     }
-    launched = next((t for t in launch_tables(table) if conv_launches == timed_steps * len(t)), None)
-    if rank == 0 and per_launch and launched and args.precision == "tf32":
-        roofline.update(layer_table(launched, per_launch, timed_steps, batch, peaks, tf32_peak))
+    launched = launch_rows(table, net.schedule())
+    if rank == 0 and per_launch and args.precision == "tf32":
+        if conv_launches == timed_steps * len(launched):
+            roofline.update(layer_table(launched, per_launch, timed_steps, batch, peaks, tf32_peak))
+        else:
+            roofline["layers_missing"] = "%d timed launches, %d in the schedule of a pass" % (conv_launches // timed_steps, len(launched))
 
     # ---- secondary figures of the benchmark definition (after the headline) ----
     extras = None
@@ -919,19 +922,16 @@ def main():
         dist.destroy_process_group()
 
 
-def launch_tables(table):
-    """The layers of a pass as launches: each its own, or a stage's projection in one launch with the reduction beside it
-    (whose input then counts once), in all stages or where the sum over the input's channels is not short."""
-    def together(shortest):
-        rows = []
-        for row in table:
-            if rows and row[0].endswith("branch2a") and rows[-1][0].endswith("branch1") and row[1] >= shortest:
-                first = rows.pop()
-                rows.append((first[0] + "+2a", first[1], first[2] + row[2]) + row[3:])
-            else:
-                rows.append(row)
-        return rows
-    return [list(table), together(256), together(0)]
+def launch_rows(table, schedule):
+    """The layers of a pass as launches, by the net's own schedule: two layers that share one are one row, whose input
+    counts once."""
+    layers = {row[0]: row for row in table}
+    rows = []
+    for step in schedule:
+        held = [layers[name] for name in step if name in layers]
+        if held:
+            rows.append(("+".join(row[0] for row in held), held[0][1], sum(row[2] for row in held)) + held[0][3:])
+    return rows
 
 
 def layer_table(table, per_launch, timed_steps, batch, peaks, tf32_peak):

@@ -73,6 +73,10 @@ class CAFFE_API Net {
   bool has_blob(const string& blob_name) const;
   const shared_ptr<Blob> blob_by_name(const string& blob_name) const;
 
+  /*! \brief the current schedule: per step the layer it runs and, behind it, one that shares its launch; a layer that is
+   *         in no step was fused into another */
+  vector<vector<string> > schedule() const;
+
   /*! \brief keep these blobs valid after Forward() */
   void MarkOutputs(const std::vector<std::string>& outs);
 

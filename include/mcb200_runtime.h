@@ -22,6 +22,11 @@ void* mcb200_current_stream(void);
 /* Block until the calling thread's stream is idle. Returns 0 or -1. */
 int mcb200_synchronize(void);
 
+/* The net's current schedule (NetHandle of c_api.h): a line per step with the name of the layer it runs and, behind a
+ * tab, of one that shares its launch.  A layer on no line was fused into another.  Valid until the thread's next call;
+ * NULL on failure.  A new batch or output set shows after the next forward pass. */
+const char* mcb200_net_schedule(void* net);
+
 /* While enabled, every tensor-core convolution launch of the calling thread is
  * bracketed by a pair of CUDA events on its stream. */
 void mcb200_kernel_timing_begin(void);

@@ -153,6 +153,16 @@ class Net(object):
     def mark_output(self, name):
         self._lib.check(self._lib.lib.CaffeNetMarkOutput(self.handle, name.encode()))
 
+    def schedule(self):
+        """[[layer, second layer of the same launch or nothing]] of the engine's steps (mcb200_runtime.h); layers that were
+        fused into others are not listed."""
+        fn = self._lib.lib.mcb200_net_schedule
+        fn.argtypes, fn.restype = [_void_p], ctypes.c_char_p
+        text = fn(self.handle)
+        if text is None:
+            raise CaffeError(self._lib.lib.CaffeGetLastError().decode("utf-8", "replace"))
+        return [line.split("\t") for line in text.decode().splitlines()]
+
     def forward(self, **inputs):
         for k, v in inputs.items():
             b = self.blob(k)

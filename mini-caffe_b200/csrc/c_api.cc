@@ -21,6 +21,7 @@ struct ThreadScratch {
   std::vector<std::string> name_storage;
   std::vector<const char*> names;
   std::vector<void*> handles;
+  std::string schedule;
 };
 
 ThreadScratch& Scratch() {
@@ -224,4 +225,19 @@ int mcb200_synchronize(void) {
   API_BEGIN();
   caffe::Context::Get().SyncAndCheck();
   API_END();
+}
+
+const char* mcb200_net_schedule(void* net) {
+  try {
+    std::string& text = Scratch().schedule;
+    text.clear();
+    for (const std::vector<std::string>& step : static_cast<Net*>(net)->schedule()) {
+      for (size_t i = 0; i < step.size(); ++i) text += (i ? "\t" : "") + step[i];
+      text += "\n";
+    }
+    return text.c_str();
+  } catch (const std::exception& err) {
+    Fail(err);
+    return nullptr;
+  }
 }

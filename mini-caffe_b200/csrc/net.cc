@@ -41,6 +41,7 @@ struct NetStep {
   int layer_id;
   std::vector<Blob*> bottoms, tops;
   std::vector<int> bottom_ids, top_ids;  // bottom_ids includes a fused residual blob
+  int sibling_id = -1;                   // layer that runs in the same launch
 };
 
 struct NetPlan {
@@ -519,6 +520,7 @@ void Net::MergeSiblings() {
       if (later.bottom_ids.size() == 1 && later.bottom_ids[0] == blob && later.top_ids.size() == 1 &&
           layers_[step.layer_id]->AcceptsSibling(layers_[later.layer_id].get())) {
         siblings[step.layer_id] = layers_[later.layer_id].get();
+        step.sibling_id = later.layer_id;
         step.tops.push_back(later.tops[0]);
         step.top_ids.push_back(later.top_ids[0]);
         plan.steps.erase(plan.steps.begin() + k);
@@ -736,6 +738,15 @@ void Net::MarkOutputs(const std::vector<std::string>& outs) {
     blob_life_time_[it->second] = static_cast<int>(layers_.size());
   }
   plan_->valid = false;  // fusion and sharing depend on the visible set
+}
+
+vector<vector<string> > Net::schedule() const {
+  vector<vector<string> > steps;
+  for (const NetStep& step : plan_->steps) {
+    steps.push_back({layer_names_[step.layer_id]});
+    if (step.sibling_id >= 0) steps.back().push_back(layer_names_[step.sibling_id]);
+  }
+  return steps;
 }
 
 void Net::ToProto(NetParameter* param) const {

@@ -343,3 +343,38 @@ def test_short_sums_share_a_launch_where_that_pays(monkeypatch, capi, gpu_engine
     assert alone[0] - together[0] == int(merged)
     for want, got in zip(alone[1:], together[1:]):
         assert np.isfinite(want).all() and np.abs(want).max() > 0 and _equal(want, got)
+
+
+@pytest.mark.parametrize("parts", ["1", "3"])
+@pytest.mark.parametrize("precision", ["fp32", "bf16"])
+@pytest.mark.parametrize("batch,size", [(7, 56), (8, 61)])
+def test_every_layer_on_its_own_gives_the_same_bits(monkeypatch, capi, gpu_engine, batch, size, precision, parts):
+    """Neither merged layers nor the march nor a pooling in its store, against all of them, whole and in parts."""
+    import test_sibling_layers_gpu as siblings
+    wl = pkg("workloads")
+    b = siblings._net(wl, batch, size)
+    weights = wl.init_params(b.params, seed=70, bn_identity=False)
+    rng = np.random.default_rng(70)
+    images = [rng.standard_normal((batch, 3, size, size)).astype(np.float32) for _ in range(3)]
+    marked = ("loc", "conf", "before", "other")
+    monkeypatch.setenv("MINICAFFE_PRECISION", precision)
+
+    def run(on, parts):
+        monkeypatch.setenv("MCB200_SIBLINGS", on)
+        monkeypatch.setenv("MCB200_MARCH", on)
+        monkeypatch.setenv("MCB200_INPUT_PARTS", parts)
+        net = capi.Net(gpu_engine, b.text(), None, from_buffer=True)
+        net.set_params(weights)
+        for name in marked:
+            net.mark_output(name)
+        got = []
+        for x in images:
+            net.forward(data=x)
+            got.append([net.blob(name).data.copy() for name in marked + ("last",)])
+        assert (["pool"] in net.schedule()) == (on == "0")
+        net.close()
+        return got
+
+    for alone, together in zip(run("0", "1"), run("1", parts)):
+        for want, got in zip(alone, together):
+            assert np.isfinite(want).all() and np.abs(want).max() > 0 and _equal(want, got)

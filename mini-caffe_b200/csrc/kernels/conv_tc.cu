@@ -73,6 +73,7 @@ constexpr int kMaxPhase = 4;      // largest deconvolution stride that phase mod
 constexpr int kOutDirect = 0;     // how results leave: from registers,
 constexpr int kOutStaged = 1;     // through shared memory as TMA tiles,
 constexpr int kOutSplit = 2;      // or after a cluster's CTAs have added up their segments of the sum over K
+constexpr int kOutStagedTwo = 3;  // as kOutStaged, for a launch of two layers
 constexpr int kMaxHaloRows = 16; // extra strip rows ((kw - 1) * dilation) the halo mode takes
 
 struct ConvTcArgs {
@@ -232,10 +233,12 @@ __global__ void __launch_bounds__(kThreads, 1)
 conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const __grid_constant__ CUtensorMap map_out, const __grid_constant__ CUtensorMap map_res,
                const ConvTcArgs args) {
-  constexpr bool kStaged = kOut == kOutStaged, kSplit = kOut == kOutSplit;
+  constexpr bool kStaged = kOut == kOutStaged || kOut == kOutStagedTwo, kSplit = kOut == kOutSplit;
   // Layers whose sum over K is cut into segments (segment_shift_of): these modes.
   constexpr bool kSegments = !kStaged && (kMode == kModeMatrix || kMode == kModeIm2col || kMode == kModeHalo);
-  constexpr bool kTwo = kMode == kModeMatrix || kMode == kModeIm2col || kMode == kModeHalo;   // may hold two layers
+  // May hold two layers.  (The staged form is compiled for either: asked per chunk whose columns it has, it was 4 to 9 % slower
+  // for every launch of one layer that its epilogue bounds, bfloat16 above all: 64 -> 128 at 56 x 56, batch 64 21.9 us, 19.9 so.)
+  constexpr bool kTwo = (kMode == kModeMatrix || kMode == kModeIm2col || kMode == kModeHalo) && kOut != kOutStaged;
   static_assert(!kSplit || (kSegments && !kPair), "a split tile belongs to one CTA per segment");
   static_assert(!(kStaged && (BN < 64 || kMode == kModeHalo || kMode == kModePhase)), "a staged tile is one box of the output");
   static_assert(!(kPair && kMode == kModeRows), "row mode runs unpaired");
@@ -265,8 +268,9 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   // 128-byte swizzled tiles must start on a 1024-byte boundary.
   const uint32_t raw_addr = smem_addr(smem_raw);
   uint8_t* tiles = smem_raw + ((1024u - (raw_addr & 1023u)) & 1023u);
-  const int stage_bytes = args.stage_bytes;
-  const int stage_b_offset = args.stage_b_offset;
+  constexpr bool kOrdinary = kStaged && kMode != kModeRows;   // tiles of 128 rows, nothing resident: a stage of fixed size
+  const int stage_bytes = kOrdinary ? Plan::kSub * (kTileABytes + Plan::kTileBBytes) : args.stage_bytes;
+  const int stage_b_offset = kOrdinary ? Plan::kSub * kTileABytes : args.stage_b_offset;
   const int a_sub_bytes = stage_b_offset / Plan::kSub;   // sub-tiles of a stage: [A ...][B ...]
   const bool resident_b = kMode == kModeRows && args.resident_b_bytes > 0;
   uint8_t* resident = tiles + stages * stage_bytes;   // stages are multiples of 1024 bytes: so is this address
@@ -1146,10 +1150,6 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #pragma unroll
           for (int j = 0; j < 8; ++j) round4(v[j]);
         }
-        if (chunk + 2 >= kChunks || col0 + 64 >= args.cout) {
-          hand_back();
-          handed = true;
-        }
         if (!has_res && g >= slots) {
           // The store that last used this slot must have finished reading it.  Asked only now,
           // with the chunk's values in registers: the query costs its thread some 200 cycles
@@ -1339,7 +1339,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         MCB200_TRACE_CHUNK();
         if (dry) break;
       }
-      if (!handed) hand_back();
+      if (!handed) hand_back();   // (staged: the arrival among the chunk's shared-memory writes cost more than it gave, 1 to 2 %)
 #pragma unroll
       for (int i = 0; i < 4; ++i) rows[i] = next_rows[i];
     }
@@ -1869,7 +1869,7 @@ CUresult encode_tile_map(CUtensorMap* map, const void* base, bool half, int cols
 
 template <int BN, int kMode, bool kPair, bool kHalf, int kOut = kOutDirect>
 cudaError_t launch_variant(const mcb200_conv_plan* plan, ConvTcArgs args, cudaStream_t stream) {
-  constexpr bool kStaged = kOut == kOutStaged, kSplit = kOut == kOutSplit;
+  constexpr bool kStaged = kOut == kOutStaged || kOut == kOutStagedTwo, kSplit = kOut == kOutSplit;
   using Plan = SmemPlan<BN, kMode, kPair>;
   auto kernel = conv_tc_kernel<BN, kMode, kPair, kHalf, kOut>;
   // The large-shared-memory opt-in is per device: do it once for each device
@@ -2421,10 +2421,12 @@ int launch_core(mcb200_conv_plan* plan, void* out, bool out_half, int out_ld, co
   a.a_bytes = (plan->im2col == kModeHalo ? plan->strip_rows : a.tile_rows) * kBlockK * 4;
   cudaError_t e = cudaErrorInvalidValue;
   const int mode = plan->im2col;
-#define MCB200_OUT(BN, MODE, PAIR, HALF)                                                           \
+#define MCB200_OUT_ONE(BN, MODE, PAIR, HALF)                                                       \
   (staged ? launch_variant<BN, MODE, PAIR, HALF, kOutStaged>(plan, a, st) : launch_variant<BN, MODE, PAIR, HALF>(plan, a, st))
+#define MCB200_OUT(BN, MODE, PAIR, HALF)                                                           \
+  (staged && second ? launch_variant<BN, MODE, PAIR, HALF, kOutStagedTwo>(plan, a, st) : MCB200_OUT_ONE(BN, MODE, PAIR, HALF))
 #define MCB200_DISPATCH(BN)                                                                        \
-  e = mode == kModeRows     ? MCB200_OUT(BN, kModeRows, false, false)                              \
+  e = mode == kModeRows     ? MCB200_OUT_ONE(BN, kModeRows, false, false)                          \
       : mode == kModeIm2col ? MCB200_OUT(BN, kModeIm2col, false, false)                            \
       : mode == kModeHalo   ? launch_variant<BN, kModeHalo, false, false>(plan, a, st)             \
       : mode == kModePhase  ? launch_variant<BN, kModePhase, false, false>(plan, a, st)            \
@@ -2498,6 +2500,7 @@ int launch_core(mcb200_conv_plan* plan, void* out, bool out_half, int out_ld, co
 #undef MCB200_DISPATCH_PAIR
 #undef MCB200_DISPATCH
 #undef MCB200_OUT
+#undef MCB200_OUT_ONE
 #undef MCB200_DISPATCH_SPLIT
   return static_cast<int>(e);
 }

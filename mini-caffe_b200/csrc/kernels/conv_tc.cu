@@ -1991,8 +1991,12 @@ cudaError_t launch_variant(const mcb200_conv_plan* plan, ConvTcArgs args, cudaSt
 // staging's bytes), which counts where a CTA has one tile whose end nothing overlaps.  But a store
 // instruction then writes 32 bytes of eight rows each, and with many tiles in flight that, not HBM, is the limit
 // (64 -> 256 columns and a residual on 56 x 56 maps, batch 64: 107 us against 80; 32 -> 64 on 112 x 112, no residual: 71
-// against 59), as 16 bytes of a bfloat16 row are.  Per launch in fp32 without a residual and with one tile per
-// CTA: 1024 -> 2048 at 14 x 14, stride 2, batch 64 37 -> 33 us, 2048 -> 512 on 7 x 7 27 -> 23.
+// against 59), as 16 bytes of a bfloat16 row are.  In fp32, without a residual and with one tile per CTA (three if the
+// layer is one tile wide) it is the quicker one for pairs of 128 columns and for no other tile.  Staged and from registers, per
+// launch: pairs of 128 columns, 640 -> 512 at 14 x 14, batch 16 10.1 and 9.5 us, 768 -> 128 at 75 x 75, two images 11.0 and 10.1,
+// 256 -> 128, 3 x 3 at stride 2, 75 x 75, batch 32 72 and 64; of 256, 768 -> 192 at 24 x 24, batch 32 14.3 and 15.1,
+// 640 -> 512 at 38 x 38, four images 13.4 and 14.0; one CTA and 128 columns, 512 -> 512 at 14 x 14, batch 16 7.9 and
+// 9.2; 64 columns, 768 -> 512 at 28 x 28, two images 8.3 and 8.7.
 bool staged_epilogue(const mcb200_conv_plan* plan, bool residual) {
   const char* force = getenv("MCB200_STAGED");   // "0" / "1": override for experiments and tests
   if (force && (force[0] == '0' || force[0] == '1')) return force[0] == '1';
@@ -2002,7 +2006,7 @@ bool staged_epilogue(const mcb200_conv_plan* plan, bool residual) {
   const long long tiles = m_tiles * ((plan->shape.cout + plan->block_n - 1) / plan->block_n);
   const long long workers = plan->cta_pair ? 74 : 148, units = plan->cta_pair ? (tiles + 1) / 2 : tiles;
   const bool one_column = plan->shape.cout <= plan->block_n;
-  return residual || plan->operand_bf16 || units > (one_column ? 3 : 1) * workers || plan->k_iters < 16;
+  return residual || plan->operand_bf16 || !plan->cta_pair || plan->block_n != 128 || units > (one_column ? 3 : 1) * workers;
 }
 
 }  // namespace
